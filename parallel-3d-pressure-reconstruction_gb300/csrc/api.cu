@@ -69,7 +69,10 @@ struct omni3d_ctx {
     double ms_geometry = 0.0;
     // per-solve buffers
     DeviceBuf in_ax, in_ay, in_az, in_aux, in_pinit;  // staging of host inputs
-    DeviceBuf f32, b16, curl;
+    DeviceBuf f32, curl;
+    Layout lay;               // layout of the walks' copies of the field, pressure and sums
+    bool lay_set = false;
+    DeviceBuf edge, pw;       // the walks' edge records (skewed layouts) and copies of the pressure
     DeviceBuf pvol_a, pvol_b, pout, cnt, pncnt, scratch, flags;
     Anchor anc;
     bool anc_cached = false;  // plain method: operator structure built for this geometry
@@ -148,16 +151,17 @@ DirEntry make_dir(float k1, float k2, float k3)
     return D;
 }
 
-// Processing order of the directions: serpentine bands of polar angle, each band ordered
-// by azimuth, so that consecutive directions are neighbours on the sphere.  Lines are
-// traced and swept in this order; the few directions in flight at a time then sweep nearly
-// coincident sheets of the volume and share the gradient and accumulator lines in L2.
+// Processing order of the directions: the step-sign octants pair by pair of opposite ones (a
+// pair walks one copy of the skewed layouts), in each octant serpentine bands of polar angle,
+// each band ordered by azimuth, so that consecutive directions are neighbours on the sphere.
+// Lines are traced and swept in this order; the few directions in flight at a time then sweep
+// nearly coincident sheets of one copy and share its gradient and accumulator lines in L2.
 std::vector<int> sphere_order(const std::vector<float> &dirs)
 {
     const int n = (int)(dirs.size() / 3);
     const double PI = 3.14159265358979323846;
     int nb = std::max(1, (int)std::lround(std::sqrt(n / 2.0)));
-    std::vector<std::pair<std::pair<int, double>, int>> key;
+    std::vector<std::tuple<int, int, double, int>> key;
     key.reserve(n);
     for (int d = 0; d < n; d++) {
         double k1 = dirs[3 * d], k2 = dirs[3 * d + 1], k3 = dirs[3 * d + 2];
@@ -165,11 +169,12 @@ std::vector<int> sphere_order(const std::vector<float> &dirs)
         double th = std::acos(std::max(-1.0, std::min(1.0, r > 0 ? k3 / r : 1.0)));
         double ph = std::atan2(k2, k1);
         int b = std::min(nb - 1, (int)(th / PI * nb));
-        key.push_back({{b, (b & 1) ? -ph : ph}, d});
+        const int signs = (k1 >= 0 ? 1 : 0) | (k2 >= 0 ? 2 : 0) | (k3 >= 0 ? 4 : 0);
+        key.push_back({2 * layout_class(signs) + (signs & 1), b, (b & 1) ? -ph : ph, d});
     }
     std::sort(key.begin(), key.end());
     std::vector<int> order(n);
-    for (int i = 0; i < n; i++) order[i] = key[i].second;
+    for (int i = 0; i < n; i++) order[i] = std::get<3>(key[i]);
     return order;
 }
 
@@ -244,6 +249,50 @@ int stage(omni3d_ctx *ctx, const float *src, bool dev, DeviceBuf &buf, long long
     return OMNI3D_OK;
 }
 
+// The layout of a context's walks, chosen at its first field: skewed copies, unless they and
+// what goes with them would take more than half of the free device memory.
+int ensure_layout(omni3d_ctx *ctx)
+{
+    const Grid &g = ctx->geo.grid;
+    if (!ctx->lay_set) {
+        ctx->lay = skewed_layout(g);
+        const omni3d_params &P = ctx->prm;
+        const size_t entry = 2 * sizeof(float4) + sizeof(float) + sizeof(int32_t) + sizeof(float2) + (P.sweep_fp64 || P.deterministic ? sizeof(double2) : 0);
+        size_t fr = 0, tot = 0;
+        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess ||
+            entry * (size_t)ctx->lay.copies * (size_t)g.V > fr / 2)
+            ctx->lay = row_major_layout(g);
+        ctx->lay_set = true;
+    }
+    const size_t n = (size_t)ctx->lay.copies * (size_t)g.V;
+    if (ctx->lay.wrap) CK(ctx, ctx->edge.ensure(2 * sizeof(float4) * n));
+    CK(ctx, ctx->pw.ensure(sizeof(float) * n));
+    CK(ctx, ctx->pncnt.ensure(sizeof(float2) * n));
+    return OMNI3D_OK;
+}
+
+// The row-major layout for a context whose skewed copies did not fit in device memory after
+// all (other contexts may have taken it): true when the call can be tried again.
+bool drop_skewed(omni3d_ctx *ctx, int rc)
+{
+    if (rc != OMNI3D_ERR_NOMEM || !ctx->lay_set || !ctx->lay.wrap) return false;
+    cudaGetLastError();
+    if (ctx->st) cudaStreamSynchronize(ctx->st);
+    ctx->lay = row_major_layout(ctx->geo.grid);
+    for (DeviceBuf *b : {&ctx->edge, &ctx->pw, &ctx->pncnt, &ctx->pncnt64}) b->release();
+    anchor_free(&ctx->anc);
+    ctx->anc_cached = ctx->anc_last = false;
+    return true;
+}
+
+// Background of the walks' pressure copies: the initial state (zero when `zero`).
+cudaError_t start_volume(const Grid &g, const Layout &lay, const float *dpinit, bool zero, float *pw, cudaStream_t st)
+{
+    if (zero) return cudaMemsetAsync(pw, 0, sizeof(float) * (size_t)lay.copies * (size_t)g.V, st);
+    if (lay.wrap) return spread_volume(g, lay, dpinit, pw, st);
+    return cudaMemcpyAsync(pw, dpinit, sizeof(float) * (size_t)g.V, cudaMemcpyDeviceToDevice, st);
+}
+
 // Build the device field (float4 ax, ay, az, curl; optional bf16 copy; curl array).
 int prepare_field(omni3d_ctx *ctx, const float *ax, const float *ay, const float *az, const float *curl,
                   const float *mask, bool dev, Field *F)
@@ -270,14 +319,13 @@ int prepare_field(omni3d_ctx *ctx, const float *ax, const float *ay, const float
     const bool bf16 = ctx->prm.grad_storage == OMNI3D_GRAD_BF16;
     CK(ctx, ctx->f32.ensure(sizeof(float4) * (size_t)V));
     F->f32 = ctx->f32.as<float4>();
+    if ((rc = ensure_layout(ctx))) return rc;
+    F->lay = ctx->lay;
+    F->edge = ctx->lay.wrap ? ctx->edge.as<float4>() : nullptr;
     float *rounded = nullptr;  // BF16 storage: every curl decision sees the rounded curl
-    if (bf16) {
-        CK(ctx, ctx->b16.ensure(sizeof(uint2) * (size_t)V));
-        F->bf16 = ctx->b16.as<uint2>();
-        if (dcurl) {
-            CK(ctx, ctx->curl.ensure(sizeof(float) * (size_t)V));
-            rounded = ctx->curl.as<float>();
-        }
+    if (bf16 && dcurl) {
+        CK(ctx, ctx->curl.ensure(sizeof(float) * (size_t)V));
+        rounded = ctx->curl.as<float>();
     }
     F->curl = rounded ? rounded : const_cast<float *>(dcurl);
     CK(ctx, pack_field(g, dax, day, daz, dcurl, F, bf16, ctx->st, rounded));
@@ -332,12 +380,32 @@ int engine_prepare(omni3d_ctx *ctx, int *engine, const Field &F, int method)
     return fail(ctx, e == cudaErrorMemoryAllocation ? OMNI3D_ERR_NOMEM : OMNI3D_ERR_CUDA, "brick passes: " + why);
 }
 
-// One full sweep with the chosen engine.
-cudaError_t engine_sweep(omni3d_ctx *ctx, int engine, const Field &F, int method, bool bf16, const float *p,
+// Layout of a sweep's pressure and sums: the brick engine's are row-major.
+Layout engine_layout(int engine, const Field &F)
+{
+    Layout l = F.lay;
+    if (engine == OMNI3D_ENGINE_BRICKS) {
+        l = Layout();
+        l.stride = F.lay.stride;
+    }
+    return l;
+}
+
+// One full sweep with the chosen engine; p and acc in engine_layout.
+cudaError_t engine_sweep(omni3d_ctx *ctx, int engine, const Field &F, int method, const float *p,
                          float2 *acc, cudaStream_t st)
 {
     if (engine == OMNI3D_ENGINE_BRICKS) return brick_sweep(ctx->geo, &ctx->bricks, method, p, acc, st);
-    return sweep_full(ctx->geo, F, method, bf16, p, acc, st);
+    return sweep_full(ctx->geo, F, method, p, acc, st);
+}
+
+// The pressure copies of a row-major volume p for a sweep in layout lay (p itself when row-major).
+cudaError_t walk_pressure(omni3d_ctx *ctx, const Layout &lay, const float *p, const float **out, cudaStream_t st)
+{
+    *out = p;
+    if (!lay.wrap) return cudaSuccess;
+    *out = ctx->pw.as<float>();
+    return spread_volume(ctx->geo.grid, lay, p, ctx->pw.as<float>(), st);
 }
 
 // The brick passes' error flag (a TMA wait that gave up) as a status.
@@ -356,8 +424,9 @@ bool prepared_for_graph(const omni3d_ctx *ctx)
 {
     const omni3d_params &P = ctx->prm;
     return P.method == OMNI3D_METHOD_PLAIN && P.solver == OMNI3D_SOLVER_ANCHOR && P.tol == 0.0 && ctx->anc_cached &&
-           ctx->f32.p && ctx->in_pinit.p && ctx->pncnt.p && ctx->pout.p && ctx->cnt.p && ctx->pvol_a.p &&
-           ctx->scratch.p && (P.grad_storage != OMNI3D_GRAD_BF16 || ctx->b16.p);
+           ctx->lay_set && ctx->f32.p && (!ctx->lay.wrap || ctx->edge.p) && ctx->pw.p && ctx->in_pinit.p &&
+           ctx->pncnt.p && ctx->pout.p && ctx->cnt.p && ctx->pvol_a.p &&
+           ctx->scratch.p;
 }
 
 // The solve of omni3d_solve for a prepared context, issued on `st` with no host
@@ -373,9 +442,11 @@ cudaError_t enqueue_prepared(omni3d_ctx *ctx, const float *dax, const float *day
     const long long ref = (long long)P.ref_i + (long long)P.ref_j * g.X + (long long)P.ref_k * g.XY;
     Field F;
     F.f32 = ctx->f32.as<float4>();
-    F.bf16 = bf16 ? ctx->b16.as<uint2>() : nullptr;
+    F.lay = ctx->lay;
+    F.edge = F.lay.wrap ? ctx->edge.as<float4>() : nullptr;
     cudaError_t e = pack_field(g, dax, day, daz, nullptr, &F, bf16, st);
     if (e != cudaSuccess) return e;
+    const bool zero = !dpinit;
     if (!dpinit) {
         if ((e = cudaMemsetAsync(ctx->in_pinit.p, 0, sizeof(float) * (size_t)V, st)) != cudaSuccess) return e;
         dpinit = ctx->in_pinit.as<float>();
@@ -391,16 +462,16 @@ cudaError_t enqueue_prepared(omni3d_ctx *ctx, const float *dax, const float *day
         std::swap(pc, pn);
     }
     float2 *acc = ctx->pncnt.as<float2>();
-    float *vol = ctx->pvol_a.as<float>(), *dout = ctx->pout.as<float>(), *dcnt = ctx->cnt.as<float>();
+    float *vol = ctx->pw.as<float>(), *dout = ctx->pout.as<float>(), *dcnt = ctx->cnt.as<float>();
     if (K == 0) {
         if ((e = cudaMemcpyAsync(dout, dpinit, sizeof(float) * (size_t)V, cudaMemcpyDeviceToDevice, st))) return e;
         if ((e = cudaMemsetAsync(dcnt, 0, sizeof(float) * (size_t)V, st))) return e;
     } else {
-        if ((e = cudaMemcpyAsync(vol, dpinit, sizeof(float) * (size_t)V, cudaMemcpyDeviceToDevice, st))) return e;
-        if ((e = anchor_scatter(A, pc, vol, st))) return e;
-        if ((e = init_accum(V, dpinit, seed && K == 1, acc, st))) return e;
-        if ((e = sweep_full(ctx->geo, F, P.method, bf16, vol, acc, st))) return e;
-        if ((e = normalize(V, acc, dpinit, dout, dcnt, st))) return e;
+        if ((e = start_volume(g, F.lay, dpinit, zero, vol, st))) return e;
+        if ((e = anchor_scatter(g, F.lay, A, pc, vol, st))) return e;
+        if ((e = init_accum(g, F.lay, dpinit, seed && K == 1, acc, st))) return e;
+        if ((e = sweep_full(ctx->geo, F, P.method, vol, acc, st))) return e;
+        if ((e = normalize(g, F.lay, acc, dpinit, dout, dcnt, st))) return e;
     }
     if ((e = apply_gauge(V, P.gauge, ref, dcnt, dout, ctx->scratch.as<double>() + 4, st))) return e;
     if (p_out && (e = cudaMemcpyAsync(p_out, dout, sizeof(float) * (size_t)V, cudaMemcpyDeviceToDevice, st))) return e;
@@ -502,9 +573,10 @@ cudaError_t tune_line_order(omni3d_ctx *ctx, std::string *err)
         if ((e = build_geometry(&geo, ctx->st, err)) != cudaSuccess) break;
         Field F;
         F.f32 = field;
-        e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, false, p, acc, ctx->st);  // warm-up
+        F.lay = row_major_layout(g);
+        e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, p, acc, ctx->st);  // warm-up
         cudaEventRecord(ctx->ev[2], ctx->st);
-        if (e == cudaSuccess) e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, false, p, acc, ctx->st);
+        if (e == cudaSuccess) e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, p, acc, ctx->st);
         cudaEventRecord(ctx->ev[3], ctx->st);
         if (e == cudaSuccess) e = cudaEventSynchronize(ctx->ev[3]);
         const float ms = ms_between(ctx->ev[2], ctx->ev[3]);
@@ -640,7 +712,7 @@ int omni3d_destroy(omni3d_ctx *ctx)
     adjoint_free(&ctx->adj);
     ctx->adj_g.release();
     ctx->adj_out.release();
-    for (DeviceBuf *b : {&ctx->in_ax, &ctx->in_ay, &ctx->in_az, &ctx->in_aux, &ctx->in_pinit, &ctx->f32, &ctx->b16,
+    for (DeviceBuf *b : {&ctx->in_ax, &ctx->in_ay, &ctx->in_az, &ctx->in_aux, &ctx->in_pinit, &ctx->f32, &ctx->edge, &ctx->pw,
                          &ctx->curl, &ctx->pvol_a, &ctx->pvol_b, &ctx->pout, &ctx->cnt, &ctx->pncnt, &ctx->scratch,
                          &ctx->flags, &ctx->centre, &ctx->pncnt64})
         b->release();
@@ -689,19 +761,35 @@ int omni3d_line_steps(omni3d_ctx *ctx, long long line, int8_t *axes, int cap)
     if (!ctx || !axes || line < 0 || line >= ctx->geo.n_lines) return fail(ctx, OMNI3D_ERR_ARG, "bad arguments");
     cudaSetDevice(ctx->prm.device);
     LineRec r;
-    uint32_t gb;
     CK(ctx, cudaMemcpyAsync(&r, ctx->geo.d_lines + line, sizeof(r), cudaMemcpyDeviceToHost, ctx->st));
-    CK(ctx, cudaMemcpyAsync(&gb, ctx->geo.d_gbase + (line >> 5), sizeof(gb), cudaMemcpyDeviceToHost, ctx->st));
+    // the last group whose first line is not beyond this one
+    GroupRec G{};
+    for (long long lo = 0, hi = ctx->geo.n_groups; lo < hi;) {
+        const long long mid = (lo + hi) / 2;
+        GroupRec q;
+        CK(ctx, cudaMemcpyAsync(&q, ctx->geo.d_groups + mid, sizeof(q), cudaMemcpyDeviceToHost, ctx->st));
+        CK(ctx, cudaStreamSynchronize(ctx->st));
+        if ((long long)q.line0 <= line) {
+            G = q;
+            lo = mid + 1;
+        } else {
+            hi = mid;
+        }
+    }
     CK(ctx, cudaStreamSynchronize(ctx->st));
     if (r.m > cap) return fail(ctx, OMNI3D_ERR_RANGE, "cap smaller than the line's step count");
-    int nw = (r.m + 15) / 16;
-    std::vector<uint32_t> words((size_t)std::max(nw, 1));
-    for (int w = 0; w < nw; w++)
-        CK(ctx, cudaMemcpyAsync(&words[w], ctx->geo.d_desc + 32ull * gb + 32ull * w + (line & 31), sizeof(uint32_t),
+    const uint32_t nw = (G.span + 15) / 16, lane = (uint32_t)(line - (long long)G.line0);
+    std::vector<uint32_t> words((size_t)std::max(nw, 1u));
+    for (uint32_t w = 0; w < nw; w++)
+        CK(ctx, cudaMemcpyAsync(&words[w], ctx->geo.d_desc + 32ull * ((size_t)G.word0 + w) + lane, sizeof(uint32_t),
                                 cudaMemcpyDeviceToHost, ctx->st));
     CK(ctx, cudaStreamSynchronize(ctx->st));
-    for (int s = 0; s < r.m; s++) axes[s] = (int8_t)((words[s >> 4] >> (2 * (s & 15))) & 3u);
-    return r.m;
+    int n = 0;
+    for (uint32_t s = 0; s < 16 * nw && n < r.m; s++) {
+        const uint32_t a = (words[s >> 4] >> (2 * (s & 15))) & 3u;
+        if (a != 3u) axes[n++] = (int8_t)a;  // 3: the group's idle code
+    }
+    return n;
 }
 
 int omni3d_gauge(omni3d_ctx *ctx, float *p, const float *count, long long n, int gauge, long long ref,
@@ -781,29 +869,28 @@ int omni3d_centre_integration(omni3d_ctx *ctx, const float *ax, const float *ay,
     return OMNI3D_OK;
 }
 
-int omni3d_sweep(omni3d_ctx *ctx, const float *ax, const float *ay, const float *az, const float *curl, const float *p,
-                 float *pn, float *count, int device_ptrs)
+namespace {
+
+int sweep_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *az, const float *curl, const float *p,
+               float *pn, float *count, bool dev)
 {
-    if (!ctx || !ax || !ay || !az || !p || !pn || !count) return fail(ctx, OMNI3D_ERR_ARG, "NULL argument");
-    if (method_uses_curl(ctx->prm.method) && !curl)
-        return fail(ctx, OMNI3D_ERR_ARG, "the selected and weighted methods need curl");
-    cudaSetDevice(ctx->prm.device);
-    const long long V = ctx->geo.grid.V;
-    const bool dev = device_ptrs != 0;
+    const Grid &g = ctx->geo.grid;
+    const long long V = g.V;
     Field F;
     int rc = prepare_field(ctx, ax, ay, az, curl, nullptr, dev, &F);
     if (rc) return rc;
     if (ctx->geo.walk_rule == 3) CK(ctx, run_walk(&ctx->geo, 3, F.curl, ctx->st));  // paths follow this field
-    const float *dp;
+    const float *dp, *wp;
     if ((rc = stage(ctx, p, dev, ctx->in_pinit, V, &dp))) return rc;
-    CK(ctx, ctx->pncnt.ensure(sizeof(float2) * (size_t)V));
     float2 *acc = ctx->pncnt.as<float2>();
     const bool bf16 = ctx->prm.grad_storage == OMNI3D_GRAD_BF16;
     int engine = choose_engine(ctx, bf16, &rc);
     if (rc) return rc;
     if ((rc = engine_prepare(ctx, &engine, F, ctx->prm.method))) return rc;
-    CK(ctx, init_accum(V, nullptr, false, acc, ctx->st));
-    CK(ctx, engine_sweep(ctx, engine, F, ctx->prm.method, bf16, dp, acc, ctx->st));
+    const Layout lay = engine_layout(engine, F);
+    CK(ctx, walk_pressure(ctx, lay, dp, &wp, ctx->st));
+    CK(ctx, init_accum(g, lay, nullptr, false, acc, ctx->st));
+    CK(ctx, engine_sweep(ctx, engine, F, ctx->prm.method, wp, acc, ctx->st));
     // add (pn, count) to the caller's arrays
     float *dpn = pn, *dcount = count;
     if (!dev) {
@@ -814,13 +901,28 @@ int omni3d_sweep(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
         CK(ctx, cudaMemcpyAsync(dpn, pn, sizeof(float) * (size_t)V, cudaMemcpyHostToDevice, ctx->st));
         CK(ctx, cudaMemcpyAsync(dcount, count, sizeof(float) * (size_t)V, cudaMemcpyHostToDevice, ctx->st));
     }
-    CK(ctx, accum_split(V, acc, dpn, dcount, ctx->st));
+    CK(ctx, accum_split(g, lay, acc, dpn, dcount, ctx->st));
     if (!dev) {
         CK(ctx, cudaMemcpyAsync(pn, dpn, sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, ctx->st));
         CK(ctx, cudaMemcpyAsync(count, dcount, sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, ctx->st));
     }
     CK(ctx, cudaStreamSynchronize(ctx->st));
     return engine_check(ctx, engine);
+}
+
+}  // namespace
+
+int omni3d_sweep(omni3d_ctx *ctx, const float *ax, const float *ay, const float *az, const float *curl, const float *p,
+                 float *pn, float *count, int device_ptrs)
+{
+    if (!ctx || !ax || !ay || !az || !p || !pn || !count) return fail(ctx, OMNI3D_ERR_ARG, "NULL argument");
+    if (method_uses_curl(ctx->prm.method) && !curl)
+        return fail(ctx, OMNI3D_ERR_ARG, "the selected and weighted methods need curl");
+    cudaSetDevice(ctx->prm.device);
+    // no allocation follows the first write of the caller's arrays, so the call can be repeated
+    int rc = sweep_impl(ctx, ax, ay, az, curl, p, pn, count, device_ptrs != 0);
+    if (drop_skewed(ctx, rc)) rc = sweep_impl(ctx, ax, ay, az, curl, p, pn, count, device_ptrs != 0);
+    return rc;
 }
 
 namespace {
@@ -888,14 +990,10 @@ cudaError_t iterate_chunk(omni3d_ctx *ctx, const Anchor &A, int gauge, long long
     return cudaSuccess;
 }
 
-}  // namespace
-
-int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float *az, const float *curl,
-                 const float *mask, const float *p_init, float *p_out, float *count_out, int device_ptrs,
-                 omni3d_stats *stats)
+int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *az, const float *curl,
+               const float *mask, const float *p_init, float *p_out, float *count_out, int device_ptrs,
+               omni3d_stats *stats)
 {
-    if (!ctx || !ax || !ay || !az || !p_out) return fail(ctx, OMNI3D_ERR_ARG, "NULL argument");
-    cudaSetDevice(ctx->prm.device);
     const omni3d_params &P = ctx->prm;
     const Grid &g = ctx->geo.grid;
     const long long V = g.V;
@@ -937,7 +1035,6 @@ int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
         }
         dpinit = ctx->in_pinit.as<float>();
     }
-    CK(ctx, ctx->pncnt.ensure(sizeof(float2) * (size_t)V));
     CK(ctx, ctx->pout.ensure(sizeof(float) * (size_t)V));
     CK(ctx, ctx->cnt.ensure(sizeof(float) * (size_t)V));
     CK(ctx, ctx->pvol_a.ensure(sizeof(float) * (size_t)V));
@@ -950,6 +1047,9 @@ int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
 
     const int K = P.max_iter;
     const bool seed = P.seed_first_iteration != 0;
+    const bool zero_init = !p_init && P.initial_guess != OMNI3D_INIT_CENTRE;
+    const Layout lay = engine_layout(engine, F);  // of the sweeps' pressure and sums
+    const float *wp = nullptr;                    // the pressure a sweep reads, in that layout
     int done = 0;
     double rel = 0.0;
     double hred[2];
@@ -971,7 +1071,7 @@ int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
         fx->hmax = 0.5 * (double)P.density * (double)std::max(std::max(std::fabs(P.dx), std::fabs(P.dy)), std::fabs(P.dz));
         fx->path = (double)g.X + (double)g.Y + (double)g.Z;
         unsigned lmax = 0;
-        CK(ctx, max_lines_through(&ctx->geo, st, &lmax));
+        CK(ctx, max_lines_through(&ctx->geo, F.lay, ctx->pw.as<uint32_t>(), st, &lmax));
         fx->lmax = (double)lmax;
         CK(ctx, fix_field_bounds(V, F.f32, *fx, st));
         CK(ctx, fix_fill_scales(*fx, st));
@@ -991,7 +1091,7 @@ int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
                 max_links = (long long)(0.8 * (double)fr / 8.0);
             }
             e = anchor_build(ctx->geo, F, P.method, P.gauge == OMNI3D_GAUGE_POINT ? ref : -1, max_links,
-                             &ctx->anc, st, &aerr, fx);
+                             &ctx->anc, st, &aerr, fx, ctx->pw.as<uint32_t>());
             ctx->anc_cached = e == cudaSuccess && P.method == OMNI3D_METHOD_PLAIN;
             adjoint_free(&ctx->adj);
         }
@@ -1028,30 +1128,31 @@ int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
         cudaEventRecord(ctx->ev[1], st);
         double2 *acc64 = nullptr;
         if (P.sweep_fp64 || det) {
-            CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)V));
+            CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)lay.copies * (size_t)V));
             acc64 = ctx->pncnt64.as<double2>();
         }
         for (int it = 1; it <= K; it++) {
+            CK(ctx, walk_pressure(ctx, lay, pc, &wp, st));
             if (det) {  // exact fixed-point sums, normalised in FP64
                 Fix2 *accf = reinterpret_cast<Fix2 *>(acc64);
                 CK(ctx, fix_sweep_scales(V, pc, *fx, st));
-                CK(ctx, init_accum_fix(V, dpinit, seed && it == 1, *fx, accf, st));
+                CK(ctx, init_accum_fix(g, lay, dpinit, seed && it == 1, *fx, accf, st));
                 cudaEventRecord(ctx->ev[5], st);
-                CK(ctx, sweep_full_fix(ctx->geo, F, P.method, bf16, pc, accf, fx->scale, st));
+                CK(ctx, sweep_full_fix(ctx->geo, F, P.method, wp, accf, fx->scale, st));
                 cudaEventRecord(ctx->ev[6], st);
-                CK(ctx, normalize_fix(V, accf, *fx, pc, pn, dcnt, st));
+                CK(ctx, normalize_fix(g, lay, accf, *fx, pc, pn, dcnt, st));
             } else if (acc64) {
-                CK(ctx, init_accum64(V, dpinit, seed && it == 1, acc64, st));
+                CK(ctx, init_accum64(g, lay, dpinit, seed && it == 1, acc64, st));
                 cudaEventRecord(ctx->ev[5], st);
-                CK(ctx, sweep_full64(ctx->geo, F, P.method, bf16, pc, acc64, st));
+                CK(ctx, sweep_full64(ctx->geo, F, P.method, wp, acc64, st));
                 cudaEventRecord(ctx->ev[6], st);
-                CK(ctx, normalize64(V, acc64, pc, pn, dcnt, st));
+                CK(ctx, normalize64(g, lay, acc64, pc, pn, dcnt, st));
             } else {
-                CK(ctx, init_accum(V, dpinit, seed && it == 1, acc, st));
+                CK(ctx, init_accum(g, lay, dpinit, seed && it == 1, acc, st));
                 cudaEventRecord(ctx->ev[5], st);
-                CK(ctx, engine_sweep(ctx, engine, F, P.method, bf16, pc, acc, st));
+                CK(ctx, engine_sweep(ctx, engine, F, P.method, wp, acc, st));
                 cudaEventRecord(ctx->ev[6], st);
-                CK(ctx, normalize(V, acc, pc, pn, dcnt, st));
+                CK(ctx, normalize(g, lay, acc, pc, pn, dcnt, st));
             }
             done = it;
             if (P.tol > 0.0) {
@@ -1107,31 +1208,38 @@ int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
         }
         cudaEventRecord(ctx->ev[2], st);
         float *vol = ctx->pvol_a.as<float>();
-        CK(ctx, cudaMemcpyAsync(vol, dpinit, sizeof(float) * (size_t)V, cudaMemcpyDeviceToDevice, st));
-        CK(ctx, anchor_scatter(A, pc, vol, st));
+        if (det || !lay.wrap) {  // row-major first: the bit-reproducible mode bounds its values
+            CK(ctx, cudaMemcpyAsync(vol, dpinit, sizeof(float) * (size_t)V, cudaMemcpyDeviceToDevice, st));
+            CK(ctx, anchor_scatter(g, row_major_layout(g), A, pc, vol, st));
+            CK(ctx, walk_pressure(ctx, lay, vol, &wp, st));
+        } else {
+            CK(ctx, start_volume(g, lay, dpinit, zero_init, ctx->pw.as<float>(), st));
+            CK(ctx, anchor_scatter(g, lay, A, pc, ctx->pw.as<float>(), st));
+            wp = ctx->pw.as<float>();
+        }
         if (det) {  // bit-reproducible: exact fixed-point sums, normalised in FP64
-            CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)V));
+            CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)lay.copies * (size_t)V));
             Fix2 *accf = reinterpret_cast<Fix2 *>(ctx->pncnt64.p);
             CK(ctx, fix_sweep_scales(V, vol, *fx, st));
-            CK(ctx, init_accum_fix(V, dpinit, seed && its == 0, *fx, accf, st));
+            CK(ctx, init_accum_fix(g, lay, dpinit, seed && its == 0, *fx, accf, st));
             cudaEventRecord(ctx->ev[5], st);
-            CK(ctx, sweep_full_fix(ctx->geo, F, P.method, bf16, vol, accf, fx->scale, st));
+            CK(ctx, sweep_full_fix(ctx->geo, F, P.method, wp, accf, fx->scale, st));
             cudaEventRecord(ctx->ev[6], st);
-            CK(ctx, normalize_fix(V, accf, *fx, dpinit, dout, dcnt, st));
+            CK(ctx, normalize_fix(g, lay, accf, *fx, dpinit, dout, dcnt, st));
         } else if (P.sweep_fp64) {  // the defect-correction sweep: FP64 sums and normalisation
-            CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)V));
+            CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)lay.copies * (size_t)V));
             double2 *acc64 = ctx->pncnt64.as<double2>();
-            CK(ctx, init_accum64(V, dpinit, seed && its == 0, acc64, st));
+            CK(ctx, init_accum64(g, lay, dpinit, seed && its == 0, acc64, st));
             cudaEventRecord(ctx->ev[5], st);
-            CK(ctx, sweep_full64(ctx->geo, F, P.method, bf16, vol, acc64, st));
+            CK(ctx, sweep_full64(ctx->geo, F, P.method, wp, acc64, st));
             cudaEventRecord(ctx->ev[6], st);
-            CK(ctx, normalize64(V, acc64, dpinit, dout, dcnt, st));
+            CK(ctx, normalize64(g, lay, acc64, dpinit, dout, dcnt, st));
         } else {
-            CK(ctx, init_accum(V, dpinit, seed && its == 0, acc, st));
+            CK(ctx, init_accum(g, lay, dpinit, seed && its == 0, acc, st));
             cudaEventRecord(ctx->ev[5], st);
-            CK(ctx, engine_sweep(ctx, engine, F, P.method, bf16, vol, acc, st));
+            CK(ctx, engine_sweep(ctx, engine, F, P.method, wp, acc, st));
             cudaEventRecord(ctx->ev[6], st);
-            CK(ctx, normalize(V, acc, dpinit, dout, dcnt, st));
+            CK(ctx, normalize(g, lay, acc, dpinit, dout, dcnt, st));
         }
         done = its + 1;
     }
@@ -1182,6 +1290,21 @@ int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
     return OMNI3D_OK;
 }
 
+}  // namespace
+
+int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float *az, const float *curl,
+                 const float *mask, const float *p_init, float *p_out, float *count_out, int device_ptrs,
+                 omni3d_stats *stats)
+{
+    if (!ctx || !ax || !ay || !az || !p_out) return fail(ctx, OMNI3D_ERR_ARG, "NULL argument");
+    cudaSetDevice(ctx->prm.device);
+    // every allocation precedes the first write of the caller's arrays, so the call can be repeated
+    int rc = solve_impl(ctx, ax, ay, az, curl, mask, p_init, p_out, count_out, device_ptrs, stats);
+    if (drop_skewed(ctx, rc))
+        rc = solve_impl(ctx, ax, ay, az, curl, mask, p_init, p_out, count_out, device_ptrs, stats);
+    return rc;
+}
+
 int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *grad_ay, float *grad_az,
                    int device_ptrs)
 {
@@ -1200,7 +1323,8 @@ int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *
     if (plain ? !ctx->anc_cached : !ctx->anc_last) {  // the last solve ran the sweep form: build it now
         Field F;
         F.f32 = ctx->f32.as<float4>();
-        F.bf16 = P.grad_storage == OMNI3D_GRAD_BF16 ? ctx->b16.as<uint2>() : nullptr;
+        F.lay = ctx->lay;
+        F.edge = F.lay.wrap ? ctx->edge.as<float4>() : nullptr;
         if (method_uses_curl(P.method)) {  // the curl the solve used, from the packed field
             CK(ctx, ctx->curl.ensure(sizeof(float) * (size_t)V));
             CK(ctx, field_curl(V, F.f32, ctx->curl.as<float>(), st));
@@ -1208,7 +1332,7 @@ int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *
         }
         std::string aerr;
         cudaError_t e = anchor_build(ctx->geo, F, P.method, P.gauge == OMNI3D_GAUGE_POINT ? ref : -1,
-                                     -1, &ctx->anc, st, &aerr);
+                                     -1, &ctx->anc, st, &aerr, nullptr, ctx->pw.as<uint32_t>());
         if (e != cudaSuccess) return fail(ctx, OMNI3D_ERR_CUDA, "anchor operator: " + aerr);
         ctx->anc_cached = plain;
         ctx->anc_last = true;

@@ -32,6 +32,12 @@ struct Fix2 {
     long long pn, cnt;
 };
 
+__device__ __forceinline__ void fold_add(Fix2 &a, const Fix2 &b)  // exact in any order
+{
+    a.pn += b.pn;
+    a.cnt += b.cnt;
+}
+
 __device__ __forceinline__ unsigned long long fix_term(float x, double s)
 {
     return (unsigned long long)__double2ll_rn((double)x * s);

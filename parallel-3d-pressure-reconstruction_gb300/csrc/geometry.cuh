@@ -310,4 +310,68 @@ struct OmWalker {
     }
 };
 
+// OmWalker for the rules that read no field (0, 1, 2) on grids of fewer than kFastWalkMax cells a
+// side: the same operations in the same order, with the coordinates kept as floats (exact there)
+// and the decisions taken without branches, which the lanes of a warp would take differently at
+// almost every step.  Plain comparisons of the squared distances decide, unless two of them are
+// within 2^-20 of each other: then the reference's comparisons of their roots.
+// 256^3 / 642 directions: 79 -> 60 ms (OmWalker: 183 instructions per step at 160^3, issue 92 % busy).
+constexpr int kFastWalkMax = 1 << 23;
+struct OmFastWalker {
+    float x, y, z, k1, k2, k3, xk1, yk2, zk3;
+    float fi, fj, fk;  // current voxel
+    float oi, oj, ok;  // exit voxel
+    float si, sj, sk;  // step toward it
+
+    __device__ __forceinline__ void init(const Grid &g, float ox, float oy, float oz, float d1, float d2, float d3, int ie,
+                                         int je, int ke, int ix, int jx, int kx)
+    {
+        OmWalker w;
+        w.init(g, ox, oy, oz, d1, d2, d3, ie, je, ke, ix, jx, kx);
+        x = w.x; y = w.y; z = w.z; k1 = w.k1; k2 = w.k2; k3 = w.k3;
+        xk1 = w.xk1; yk2 = w.yk2; zk3 = w.zk3;
+        fi = (float)ie; fj = (float)je; fk = (float)ke;
+        oi = (float)ix; oj = (float)jx; ok = (float)kx;
+        si = ie < ix ? 1.0f : -1.0f; sj = je < jx ? 1.0f : -1.0f; sk = ke < kx ? 1.0f : -1.0f;
+    }
+
+    // One step: the axis moved along, or -1 when no candidate qualifies.
+    template <int RULE>
+    __device__ __forceinline__ int step()
+    {
+        static_assert(RULE != 3, "the minimum-curl walk reads a field");
+        const bool mi = fi != oi, mj = fj != oj, mk = fk != ok;
+        const float f1 = OM_ADD(fi, mi ? si : -60000.0f), f2 = OM_ADD(fj, mj ? sj : -60000.0f),
+                    f3 = OM_ADD(fk, mk ? sk : -60000.0f);
+        const float k2jl = OM_MUL(k2, fj), k3kl = OM_MUL(k3, fk);
+        const float A = OM_SUB(OM_MUL(k1, fi), xk1);
+        const float r1 = OM_SUB(OM_ADD(OM_SUB(OM_ADD(OM_SUB(OM_MUL(k1, f1), xk1), k2jl), yk2), k3kl), zk3);
+        const float r2 = OM_SUB(OM_ADD(OM_SUB(OM_ADD(A, OM_MUL(k2, f2)), yk2), k3kl), zk3);
+        const float r3 = OM_SUB(OM_ADD(OM_SUB(OM_ADD(A, k2jl), yk2), OM_MUL(k3, f3)), zk3);
+        const float q1 = om_dist2(x, y, z, k1, k2, k3, r1, f1, fj, fk);
+        const float q2 = om_dist2(x, y, z, k1, k2, k3, r2, fi, f2, fk);
+        const float q3 = om_dist2(x, y, z, k1, k2, k3, r3, fi, fj, f3);
+        constexpr float c = 9.5367431640625e-7f;  // 2^-20
+        const bool near = (fabsf(OM_SUB(q1, q2)) <= OM_MUL(c, fminf(q1, q2))) | (fabsf(OM_SUB(q1, q3)) <= OM_MUL(c, fminf(q1, q3))) |
+                          (fabsf(OM_SUB(q2, q3)) <= OM_MUL(c, fminf(q2, q3)));
+        bool b0, b1, b2;
+        if (near) {
+            b0 = (RULE == 2 ? om_sqrt_lt(q1, q2) : om_sqrt_le(q1, q2)) & om_sqrt_le(q1, q3);
+            b1 = (RULE == 2 ? om_sqrt_le(q2, q1) : om_sqrt_lt(q2, q1)) & om_sqrt_le(q2, q3);
+            b2 = om_sqrt_lt(q3, q1) & om_sqrt_lt(q3, q2);
+        } else {
+            b0 = (RULE == 2 ? q1 < q2 : q1 <= q2) & (q1 <= q3);
+            b1 = (RULE == 2 ? q2 <= q1 : q2 < q1) & (q2 <= q3);
+            b2 = (q3 < q1) & (q3 < q2);
+        }
+        b0 = b0 & mi & ((RULE != 2) | (fj != 0.0f));
+        b1 = b1 & mj & ((RULE == 0) | (f2 != 0.0f)) & !b0;
+        b2 = b2 & mk & ((RULE != 2) | (fj != 0.0f)) & !b0 & !b1;
+        fi = b0 ? f1 : fi;
+        fj = b1 ? f2 : fj;
+        fk = b2 ? f3 : fk;
+        return b0 ? 0 : (b1 ? 1 : (b2 ? 2 : -1));
+    }
+};
+
 }  // namespace omni3d

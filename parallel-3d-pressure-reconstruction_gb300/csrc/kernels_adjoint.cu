@@ -25,36 +25,11 @@
 #include <utility>
 
 #include "omni3d_internal.h"
+#include "walk.cuh"
 
 namespace omni3d {
 
 namespace {
-
-struct AdjWalk {
-    long long v;
-    int d0, d1, d2;
-    float h0, h1, h2;
-    int m;
-    const uint32_t *dp;
-    __device__ __forceinline__ void init(const Grid &g, const LineRec &r, const uint32_t *gbase, const uint32_t *desc,
-                                         long long li)
-    {
-        int ie = (int)(r.e % (uint32_t)g.X), je = (int)((r.e / (uint32_t)g.X) % (uint32_t)g.Y),
-            ke = (int)(r.e / (uint32_t)g.XY);
-        int ix = (int)(r.x % (uint32_t)g.X), jx = (int)((r.x / (uint32_t)g.X) % (uint32_t)g.Y),
-            kx = (int)(r.x / (uint32_t)g.XY);
-        int si = ix > ie ? 1 : -1, sj = jx > je ? 1 : -1, sk = kx > ke ? 1 : -1;
-        d0 = si;
-        d1 = sj * g.X;
-        d2 = sk * (int)g.XY;
-        h0 = __fmul_rn(-g.rho * (float)si, g.dx) * 0.5f;
-        h1 = __fmul_rn(-g.rho * (float)sj, g.dy) * 0.5f;
-        h2 = __fmul_rn(-g.rho * (float)sk, g.dz) * 0.5f;
-        v = r.e;
-        m = r.m;
-        dp = desc + 32ull * gbase[li >> 5] + (li & 31);
-    }
-};
 
 // The per-line program of a method's accumulation (the forward kernels' state machines and
 // weight arithmetic): init() at the entry gives the entry's contribution weight and whether
@@ -130,26 +105,28 @@ struct LineProg {
     }
 };
 
-// Step decoder over a line's staircase (2-bit steps, lane-interleaved words).
+// Step decoder over a line's staircase (2-bit steps between its group's idle codes).
 struct StepCursor {
-    const uint32_t *dp;
     uint32_t word;
-    int s, m;
-    long long v;
-    __device__ __forceinline__ bool next(const AdjWalk &L, int &a, long long &prev)
+    uint32_t s;
+    uint32_t v;
+    __device__ __forceinline__ bool next(const LineWalk &L, int &a, uint32_t &prev)
     {
-        if (s >= m) return false;
-        if ((s & 15) == 0) word = __ldg(dp + 32 * (s >> 4));
-        a = (int)(word & 3u);
-        word >>= 2;
+        do {
+            if (s >= L.span) return false;
+            if ((s & 15) == 0) word = __ldg(L.dp + 32 * (s >> 4));
+            a = (int)(word & 3u);
+            word >>= 2;
+            s++;
+        } while (a == kIdle);
         prev = v;
-        v += a == 0 ? L.d0 : (a == 1 ? L.d1 : L.d2);
-        s++;
+        v += (uint32_t)(a == 0 ? L.d0 : (a == 1 ? L.d1 : L.d2));
+        v = min(v, v + L.wv);
         return true;
     }
 };
 
-__device__ __forceinline__ float curl_at(const float4 *f32, long long v) { return __ldg(&f32[v].w); }
+__device__ __forceinline__ float curl_at(const float4 *f32, uint32_t v) { return __ldg(&f32[v].w); }
 
 // mu = g / c where c > 0, else 0
 __global__ void k_adj_mu(long long V, const float *g, const float *cnt, float *mu)
@@ -160,26 +137,21 @@ __global__ void k_adj_mu(long long V, const float *g, const float *cnt, float *m
 
 // lambda[id(start)] += sum of w mu over each segment (S^T mu)
 template <int ACC>
-__global__ void __launch_bounds__(256) k_adj_gather(Grid g, const LineRec *__restrict__ lines,
-                                                    const uint32_t *__restrict__ gbase,
-                                                    const uint32_t *__restrict__ desc, long long n_lines,
+__global__ void __launch_bounds__(256) k_adj_gather(Grid g, Layout lay, WalkLines W,
                                                     const float4 *__restrict__ f32, const float *__restrict__ mu,
                                                     const int32_t *__restrict__ id, float *lam)
 {
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    AdjWalk L;
-    L.init(g, r, gbase, desc, li);
+    LineWalk L;
+    if (!L.init(g, lay, W) || !L.on) return;
     LineProg<ACC> P;
     float w;
     bool seg;
     P.init(curl_at(f32, L.v), g.thr, w, seg);
-    long long start = seg ? L.v : -1;
+    long long start = seg ? (long long)L.v : -1;
     float t = w != 0.0f ? w * __ldg(mu + L.v) : 0.0f;
-    StepCursor c{L.dp, 0u, 0, L.m, L.v};
+    StepCursor c{0u, 0u, L.v};
     int a;
-    long long prev;
+    uint32_t prev;
     while (c.next(L, a, prev)) {
         bool term, restart;
         P.step(a, curl_at(f32, c.v), g.thr, w, term, restart);
@@ -202,12 +174,12 @@ __global__ void __launch_bounds__(256) k_adj_gather(Grid g, const LineRec *__res
 // The sum of w dB over the contributions of the segment that follows the cursor's position
 // (up to the next segment start or the end of the line), without moving the cursor.
 template <int ACC>
-__device__ __forceinline__ float segment_total(const Grid &g, const AdjWalk &L, StepCursor c, LineProg<ACC> P,
+__device__ __forceinline__ float segment_total(const Grid &g, const LineWalk &L, StepCursor c, LineProg<ACC> P,
                                                const float4 *f32, const float *dB)
 {
     float T = 0.0f;
     int a;
-    long long prev;
+    uint32_t prev;
     while (c.next(L, a, prev)) {
         float w;
         bool term, restart;
@@ -220,25 +192,20 @@ __device__ __forceinline__ float segment_total(const Grid &g, const AdjWalk &L, 
 
 // dL/da along every segment: suffix sums R_t of w dB times the trapezoid coefficients
 template <int ACC>
-__global__ void __launch_bounds__(256) k_adj_grad(Grid g, const LineRec *__restrict__ lines,
-                                                  const uint32_t *__restrict__ gbase,
-                                                  const uint32_t *__restrict__ desc, long long n_lines,
+__global__ void __launch_bounds__(256) k_adj_grad(Grid g, Layout lay, WalkLines W,
                                                   const float4 *__restrict__ f32, const float *__restrict__ dB,
                                                   float *gx, float *gy, float *gz)
 {
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    AdjWalk L;
-    L.init(g, r, gbase, desc, li);
+    LineWalk L;
+    if (!L.init(g, lay, W) || !L.on) return;
     LineProg<ACC> P;
     float w;
     bool seg;
     P.init(curl_at(f32, L.v), g.thr, w, seg);
-    StepCursor c{L.dp, 0u, 0, L.m, L.v};
+    StepCursor c{0u, 0u, L.v};
     float R = seg ? segment_total<ACC>(g, L, c, P, f32, dB) : 0.0f;
     int a;
-    long long prev;
+    uint32_t prev;
     while (c.next(L, a, prev)) {
         bool term, restart;
         P.step(a, curl_at(f32, c.v), g.thr, w, term, restart);
@@ -418,12 +385,14 @@ template <int ACC>
 void launch_adj_lines(const Geometry &geo, bool gather, const float4 *f32, const float *in, const int32_t *id,
                       float *lam, float *gx, float *gy, float *gz, cudaStream_t st)
 {
-    const unsigned lblocks = (unsigned)((geo.n_lines + 255) / 256);
+    const unsigned lblocks = group_blocks(geo, 256);
+    const Layout lay = row_major_layout(geo.grid);
+    const WalkLines W{geo.d_groups, geo.n_groups, geo.d_lines, geo.d_desc};
     if (gather)
-        k_adj_gather<ACC><<<lblocks, 256, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc, geo.n_lines, f32, in,
+        k_adj_gather<ACC><<<lblocks, 256, 0, st>>>(geo.grid, lay, W, f32, in,
                                                    id, lam);
     else
-        k_adj_grad<ACC><<<lblocks, 256, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc, geo.n_lines, f32, in,
+        k_adj_grad<ACC><<<lblocks, 256, 0, st>>>(geo.grid, lay, W, f32, in,
                                                  gx, gy, gz);
     OM_COUNT_LAUNCH();
 }

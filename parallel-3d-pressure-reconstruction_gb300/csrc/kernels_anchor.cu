@@ -17,17 +17,18 @@
 // the anchors, the geometry's line counts size each anchor's row, a filling pass writes
 // (column = start anchor, weight) pairs and accumulates b and c.  The filling pass learns
 // whether a visited voxel is an anchor from the field gather itself: for the duration of
-// the pass the anchors' packed field entries carry a flag in a bit no value uses (the sign
-// of the curl in .w, curl being non-negative), so a step costs one gather instead of a
-// gather and a bitmap load.  A field with a negative curl value keeps the bitmap.  The
-// operator passes read the float4 entries, which with BF16 storage hold the stored values
-// (k_pack): they are bound by instruction issue, not by their gathers, and so read nothing
-// that needs unpacking.
+// the pass the anchors' field records carry a flag in a bit no value uses (the sign
+// of the curl in .w, curl being non-negative), so a step costs one gather.  A field with a
+// negative curl value gathers the anchor id beside it.
 //
 // The filling pass sums each line's integral in plain FP32 in step order, as the reference
 // does (K:1816-1834); the final sweep, whose integrals reach every voxel directly, keeps
-// compensated sums.  The filling pass is bound by instruction issue, and the three
-// additions of the compensation took 2.7 ms of its 52.7 ms at 256^3 / 642 directions.
+// compensated sums (the compensation took 2.7 ms of the pass's 52.7 ms at 256^3 / 642 directions).
+//
+// What bounds the filling pass (160^3, 642 directions, ncu): the plain method's the L1 data pipe
+// (82-86 %: the 16-byte gathers), the selected method's the same pipe (73 %) beside the
+// half-rate integer and selection pipe (62 %, 47 instructions per step).  256^3 / 642 directions,
+// selected method, with the pass's setup: 44.3 -> 33.8 ms against the row-major walk.
 #include <algorithm>
 
 #include "fixed.cuh"
@@ -36,39 +37,31 @@
 
 namespace omni3d {
 
-// Steps whose gathers a walk issues together (walk.cuh): 4 beat 3 and 2 by 0.3 and 1.5 ms at
-// 256^3 / 642 directions; 5 and 6 spill.
+// Steps whose gathers a walk issues together: 4 beat 8 and 2 by 6 and 2 ms at 256^3 / 642
+// directions.
 constexpr int kWalkBatch = 4;
-// Launch shape of the operator passes: the filling pass waits on its gathers and issues many
-// instructions per step, and 40 resident warps per SM (48 registers, a few bytes spilled to
-// L1) beat 32 (64 registers, no spill) and 48 (more spills): with CTAs of 256 threads 50.0
-// against 55.1 and 56.2 ms at 256^3 / 642 directions.  Small CTAs then free their slots as
-// soon as their own few lines end, where a CTA of 8 warps waits for its longest line: 20
-// CTAs of 64 threads took the pass from 46.9 to 44.2 ms (10 of 128: 44.8 ms; 32 warps
-// without spills, 32 CTAs of 32 threads or 16 of 64: 48.1 ms).
-constexpr int kFillBlocks = 20;
+// Launch shape of the operator passes: 64 registers hold a batch with its records; at 48 (20
+// CTAs) the selected method's pass spills 90 bytes and took 39.5 instead of 36.9 ms.  Small CTAs
+// free their slots as soon as their own few lines end.
+constexpr int kFillBlocks = 16;
 constexpr int kFillThreads = 64;  // threads per CTA (whole warps: one line per thread)
+constexpr uint32_t kAllIdle = 0x55555555u & ((1u << (2 * kWalkBatch)) - 1u);  // no step of the batch is the lane's
 
 namespace {
 
-// Anchor flag of a gathered voxel: with FB the sign bit of its .w (the flag the filling
-// pass sets in the field), else its bit of the bitmap word gathered beside it.
+// Whether a gathered voxel is an anchor: with FB the sign bit of its curl (the flag the filling
+// pass sets in the field), else its anchor id gathered beside it.
 template <bool FB>
-__device__ __forceinline__ bool anchor_of(const float4 &gv, uint32_t word, long long v)
+__device__ __forceinline__ bool anchor_of(const float4 &gv, int32_t id)
 {
-    return FB ? (__float_as_uint(gv.w) >> 31) != 0u : ((word >> (v & 31)) & 1u) != 0u;
+    return FB ? (__float_as_uint(gv.w) >> 31) != 0u : id >= 0;
 }
 
-// Curl from .w of the FP32 field: under FB its sign bit is the anchor flag.
+// Curl of a gathered voxel: under FB its sign bit is the anchor flag.
 template <bool FB>
 __device__ __forceinline__ float curl_of(const float4 &gv)
 {
     return FB ? fabsf(gv.w) : gv.w;
-}
-
-__device__ __forceinline__ float sel3(int a, float x, float y, float z)
-{
-    return a == 0 ? x : (a == 1 ? y : z);
 }
 
 __device__ __forceinline__ void kahan_add(float &s, float &c, float x)
@@ -79,17 +72,11 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float x)
     s = t;
 }
 
-__device__ __forceinline__ bool is_anchor(const uint32_t *bits, long long v)
-{
-    return (__ldg(bits + (v >> 5)) >> (v & 31)) & 1u;
-}
-
 enum Pass { kMark = 0, kFill = 2, kRhs = 3 };
 
 struct Sink {
-    const uint32_t *bits;
-    const int32_t *id;
-    uint8_t *flag;
+    const int32_t *id;   // the walks' copies of the anchor ids (-1: no anchor)
+    uint8_t *flag;       // row-major (the marking pass walks the row-major layout)
     unsigned long long *next;  // per row: the next free link slot (starts at the row's first slot)
     uint32_t *col;   // unit-weight operators: the start anchor of each link
     uint2 *cw;       // weighted operators: (start anchor, weight bits) of each link
@@ -98,16 +85,13 @@ struct Sink {
     const double *fix;  // its scales (fixed.cuh)
 };
 
-// Record one contribution of weight wt and integral I into voxel v from the segment whose
-// start anchor is scol (its id, loaded once per segment).  A link costs one row lookup, one
-// 64-bit slot atomic, one store and one vector reduction of (b, c); UNIT operators (every
-// weight 1) store no weight.
+// Record one contribution of weight wt and integral I into the anchor row `row` (-1: none) from
+// the segment whose start anchor is scol (its id, loaded once per segment).  A link costs one
+// row lookup, one 64-bit slot atomic, one store and one vector reduction of (b, c); UNIT
+// operators (every weight 1) store no weight.
 template <int PASS, bool UNIT>
-__device__ __forceinline__ void emit_w(const Sink &S, uint32_t v, uint32_t scol, float wt, float I, bool anchor)
+__device__ __forceinline__ void emit_w(const Sink &S, int row, uint32_t scol, float wt, float I)
 {
-    if (PASS == kMark) return;
-    if (!anchor) return;
-    int row = __ldg(S.id + v);
     if (row < 0) return;  // not an anchor after all: nothing to index
     if (PASS == kFill && (int)scol < 0) return;  // a start that is no anchor: no column to link
     if (PASS == kRhs) {  // plain method, operator cached: only b = sum I is field-dependent
@@ -134,202 +118,292 @@ __device__ __forceinline__ uint32_t start_col(const Sink &S, uint32_t start)
     return PASS == kFill ? (uint32_t)__ldg(S.id + start) : 0u;
 }
 
-struct Walk {
-    uint32_t v;
-    int d0, d1, d2;
-    float h0, h1, h2;
-    int m;
-    const uint32_t *dp;
-    __device__ __forceinline__ void init(const Grid &g, const LineRec &r, const uint32_t *gbase,
-                                         const uint32_t *desc, long long li)
+// Element q of a batch's registers, q not known at compile time.
+template <typename T>
+__device__ __forceinline__ T pick(const T (&x)[kWalkBatch], int q)
+{
+    T r = x[0];
+#pragma unroll
+    for (int i = 1; i < kWalkBatch; i++) r = q == i ? x[i] : r;
+    return r;
+}
+
+// Bits 2q of the batch's steps that enter an anchor.
+template <bool FB>
+__device__ __forceinline__ uint32_t anchor_steps(uint32_t idle, const float4 (&g)[kWalkBatch], const int32_t (&id)[kWalkBatch])
+{
+    uint32_t m = 0u;
+#pragma unroll
+    for (int q = 0; q < kWalkBatch; q++)
+        m += (FB ? __float_as_uint(g[q].w) >> 31 : (uint32_t)~id[q] >> 31) << (2 * q);
+    return m & ~idle;
+}
+
+// Whether any lane's batch may enter an anchor (an idle step's sample counts too: a false alarm
+// costs the slower form, no record).
+template <bool FB>
+__device__ __forceinline__ bool any_anchor(const float4 (&g)[kWalkBatch], const int32_t (&id)[kWalkBatch])
+{
+    uint32_t m = 0u;
+#pragma unroll
+    for (int q = 0; q < kWalkBatch; q++) m |= FB ? __float_as_uint(g[q].w) : ~(uint32_t)id[q];
+    return __any_sync(0xffffffffu, (int32_t)m < 0);
+}
+
+// What every operator pass keeps along a line.  A batch without an anchor only sums; in one
+// with anchors the sums at its steps stay in registers and the lanes then record their
+// contributions together, each lane its next one per round, instead of step by step with the
+// few lanes that enter an anchor at that step (three of 32 on average): a record waits for a
+// row lookup and an atomic, and a round of them waits once.
+template <int GRAD>
+struct FillLine {
+    const LineWalk &L;
+    const Sink S;      // ids of the lane's copy
+    float4 gl;         // sample of the last voxel
+    float I = 0.0f;
+
+    // I += the trapezoid increment of step q of a batch, or 0 on a lane that does not take it
+    __device__ __forceinline__ void integrate(uint32_t c, int q, const float4 &gv, bool t)
     {
-        int ie = (int)(r.e % (uint32_t)g.X), je = (int)((r.e / (uint32_t)g.X) % (uint32_t)g.Y),
-            ke = (int)(r.e / (uint32_t)g.XY);
-        int ix = (int)(r.x % (uint32_t)g.X), jx = (int)((r.x / (uint32_t)g.X) % (uint32_t)g.Y),
-            kx = (int)(r.x / (uint32_t)g.XY);
-        int si = ix > ie ? 1 : -1, sj = jx > je ? 1 : -1, sk = kx > ke ? 1 : -1;
-        d0 = si;
-        d1 = sj * g.X;
-        d2 = sk * (int)g.XY;
-        h0 = __fmul_rn(-g.rho * (float)si, g.dx) * 0.5f;
-        h1 = __fmul_rn(-g.rho * (float)sj, g.dy) * 0.5f;
-        h2 = __fmul_rn(-g.rho * (float)sk, g.dz) * 0.5f;
-        v = r.e;
-        m = r.m;
-        dp = desc + 32ull * gbase[li >> 5] + (li & 31);
+        const float x = step_h(L, c, q) * step_sum<GRAD>(c, q, gv, gl);
+        I += t ? x : 0.0f;
+        if (GRAD != kGradEdge) gl = gv;
     }
 };
 
-// The trapezoid increment of a step along axis a, h_a (g_a(v) + g_a(previous voxel)), formed
-// for all three axes and then selected: one selection instead of three.  The filling pass is
-// bound by instruction issue with the selections' pipe the busiest, and this took 0.8 ms off
-// its 50 ms at 256^3 / 642 directions.
-__device__ __forceinline__ float step_term(int a, const Walk &L, const float4 &gv, const float4 &gl)
-{
-    return sel3(a, L.h0 * (gv.x + gl.x), L.h1 * (gv.y + gl.y), L.h2 * (gv.z + gl.z));
-}
-
 // Plain method: anchors are the entries; every voxel of a line takes (p[entry] + I, 1).
+template <int GRAD, int PASS, bool FB>
+struct PlainFill : FillLine<GRAD> {
+    uint32_t ecol;
+    template <bool MASK>
+    __device__ __forceinline__ bool quick(uint32_t, const float4 (&)[kWalkBatch], const int32_t (&)[kWalkBatch]) const
+    {
+        return true;
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void batch(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                          const float4 (&g)[kWalkBatch], const int32_t (&id)[kWalkBatch])
+    {
+        if (!any_anchor<FB>(g, id)) {
+#pragma unroll
+            for (int q = 0; q < kWalkBatch; q++) this->integrate(c, q, g[q], taken<MASK>(idle, q));
+            return;
+        }
+        float Is[kWalkBatch];
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) {
+            this->integrate(c, q, g[q], taken<MASK>(idle, q));
+            Is[q] = this->I;
+        }
+        for (uint32_t todo = anchor_steps<FB>(idle, g, id); todo; todo &= todo - 1u) {
+            const int q = (__ffs(todo) - 1) >> 1;
+            emit_w<PASS, true>(this->S, __ldg(this->S.id + pick(v, q)), ecol, 1.0f, pick(Is, q));
+        }
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void general(uint32_t, uint32_t, const uint32_t (&)[kWalkBatch],
+                                            const float4 (&)[kWalkBatch], const int32_t (&)[kWalkBatch])
+    {
+    }
+};
+
 // SELF = false leaves the entry's own term out (the minimum-curl plain variant).
-template <int PASS, bool SELF, bool FB>
+template <int GRAD, int PASS, bool SELF, bool FB>
 __global__ void __launch_bounds__(kFillThreads, kFillBlocks)
-k_anchor_plain(Grid g, const LineRec *__restrict__ lines,
-               const uint32_t *__restrict__ gbase,
-               const uint32_t *__restrict__ desc, long long n_lines,
-               const float4 *__restrict__ f32, Sink S)
+k_anchor_plain(Grid g, Layout lay, WalkLines W, WalkField F, Sink S)
 {
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
+    LineWalk L;
+    if (!L.init(g, lay, W)) return;
     if (PASS == kMark) {
-        S.flag[r.e] = 1;
+        if (L.on) S.flag[L.e] = 1;
         return;
     }
-    Walk L;
-    L.init(g, r, gbase, desc, li);
-    const uint32_t e = r.e;
-    const uint32_t ecol = start_col<PASS>(S, e);
-    if (SELF) emit_w<PASS, true>(S, e, ecol, 1.0f, 0.0f, is_anchor(S.bits, e));
-    float4 gl = __ldg(f32 + e);
-    float I = 0.0f;
-    // the field (and without FB the anchor bitmap word) of every voxel gathered in batches
-    walk_steps<kWalkBatch, kGradF32, !FB>(
-        L.v, L.d0, L.d1, L.d2, L.m, L.dp, f32, nullptr, S.bits, [&](int a, uint32_t v, const float4 &gv, uint32_t word) {
-            I += step_term(a, L, gv, gl);
-            gl = gv;
-            emit_w<PASS, true>(S, v, ecol, 1.0f, I, anchor_of<FB>(gv, word, v));
-        });
+    const float4 *field = lane_field<GRAD>(F, lay, L);
+    S.id += L.copy;
+    PlainFill<GRAD, PASS, FB> f{{L, S, sample<GRAD>(field, L.v)}, start_col<PASS>(S, L.v)};
+    if (SELF && L.on) emit_w<PASS, true>(S, __ldg(S.id + L.v), f.ecol, 1.0f, 0.0f);
+    walk_steps<kWalkBatch, GRAD, !FB>(L, field, S.id, f);
 }
 
-// Weighted method: the walk of k_sweep_weighted (K:1993-2135); anchors are the entries
-// (the marking pass is the plain method's), the entry itself receives nothing.
-template <int PASS, bool FB>
-__global__ void __launch_bounds__(kFillThreads, kFillBlocks)
-k_anchor_weighted(Grid g, const LineRec *__restrict__ lines,
-                  const uint32_t *__restrict__ gbase,
-                  const uint32_t *__restrict__ desc, long long n_lines,
-                  const float4 *__restrict__ f32,
-                  const float *__restrict__ curl, Sink S)
-{
-    static_assert(PASS == kFill, "the weighted operator has only a filling pass");
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    Walk L;
-    L.init(g, r, gbase, desc, li);
-    const uint32_t e = r.e;
-    const uint32_t ecol = start_col<PASS>(S, e);
-    float4 gl = __ldg(f32 + e);
-    float I = 0.0f, csum = 0.0f, nseg = 0.0f;
-    walk_steps<kWalkBatch, kGradF32, !FB>(
-        L.v, L.d0, L.d1, L.d2, L.m, L.dp, f32, nullptr, S.bits, [&](int a, uint32_t v, const float4 &gv, uint32_t word) {
-            float cn = curl_of<FB>(gv);
-            I += step_term(a, L, gv, gl);
-            csum += __fdiv_rn(cn, 1.0e4f);  // the weights as in k_sweep_weighted
-            nseg += 1.0f;
-            if (csum != 0.0f) emit_w<PASS, false>(S, v, ecol, __fdividef(nseg, csum), I, anchor_of<FB>(gv, word, v));
-            gl = gv;
-        });
-}
+// Weighted methods: the walks of k_sweep_weighted (K:1993-2135, RAW: K:2937-3085); anchors are
+// the entries (the marking pass is the plain method's).  The entry itself receives nothing, or
+// with RAW its own term.
+template <int GRAD, bool RAW, bool FB>
+struct WeightedFill : FillLine<GRAD> {
+    uint32_t ecol;
+    float csum, nseg;
+    template <bool MASK>
+    __device__ __forceinline__ bool quick(uint32_t, const float4 (&)[kWalkBatch], const int32_t (&)[kWalkBatch]) const
+    {
+        return true;
+    }
+    template <bool FLAGS>  // FLAGS: the curl may carry an anchor flag
+    __device__ __forceinline__ void step(uint32_t c, int q, const float4 &gv, bool t)
+    {
+        const float cn = t ? curl_of<FLAGS>(gv) : 0.0f;
+        csum += RAW ? cn : __fdiv_rn(cn, 1.0e4f);
+        this->integrate(c, q, gv, t);
+        nseg += t ? 1.0f : 0.0f;
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void batch(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                          const float4 (&g)[kWalkBatch], const int32_t (&id)[kWalkBatch])
+    {
+        if (!any_anchor<FB>(g, id)) {
+#pragma unroll
+            for (int q = 0; q < kWalkBatch; q++) step<false>(c, q, g[q], taken<MASK>(idle, q));
+            return;
+        }
+        uint32_t todo = anchor_steps<FB>(idle, g, id);
+        float Is[kWalkBatch], ws[kWalkBatch];
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) {
+            step<FB>(c, q, g[q], taken<MASK>(idle, q));
+            Is[q] = this->I;
+            ws[q] = __fdividef(nseg, csum);
+            if (!RAW) todo &= csum == 0.0f ? ~(1u << (2 * q)) : ~0u;
+        }
+        for (; todo; todo &= todo - 1u) {
+            const int q = (__ffs(todo) - 1) >> 1;
+            emit_w<kFill, false>(this->S, __ldg(this->S.id + pick(v, q)), ecol, pick(ws, q), pick(Is, q));
+        }
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void general(uint32_t, uint32_t, const uint32_t (&)[kWalkBatch],
+                                            const float4 (&)[kWalkBatch], const int32_t (&)[kWalkBatch])
+    {
+    }
+};
 
-// Weighted method with raw curl sums (the minimum-curl variant): the walk of
-// k_sweep_weighted_raw; anchors are the entries, the entry takes its own term.
-template <int PASS, bool FB>
+template <int GRAD, bool RAW, bool FB>
 __global__ void __launch_bounds__(kFillThreads, kFillBlocks)
-k_anchor_weighted_raw(Grid g, const LineRec *__restrict__ lines,
-                      const uint32_t *__restrict__ gbase,
-                      const uint32_t *__restrict__ desc, long long n_lines,
-                      const float4 *__restrict__ f32,
-                      const float *__restrict__ curl, Sink S)
+k_anchor_weighted(Grid g, Layout lay, WalkLines W, WalkField F, Sink S)
 {
-    static_assert(PASS == kFill, "the raw-curl weighted operator has only a filling pass");
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    Walk L;
-    L.init(g, r, gbase, desc, li);
-    const uint32_t e = r.e;
-    const uint32_t ecol = start_col<PASS>(S, e);
-    float4 gl = __ldg(f32 + e);
-    float csum = curl_of<FB>(gl), nseg = 1.0f;
-    emit_w<PASS, false>(S, e, ecol, __frcp_rn(csum), 0.0f, FB ? anchor_of<FB>(gl, 0u, e) : is_anchor(S.bits, e));
-    float I = 0.0f;
-    walk_steps<kWalkBatch, kGradF32, !FB>(
-        L.v, L.d0, L.d1, L.d2, L.m, L.dp, f32, nullptr, S.bits, [&](int a, uint32_t v, const float4 &gv, uint32_t word) {
-            float cn = curl_of<FB>(gv);
-            I += step_term(a, L, gv, gl);
-            csum += cn;
-            nseg += 1.0f;
-            emit_w<PASS, false>(S, v, ecol, __fdividef(nseg, csum), I, anchor_of<FB>(gv, word, v));
-            gl = gv;
-        });
+    LineWalk L;
+    if (!L.init(g, lay, W)) return;
+    const float4 *field = lane_field<GRAD>(F, lay, L);
+    S.id += L.copy;
+    WeightedFill<GRAD, RAW, FB> f{{L, S, sample<GRAD>(field, L.v)}, start_col<kFill>(S, L.v), 0.0f, 0.0f};
+    if (RAW) {
+        f.csum = curl_of<FB>(f.gl);
+        f.nseg = 1.0f;
+        if (L.on) emit_w<kFill, false>(S, __ldg(S.id + L.v), f.ecol, __frcp_rn(f.csum), 0.0f);
+    }
+    walk_steps<kWalkBatch, GRAD, !FB>(L, field, S.id, f);
 }
 
 // Selected method: the state machine of k_sweep_select (K:2280-2537); anchors are the
-// segment starts.
-template <int PASS, bool FB>
-__global__ void __launch_bounds__(kFillThreads, kFillBlocks)
-k_anchor_select(Grid g, const LineRec *__restrict__ lines,
-                const uint32_t *__restrict__ gbase,
-                const uint32_t *__restrict__ desc, long long n_lines,
-                const float4 *__restrict__ f32,
-                const float *__restrict__ curl, Sink S)
-{
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    Walk L;
-    L.init(g, r, gbase, desc, li);
-    const float thr = g.thr;
-    float4 gl = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (PASS == kFill) gl = __ldg(f32 + L.v);
-    // the field carries curl (.w of its entries): one gather per step in the filling pass
-    constexpr bool kW = PASS == kFill;
-    float ce = kW ? curl_of<FB>(gl) : __ldg(curl + L.v);
-    bool started = !(ce == 0.0f || ce > thr);
-    bool paused = false;
-    uint32_t start = L.v;
-    if (PASS == kMark && started) S.flag[start] = 1;
-    uint32_t scol = started ? start_col<PASS>(S, start) : 0u;
-    float I = 0.0f, csum = 0.0f, nseg = 0.0f;
-    // the filling pass gathers the field (and without FB the anchor bitmap word) of every
-    // voxel in batches
-    constexpr int kGrad = PASS == kFill ? kGradF32 : kNoGrad;
-    walk_steps<kWalkBatch, kGrad, PASS == kFill && !FB>(
-        L.v, L.d0, L.d1, L.d2, L.m, L.dp, f32, nullptr, S.bits, [&](int a, uint32_t v, const float4 &gv, uint32_t word) {
-            const float cn = kW ? curl_of<FB>(gv) : __ldg(curl + v);
-            if (!started) {
-                bool ok = (a == 0) ? (cn != 0.0f && cn < thr) : (cn != 0.0f);
-                if (ok) {
-                    start = v;
-                    if (PASS == kMark) S.flag[start] = 1;
-                    scol = start_col<PASS>(S, start);
-                    started = true;
-                    I = 0.0f; nseg = 0.0f; csum = 0.0f;
-                }
-            } else {
-                bool good = cn < thr && cn != 0.0f;
-                if (!paused && good) {
-                    if (PASS == kFill)
-                        I += step_term(a, L, gv, gl);
-                    csum += cn * 1.0e-4f;  // the weights as in k_sweep_select
-                    nseg += 1.0f;
-                    if (PASS == kFill)
-                        emit_w<PASS, false>(S, v, scol, __fdividef(nseg, csum), I, anchor_of<FB>(gv, word, v));
-                }
-                bool enter_bad = (a == 0) ? ((!paused && cn >= thr) || cn == 0.0f) : (!paused && cn >= thr);
-                if (enter_bad) paused = true;
-                if (paused && good) {
-                    start = v;
-                    if (PASS == kMark) S.flag[start] = 1;
-                    scol = start_col<PASS>(S, start);
-                    I = 0.0f;
-                    paused = false;
-                    if (a != 2) { nseg = 0.0f; csum = 0.0f; }
-                }
+// segment starts.  The marking pass reads the curl alone, row-major.
+template <int GRAD, int PASS, bool FB>
+struct SelectFill : FillLine<GRAD> {
+    const float *curl;
+    float thr;
+    SelectState st;
+    uint32_t scol;
+    float csum = 0.0f, nseg = 0.0f;
+
+    // every step adds to a running segment
+    template <bool MASK>
+    __device__ __forceinline__ bool quick(uint32_t idle, const float4 (&g)[kWalkBatch], const int32_t (&)[kWalkBatch]) const
+    {
+        if (PASS == kMark) return false;
+        if (!MASK && FB) {
+            float lo, hi;
+            curl_range<true>(g, lo, hi);
+            return st.run & (lo > 0.0f) & (hi < thr);
+        }
+        bool ok = st.run;
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) {
+            const float cn = curl_of<FB>(g[q]);
+            ok = ok & (((cn < thr) & (cn != 0.0f)) | !taken<MASK>(idle, q));
+        }
+        return ok | (MASK & (idle == kAllIdle));
+    }
+    template <bool FLAGS>  // FLAGS: the curl may carry an anchor flag
+    __device__ __forceinline__ void step(uint32_t c, int q, const float4 &gv, bool t)
+    {
+        csum += (t ? curl_of<FLAGS>(gv) : 0.0f) * 1.0e-4f;  // the weights as in k_sweep_select
+        this->integrate(c, q, gv, t);
+        nseg += t ? 1.0f : 0.0f;
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void batch(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                          const float4 (&g)[kWalkBatch], const int32_t (&id)[kWalkBatch])
+    {
+        if (!any_anchor<FB>(g, id)) {
+#pragma unroll
+            for (int q = 0; q < kWalkBatch; q++) step<false>(c, q, g[q], taken<MASK>(idle, q));
+            return;
+        }
+        float Is[kWalkBatch], ws[kWalkBatch];
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) {
+            step<FB>(c, q, g[q], taken<MASK>(idle, q));
+            Is[q] = this->I;
+            ws[q] = __fdividef(nseg, csum);
+        }
+        for (uint32_t todo = anchor_steps<FB>(idle, g, id); todo; todo &= todo - 1u) {
+            const int q = (__ffs(todo) - 1) >> 1;
+            emit_w<PASS, false>(this->S, __ldg(this->S.id + pick(v, q)), scol, pick(ws, q), pick(Is, q));
+        }
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void general(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                            const float4 (&g)[kWalkBatch], const int32_t (&id)[kWalkBatch])
+    {
+        if (PASS == kMark) {
+            float cn[kWalkBatch];
+#pragma unroll
+            for (int q = 0; q < kWalkBatch; q++) cn[q] = __ldg(curl + v[q]);
+#pragma unroll
+            for (int q = 0; q < kWalkBatch; q++) {
+                bool add, start, clear;
+                st.step(is_x(c, q), is_y(c, q), taken<MASK>(idle, q), cn[q], thr, add, start, clear);
+                if (start) this->S.flag[v[q]] = 1;
             }
-            gl = gv;
-        });
+            return;
+        }
+        // the ids of the voxels that are anchors or may start a segment, loaded together
+        int32_t rows[kWalkBatch];
+        bool open = !st.run;
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) {
+            rows[q] = -1;
+            if (open | anchor_of<FB>(g[q], id[q])) rows[q] = __ldg(this->S.id + v[q]);
+            open = st.may_start_after(curl_of<FB>(g[q]), thr) | !taken<MASK>(idle, q);
+        }
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) {
+            bool add, start, clear;
+            st.step(is_x(c, q), is_y(c, q), taken<MASK>(idle, q), curl_of<FB>(g[q]), thr, add, start, clear);
+            if (add) {
+                step<FB>(c, q, g[q], true);
+                if (rows[q] >= 0) emit_w<PASS, false>(this->S, rows[q], scol, __fdividef(nseg, csum), this->I);
+            }
+            if (GRAD != kGradEdge) this->gl = g[q];
+            scol = start ? (uint32_t)rows[q] : scol;
+            this->I = start ? 0.0f : this->I;
+            nseg = clear ? 0.0f : nseg;
+            csum = clear ? 0.0f : csum;
+        }
+    }
+};
+
+template <int GRAD, int PASS, bool FB>
+__global__ void __launch_bounds__(kFillThreads, kFillBlocks)
+k_anchor_select(Grid g, Layout lay, WalkLines W, WalkField F, const float *__restrict__ curl, Sink S)
+{
+    LineWalk L;
+    if (!L.init(g, lay, W)) return;
+    const float4 *field = lane_field<GRAD>(F, lay, L);
+    const float4 gl = sample<GRAD>(field, L.v);
+    if (PASS == kFill) S.id += L.copy;
+    SelectState st;
+    st.enter(PASS == kFill ? curl_of<FB>(gl) : __ldg(curl + L.v), g.thr);
+    if (PASS == kMark && st.run && L.on) S.flag[L.v] = 1;
+    SelectFill<GRAD, PASS, FB> f{{L, S, gl}, curl, g.thr, st, st.run ? start_col<PASS>(S, L.v) : 0u};
+    walk_steps<kWalkBatch, GRAD, PASS == kFill && !FB>(L, field, S.id, f);
 }
 
 // Selected method: a voxel can start a segment only if it is on the boundary (a line entry)
@@ -369,20 +443,25 @@ __global__ void k_flag_to_u32(long long V, const uint8_t *flag, uint32_t *out)
         out[v] = flag[v];
 }
 
-// id[v] = position among anchors or -1; vox[id] = v; bits = one bit per voxel.
-__global__ void k_assign_ids(long long V, const uint8_t *flag, const uint32_t *pos, int32_t *id, uint32_t *vox,
-                             uint32_t *bits)
+// id[v] = position among anchors or -1; vox[id] = v; the walks' copies of id (set to -1
+// before) at the anchors.
+__global__ void k_assign_ids(Grid g, Layout lay, const uint8_t *flag, const uint32_t *pos, int32_t *id, uint32_t *vox,
+                             int32_t *wid)
 {
-    long long nthr = ((V + 31) / 32) * 32;
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nthr;
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < g.V;
          v += (long long)gridDim.x * blockDim.x) {
-        bool f = v < V && flag[v];
-        unsigned b = __ballot_sync(0xffffffffu, f);
-        if (v < V) {
-            id[v] = f ? (int32_t)pos[v] : -1;
-            if (f) vox[pos[v]] = (uint32_t)v;
+        if (!flag[v]) {
+            id[v] = -1;
+            continue;
         }
-        if ((threadIdx.x & 31) == 0) bits[v >> 5] = b;
+        const int32_t a = (int32_t)pos[v];
+        id[v] = a;
+        vox[a] = (uint32_t)v;
+        if (!lay.wrap) continue;
+        const VoxelAt q(g, v);
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            wid[(size_t)c * (size_t)lay.stride + layout_index(lay, g.X, g.Y, c, q.i, q.j, q.k)] = a;
     }
 }
 
@@ -614,10 +693,21 @@ __global__ void k_converged(const double *red2, double tol, int j, int *stop, do
     if (rel < tol) *stop = j + 1;
 }
 
-__global__ void k_scatter(long long n, const uint32_t *vox, const float *pa, float *vol)
+// The anchor values into the walks' copies of the pressure.
+__global__ void k_scatter(Grid g, Layout lay, long long n, const uint32_t *vox, const float *pa, float *vol)
 {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        vol[vox[i]] = pa[i];
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const uint32_t v = vox[i];
+        const float x = pa[i];
+        if (!lay.wrap) {
+            vol[v] = x;
+            continue;
+        }
+        const VoxelAt q(g, v);
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            vol[(size_t)c * (size_t)lay.stride + layout_index(lay, g.X, g.Y, c, q.i, q.j, q.k)] = x;
+    }
 }
 
 __global__ void k_gather(long long n, const uint32_t *vox, const float *vol, float *pa)
@@ -641,27 +731,28 @@ __global__ void k_clear_b(long long n, float2 *bc)
         bc[i].x = 0.0f;
 }
 
-// After the filling pass: each row's length from its next free slot, and (flags = 1) the
-// anchor flags cleared from the field entries.
-__global__ void k_fill_finish(long long n, const unsigned long long *__restrict__ rowptr,
-                              const unsigned long long *__restrict__ next, uint32_t *rowlen, int flags,
-                              const uint32_t *__restrict__ vox, float4 *f32)
+// After the filling pass: each row's length from its next free slot.
+__global__ void k_row_lengths(long long n, const unsigned long long *__restrict__ rowptr,
+                              const unsigned long long *__restrict__ next, uint32_t *rowlen)
 {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         rowlen[i] = (uint32_t)(next[i] - rowptr[i]);
-        if (flags) {
-            uint32_t *u = reinterpret_cast<uint32_t *>(&f32[vox[i]].w);
-            *u &= 0x7fffffffu;
-        }
-    }
 }
 
-// Set (set = 1) or clear the anchor flag, the sign bit of .w, in the field entries of the n
-// anchors.
-__global__ void k_field_flags(long long n, const uint32_t *__restrict__ vox, float4 *f32, int set)
+// Set (set = 1) or clear the anchor flag, the sign bit of the curl, in the n anchors' field
+// records that the walks read.
+__global__ void k_field_flags(Grid g, Layout lay, long long n, const uint32_t *__restrict__ vox, float4 *field, int set)
 {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        uint32_t *u = reinterpret_cast<uint32_t *>(&f32[vox[i]].w);
+    const int per = lay.wrap ? 8 : 1;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n * per; i += (long long)gridDim.x * blockDim.x) {
+        const uint32_t v = vox[i / per];
+        size_t at = v;
+        if (lay.wrap) {
+            const int oct = (int)(i % per);
+            const VoxelAt q(g, v);
+            at = (size_t)oct * (size_t)lay.stride + layout_index(lay, g.X, g.Y, oct >> 1, q.i, q.j, q.k);
+        }
+        uint32_t *u = reinterpret_cast<uint32_t *>(&field[at].w);
         *u = set ? (*u | 0x80000000u) : (*u & 0x7fffffffu);
     }
 }
@@ -676,44 +767,38 @@ __global__ void k_sign_any(long long V, const float *__restrict__ curl, uint32_t
 }
 
 // Launch the pass for the method's accumulation kind.  FB: the anchors are flagged in the
-// field (bitmap otherwise).
-template <int PASS, bool FB>
+// field.
+template <int GRAD, int PASS, bool FB>
 void launch_pass(int acc, const Geometry &geo, const Field &f, const Sink &S, cudaStream_t st)
 {
-    const unsigned blocks = (unsigned)((geo.n_lines + kFillThreads - 1) / kFillThreads);
+    const unsigned blocks = group_blocks(geo, kFillThreads);
     const Grid &g = geo.grid;
+    const Layout lay = PASS == kMark ? row_major_layout(g) : f.lay;
+    const WalkLines W{geo.d_groups, geo.n_groups, geo.d_lines, geo.d_desc};
+    const WalkField F{f.f32, f.edge};
+    OM_COUNT_LAUNCH();
     if constexpr (PASS == kFill) {
         if (acc == kAccWeightedRawCurl) {
-            k_anchor_weighted_raw<kFill, FB><<<blocks, kFillThreads, 0, st>>>(g, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                                     geo.n_lines, f.f32, f.curl, S);
-            OM_COUNT_LAUNCH();
+            k_anchor_weighted<GRAD, true, FB><<<blocks, kFillThreads, 0, st>>>(g, lay, W, F, S);
             return;
         }
         if (acc == kAccWeighted) {
-            k_anchor_weighted<kFill, FB><<<blocks, kFillThreads, 0, st>>>(g, geo.d_lines, geo.d_gbase, geo.d_desc, geo.n_lines,
-                                                                 f.f32, f.curl, S);
-            OM_COUNT_LAUNCH();
+            k_anchor_weighted<GRAD, false, FB><<<blocks, kFillThreads, 0, st>>>(g, lay, W, F, S);
             return;
         }
         if (acc == kAccPlainNoEntry) {
-            k_anchor_plain<kFill, false, FB><<<blocks, kFillThreads, 0, st>>>(g, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                                     geo.n_lines, f.f32, S);
-            OM_COUNT_LAUNCH();
+            k_anchor_plain<GRAD, kFill, false, FB><<<blocks, kFillThreads, 0, st>>>(g, lay, W, F, S);
             return;
         }
     }
     if constexpr (PASS != kRhs) {
         if (acc == kAccSelect) {
-            k_anchor_select<PASS, FB><<<blocks, kFillThreads, 0, st>>>(g, geo.d_lines, geo.d_gbase, geo.d_desc, geo.n_lines,
-                                                              f.f32, f.curl, S);
-            OM_COUNT_LAUNCH();
+            k_anchor_select<GRAD, PASS, FB><<<blocks, kFillThreads, 0, st>>>(g, lay, W, F, f.curl, S);
             return;
         }
     }
     // plain method, and the marking pass of every method whose anchors are the entries
-    k_anchor_plain<PASS, true, FB><<<blocks, kFillThreads, 0, st>>>(g, geo.d_lines, geo.d_gbase, geo.d_desc, geo.n_lines,
-                                                           f.f32, S);
-    OM_COUNT_LAUNCH();
+    k_anchor_plain<GRAD, PASS, true, FB><<<blocks, kFillThreads, 0, st>>>(g, lay, W, F, S);
 }
 
 // fb: the anchors' field entries carry the anchor flag (k_field_flags): possible when no
@@ -724,20 +809,21 @@ cudaError_t run_pass(const Geometry &geo, const Field &f, int method, bool fb, c
     if (geo.n_lines == 0) return cudaSuccess;
     // every pointer the pass dereferences must be set: refuse to launch otherwise
     const bool need_field = PASS == kFill || PASS == kRhs;
-    bool ok = geo.d_lines && geo.d_gbase && geo.d_desc;
+    bool ok = geo.d_lines && geo.d_groups && geo.d_desc;
     if (PASS == kMark) ok = ok && S.flag;
-    else ok = ok && S.bits && S.id && S.bc;
+    else ok = ok && S.id && S.bc;
     const bool unit_links = method_accum(method) == kAccPlain || method_accum(method) == kAccPlainNoEntry;
     if (PASS == kFill) ok = ok && S.next && (unit_links ? S.col != nullptr : S.cw != nullptr);
-    if (need_field) ok = ok && f.f32 != nullptr;
+    if (need_field) ok = ok && (f.lay.wrap ? f.edge != nullptr : f.f32 != nullptr);
     const int acc = method_accum(method);
     const bool weighted = acc == kAccWeighted || acc == kAccWeightedRawCurl;
-    if (acc == kAccSelect || (weighted && PASS == kFill)) ok = ok && f.curl && f.f32;
+    if (acc == kAccSelect || (weighted && PASS == kFill)) ok = ok && f.curl;
     if (PASS == kRhs && acc != kAccPlain) ok = false;  // only the plain operator is cached
     if (!ok) return cudaErrorInvalidValue;
-    if (PASS == kMark) launch_pass<kMark, false>(acc, geo, f, S, st);  // reads no field
-    else if (fb) launch_pass<PASS, true>(acc, geo, f, S, st);
-    else launch_pass<PASS, false>(acc, geo, f, S, st);
+    if constexpr (PASS == kMark) launch_pass<kNoGrad, kMark, false>(acc, geo, f, S, st);  // reads no packed field
+    else if (f.lay.wrap) fb ? launch_pass<kGradEdge, PASS, true>(acc, geo, f, S, st)
+                            : launch_pass<kGradEdge, PASS, false>(acc, geo, f, S, st);
+    else fb ? launch_pass<kGradVoxel, PASS, true>(acc, geo, f, S, st) : launch_pass<kGradVoxel, PASS, false>(acc, geo, f, S, st);
     return cudaGetLastError();
 }
 
@@ -770,7 +856,7 @@ cudaError_t grow(T *&p, size_t &cap, size_t bytes)
 
 void anchor_free(Anchor *A)
 {
-    cudaFree(A->flag); cudaFree(A->bits); cudaFree(A->id); cudaFree(A->vox); cudaFree(A->rowptr);
+    cudaFree(A->flag); cudaFree(A->wid); cudaFree(A->id); cudaFree(A->vox); cudaFree(A->rowptr);
     cudaFree(A->col); cudaFree(A->cw); cudaFree(A->bc); cudaFree(A->pa); cudaFree(A->pb);
     cudaFree(A->red); cudaFree(A->rowlen); cudaFree(A->u); cudaFree(A->pos); cudaFree(A->tmp); cudaFree(A->cnt64); cudaFree(A->tmp64);
     cudaFree(A->neg); cudaFree(A->next);
@@ -778,12 +864,16 @@ void anchor_free(Anchor *A)
 }
 
 cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long ref_voxel,
-                         long long max_nnz, Anchor *A, cudaStream_t st, std::string *err, Fixed *fx)
+                         long long max_nnz, Anchor *A, cudaStream_t st, std::string *err, Fixed *fx, uint32_t *scratch)
 {
     const long long V = geo.grid.V;
     size_t *cap = A->cap;
     AN_TRY(grow(A->flag, cap[0], (size_t)V));
-    AN_TRY(grow(A->bits, cap[1], sizeof(uint32_t) * (size_t)((V + 31) / 32)));
+    const Layout &lay = f.lay;
+    if (lay.wrap) {
+        AN_TRY(grow(A->wid, cap[1], sizeof(int32_t) * (size_t)lay.copies * (size_t)V));
+        AN_TRY(cudaMemsetAsync(A->wid, 0xff, sizeof(int32_t) * (size_t)lay.copies * (size_t)V, st));
+    }
     AN_TRY(grow(A->id, cap[2], sizeof(int32_t) * (size_t)V));
     AN_TRY(grow(A->u, cap[3], sizeof(uint32_t) * (size_t)V));
     AN_TRY(grow(A->pos, cap[4], sizeof(uint32_t) * (size_t)(V + 1)));
@@ -832,13 +922,13 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     A->n = n;
     const bool fb = neg == 0u;
     AN_TRY(grow(A->vox, cap[7], sizeof(uint32_t) * (size_t)n));
-    k_assign_ids<<<grid_for(V), 256, 0, st>>>(V, A->flag, A->pos, A->id, A->vox, A->bits);
+    k_assign_ids<<<grid_for(V), 256, 0, st>>>(geo.grid, lay, A->flag, A->pos, A->id, A->vox, A->wid);
     OM_COUNT_LAUNCH();
     AN_TRY(cudaGetLastError());
 
     // rows: a voxel receives at most one contribution per line through it, so the
     // geometry-only line counts size the rows and no counting pass is needed
-    AN_TRY(ensure_lines_through(&geo, st));
+    AN_TRY(ensure_lines_through(&geo, f.lay, scratch, st));
     AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * (size_t)n));
     AN_TRY(grow(A->tmp64, cap[9], sizeof(unsigned long long) * scan_tmp_elems(n)));
     AN_TRY(grow(A->rowptr, cap[10], sizeof(unsigned long long) * (size_t)(n + 1)));
@@ -865,8 +955,7 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     AN_TRY(grow(A->next, cap[19], sizeof(unsigned long long) * (size_t)std::max<long long>(n, 1)));
     if (n) AN_TRY(cudaMemcpyAsync(A->next, A->rowptr, sizeof(unsigned long long) * (size_t)n, cudaMemcpyDeviceToDevice, st));
     AN_TRY(cudaMemsetAsync(A->bc, 0, sizeof(float2) * (size_t)std::max<long long>(n, 1), st));
-    S.bits = A->bits;
-    S.id = A->id;
+    S.id = lay.wrap ? A->wid : A->id;
     S.next = A->next;
     S.col = unit_links ? A->col : nullptr;
     S.cw = unit_links ? nullptr : A->cw;
@@ -878,15 +967,19 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
         S.fix = fx->scale;
     }
     if (fb && n) {
-        k_field_flags<<<grid_for(n), 256, 0, st>>>(n, A->vox, f.f32, 1);
+        k_field_flags<<<grid_for(n * 8), 256, 0, st>>>(geo.grid, f.lay, n, A->vox, f.lay.wrap ? f.edge : f.f32, 1);
         OM_COUNT_LAUNCH();
         AN_TRY(cudaGetLastError());
     }
     AN_TRY(run_pass<kFill>(geo, f, method, fb, S, st));
     if (fx) AN_TRY(fix_rows_to_float(n, *fx, A->bc, false, st));
-    if (n) {  // row lengths; the sweeps read the field unflagged
-        k_fill_finish<<<grid_for(n), 256, 0, st>>>(n, A->rowptr, A->next, A->rowlen, fb ? 1 : 0, A->vox, f.f32);
+    if (n) {
+        k_row_lengths<<<grid_for(n), 256, 0, st>>>(n, A->rowptr, A->next, A->rowlen);
         OM_COUNT_LAUNCH();
+        if (fb) {  // the sweeps read the field unflagged
+            k_field_flags<<<grid_for(n * 8), 256, 0, st>>>(geo.grid, f.lay, n, A->vox, f.lay.wrap ? f.edge : f.f32, 0);
+            OM_COUNT_LAUNCH();
+        }
         AN_TRY(cudaGetLastError());
     }
     A->unit_weights = method_accum(method) == kAccPlain || method_accum(method) == kAccPlainNoEntry;
@@ -989,8 +1082,7 @@ cudaError_t anchor_refresh_rhs(const Geometry &geo, const Field &f, Anchor *A, c
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     Sink S{};
-    S.bits = A->bits;
-    S.id = A->id;
+    S.id = f.lay.wrap ? A->wid : A->id;
     S.bc = A->bc;
     if (fx) {
         if ((e = cudaMemsetAsync(fx->bc64, 0, sizeof(long long) * 2 * (size_t)A->n, st)) != cudaSuccess) return e;
@@ -1000,21 +1092,22 @@ cudaError_t anchor_refresh_rhs(const Geometry &geo, const Field &f, Anchor *A, c
     // the plain method's field carries no curl (.w = +0), so the anchors can be flagged in it
     const bool fb = f.curl == nullptr;
     if (fb) {
-        k_field_flags<<<grid_for(A->n), 256, 0, st>>>(A->n, A->vox, f.f32, 1);
+        k_field_flags<<<grid_for(A->n * 8), 256, 0, st>>>(geo.grid, f.lay, A->n, A->vox, f.lay.wrap ? f.edge : f.f32, 1);
         OM_COUNT_LAUNCH();
     }
     e = run_pass<kRhs>(geo, f, OMNI3D_METHOD_PLAIN, fb, S, st);
     if (e == cudaSuccess && fx) e = fix_rows_to_float(A->n, *fx, A->bc, true, st);
     if (e != cudaSuccess || !fb) return e;
-    k_field_flags<<<grid_for(A->n), 256, 0, st>>>(A->n, A->vox, f.f32, 0);
+    k_field_flags<<<grid_for(A->n * 8), 256, 0, st>>>(geo.grid, f.lay, A->n, A->vox, f.lay.wrap ? f.edge : f.f32, 0);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
 
-cudaError_t anchor_scatter(const Anchor &A, const float *pa, float *vol, cudaStream_t st)
+cudaError_t anchor_scatter(const Grid &g, const Layout &lay, const Anchor &A, const float *pa, float *vol,
+                           cudaStream_t st)
 {
     if (A.n == 0) return cudaSuccess;
-    k_scatter<<<grid_for(A.n), 256, 0, st>>>(A.n, A.vox, pa, vol);
+    k_scatter<<<grid_for(A.n), 256, 0, st>>>(g, lay, A.n, A.vox, pa, vol);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }

@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "omni3d_internal.h"
+#include "walk.cuh"
 
 namespace omni3d {
 
@@ -124,25 +125,28 @@ __device__ __forceinline__ void fence_proxy_async()
 struct LineStart {
     int i, j, k;          // entry voxel coordinates
     int si, sj, sk;       // step signs
-    int m;
+    uint32_t e;           // entry voxel
+    long long li;
+    uint32_t span;        // steps of the group, idle ones included
     const uint32_t *dp;
 };
 
-__device__ __forceinline__ LineStart line_start(const Grid &g, const LineRec &r, const uint32_t *gbase,
-                                                const uint32_t *desc, long long li)
+// The line of this thread (its lane of a group); false when it has none.
+__device__ __forceinline__ bool line_start(const Grid &g, const WalkLines &W, LineStart &s)
 {
-    LineStart s;
-    s.i = (int)(r.e % (uint32_t)g.X);
-    s.j = (int)((r.e / (uint32_t)g.X) % (uint32_t)g.Y);
-    s.k = (int)(r.e / (uint32_t)g.XY);
-    int ix = (int)(r.x % (uint32_t)g.X), jx = (int)((r.x / (uint32_t)g.X) % (uint32_t)g.Y),
-        kx = (int)(r.x / (uint32_t)g.XY);
-    s.si = ix > s.i ? 1 : -1;
-    s.sj = jx > s.j ? 1 : -1;
-    s.sk = kx > s.k ? 1 : -1;
-    s.m = r.m;
-    s.dp = desc + 32ull * gbase[li >> 5] + (li & 31);
-    return s;
+    LineWalk L;
+    if (!L.init(g, Layout(), W) || !L.on) return false;
+    s.e = L.e;
+    s.i = (int)(L.e % (uint32_t)g.X);
+    s.j = (int)((L.e / (uint32_t)g.X) % (uint32_t)g.Y);
+    s.k = (int)(L.e / (uint32_t)g.XY);
+    s.si = L.d0 > 0 ? 1 : -1;
+    s.sj = L.d1 > 0 ? 1 : -1;
+    s.sk = L.d2 > 0 ? 1 : -1;
+    s.li = (long long)L.line;
+    s.span = L.span;
+    s.dp = L.dp;
+    return true;
 }
 
 // Does a step of sign s that ends at coordinate c cross a brick boundary?
@@ -159,23 +163,20 @@ __device__ __forceinline__ long long seg_key(int i, int j, int k, int nbx, int n
     return ((i >> 4) + (long long)(j >> 4) * nbx + (long long)(k >> 4) * nbx * nby) * kLenKeys + nv;
 }
 
-__global__ void __launch_bounds__(256) k_seg_count(Grid g, const LineRec *__restrict__ lines,
-                                                   const uint32_t *__restrict__ gbase,
-                                                   const uint32_t *__restrict__ desc, long long n_lines, int nbx,
+__global__ void __launch_bounds__(256) k_seg_count(Grid g, WalkLines W, int nbx,
                                                    int nby, uint32_t *key_count, uint32_t *line_nseg)
 {
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    LineStart L = line_start(g, r, gbase, desc, li);
+    LineStart L;
+    if (!line_start(g, W, L)) return;
+    const long long li = L.li;
     int i = L.i, j = L.j, k = L.k;
     uint32_t nseg = 1;
     int nv = 1;
-    for (int s0 = 0; s0 < L.m; s0 += 16) {
+    for (uint32_t s0 = 0; s0 < L.span; s0 += 16) {
         uint32_t w = __ldg(L.dp + 32 * (s0 >> 4));
-        int n = min(16, L.m - s0);
-        for (int t = 0; t < n; t++, w >>= 2) {
+        for (int t = 0; t < 16; t++, w >>= 2) {
             int a = (int)(w & 3u);
+            if (a == kIdle) continue;  // before the line enters or after it leaves
             bool cr;
             if (a == 0) { i += L.si; cr = crossed(i, L.si); }
             else if (a == 1) { j += L.sj; cr = crossed(j, L.sj); }
@@ -222,31 +223,28 @@ __device__ __forceinline__ void emit_segment(const SegOut &O, int fi, int fj, in
     O.rec[2ull * slot + 1] = rb;
 }
 
-__global__ void __launch_bounds__(256) k_seg_fill(Grid g, const LineRec *__restrict__ lines,
-                                                  const uint32_t *__restrict__ gbase,
-                                                  const uint32_t *__restrict__ desc, long long n_lines, SegOut O)
+__global__ void __launch_bounds__(256) k_seg_fill(Grid g, WalkLines W, SegOut O)
 {
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    LineStart L = line_start(g, r, gbase, desc, li);
+    LineStart L;
+    if (!line_start(g, W, L)) return;
+    const long long li = L.li;
     const int signs = (L.si > 0 ? 1 : 0) | (L.sj > 0 ? 2 : 0) | (L.sk > 0 ? 4 : 0);
     int i = L.i, j = L.j, k = L.k;
     int fi = i, fj = j, fk = k;  // first voxel of the open segment
     int nv = 1, ns = 0, first_entry = 1;
     uint32_t w3[3] = {0u, 0u, 0u};
     uint32_t id = O.line_seg[li];
-    for (int s0 = 0; s0 < L.m; s0 += 16) {
+    for (uint32_t s0 = 0; s0 < L.span; s0 += 16) {
         uint32_t w = __ldg(L.dp + 32 * (s0 >> 4));
-        int n = min(16, L.m - s0);
-        for (int t = 0; t < n; t++, w >>= 2) {
+        for (int t = 0; t < 16; t++, w >>= 2) {
             int a = (int)(w & 3u);
+            if (a == kIdle) continue;  // before the line enters or after it leaves
             bool cr;
             if (a == 0) { i += L.si; cr = crossed(i, L.si); }
             else if (a == 1) { j += L.sj; cr = crossed(j, L.sj); }
             else { k += L.sk; cr = crossed(k, L.sk); }
             if (cr) {
-                emit_segment(O, fi, fj, fk, nv, signs, first_entry, r.e, w3, id, (uint32_t)li);
+                emit_segment(O, fi, fj, fk, nv, signs, first_entry, L.e, w3, id, (uint32_t)li);
                 id++;
                 fi = i; fj = j; fk = k;
                 nv = 0; ns = 0; first_entry = 0;
@@ -260,7 +258,7 @@ __global__ void __launch_bounds__(256) k_seg_fill(Grid g, const LineRec *__restr
             nv++;
         }
     }
-    emit_segment(O, fi, fj, fk, nv, signs, first_entry, r.e, w3, id, (uint32_t)li);
+    emit_segment(O, fi, fj, fk, nv, signs, first_entry, L.e, w3, id, (uint32_t)li);
 }
 
 // ------------------------------------------------------------------ segment decoding
@@ -787,9 +785,10 @@ cudaError_t build_bricks(const Geometry &geo, Bricks *B, cudaStream_t st, std::s
         cleanup();
         return fail(e, "brick segment counts");
     }
-    const unsigned lblocks = (unsigned)((nl + 255) / 256);
+    const unsigned lblocks = group_blocks(geo, 256);
+    const WalkLines W{geo.d_groups, geo.n_groups, geo.d_lines, geo.d_desc};
     cudaMemsetAsync(kcount, 0, sizeof(uint32_t) * (size_t)nkeys, st);
-    k_seg_count<<<lblocks, 256, 0, st>>>(g, geo.d_lines, geo.d_gbase, geo.d_desc, nl, B->nbx, B->nby, kcount, lnseg);
+    k_seg_count<<<lblocks, 256, 0, st>>>(g, W, B->nbx, B->nby, kcount, lnseg);
     OM_COUNT_LAUNCH();
     if ((e = cudaGetLastError()) != cudaSuccess) { cleanup(); return fail(e, "k_seg_count"); }
     if ((e = exclusive_scan_u32(lnseg, B->line_seg, nl, tmp, st)) != cudaSuccess) {
@@ -839,7 +838,7 @@ cudaError_t build_bricks(const Geometry &geo, Bricks *B, cudaStream_t st, std::s
     O.nbx = B->nbx;
     O.nby = B->nby;
     cudaMemsetAsync(kcount, 0, sizeof(uint32_t) * (size_t)nkeys, st);
-    k_seg_fill<<<lblocks, 256, 0, st>>>(g, geo.d_lines, geo.d_gbase, geo.d_desc, nl, O);
+    k_seg_fill<<<lblocks, 256, 0, st>>>(g, W, O);
     OM_COUNT_LAUNCH();
     if ((e = cudaGetLastError()) != cudaSuccess) { cleanup(); return fail(e, "k_seg_fill"); }
     // work items: a brick, or a slice of a large brick, so that every SM has several

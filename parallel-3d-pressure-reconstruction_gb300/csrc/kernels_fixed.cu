@@ -2,7 +2,9 @@
 #include <cfloat>
 
 #include "fixed.cuh"
+#include "fold.cuh"
 #include "omni3d_internal.h"
+#include "walk.cuh"
 
 namespace omni3d {
 
@@ -132,26 +134,33 @@ __global__ void k_rows_to_float(long long n, const long long *__restrict__ bc64,
     }
 }
 
-__global__ void k_init_fix(long long V, const float *__restrict__ p_init, int seed, const double *__restrict__ scale,
-                           Fix2 *acc)
+// The seed of a sweep that accumulates on top of p_init: into the first copy.
+__global__ void k_seed_fix(Grid g, Layout lay, const float *__restrict__ p_init, const double *__restrict__ scale, Fix2 *acc)
 {
     const double sp = scale[kFixPn];
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x)
-        acc[v] = Fix2{seed && p_init ? (long long)fix_term(p_init[v], sp) : 0LL, 0LL};
-}
-
-__global__ void k_normalize_fix(long long V, const Fix2 *__restrict__ acc, const double *__restrict__ scale,
-                                const float *__restrict__ p_keep, float *p_out, float *cnt_out)
-{
-    const double sp = scale[kFixPn], sc = scale[kFixCnt];
+    const long long V = g.V;
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
-        const Fix2 a = acc[v];
-        const double c = (double)a.cnt / sc;
-        const float pk = p_keep ? p_keep[v] : 0.0f;
-        if (p_out) p_out[v] = c > 0.0 ? (float)(((double)a.pn / sp) / c) : pk;
-        if (cnt_out) cnt_out[v] = (float)c;
+        size_t at = (size_t)v;
+        if (lay.wrap) {
+            const VoxelAt q(g, v);
+            at = layout_index(lay, g.X, g.Y, 0, q.i, q.j, q.k);
+        }
+        acc[at].pn = (long long)fix_term(p_init[v], sp);
     }
 }
+
+struct NormalizeFix {
+    const double *scale;
+    const float *p_keep;
+    float *p_out, *cnt_out;
+    __device__ __forceinline__ void operator()(long long v, const Fix2 &a) const
+    {
+        const double c = (double)a.cnt / scale[kFixCnt];
+        const float pk = p_keep ? p_keep[v] : 0.0f;
+        if (p_out) p_out[v] = c > 0.0 ? (float)(((double)a.pn / scale[kFixPn]) / c) : pk;
+        if (cnt_out) cnt_out[v] = (float)c;
+    }
+};
 
 }  // namespace
 
@@ -198,17 +207,20 @@ cudaError_t fix_rows_to_float(long long n, const Fixed &fx, float2 *bc, bool kee
     return cudaGetLastError();
 }
 
-cudaError_t init_accum_fix(long long V, const float *p_init, bool seed, const Fixed &fx, Fix2 *acc, cudaStream_t st)
+cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, Fix2 *acc,
+                           cudaStream_t st)
 {
-    k_init_fix<<<grid_for(V), 256, 0, st>>>(V, p_init, seed ? 1 : 0, fx.scale, acc);
+    cudaError_t e = cudaMemsetAsync(acc, 0, sizeof(Fix2) * (size_t)lay.copies * (size_t)g.V, st);
+    if (e != cudaSuccess || !seed || !p_init) return e;
+    k_seed_fix<<<grid_for(g.V), 256, 0, st>>>(g, lay, p_init, fx.scale, acc);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
 
-cudaError_t normalize_fix(long long V, const Fix2 *acc, const Fixed &fx, const float *p_keep, float *p_out,
-                          float *cnt_out, cudaStream_t st)
+cudaError_t normalize_fix(const Grid &g, const Layout &lay, const Fix2 *acc, const Fixed &fx, const float *p_keep,
+                          float *p_out, float *cnt_out, cudaStream_t st)
 {
-    k_normalize_fix<<<grid_for(V), 256, 0, st>>>(V, acc, fx.scale, p_keep, p_out, cnt_out);
+    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, acc, NormalizeFix{fx.scale, p_keep, p_out, cnt_out});
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }

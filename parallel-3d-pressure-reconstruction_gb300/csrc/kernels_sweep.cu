@@ -3,80 +3,39 @@
 // (K:2280-2537), the normalisation
 // devidecountInner (K:6746-6759), the curl indicator (K:8352-8378) and the gauge.
 //
-// One thread walks one line by decoding its 2-bit staircase; a warp holds 32 neighbouring
-// lines of one direction, whose step words are interleaved so that every word load is one
-// coalesced 128-byte transaction.  The gradient and curl of each visited voxel are one
-// 16-byte (FP32) or 8-byte (BF16) gather; contributions go to an interleaved (pn, count) pair with
-// one vector reduction (red.global.add.v2.f32) per visited voxel.  The trapezoid prefix
-// integral along the line is a compensated (Kahan) FP32 sum.
+// One thread walks one line by decoding its 2-bit staircase; a warp holds a group (walk.cuh):
+// the lines of one direction through a lattice tile, all at the same level of the volume.  The
+// edge record of each visited voxel is one 16-byte gather; contributions go to an interleaved
+// (pn, count) pair with one vector reduction (red.global.add.v2.f32) per visited voxel.  The
+// trapezoid prefix integral along the line is a compensated (Kahan) FP32 sum.
+//
+// What bounds the full sweep (selected method, 160^3, 642 directions, ncu): the L1 data pipe, 82 %
+// busy -- eight cycles to write back a warp's 16-byte gather, four wavefronts for its lines, and
+// about eight for the reduction -- and, with 0.48 reduction sectors per visit, the L2's atomic
+// rate (the chip takes about 200 G sector operations per second whatever their width).  In the
+// row-major volume the same sweep had 0.76 sectors per visit and 14 wavefronts for gather and
+// reduction instead of 7.5; 256^3 / 642 directions: 73.6 -> 44.2 ms.  With the gathers taken out it would
+// take 32 ms, with the reductions taken out 34.
 #include <cuda_bf16.h>
 
 #include <algorithm>
 #include <type_traits>
 
 #include "fixed.cuh"
+#include "fold.cuh"
 #include "omni3d_internal.h"
 #include "walk.cuh"
 
 namespace omni3d {
 
-// Steps whose gathers a walk issues together (walk.cuh); the batched kernels run 4 CTAs of
-// 256 threads per SM (64 registers: the batch's gathers stay in registers).  CTAs of 128 or
-// 64 threads changed nothing (73.7 and 73.9 against 73.8 ms at 256^3 / 642 directions): the
-// full sweep is bound by its scattered reductions.
+// Steps whose gathers a walk issues together, and the launch shape: 32 warps per SM at 64
+// registers, in small CTAs that free their slots as soon as their own lines end.  256^3 / 642
+// directions: batches of 4 in 16 CTAs of 64 threads 44.7 ms, 4 CTAs of 256 46.2, 20 of 64 (48
+// registers) 51.9; batches of 2 45.3, of 8 49.1 or more (fewer warps, or spills).
 constexpr int kWalkBatch = 4;
-constexpr int kSweepThreads = 256, kSweepBlocks = 4;  // threads per CTA, CTAs per SM
+constexpr int kSweepThreads = 64, kSweepBlocks = 16;  // threads per CTA, CTAs per SM
 
 namespace {
-
-__device__ __forceinline__ float bf_lo(uint32_t u) { return __uint_as_float(u << 16); }
-__device__ __forceinline__ float bf_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
-
-// (ax, ay, az, curl) of voxel v from either storage.
-template <bool BF16>
-__device__ __forceinline__ float4 load_grad(const float4 *f32, const uint2 *b16, long long v)
-{
-    if (BF16) {
-        uint2 u = __ldg(b16 + v);
-        return make_float4(bf_lo(u.x), bf_hi(u.x), bf_lo(u.y), bf_hi(u.y));
-    } else {
-        return __ldg(f32 + v);
-    }
-}
-
-__device__ __forceinline__ float sel3(int a, float x, float y, float z)
-{
-    return a == 0 ? x : (a == 1 ? y : z);
-}
-
-// Per-line constants of the accumulation walk.
-struct LineWalk {
-    uint32_t v;           // current voxel
-    int d0, d1, d2;       // signed strides of a step along x, y, z
-    float h0, h1, h2;     // -rho * sign * spacing / 2 per axis (K:1816, 1825, 1834)
-    int m;
-    const uint32_t *dp;   // this lane's first step word
-
-    __device__ __forceinline__ void init(const Grid &g, const LineRec &r, const uint32_t *gbase,
-                                         const uint32_t *desc, long long li)
-    {
-        int ie = (int)(r.e % (uint32_t)g.X), je = (int)((r.e / (uint32_t)g.X) % (uint32_t)g.Y),
-            ke = (int)(r.e / (uint32_t)g.XY);
-        int ix = (int)(r.x % (uint32_t)g.X), jx = (int)((r.x / (uint32_t)g.X) % (uint32_t)g.Y),
-            kx = (int)(r.x / (uint32_t)g.XY);
-        int si = ix > ie ? 1 : -1, sj = jx > je ? 1 : -1, sk = kx > ke ? 1 : -1;
-        d0 = si;
-        d1 = sj * g.X;
-        d2 = sk * (int)g.XY;
-        // the reference forms -rho*s*dl in float and halves it in double (exact)
-        h0 = __fmul_rn(-g.rho * (float)si, g.dx) * 0.5f;
-        h1 = __fmul_rn(-g.rho * (float)sj, g.dy) * 0.5f;
-        h2 = __fmul_rn(-g.rho * (float)sk, g.dz) * 0.5f;
-        v = r.e;
-        m = r.m;
-        dp = desc + 32ull * gbase[li >> 5] + (li & 31);
-    }
-};
 
 // Contributions into the (pn, count) accumulators: one FP32 vector reduction, (the FP64
 // defect-correction sweep) two FP64 reductions, each a native L2 atomic, or (the
@@ -96,7 +55,7 @@ __device__ __forceinline__ FixScale load_fix(const double *fix)
 }
 __device__ __forceinline__ void acc_add(const FixScale &, float2 *a, float x, float y)
 {
-    atomicAdd(a, make_float2(x, y));
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(__cvta_generic_to_global(a)), "f"(x), "f"(y) : "memory");
 }
 __device__ __forceinline__ void acc_add(const FixScale &, double2 *a, float x, float y)
 {
@@ -117,115 +76,160 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float x)
     s = t;
 }
 
-// Plain method: every voxel of the line, the entry included, receives p[entry] + I(v).
-// SELF = false leaves the entry out (the minimum-curl plain variant, K:2797-2936).
-template <bool BF16, bool SELF, typename ACC>
-__global__ void __launch_bounds__(kSweepThreads, kSweepBlocks)
-k_sweep_plain(Grid g, const LineRec *__restrict__ lines,
-              const uint32_t *__restrict__ gbase,
-              const uint32_t *__restrict__ desc, long long n_lines,
-              const float4 *__restrict__ f32,
-              const uint2 *__restrict__ b16,
-              const float *__restrict__ p, ACC *pncnt,
-              const double *__restrict__ fix)
+// n / csum for a batch of the walk (f.quick has seen csum far from the subnormal range): the
+// reciprocal's and the product's rounding, as __fdividef's within 2 ulp, without its scaling.
+__device__ __forceinline__ float quick_div(float n, float csum)
 {
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    LineWalk L;
-    L.init(g, r, gbase, desc, li);
-    const FixScale fs = load_fix<ACC>(fix);
-    const float pe = __ldg(p + r.e);
-    if (SELF) acc_add(fs, pncnt + r.e, pe, 1.0f);
-    float4 gl = load_grad<BF16>(f32, b16, L.v);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(csum));
+    return n * r;
+}
+constexpr float kQuickMin = 1e-30f;  // least csum of a batch that uses quick_div
+constexpr float kQuickCurl = 1e-25f; // least curl of one that starts a sum
+constexpr uint32_t kAllIdle = 0x55555555u & ((1u << (2 * kWalkBatch)) - 1u);  // no step of the batch is the lane's
+
+// What every accumulation keeps along a line.
+template <int GRAD, typename ACC>
+struct LineSum {
+    const LineWalk &L;
+    ACC *acc;          // the lane's copy
+    const FixScale fs;
+    float4 gl;         // sample of the last voxel
     float I = 0.0f, comp = 0.0f;
-    walk_steps<kWalkBatch, BF16 ? kGradBF16 : kGradF32, false>(
-        L.v, L.d0, L.d1, L.d2, L.m, L.dp, f32, b16, nullptr, [&](int a, uint32_t v, const float4 &gv, uint32_t) {
-            float term = sel3(a, L.h0, L.h1, L.h2) * (sel3(a, gv.x, gv.y, gv.z) + sel3(a, gl.x, gl.y, gl.z));
-            kahan_add(I, comp, term);
-            acc_add(fs, pncnt + v, pe + I, 1.0f);
-            gl = gv;
-        });
-}
 
-// Weighted method (K:1993-2135): the entry receives nothing; step s of the line (s = 1..m)
-// adds w_s (p[entry] + I_s) and w_s, w_s = s / sum_{t<=s} curl_t/1e4, once that sum is
-// nonzero.  Each curl/1e4 term is the reference's correctly rounded float division, so the
-// "sum != 0" decision (all curls so far zero) is the reference's.
-template <bool BF16, typename ACC>
-__global__ void __launch_bounds__(kSweepThreads, kSweepBlocks)
-k_sweep_weighted(Grid g, const LineRec *__restrict__ lines,
-                 const uint32_t *__restrict__ gbase,
-                 const uint32_t *__restrict__ desc, long long n_lines,
-                 const float4 *__restrict__ f32,
-                 const uint2 *__restrict__ b16,
-                 const float *__restrict__ curl,
-                 const float *__restrict__ p, ACC *pncnt,
-                 const double *__restrict__ fix)
-{
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    LineWalk L;
-    L.init(g, r, gbase, desc, li);
-    const FixScale fs = load_fix<ACC>(fix);
-    const float pe = __ldg(p + r.e);
-    float4 gl = load_grad<BF16>(f32, b16, L.v);
-    float I = 0.0f, comp = 0.0f, csum = 0.0f, nseg = 0.0f;
-    walk_steps<kWalkBatch, BF16 ? kGradBF16 : kGradF32, false>(
-        L.v, L.d0, L.d1, L.d2, L.m, L.dp, f32, b16, nullptr, [&](int a, uint32_t v, const float4 &gv, uint32_t) {
-            float cn = gv.w;
-            float term = sel3(a, L.h0, L.h1, L.h2) * (sel3(a, gv.x, gv.y, gv.z) + sel3(a, gl.x, gl.y, gl.z));
-            kahan_add(I, comp, term);
-            csum += __fdiv_rn(cn, 1.0e4f);
-            nseg += 1.0f;
-            if (csum != 0.0f) {
-                float wc = __fdividef(nseg, csum);
-                acc_add(fs, pncnt + v, (pe + I) * wc, wc);
-            }
-            gl = gv;
-        });
-}
-
-// Weighted method with raw curl sums (the minimum-curl variant, K:2937-3085): the sum starts
-// at the entry's curl and the entry receives (p[entry], 1) / C; step s adds its curl (not
-// divided by 1e4) and contributes w (p[entry] + I), w = (s + 1) / C, with no test for a zero
-// sum: a zero sum gives infinities, as in the reference.
-template <bool BF16, typename ACC>
-__global__ void __launch_bounds__(kSweepThreads, kSweepBlocks)
-k_sweep_weighted_raw(Grid g, const LineRec *__restrict__ lines,
-                     const uint32_t *__restrict__ gbase,
-                     const uint32_t *__restrict__ desc, long long n_lines,
-                     const float4 *__restrict__ f32,
-                     const uint2 *__restrict__ b16,
-                     const float *__restrict__ curl,
-                     const float *__restrict__ p, ACC *pncnt,
-                     const double *__restrict__ fix)
-{
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    LineWalk L;
-    L.init(g, r, gbase, desc, li);
-    const FixScale fs = load_fix<ACC>(fix);
-    const float pe = __ldg(p + r.e);
-    float4 gl = load_grad<BF16>(f32, b16, L.v);
-    float csum = gl.w, nseg = 1.0f;
+    __device__ __forceinline__ void add(uint32_t v, float x, float y) const
     {
-        const float w0 = __frcp_rn(csum);
-        acc_add(fs, pncnt + L.v, pe * w0, w0);
+        acc_add(fs, acc + v, x, y);
     }
-    float I = 0.0f, comp = 0.0f;
-    walk_steps<kWalkBatch, BF16 ? kGradBF16 : kGradF32, false>(
-        L.v, L.d0, L.d1, L.d2, L.m, L.dp, f32, b16, nullptr, [&](int a, uint32_t v, const float4 &gv, uint32_t) {
-            float cn = gv.w;
-            kahan_add(I, comp, sel3(a, L.h0, L.h1, L.h2) * (sel3(a, gv.x, gv.y, gv.z) + sel3(a, gl.x, gl.y, gl.z)));
-            csum += cn;
-            nseg += 1.0f;
-            const float wc = __fdividef(nseg, csum);
-            acc_add(fs, pncnt + v, (pe + I) * wc, wc);
-            gl = gv;
-        });
+    // I += the trapezoid increment of step q of a batch, or 0 on a lane that does not take it
+    // (`t` false: the lane's line is not in the volume, so that its sums are still zero or not
+    // read again).  No branch: the lanes of a step mostly agree, and selections cost less.
+    __device__ __forceinline__ void integrate(uint32_t c, int q, const float4 &gv, bool t)
+    {
+        const float x = step_h(L, c, q) * step_sum<GRAD>(c, q, gv, gl);
+        kahan_add(I, comp, t ? x : 0.0f);
+        if (GRAD != kGradEdge) gl = gv;
+    }
+};
+
+// Plain method: every voxel of the line, the entry included, receives p[entry] + I(v).
+template <int GRAD, typename ACC>
+struct PlainWalk : LineSum<GRAD, ACC> {
+    float pe;
+    template <bool MASK>
+    __device__ __forceinline__ bool quick(uint32_t, const float4 (&)[kWalkBatch], const int32_t (&)[kWalkBatch]) const
+    {
+        return true;
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void batch(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                          const float4 (&g)[kWalkBatch], const int32_t (&)[kWalkBatch])
+    {
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++)
+        {
+            const bool t = taken<MASK>(idle, q);
+            this->integrate(c, q, g[q], t);
+            if (t) this->add(v[q], pe + this->I, 1.0f);
+        }
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void general(uint32_t, uint32_t, const uint32_t (&)[kWalkBatch],
+                                            const float4 (&)[kWalkBatch], const int32_t (&)[kWalkBatch])
+    {
+    }
+};
+
+// SELF = false leaves the entry out (the minimum-curl plain variant, K:2797-2936).
+template <int GRAD, bool SELF, typename ACC>
+__global__ void __launch_bounds__(kSweepThreads, kSweepBlocks)
+k_sweep_plain(Grid g, Layout lay, WalkLines W,
+              WalkField F, const float *__restrict__ p, ACC *pncnt, const double *__restrict__ fix)
+{
+    LineWalk L;
+    if (!L.init(g, lay, W)) return;
+    const float4 *field = lane_field<GRAD>(F, lay, L);
+    PlainWalk<GRAD, ACC> f{{L, pncnt + L.copy, load_fix<ACC>(fix), sample<GRAD>(field, L.v)}, __ldg(p + L.copy + L.v)};
+    if (SELF && L.on) f.add(L.v, f.pe, 1.0f);
+    walk_steps<kWalkBatch, GRAD, false>(L, field, nullptr, f);
+}
+
+// Weighted methods.  RAW = false (K:1993-2135): the entry receives nothing; step s of the line
+// (s = 1..m) adds w_s (p[entry] + I_s) and w_s, w_s = s / sum_{t<=s} curl_t/1e4, once that sum
+// is nonzero.  Each curl/1e4 term is the reference's correctly rounded float division, so the
+// "sum != 0" decision (all curls so far zero) is the reference's.
+// RAW = true (the minimum-curl variant, K:2937-3085): the sum starts at the entry's curl and the
+// entry receives (p[entry], 1) / C; step s adds its curl (not divided by 1e4) and contributes
+// w (p[entry] + I), w = (s + 1) / C, with no test for a zero sum: a zero sum gives infinities,
+// as in the reference.
+template <int GRAD, bool RAW, typename ACC>
+struct WeightedWalk : LineSum<GRAD, ACC> {
+    float pe;
+    float csum, nseg;
+    template <bool MASK>
+    __device__ __forceinline__ bool quick(uint32_t idle, const float4 (&g)[kWalkBatch], const int32_t (&)[kWalkBatch]) const
+    {
+        if (!MASK) {
+            float lo, hi;
+            curl_range<false>(g, lo, hi);
+            return (csum >= kQuickMin) & (lo >= 0.0f);
+        }
+        bool ok = csum >= kQuickMin;
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) ok = ok & ((g[q].w >= 0.0f) | !taken<MASK>(idle, q));
+        return ok | (MASK & (idle == kAllIdle));
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void batch(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                          const float4 (&g)[kWalkBatch], const int32_t (&)[kWalkBatch])
+    {
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++)
+        {
+            const bool t = taken<MASK>(idle, q);
+            const float cn = t ? g[q].w : 0.0f;
+            csum += RAW ? cn : __fdiv_rn(cn, 1.0e4f);
+            this->integrate(c, q, g[q], t);
+            nseg += t ? 1.0f : 0.0f;
+            const float w = quick_div(nseg, csum);
+            if (t) this->add(v[q], (pe + this->I) * w, w);
+        }
+    }
+    template <bool MASK>
+    __device__ __forceinline__ void general(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                            const float4 (&g)[kWalkBatch], const int32_t (&)[kWalkBatch])
+    {
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++)
+        {
+            const bool t = taken<MASK>(idle, q);
+            const float cn = t ? g[q].w : 0.0f;
+            csum += RAW ? cn : __fdiv_rn(cn, 1.0e4f);
+            this->integrate(c, q, g[q], t);
+            nseg += t ? 1.0f : 0.0f;
+            const float w = __fdividef(nseg, csum);
+            if (t & (RAW | (csum != 0.0f))) this->add(v[q], (pe + this->I) * w, w);
+        }
+    }
+};
+
+template <int GRAD, bool RAW, typename ACC>
+__global__ void __launch_bounds__(kSweepThreads, kSweepBlocks)
+k_sweep_weighted(Grid g, Layout lay, WalkLines W,
+                 WalkField F, const float *__restrict__ p, ACC *pncnt, const double *__restrict__ fix)
+{
+    LineWalk L;
+    if (!L.init(g, lay, W)) return;
+    const float4 *field = lane_field<GRAD>(F, lay, L);
+    WeightedWalk<GRAD, RAW, ACC> f{{L, pncnt + L.copy, load_fix<ACC>(fix), sample<GRAD>(field, L.v)},
+                                   __ldg(p + L.copy + L.v), 0.0f, 0.0f};
+    if (RAW) {
+        f.csum = f.gl.w;
+        f.nseg = 1.0f;
+        const float w0 = __frcp_rn(f.csum);
+        if (L.on) f.add(L.v, f.pe * w0, w0);
+    }
+    walk_steps<kWalkBatch, GRAD, false>(L, field, nullptr, f);
 }
 
 // Selected method (K:2280-2537), state machine and asymmetries included: the entry is a
@@ -234,94 +238,148 @@ k_sweep_weighted_raw(Grid g, const LineRec *__restrict__ lines,
 // also pauses on curl == 0, a y/z step walks through it without adding that step's
 // increment); a good voxel after a pause restarts the segment at that voxel; the z
 // branch keeps the running curl/count sums on restart.
-template <bool BF16, typename ACC>
-__global__ void __launch_bounds__(kSweepThreads, kSweepBlocks)
-k_sweep_select(Grid g, const LineRec *__restrict__ lines,
-               const uint32_t *__restrict__ gbase,
-               const uint32_t *__restrict__ desc, long long n_lines,
-               const float4 *__restrict__ f32,
-               const uint2 *__restrict__ b16,
-               const float *__restrict__ curl,
-               const float *__restrict__ p, ACC *pncnt,
-               const double *__restrict__ fix)
-{
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    LineWalk L;
-    L.init(g, r, gbase, desc, li);
-    const FixScale fs = load_fix<ACC>(fix);
-    const float thr = g.thr;
-    float4 gl = load_grad<BF16>(f32, b16, L.v);
-    float ce = gl.w;
-    bool started = !(ce == 0.0f || ce > thr);
-    bool paused = false;
-    float p0 = started ? __ldg(p + L.v) : 0.0f;
-    float I = 0.0f, comp = 0.0f, csum = 0.0f, nseg = 0.0f;
-    walk_steps<kWalkBatch, BF16 ? kGradBF16 : kGradF32, false>(
-        L.v, L.d0, L.d1, L.d2, L.m, L.dp, f32, b16, nullptr, [&](int a, uint32_t v, const float4 &gv, uint32_t) {
-            const float cn = gv.w;
-            if (!started) {
-                bool ok = (a == 0) ? (cn != 0.0f && cn < thr) : (cn != 0.0f);
-                if (ok) {
-                    p0 = __ldg(p + v);
-                    started = true;
-                    I = 0.0f; comp = 0.0f; nseg = 0.0f; csum = 0.0f;
-                }
-            } else {
-                bool good = cn < thr && cn != 0.0f;
-                if (!paused && good) {
-                    float term = sel3(a, L.h0, L.h1, L.h2) * (sel3(a, gv.x, gv.y, gv.z) + sel3(a, gl.x, gl.y, gl.z));
-                    kahan_add(I, comp, term);
-                    // weight n / sum(curl / 1e4) of the reference (K:2390-2392), as one fast
-                    // division (within 2 ulp) instead of its two correctly rounded ones: the
-                    // weights only scale averages, and the FP64-oracle bars hold (the 256^3
-                    // solve took 127.9 against 130.5 ms with a correctly rounded reciprocal)
-                    csum += cn * 1.0e-4f;
-                    nseg += 1.0f;
-                    float wc = __fdividef(nseg, csum);
-                    acc_add(fs, pncnt + v, (p0 + I) * wc, wc);
-                }
-                bool enter_bad = (a == 0) ? ((!paused && cn >= thr) || cn == 0.0f) : (!paused && cn >= thr);
-                if (enter_bad) paused = true;
-                if (paused && good) {
-                    p0 = __ldg(p + v);
-                    I = 0.0f; comp = 0.0f;
-                    paused = false;
-                    if (a != 2) { nseg = 0.0f; csum = 0.0f; }
-                }
-            }
-            gl = gv;
-        });
-}
+template <int GRAD, typename ACC>
+struct SelectWalk : LineSum<GRAD, ACC> {
+    const float *p;    // the lane's copy
+    float thr;
+    SelectState st;
+    float p0;
+    float csum = 0.0f, nseg = 0.0f;
 
-__global__ void k_normalize(long long V, const float2 *__restrict__ pncnt, const float *__restrict__ p_keep,
-                            float *p_out, float *cnt_out)
-{
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
-         v += (long long)gridDim.x * blockDim.x) {
-        float2 a = pncnt[v];
-        float pk = p_keep ? p_keep[v] : 0.0f;
-        if (p_out) p_out[v] = a.y > 0.0f ? __fdiv_rn(a.x, a.y) : pk;
-        if (cnt_out) cnt_out[v] = a.y;
+    // every step adds to a running segment
+    template <bool MASK>
+    __device__ __forceinline__ bool quick(uint32_t idle, const float4 (&g)[kWalkBatch], const int32_t (&)[kWalkBatch]) const
+    {
+        if (!MASK) {
+            float lo, hi;
+            curl_range<false>(g, lo, hi);
+            return st.run & (csum >= kQuickMin) & (lo > 0.0f) & (hi < thr);
+        }
+        bool ok = st.run & ((csum >= kQuickMin) | (nseg == 0.0f));
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++)
+            ok = ok & (((g[q].w >= kQuickCurl) & (g[q].w < thr)) | !taken<true>(idle, q));
+        return ok | (idle == kAllIdle);
     }
+    template <bool MASK>
+    __device__ __forceinline__ void batch(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                          const float4 (&g)[kWalkBatch], const int32_t (&)[kWalkBatch])
+    {
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++)
+        {
+            const bool t = taken<MASK>(idle, q);
+            csum += (t ? g[q].w : 0.0f) * 1.0e-4f;
+            this->integrate(c, q, g[q], t);
+            nseg += t ? 1.0f : 0.0f;
+            const float w = quick_div(nseg, csum);
+            if (t) this->add(v[q], (p0 + this->I) * w, w);
+        }
+    }
+    // The p values of the voxels that may start a segment are loaded together, before the sums
+    // that wait for them: a segment starts only after a voxel that is not good.
+    template <bool MASK>
+    __device__ __forceinline__ void general(uint32_t c, uint32_t idle, const uint32_t (&v)[kWalkBatch],
+                                            const float4 (&g)[kWalkBatch], const int32_t (&)[kWalkBatch])
+    {
+        float ps[kWalkBatch];
+        bool open = !st.run;
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) {
+            ps[q] = 0.0f;
+            if (open) ps[q] = __ldg(p + v[q]);
+            open = st.may_start_after(g[q].w, thr) | !taken<MASK>(idle, q);
+        }
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++) {
+            bool add, start, clear;
+            st.step(is_x(c, q), is_y(c, q), taken<MASK>(idle, q), g[q].w, thr, add, start, clear);
+            if (add) {
+                // weight n / sum(curl / 1e4) of the reference (K:2390-2392), as one fast
+                // division (within 2 ulp) instead of its two correctly rounded ones: the
+                // weights only scale averages, and the FP64-oracle bars hold
+                csum += g[q].w * 1.0e-4f;
+                nseg += 1.0f;
+                this->integrate(c, q, g[q], true);
+                const float w = __fdividef(nseg, csum);
+                this->add(v[q], (p0 + this->I) * w, w);
+            }
+            if (GRAD != kGradEdge) this->gl = g[q];
+            p0 = start ? ps[q] : p0;
+            this->I = start ? 0.0f : this->I;
+            this->comp = start ? 0.0f : this->comp;
+            nseg = clear ? 0.0f : nseg;
+            csum = clear ? 0.0f : csum;
+        }
+    }
+};
+
+template <int GRAD, typename ACC>
+__global__ void __launch_bounds__(kSweepThreads, kSweepBlocks)
+k_sweep_select(Grid g, Layout lay, WalkLines W,
+               WalkField F, const float *__restrict__ p, ACC *pncnt, const double *__restrict__ fix)
+{
+    LineWalk L;
+    if (!L.init(g, lay, W)) return;
+    const float4 *field = lane_field<GRAD>(F, lay, L);
+    p += L.copy;
+    const float4 gl = sample<GRAD>(field, L.v);
+    SelectState st;
+    st.enter(gl.w, g.thr);
+    SelectWalk<GRAD, ACC> f{{L, pncnt + L.copy, load_fix<ACC>(fix), gl}, p, g.thr, st,
+                            st.run ? __ldg(p + L.v) : 0.0f};
+    walk_steps<kWalkBatch, GRAD, false>(L, field, nullptr, f);
 }
 
-__global__ void k_accum_split(long long V, const float2 *__restrict__ acc, float *pn, float *cnt)
-{
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
-         v += (long long)gridDim.x * blockDim.x) {
-        float2 a = acc[v];
+// p = pn / count where count > 0, else the kept value; a pair of sums in FP32 or FP64.
+template <typename ACC>
+struct Normalize {
+    const float *p_keep;
+    float *p_out, *cnt_out;
+    __device__ __forceinline__ void operator()(long long v, const ACC &a) const
+    {
+        const float pk = p_keep ? p_keep[v] : 0.0f;
+        if (p_out) p_out[v] = a.y > 0 ? quotient(a) : pk;
+        if (cnt_out) cnt_out[v] = (float)a.y;
+    }
+    static __device__ __forceinline__ float quotient(const float2 &a) { return __fdiv_rn(a.x, a.y); }
+    static __device__ __forceinline__ float quotient(const double2 &a) { return (float)(a.x / a.y); }
+};
+
+struct AddTo {
+    float *pn, *cnt;
+    __device__ __forceinline__ void operator()(long long v, const float2 &a) const
+    {
         pn[v] += a.x;
         cnt[v] += a.y;
     }
+};
+
+// The seed of a sweep that accumulates on top of p_init: into the first copy.
+template <typename ACC>
+__global__ void k_seed_accum(Grid g, Layout lay, const float *__restrict__ p_init, ACC *pncnt)
+{
+    const long long V = g.V;
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
+         v += (long long)gridDim.x * blockDim.x) {
+        size_t at = (size_t)v;
+        if (lay.wrap) {
+            const VoxelAt q(g, v);
+            at = layout_index(lay, g.X, g.Y, 0, q.i, q.j, q.k);
+        }
+        pncnt[at].x = p_init[v];
+    }
 }
 
-__global__ void k_init_accum(long long V, const float *__restrict__ p_init, int seed, float2 *pncnt)
+// out = the copies of the row-major volume in.
+__global__ void __launch_bounds__(kTileThreads) k_spread(Grid g, Layout lay, const float *__restrict__ in, float *out)
 {
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
-         v += (long long)gridDim.x * blockDim.x)
-        pncnt[v] = make_float2(seed && p_init ? p_init[v] : 0.0f, 0.0f);
+    __shared__ float tile[kTile * kTile];
+    const TileAt at(g);
+    at.rows(g, [&](int p, long long v, int, int) { tile[p] = in[v]; });
+    __syncthreads();
+    for (int c = 0; c < 4; c++)
+        at.diagonals(g, lay, c, [&](int p, uint32_t q) { out[(size_t)c * (size_t)lay.stride + q] = tile[p]; });
 }
 
 __device__ __forceinline__ uint32_t to_bf16(float x)
@@ -353,31 +411,54 @@ __device__ __forceinline__ uint32_t curl_bf16(float c, const Grid &g)
     return v;
 }
 
-// The packed field: float4 (ax, ay, az, curl) and, for BF16 storage, the 8-byte record
-// {ax | ay << 16, az | curl << 16} of round-to-nearest-even BF16 values (the curl by
-// curl_bf16).  With BF16 storage the FP32 entry holds the stored values as floats, and
-// curl_out (which may be the curl array itself) the stored curl: every pass then sees the
-// same field, the full sweeps gathering the 8-byte records and the anchor operator's filling
-// pass, which is bound by instruction issue rather than by its gathers, the float4 entries
-// (nothing to unpack: 1.8 ms of its 50.9 ms at 256^3 / 642 directions).
-__global__ void k_pack(Grid g, const float *__restrict__ ax, const float *__restrict__ ay,
-                       const float *__restrict__ az, const float *curl, float4 *f32, uint2 *b16, float *curl_out)
+// The packed field, float4 (ax, ay, az, curl), row-major, and for skewed layouts the walks'
+// edge records: per step-sign octant a copy of float4 (ex, ey, ez, curl) in the octant's class,
+// e_a(v) the sum of component a at v and at the voxel from which a line of the octant steps
+// into v along a (the step's trapezoid increment without its coefficient; 0 where that voxel
+// lies outside).  A step then needs the one record of the voxel it enters.
+// With BF16 storage every component and the curl (curl_bf16) is rounded to BF16 first, and
+// curl_out (which may be the curl array itself) receives the rounded curl: every pass sees the
+// same field.
+// The records of a tile are put together in shared memory and written diagonal by diagonal
+// (fold.cuh): 256^3, 2.46 -> 0.50 ms against eight scattered records per voxel.
+__global__ void __launch_bounds__(kTileThreads) k_pack(Grid g, const float *__restrict__ ax, const float *__restrict__ ay,
+                       const float *__restrict__ az, const float *curl, float4 *f32, Layout lay, float4 *edge,
+                       float *curl_out, int round16)
 {
-    const long long V = g.V;
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
-         v += (long long)gridDim.x * blockDim.x) {
-        float x = ax[v], y = ay[v], z = az[v];
+    __shared__ float sxl[kTile * kTile], sxu[kTile * kTile], syl[kTile * kTile], syu[kTile * kTile], szl[kTile * kTile],
+        szu[kTile * kTile], sc[kTile * kTile];
+    // a component as stored
+    auto stored = [&](float x) { return round16 ? __uint_as_float(to_bf16(x) << 16) : x; };
+    const TileAt at(g);
+    at.rows(g, [&](int p, long long v, int i, int j) {
+        const float x = stored(ax[v]), y = stored(ay[v]), z = stored(az[v]);
         float c = curl ? curl[v] : 0.0f;
-        if (b16) {
-            const uint32_t bx = to_bf16(x), by = to_bf16(y), bz = to_bf16(z), cb = curl_bf16(c, g);
-            b16[v] = make_uint2(bx | (by << 16), bz | (cb << 16));
-            x = __uint_as_float(bx << 16);
-            y = __uint_as_float(by << 16);
-            z = __uint_as_float(bz << 16);
-            c = __uint_as_float(cb << 16);
+        if (round16) {
+            c = __uint_as_float(curl_bf16(c, g) << 16);
             if (curl_out) curl_out[v] = c;
         }
         f32[v] = make_float4(x, y, z, c);
+        if (!lay.wrap) return;
+        // the sums over each axis' two edges
+        sxl[p] = i > 0 ? x + stored(ax[v - 1]) : 0.0f;
+        sxu[p] = i < g.X - 1 ? x + stored(ax[v + 1]) : 0.0f;
+        syl[p] = j > 0 ? y + stored(ay[v - g.X]) : 0.0f;
+        syu[p] = j < g.Y - 1 ? y + stored(ay[v + g.X]) : 0.0f;
+        szl[p] = at.k > 0 ? z + stored(az[v - g.XY]) : 0.0f;
+        szu[p] = at.k < g.Z - 1 ? z + stored(az[v + g.XY]) : 0.0f;
+        sc[p] = c;
+    });
+    if (!lay.wrap) return;
+    __syncthreads();
+    for (int c = 0; c < 4; c++) {
+        // a step upward along an axis crosses the voxel's lower edge
+        const float *yd = (c & 1) ? syl : syu, *yu = (c & 1) ? syu : syl;
+        const float *zd = (c & 2) ? szl : szu, *zu = (c & 2) ? szu : szl;
+        at.diagonals(g, lay, c, [&](int p, uint32_t q) {
+            const float w = sc[p];
+            edge[(size_t)(2 * c) * (size_t)lay.stride + q] = make_float4(sxu[p], yd[p], zd[p], w);
+            edge[(size_t)(2 * c + 1) * (size_t)lay.stride + q] = make_float4(sxl[p], yu[p], zu[p], w);
+        });
     }
 }
 
@@ -515,147 +596,114 @@ unsigned grid_for(long long n, int threads = 256)
     return (unsigned)b;
 }
 
+// p and pncnt are the walks' copies (f.lay) of the pressure and of the accumulators.
 template <typename ACC>
-cudaError_t sweep_full_t(const Geometry &geo, const Field &f, int method, bool bf16, const float *p, ACC *pncnt,
+cudaError_t sweep_full_t(const Geometry &geo, const Field &f, int method, const float *p, ACC *pncnt,
                          cudaStream_t st, const double *fix = nullptr)
 {
     if (geo.n_lines == 0) return cudaSuccess;
     // every pointer the kernels dereference must be set: refuse to launch otherwise
-    if (!geo.d_lines || !geo.d_gbase || !geo.d_desc || !p || !pncnt || (bf16 ? !f.bf16 : !f.f32) ||
-        (method_uses_curl(method) && !f.curl))
-        return cudaErrorInvalidValue;
-    unsigned blocks = (unsigned)((geo.n_lines + kSweepThreads - 1) / kSweepThreads);
-    const int acc = method_accum(method);
-    if (acc == kAccWeighted) {
-        if (bf16)
-            k_sweep_weighted<true, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                           geo.n_lines, f.f32, f.bf16, f.curl, p, pncnt, fix);
-        else
-            k_sweep_weighted<false, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                            geo.n_lines, f.f32, f.bf16, f.curl, p, pncnt, fix);
+    const bool edge = f.lay.wrap != 0;
+    if (!geo.d_lines || !geo.d_groups || !geo.d_desc || !p || !pncnt || (edge ? !f.edge : !f.f32)) return cudaErrorInvalidValue;
+    const unsigned blocks = group_blocks(geo, kSweepThreads);
+    const WalkLines W{geo.d_groups, geo.n_groups, geo.d_lines, geo.d_desc};
+    const WalkField F{f.f32, f.edge};
+    auto launch = [&](auto e, auto v) {
+        auto kernel = edge ? e : v;
+        kernel<<<blocks, kSweepThreads, 0, st>>>(geo.grid, f.lay, W, F, p, pncnt, fix);
         OM_COUNT_LAUNCH();
-    } else if (acc == kAccWeightedRawCurl) {
-        if (bf16)
-            k_sweep_weighted_raw<true, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                               geo.n_lines, f.f32, f.bf16, f.curl, p, pncnt, fix);
-        else
-            k_sweep_weighted_raw<false, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                                geo.n_lines, f.f32, f.bf16, f.curl, p, pncnt, fix);
-        OM_COUNT_LAUNCH();
-    } else if (acc == kAccSelect) {
-        if (bf16)
-            k_sweep_select<true, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc, geo.n_lines,
-                                                         f.f32, f.bf16, f.curl, p, pncnt, fix);
-        else
-            k_sweep_select<false, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc, geo.n_lines,
-                                                          f.f32, f.bf16, f.curl, p, pncnt, fix);
-        OM_COUNT_LAUNCH();
-    } else if (acc == kAccPlainNoEntry) {
-        if (bf16)
-            k_sweep_plain<true, false, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                               geo.n_lines, f.f32, f.bf16, p, pncnt, fix);
-        else
-            k_sweep_plain<false, false, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                                geo.n_lines, f.f32, f.bf16, p, pncnt, fix);
-        OM_COUNT_LAUNCH();
-    } else {
-        if (bf16)
-            k_sweep_plain<true, true, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                              geo.n_lines, f.f32, f.bf16, p, pncnt, fix);
-        else
-            k_sweep_plain<false, true, ACC><<<blocks, kSweepThreads, 0, st>>>(geo.grid, geo.d_lines, geo.d_gbase, geo.d_desc,
-                                                               geo.n_lines, f.f32, f.bf16, p, pncnt, fix);
-        OM_COUNT_LAUNCH();
+    };
+    switch (method_accum(method)) {
+    case kAccWeighted: launch(k_sweep_weighted<kGradEdge, false, ACC>, k_sweep_weighted<kGradVoxel, false, ACC>); break;
+    case kAccWeightedRawCurl: launch(k_sweep_weighted<kGradEdge, true, ACC>, k_sweep_weighted<kGradVoxel, true, ACC>); break;
+    case kAccSelect: launch(k_sweep_select<kGradEdge, ACC>, k_sweep_select<kGradVoxel, ACC>); break;
+    case kAccPlainNoEntry: launch(k_sweep_plain<kGradEdge, false, ACC>, k_sweep_plain<kGradVoxel, false, ACC>); break;
+    default: launch(k_sweep_plain<kGradEdge, true, ACC>, k_sweep_plain<kGradVoxel, true, ACC>); break;
     }
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t sweep_full(const Geometry &geo, const Field &f, int method, bool bf16, const float *p, float2 *pncnt,
+cudaError_t sweep_full(const Geometry &geo, const Field &f, int method, const float *p, float2 *pncnt,
                        cudaStream_t st)
 {
-    return sweep_full_t(geo, f, method, bf16, p, pncnt, st);
+    return sweep_full_t(geo, f, method, p, pncnt, st);
 }
 
-cudaError_t sweep_full64(const Geometry &geo, const Field &f, int method, bool bf16, const float *p, double2 *pncnt,
+cudaError_t sweep_full64(const Geometry &geo, const Field &f, int method, const float *p, double2 *pncnt,
                          cudaStream_t st)
 {
-    return sweep_full_t(geo, f, method, bf16, p, pncnt, st);
+    return sweep_full_t(geo, f, method, p, pncnt, st);
 }
 
-cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, bool bf16, const float *p, Fix2 *pncnt,
+cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, Fix2 *pncnt,
                            const double *scale, cudaStream_t st)
 {
     if (!scale) return cudaErrorInvalidValue;
-    return sweep_full_t(geo, f, method, bf16, p, pncnt, st, scale);
+    return sweep_full_t(geo, f, method, p, pncnt, st, scale);
 }
 
 namespace {
 
-__global__ void k_init_accum64(long long V, const float *__restrict__ p_init, int seed, double2 *pncnt)
+template <typename ACC>
+cudaError_t init_accum_t(const Grid &g, const Layout &lay, const float *p_init, bool seed, ACC *pncnt, cudaStream_t st)
 {
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
-         v += (long long)gridDim.x * blockDim.x)
-        pncnt[v] = make_double2(seed && p_init ? (double)p_init[v] : 0.0, 0.0);
-}
-
-__global__ void k_normalize64(long long V, const double2 *__restrict__ pncnt, const float *__restrict__ p_keep,
-                              float *p_out, float *cnt_out)
-{
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V;
-         v += (long long)gridDim.x * blockDim.x) {
-        const double2 a = pncnt[v];
-        const float pk = p_keep ? p_keep[v] : 0.0f;
-        if (p_out) p_out[v] = a.y > 0.0 ? (float)(a.x / a.y) : pk;
-        if (cnt_out) cnt_out[v] = (float)a.y;
-    }
+    cudaError_t e = cudaMemsetAsync(pncnt, 0, sizeof(ACC) * (size_t)lay.copies * (size_t)g.V, st);
+    if (e != cudaSuccess || !seed || !p_init) return e;
+    k_seed_accum<ACC><<<grid_for(g.V), 256, 0, st>>>(g, lay, p_init, pncnt);
+    OM_COUNT_LAUNCH();
+    return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t init_accum64(long long V, const float *p_init, bool seed, double2 *pncnt, cudaStream_t st)
+cudaError_t init_accum64(const Grid &g, const Layout &lay, const float *p_init, bool seed, double2 *pncnt, cudaStream_t st)
 {
-    k_init_accum64<<<grid_for(V), 256, 0, st>>>(V, p_init, seed ? 1 : 0, pncnt);
+    return init_accum_t(g, lay, p_init, seed, pncnt, st);
+}
+
+cudaError_t normalize64(const Grid &g, const Layout &lay, const double2 *pncnt, const float *p_keep, float *p_out,
+                        float *cnt_out, cudaStream_t st)
+{
+    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, pncnt, Normalize<double2>{p_keep, p_out, cnt_out});
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
 
-cudaError_t normalize64(long long V, const double2 *pncnt, const float *p_keep, float *p_out, float *cnt_out,
-                        cudaStream_t st)
+cudaError_t normalize(const Grid &g, const Layout &lay, const float2 *pncnt, const float *p_keep, float *p_out,
+                      float *cnt_out, cudaStream_t st)
 {
-    k_normalize64<<<grid_for(V), 256, 0, st>>>(V, pncnt, p_keep, p_out, cnt_out);
+    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, pncnt, Normalize<float2>{p_keep, p_out, cnt_out});
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
 
-cudaError_t normalize(long long V, const float2 *pncnt, const float *p_keep, float *p_out, float *cnt_out,
-                      cudaStream_t st)
+cudaError_t accum_split(const Grid &g, const Layout &lay, const float2 *acc, float *pn, float *cnt, cudaStream_t st)
 {
-    k_normalize<<<grid_for(V), 256, 0, st>>>(V, pncnt, p_keep, p_out, cnt_out);
+    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, acc, AddTo{pn, cnt});
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
 
-cudaError_t accum_split(long long V, const float2 *acc, float *pn, float *cnt, cudaStream_t st)
+cudaError_t init_accum(const Grid &g, const Layout &lay, const float *p_init, bool seed, float2 *pncnt, cudaStream_t st)
 {
-    k_accum_split<<<grid_for(V), 256, 0, st>>>(V, acc, pn, cnt);
-    OM_COUNT_LAUNCH();
-    return cudaGetLastError();
+    return init_accum_t(g, lay, p_init, seed, pncnt, st);
 }
 
-cudaError_t init_accum(long long V, const float *p_init, bool seed, float2 *pncnt, cudaStream_t st)
+cudaError_t spread_volume(const Grid &g, const Layout &lay, const float *in, float *out, cudaStream_t st)
 {
-    k_init_accum<<<grid_for(V), 256, 0, st>>>(V, p_init, seed ? 1 : 0, pncnt);
+    if (!lay.wrap) return in == out ? cudaSuccess : cudaErrorInvalidValue;
+    k_spread<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, in, out);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
 
 cudaError_t pack_field(const Grid &g, const float *ax, const float *ay, const float *az, const float *curl,
-                       Field *f, bool make_bf16, cudaStream_t st, float *curl_rounded)
+                       Field *f, bool round_bf16, cudaStream_t st, float *curl_rounded)
 {
-    k_pack<<<grid_for(g.V), 256, 0, st>>>(g, ax, ay, az, curl, f->f32, make_bf16 ? f->bf16 : nullptr,
-                                          make_bf16 ? curl_rounded : nullptr);
+    if (!f->f32 || (f->lay.wrap && !f->edge)) return cudaErrorInvalidValue;
+    k_pack<<<tile_blocks(g), kTileThreads, 0, st>>>(g, ax, ay, az, curl, f->f32, f->lay, f->edge, curl_rounded, round_bf16 ? 1 : 0);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }

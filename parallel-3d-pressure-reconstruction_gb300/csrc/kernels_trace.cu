@@ -4,16 +4,20 @@
 // geometry instead of once per line per iteration.
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 #include <vector>
 
+#include "fold.cuh"
 #include "geometry.cuh"
 #include "omni3d_internal.h"
+#include "walk.cuh"
 
 namespace omni3d {
 
 namespace {
 
 constexpr int kTraceBlock = 256;
+constexpr int kWalkThreads = 64;  // a CTA leaves when its own two groups end
 constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 4;  // items per thread
 constexpr long long kScanTile = (long long)kScanBlock * kScanItems;
@@ -88,10 +92,11 @@ __device__ __forceinline__ bool trace_candidate(const Grid &g, const DirEntry *d
     return om_line_valid(g, in, out);
 }
 
-// Pass 1: number of valid lines per block of candidates.
+// The 32 candidates of a warp are one tile of one direction: its valid lines form one group.
+// Pass 1: lines (low word) and groups (high word) per block of candidates.
 __global__ void __launch_bounds__(kTraceBlock) k_trace_count(Grid g, const DirEntry *dirs,
                                                              long long ncand, CandOrder co,
-                                                             uint32_t *blk_cnt)
+                                                             unsigned long long *blk_cnt)
 {
     __shared__ uint32_t warp_cnt[kTraceBlock / 32];
     long long c = (long long)blockIdx.x * kTraceBlock + threadIdx.x;
@@ -105,17 +110,17 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_count(Grid g, const DirEn
     if ((threadIdx.x & 31) == 0) warp_cnt[threadIdx.x >> 5] = __popc(b);
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t s = 0;
-        for (int w = 0; w < kTraceBlock / 32; w++) s += warp_cnt[w];
+        unsigned long long s = 0;
+        for (int w = 0; w < kTraceBlock / 32; w++) s += warp_cnt[w] ? (1ull << 32) + warp_cnt[w] : 0ull;
         blk_cnt[blockIdx.x] = s;
     }
 }
 
-// Pass 2: write the valid lines of each block at its offset, in candidate order.
+// Pass 2: write the valid lines and the groups of each block at its offsets, in candidate order.
 __global__ void __launch_bounds__(kTraceBlock) k_trace_emit(Grid g, const DirEntry *dirs,
                                                             long long ncand, CandOrder co,
-                                                            const uint32_t *blk_off,
-                                                            LineRec *lines, float4 *off)
+                                                            const unsigned long long *blk_off,
+                                                            LineRec *lines, float4 *off, GroupRec *groups)
 {
     __shared__ uint32_t warp_cnt[kTraceBlock / 32];
     long long c = (long long)blockIdx.x * kTraceBlock + threadIdx.x;
@@ -128,9 +133,19 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_emit(Grid g, const DirEnt
     if (lane == 0) warp_cnt[warp] = __popc(b);
     __syncthreads();
     if (!valid) return;
-    uint32_t base = blk_off[blockIdx.x];
-    for (int w = 0; w < warp; w++) base += warp_cnt[w];
-    base += __popc(b & ((1u << lane) - 1u));
+    const unsigned long long at = blk_off[blockIdx.x];
+    uint32_t base = (uint32_t)at, grp = (uint32_t)(at >> 32);
+    for (int w = 0; w < warp; w++) {
+        base += warp_cnt[w];
+        grp += warp_cnt[w] ? 1u : 0u;
+    }
+    const uint32_t rank = __popc(b & ((1u << lane) - 1u));
+    if (rank == 0) {
+        const DirEntry D = dirs[d];
+        const uint32_t sg = (D.k1 >= 0.0f ? 1u : 0u) | (D.k2 >= 0.0f ? 2u : 0u) | (D.k3 >= 0.0f ? 4u : 0u);
+        groups[grp] = GroupRec{base, 0u, 0u, (uint32_t)__popc(b) | (sg << kGroupSigns)};
+    }
+    base += rank;
     LineRec r;
     r.e = (uint32_t)(in[0] + (long long)in[1] * g.X + (long long)in[2] * g.XY);
     r.x = (uint32_t)(out[0] + (long long)out[1] * g.X + (long long)out[2] * g.XY);
@@ -140,84 +155,125 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_emit(Grid g, const DirEnt
     off[base] = make_float4(o[0], o[1], o[2], 0.0f);
 }
 
-// Words per lane of every group of 32 lines: ceil(max steps / 16).
-__global__ void k_group_words(const LineRec *lines, long long n_lines, long long n_groups,
-                              uint32_t *gw)
+// A lane's line of a group: its end voxels, its staircase length and the idle steps before it
+// enters, which bring the group's lines to one level.  A line that moves against its
+// direction's signs (directions with k3 = 0 have some, see om_cross2point) starts at once.
+// Every lane of the warp calls it; the lanes beyond the group's lines repeat the last one, so
+// that the walks need no test for them but where they write.
+struct LaneLine {
+    int ie, je, ke, ix, jx, kx, m, lag;
+};
+__device__ __forceinline__ LaneLine lane_line(const Grid &g, const LineRec &r, int dir_signs)
 {
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if ((li >> 5) >= n_groups) return;  // whole warps only (blockDim is a multiple of 32)
-    int m = li < n_lines ? lines[li].m : 0;
-    int mx = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) gw[li >> 5] = (uint32_t)((mx + 15) >> 4);
+    LaneLine L;
+    L.ie = (int)(r.e % (uint32_t)g.X); L.je = (int)((r.e / (uint32_t)g.X) % (uint32_t)g.Y); L.ke = (int)(r.e / (uint32_t)g.XY);
+    L.ix = (int)(r.x % (uint32_t)g.X); L.jx = (int)((r.x / (uint32_t)g.X) % (uint32_t)g.Y); L.kx = (int)(r.x / (uint32_t)g.XY);
+    L.m = abs(L.ix - L.ie) + abs(L.jx - L.je) + abs(L.kx - L.ke);
+    const bool regular = line_signs(L.ie, L.je, L.ke, L.ix, L.jx, L.kx, dir_signs) == (dir_signs & 7);
+    const int level = ((dir_signs & 1) ? L.ie : -L.ie) + ((dir_signs & 2) ? L.je : -L.je) + ((dir_signs & 4) ? L.ke : -L.ke);
+    const int low = __reduce_min_sync(0xffffffffu, regular ? level : 0x7fffffff);
+    L.lag = regular ? level - low : 0;
+    return L;
 }
 
-// Walk every line once (K:1762-1861) and store its staircase, 2 bits per step.  RULE is
-// the walk rule of OmWalker::step; rule 3 reads `curl`.  The full path length
-// |di| + |dj| + |dk| bounds every walk (each step moves one axis toward the exit), so a
-// re-walk with another field fits the words reserved for the line.  counters[0] counts
-// walks that stopped early under rule 0 (the reference's "Wrong Point" error; under the
-// other rules stopping early is their design), counters[1] the voxel visits.
-template <int RULE>
-__global__ void __launch_bounds__(256) k_walk(Grid g, const DirEntry *dirs, LineRec *lines,
-                                              const float4 *off, const uint32_t *gbase,
-                                              uint32_t *desc, long long n_lines,
-                                              unsigned long long *counters, const float *curl)
+// Steps of every group, idle ones included, and its words per lane.
+__global__ void k_group_words(Grid g, const LineRec *lines, long long n_groups, GroupRec *groups, uint32_t *gw)
 {
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned mask = __ballot_sync(0xffffffffu, li < n_lines);
-    if (li >= n_lines) return;  // the tail of the last warp only
-    LineRec r = lines[li];
-    float4 o = off[li];
-    DirEntry D = dirs[r.dir];
-    int ie = (int)(r.e % g.X), je = (int)((r.e / g.X) % g.Y), ke = (int)(r.e / g.XY);
-    int ix = (int)(r.x % g.X), jx = (int)((r.x / g.X) % g.Y), kx = (int)(r.x / g.XY);
-    OmWalker w;
-    w.init(g, o.x, o.y, o.z, D.k1, D.k2, D.k3, ie, je, ke, ix, jx, kx);
-    uint32_t *dp = desc + 32ull * gbase[li >> 5] + (li & 31);
-    uint32_t word = 0;
-    int s = 0;
-    const int m = abs(ix - ie) + abs(jx - je) + abs(kx - ke);
-    for (; s < m; s++) {
-        int a = w.step<RULE>(curl, g.X, g.XY, g.V);
-        if (a < 0) break;
-        word |= (uint32_t)a << (2 * (s & 15));
-        if ((s & 15) == 15) { dp[32 * (s >> 4)] = word; word = 0; }
+    const long long gi = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (gi >= n_groups) return;  // whole warps
+    const int lane = threadIdx.x & 31;
+    const GroupRec G = groups[gi];
+    const uint32_t count = G.info & kGroupCount;
+    const LaneLine L = lane_line(g, lines[G.line0 + min((uint32_t)lane, count - 1u)], (int)(G.info >> kGroupSigns));
+    const int span = __reduce_max_sync(0xffffffffu, L.lag + L.m);
+    if (lane == 0) {
+        groups[gi].span = (uint32_t)span;
+        gw[gi] = (uint32_t)((span + 15) >> 4);
     }
-    if (s & 15) dp[32 * (s >> 4)] = word;
-    if (s != r.m) lines[li].m = s;  // the reference keeps the contributions of the steps taken
-    if (s != m && RULE == 0) atomicAdd(&counters[0], 1ull);
+}
+
+__global__ void k_group_offsets(long long n_groups, const uint32_t *off, GroupRec *groups)
+{
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_groups; i += (long long)gridDim.x * blockDim.x)
+        groups[i].word0 = off[i];
+}
+
+// Walk every line once (K:1762-1861) and store its staircase, 2 bits per step, between the
+// idle codes of its group.  RULE is the walk rule of OmWalker::step; rule 3 reads `curl`.  The
+// full path length |di| + |dj| + |dk| bounds every walk (each step moves one axis toward the
+// exit), so a re-walk with another field fits the words reserved for the line.  counters[0]
+// counts walks that stopped early under rule 0 (the reference's "Wrong Point" error; under the
+// other rules stopping early is their design), counters[1] the voxel visits.
+template <int RULE, bool FAST>
+__global__ void __launch_bounds__(kWalkThreads) k_walk(Grid g, const DirEntry *dirs, LineRec *lines,
+                                                       const float4 *off, const GroupRec *groups,
+                                                       uint32_t *desc, long long n_groups,
+                                                       unsigned long long *counters, const float *curl)
+{
+    const long long gi = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (gi >= n_groups) return;  // whole warps
+    const int lane = threadIdx.x & 31;
+    const GroupRec G = groups[gi];
+    const uint32_t count = G.info & kGroupCount;
+    const bool on = (uint32_t)lane < count;
+    const long long li = (long long)G.line0 + min((uint32_t)lane, count - 1u);
+    const LineRec r = lines[li];
+    const float4 o = off[li];
+    const DirEntry D = dirs[r.dir];
+    const LaneLine L = lane_line(g, r, (int)(G.info >> kGroupSigns));
+    std::conditional_t<FAST, OmFastWalker, OmWalker> w;
+    w.init(g, o.x, o.y, o.z, D.k1, D.k2, D.k3, L.ie, L.je, L.ke, L.ix, L.jx, L.kx);
+    uint32_t *dp = desc + 32ull * G.word0 + lane;
+    int s = 0;
+    const int first = L.lag;
+    int end = first + L.m;  // position after the last step
+    for (int t0 = 0; t0 < (int)G.span; t0 += 16) {
+        uint32_t word = 0xffffffffu;  // idle
+        const int n1 = min(16, end - t0);
+        for (int t = max(0, first - t0); t < n1; t++) {
+            int a;
+            if constexpr (FAST) a = w.template step<RULE>();
+            else a = w.template step<RULE>(curl, g.X, g.XY, g.V);
+            if (a < 0) {  // the reference's loop ends here and keeps the steps taken
+                end = 0;
+                break;
+            }
+            word ^= (uint32_t)(kIdle ^ a) << (2 * t);
+            s++;
+        }
+        dp[2 * t0] = word;
+    }
+    if (on && s != r.m) lines[li].m = s;
+    if (on && s != L.m && RULE == 0) atomicAdd(&counters[0], 1ull);
     // voxel-direction updates: entry + one per step
-    unsigned u = __reduce_add_sync(mask, (unsigned)(s + 1));
-    if ((threadIdx.x & 31) == (__ffs(mask) - 1)) atomicAdd(&counters[1], (unsigned long long)u);
+    const unsigned u = __reduce_add_sync(0xffffffffu, on ? (unsigned)(s + 1) : 0u);
+    if (lane == 0) atomicAdd(&counters[1], (unsigned long long)u);
 }
 
 // Number of lines through every voxel (entry included): a geometry-only bound on the
 // contributions any voxel can receive in one sweep.
-__global__ void __launch_bounds__(256) k_lines_through(Grid g, const LineRec *__restrict__ lines,
-                                                       const uint32_t *__restrict__ gbase,
-                                                       const uint32_t *__restrict__ desc, long long n_lines,
-                                                       uint32_t *cnt)
-{
-    long long li = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_lines) return;
-    LineRec r = lines[li];
-    int ie = (int)(r.e % (uint32_t)g.X), je = (int)((r.e / (uint32_t)g.X) % (uint32_t)g.Y),
-        ke = (int)(r.e / (uint32_t)g.XY);
-    int ix = (int)(r.x % (uint32_t)g.X), jx = (int)((r.x / (uint32_t)g.X) % (uint32_t)g.Y),
-        kx = (int)(r.x / (uint32_t)g.XY);
-    const int d0 = ix > ie ? 1 : -1, d1 = (jx > je ? 1 : -1) * g.X, d2 = (kx > ke ? 1 : -1) * (int)g.XY;
-    long long v = r.e;
-    atomicAdd(cnt + v, 1u);
-    const uint32_t *dp = desc + 32ull * gbase[li >> 5] + (li & 31);
-    for (int s0 = 0; s0 < r.m; s0 += 16) {
-        uint32_t w = __ldg(dp + 32 * (s0 >> 4));
-        int n = min(16, r.m - s0);
-        for (int t = 0; t < n; t++, w >>= 2) {
-            int a = (int)(w & 3u);
-            v += a == 0 ? d0 : (a == 1 ? d1 : d2);
-            atomicAdd(cnt + v, 1u);
-        }
+struct CountVisits {
+    uint32_t *cnt;
+    template <bool MASK>
+    __device__ __forceinline__ bool quick(uint32_t, const float4 (&)[4], const int32_t (&)[4]) const { return true; }
+    template <bool MASK>
+    __device__ __forceinline__ void batch(uint32_t, uint32_t idle, const uint32_t (&v)[4], const float4 (&)[4], const int32_t (&)[4]) const
+    {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (taken<MASK>(idle, q)) atomicAdd(cnt + v[q], 1u);
     }
+    template <bool MASK>
+    __device__ __forceinline__ void general(uint32_t, uint32_t, const uint32_t (&)[4], const float4 (&)[4], const int32_t (&)[4]) const {}
+};
+
+__global__ void __launch_bounds__(kWalkThreads) k_lines_through(Grid g, Layout lay, WalkLines W, uint32_t *cnt)
+{
+    LineWalk L;
+    if (!L.init(g, lay, W)) return;
+    CountVisits f{cnt + L.copy};
+    if (L.on) atomicAdd(f.cnt + L.v, 1u);
+    walk_steps<4, kNoGrad, false>(L, nullptr, nullptr, f);
 }
 
 // ---------------------------------------------------------------- scan
@@ -358,15 +414,31 @@ struct TmpBuf {
 };
 }  // namespace
 
-cudaError_t ensure_lines_through(Geometry *g, cudaStream_t st)
+namespace {
+struct StoreCount {
+    uint32_t *out;
+    __device__ __forceinline__ void operator()(long long v, uint32_t n) const { out[v] = n; }
+};
+}  // namespace
+
+cudaError_t ensure_lines_through(Geometry *g, const Layout &lay, uint32_t *scratch, cudaStream_t st)
 {
     if (g->d_lines_through) return cudaSuccess;
-    cudaError_t e = cudaMalloc(&g->d_lines_through, sizeof(uint32_t) * (size_t)std::max(g->grid.V, 1LL));
+    const long long V = g->grid.V;
+    cudaError_t e = cudaMalloc(&g->d_lines_through, sizeof(uint32_t) * (size_t)std::max(V, 1LL));
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(g->d_lines_through, 0, sizeof(uint32_t) * (size_t)g->grid.V, st);
-    if (e != cudaSuccess || g->n_lines == 0) return e;
-    k_lines_through<<<(unsigned)((g->n_lines + 255) / 256), 256, 0, st>>>(g->grid, g->d_lines, g->d_gbase, g->d_desc,
-                                                                          g->n_lines, g->d_lines_through);
+    // counted in the layout's copies: 256^3 / 642 directions, 47 ms row-major, 25.5 ms skewed
+    const bool fold = lay.wrap && scratch;
+    uint32_t *cnt = fold ? scratch : g->d_lines_through;
+    e = cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (size_t)(fold ? lay.copies : 1) * (size_t)V, st);
+    if (e != cudaSuccess || (g->n_lines == 0 && !fold)) return e;
+    if (g->n_lines) {
+        k_lines_through<<<group_blocks(*g, kWalkThreads), kWalkThreads, 0, st>>>(
+            g->grid, fold ? lay : row_major_layout(g->grid), WalkLines{g->d_groups, g->n_groups, g->d_lines, g->d_desc}, cnt);
+        OM_COUNT_LAUNCH();
+        if ((e = cudaGetLastError()) != cudaSuccess || !fold) return e;
+    }
+    k_fold<<<tile_blocks(g->grid), kTileThreads, 0, st>>>(g->grid, lay, (const uint32_t *)cnt, StoreCount{g->d_lines_through});
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
@@ -383,14 +455,14 @@ __global__ void k_max_u32(long long n, const uint32_t *__restrict__ x, unsigned 
 }
 }  // namespace
 
-cudaError_t max_lines_through(Geometry *g, cudaStream_t st, unsigned *out)
+cudaError_t max_lines_through(Geometry *g, const Layout &lay, uint32_t *scratch, cudaStream_t st, unsigned *out)
 {
     if (!g->d_lines_through) g->max_through = 0;
     if (g->max_through) {
         *out = g->max_through;
         return cudaSuccess;
     }
-    cudaError_t e = ensure_lines_through(g, st);
+    cudaError_t e = ensure_lines_through(g, lay, scratch, st);
     if (e != cudaSuccess) return e;
     TmpBuf tb;
     unsigned *d = nullptr;
@@ -418,11 +490,11 @@ void free_geometry(Geometry *g)
     g->d_counters = nullptr;
     cudaFree(g->d_off);
     cudaFree(g->d_lines);
-    cudaFree(g->d_gbase);
+    cudaFree(g->d_groups);
     cudaFree(g->d_desc);
     g->d_off = nullptr;
     g->d_lines = nullptr;
-    g->d_gbase = nullptr;
+    g->d_groups = nullptr;
     g->d_desc = nullptr;
     g->n_lines = g->n_groups = g->n_words = g->n_units = g->walk_errors = 0;
 }
@@ -450,43 +522,46 @@ cudaError_t build_geometry(Geometry *g, cudaStream_t st, std::string *err)
     }
     // temporaries of the build, freed on every exit
     TmpBuf tb_blk, tb_tmp, tb_gw, tb_gtmp;
-    uint32_t *blk = nullptr, *tmp = nullptr;
+    unsigned long long *blk = nullptr, *tmp = nullptr;
     OM_TRY(tb_blk.alloc(&blk, (size_t)(2 * nblk + 1)));
     OM_TRY(tb_tmp.alloc(&tmp, scan_tmp_elems(nblk)));
-    uint32_t *blk_off = blk + nblk;
+    unsigned long long *blk_off = blk + nblk;
     k_trace_count<<<(unsigned)nblk, kTraceBlock, 0, st>>>(G, g->d_dirs, ncand, co, blk);
     OM_COUNT_LAUNCH();
     OM_TRY(cudaGetLastError());
-    OM_TRY(exclusive_scan_u32(blk, blk_off, nblk, tmp, st));
-    uint32_t total = 0;
-    OM_TRY(cudaMemcpyAsync(&total, blk_off + nblk, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    OM_TRY(exclusive_scan_u64(blk, blk_off, nblk, tmp, st));
+    unsigned long long total = 0;
+    OM_TRY(cudaMemcpyAsync(&total, blk_off + nblk, sizeof(total), cudaMemcpyDeviceToHost, st));
     OM_TRY(cudaStreamSynchronize(st));
-    g->n_lines = total;
-    g->n_groups = (total + 31) / 32;
-    if (total == 0) {
+    g->n_lines = (long long)(total & 0xffffffffull);
+    g->n_groups = (long long)(total >> 32);
+    if (g->n_lines == 0) {
         g->n_words = 0;
         g->n_units = 0;
         return cudaSuccess;
     }
-    OM_TRY(cudaMalloc(&g->d_lines, sizeof(LineRec) * (size_t)total));
-    OM_TRY(cudaMalloc(&g->d_off, sizeof(float4) * (size_t)total));
+    OM_TRY(cudaMalloc(&g->d_lines, sizeof(LineRec) * (size_t)g->n_lines));
+    OM_TRY(cudaMalloc(&g->d_off, sizeof(float4) * (size_t)g->n_lines));
+    OM_TRY(cudaMalloc(&g->d_groups, sizeof(GroupRec) * (size_t)g->n_groups));
     k_trace_emit<<<(unsigned)nblk, kTraceBlock, 0, st>>>(G, g->d_dirs, ncand, co, blk_off, g->d_lines,
-                                                         g->d_off);
+                                                         g->d_off, g->d_groups);
     OM_COUNT_LAUNCH();
     OM_TRY(cudaGetLastError());
 
-    // words per group -> prefix offsets
+    // steps and words per group -> prefix offsets
     uint32_t *gw = nullptr, *gtmp = nullptr;
-    OM_TRY(tb_gw.alloc(&gw, (size_t)g->n_groups));
-    OM_TRY(cudaMalloc(&g->d_gbase, sizeof(uint32_t) * (size_t)(g->n_groups + 1)));
+    OM_TRY(tb_gw.alloc(&gw, (size_t)(2 * g->n_groups + 1)));
     OM_TRY(tb_gtmp.alloc(&gtmp, scan_tmp_elems(g->n_groups)));
-    long long nthr = g->n_groups * 32;
-    k_group_words<<<(unsigned)((nthr + 255) / 256), 256, 0, st>>>(g->d_lines, g->n_lines, g->n_groups, gw);
+    uint32_t *goff = gw + g->n_groups;
+    k_group_words<<<group_blocks(*g, 256), 256, 0, st>>>(G, g->d_lines, g->n_groups, g->d_groups, gw);
     OM_COUNT_LAUNCH();
     OM_TRY(cudaGetLastError());
-    OM_TRY(exclusive_scan_u32(gw, g->d_gbase, g->n_groups, gtmp, st));
+    OM_TRY(exclusive_scan_u32(gw, goff, g->n_groups, gtmp, st));
+    k_group_offsets<<<(unsigned)std::min<long long>((g->n_groups + 255) / 256, 152LL * 64), 256, 0, st>>>(g->n_groups, goff,
+                                                                                                         g->d_groups);
+    OM_COUNT_LAUNCH();
     uint32_t words_per_lane_total = 0;
-    OM_TRY(cudaMemcpyAsync(&words_per_lane_total, g->d_gbase + g->n_groups, sizeof(uint32_t),
+    OM_TRY(cudaMemcpyAsync(&words_per_lane_total, goff + g->n_groups, sizeof(uint32_t),
                            cudaMemcpyDeviceToHost, st));
     OM_TRY(cudaStreamSynchronize(st));
     g->n_words = 32LL * words_per_lane_total;
@@ -504,17 +579,17 @@ cudaError_t run_walk(Geometry *g, int rule, const float *curl, cudaStream_t st)
     if (!g->d_counters || !g->d_lines || !g->d_desc || (rule == 3 && !curl)) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(g->d_counters, 0, 2 * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    const unsigned blocks = (unsigned)((g->n_lines + 255) / 256);
     const Grid &G = g->grid;
+    const bool fast = std::max(std::max(G.X, G.Y), G.Z) < kFastWalkMax;
+    auto launch = [&](auto kernel) {
+        kernel<<<group_blocks(*g, kWalkThreads), kWalkThreads, 0, st>>>(G, g->d_dirs, g->d_lines, g->d_off, g->d_groups, g->d_desc,
+                                                                        g->n_groups, g->d_counters, curl);
+    };
     switch (rule) {
-    case 1: k_walk<1><<<blocks, 256, 0, st>>>(G, g->d_dirs, g->d_lines, g->d_off, g->d_gbase, g->d_desc, g->n_lines,
-                                              g->d_counters, curl); break;
-    case 2: k_walk<2><<<blocks, 256, 0, st>>>(G, g->d_dirs, g->d_lines, g->d_off, g->d_gbase, g->d_desc, g->n_lines,
-                                              g->d_counters, curl); break;
-    case 3: k_walk<3><<<blocks, 256, 0, st>>>(G, g->d_dirs, g->d_lines, g->d_off, g->d_gbase, g->d_desc, g->n_lines,
-                                              g->d_counters, curl); break;
-    default: k_walk<0><<<blocks, 256, 0, st>>>(G, g->d_dirs, g->d_lines, g->d_off, g->d_gbase, g->d_desc, g->n_lines,
-                                               g->d_counters, curl); break;
+    case 1: fast ? launch(k_walk<1, true>) : launch(k_walk<1, false>); break;
+    case 2: fast ? launch(k_walk<2, true>) : launch(k_walk<2, false>); break;
+    case 3: launch(k_walk<3, false>); break;
+    default: fast ? launch(k_walk<0, true>) : launch(k_walk<0, false>); break;
     }
     OM_COUNT_LAUNCH();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
