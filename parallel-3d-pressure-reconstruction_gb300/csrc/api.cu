@@ -458,7 +458,7 @@ cudaError_t enqueue_prepared(omni3d_ctx *ctx, const float *dax, const float *day
     const bool seed = P.seed_first_iteration != 0;
     float *pc = A.pa, *pn = A.pb;
     for (int it = 1; it <= K - 1; it++) {
-        if ((e = anchor_step(A, dpinit, seed && it == 1, P.gauge, -1, pc, pn, nullptr, st)) != cudaSuccess) return e;
+        if ((e = anchor_step(A, dpinit, seed && it == 1, it == 1, P.gauge, -1, pc, pn, nullptr, st)) != cudaSuccess) return e;
         std::swap(pc, pn);
     }
     float2 *acc = ctx->pncnt.as<float2>();
@@ -930,7 +930,7 @@ namespace {
 // Tolerance-driven anchor iterations in CUDA-graph chunks.  Checking the relative change on
 // the host after every step costs a stream synchronisation per iteration (about 70 us,
 // several times the step itself on small grids).  A chunk of kIterChunk steps is captured
-// once into a graph; each step is followed by a one-thread convergence test that sets a
+// once into a graph; the last block of each step tests the convergence and sets a
 // device stop word, and every later kernel of the chunk sees the word and returns.  The host
 // synchronises once per chunk and learns from the word which step met the tolerance, so the
 // iterate and the iteration count are those of the step-by-step loop.
@@ -960,8 +960,8 @@ cudaError_t iterate_chunk(omni3d_ctx *ctx, const Anchor &A, int gauge, long long
         for (int j = 0; j < kIterChunk && ce == cudaSuccess; j++) {
             const float *from = (j % 2 == 0) ? pc : pn;
             float *to = (j % 2 == 0) ? pn : pc;
-            ce = anchor_step(A, nullptr, false, gauge, ref_anchor, from, to, red2, st, stop, fx);
-            if (ce == cudaSuccess) ce = converged_test_launch(red2, tol, j, stop, rels, st);
+            const ChunkTest test{tol, j, stop, rels};
+            ce = anchor_step(A, nullptr, false, false, gauge, ref_anchor, from, to, red2, st, &test, fx);
         }
         cudaGraph_t graph = nullptr;
         e = cudaStreamEndCapture(st, &graph);
@@ -1194,7 +1194,7 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
                 it += kIterChunk;
                 continue;
             }
-            CK(ctx, anchor_step(A, dpinit, seed && it == 1, P.gauge, ref_anchor, pc, pn, P.tol > 0.0 ? red2 : nullptr, st,
+            CK(ctx, anchor_step(A, dpinit, seed && it == 1, it == 1, P.gauge, ref_anchor, pc, pn, P.tol > 0.0 ? red2 : nullptr, st,
                                 nullptr, fx));
             its = it;
             std::swap(pc, pn);

@@ -472,15 +472,21 @@ __global__ void k_row_capacity(long long n, const uint32_t *vox, const uint32_t 
         out[i] = lines_through[vox[i]];
 }
 
-// Row sums of the anchor iteration: compensated (Kahan) FP32 per lane, the 32 lane sums
-// and the numerator in FP64.  A row gathers about as many terms as lines cross its voxel
-// (~1000 at 642 directions); plain FP32 sums of that many terms leave a rounding floor near
-// 1e-6 in the iteration's relative change, above the tolerances the solver is asked for.
-__device__ __forceinline__ double warp_sum_compensated(float s, float comp)
+// Row sums of the anchor iteration: compensated (Kahan) FP32 per lane, the lane sums added as
+// unevaluated pairs (hi, lo) with error-free additions, about 46 bits, and the row's update in
+// FP64.  A row gathers about as many terms as lines cross its voxel (~1000 at 642 directions);
+// plain FP32 sums of that many terms leave a rounding floor near 1e-6 in the iteration's
+// relative change, above the tolerances the solver is asked for.
+__device__ __forceinline__ void warp_sum_pair(float &hi, float &lo)
 {
-    double d = (double)s - (double)comp;
-    for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-    return d;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const float h2 = __shfl_xor_sync(0xffffffffu, hi, o), l2 = __shfl_xor_sync(0xffffffffu, lo, o);
+        const float t = __fadd_rn(hi, h2), b = __fsub_rn(t, hi);
+        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(h2, b));  // hi + h2 = t + e exactly
+        lo = __fadd_rn(__fadd_rn(lo, l2), e);
+        hi = t;
+    }
 }
 
 // The warp's exact sum of fixed-point lane sums (integer additions: order-independent).
@@ -490,75 +496,178 @@ __device__ __forceinline__ long long warp_sum_fixed(long long t)
     return t;
 }
 
-__device__ __forceinline__ float anchor_update(double sum, long long row, const float2 *bc,
-                                               const uint32_t *vox, const float *p_init, int seed, const float *pc)
+__device__ __forceinline__ double warp_sum_double(double x)
 {
-    const float2 q = bc[row];
-    const float cc = q.y;
-    double numer = (double)q.x + sum;
-    if (seed && p_init) numer += (double)p_init[vox[row]];
-    return cc > 0.0f ? (float)(numer / (double)cc) : pc[row];
+    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
 }
 
-// One anchor iteration, a warp per row.
-__global__ void __launch_bounds__(256) k_anchor_spmv(long long n, const unsigned long long *__restrict__ rowptr,
-                                                     const uint32_t *__restrict__ rowlen,
-                                                     const uint2 *__restrict__ cw, const float2 *__restrict__ bc,
-                                                     const uint32_t *__restrict__ vox, const float *__restrict__ p_init,
-                                                     int seed, const float *__restrict__ pc, float *__restrict__ pn,
-                                                     const int *stop, const double *__restrict__ fix)
+// The convergence measure of an iteration (tolerance-driven solves): the gauged squared change
+// and norm over all anchors, sum (d - sd)^2 and sum (p - sp)^2 with d = pn - pc.  The shifts
+// (the reference entry's change and value, the means, or 0) are not known before every row is
+// done, so the sums are taken about the last iteration's shifts (`about`, 0 in the first) and
+// moved to this one's at the end, where little is left to cancel.
+struct ChangeOut {
+    double *red2;        // {change, norm} (null: no measure)
+    double *about;       // 2: the shifts of the last iteration
+    unsigned *arrived;   // blocks done (wraps to 0)
+    double *part;        // 4 per block
+    int gauge;
+    long long ref;
+    double tol;          // with stop: the chunk's test, see iterate_chunk
+    int step;
+    int *stop;
+    double *rel_out;
+};
+
+// Rows per warp: the FP64 work of a row -- its update, one division among it -- is done for a
+// warp's rows together, a lane each, since this GPU's FP64 units take 16 cycles per warp
+// instruction and SM: with a row per warp and FP64 lane sums they alone took 0.1 ms of the
+// 0.165 of an iteration at 128^3 / 642 directions (97 K rows).
+constexpr int kIterThreads = 256, kIterRowsMax = 16, kIterWarps = 152 * 48;
+inline int iter_rows(long long n) { return (int)std::max(1LL, std::min<long long>(kIterRowsMax, (n + kIterWarps - 1) / kIterWarps)); }
+inline unsigned iter_blocks(long long n)
+{
+    const long long per = (long long)iter_rows(n) * (kIterThreads / 32);
+    return (unsigned)((n + per - 1) / per);
+}
+
+// One anchor iteration, p_next = (b + seed p_init + M p_cur) / c; UNIT: every weight is 1 (plain
+// method), a row is a sum of gathered anchor values; FIX: the bit-reproducible mode's exact
+// fixed-point sums, whatever the entries' order.
+template <bool UNIT, bool FIX>
+__global__ void __launch_bounds__(kIterThreads) k_anchor_iterate(
+    long long n, int rows, const unsigned long long *__restrict__ rowptr, const uint32_t *__restrict__ rowlen,
+    const uint32_t *__restrict__ col, const uint2 *__restrict__ cw, const float2 *__restrict__ bc,
+    const uint32_t *__restrict__ vox, const float *__restrict__ p_init, int seed, const float *__restrict__ pc, float *pn,
+    const int *stop, const double *__restrict__ fix, ChangeOut C)
 {
     if (stop && *stop) return;  // a graph-captured chunk that has met its tolerance
-    long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (row >= n) return;  // whole warps
-    unsigned long long j0 = rowptr[row], j1 = j0 + rowlen[row];
-    double sum;
-    if (fix) {  // bit-reproducible: exact fixed-point sum, whatever the entries' order
-        const double sr = fix[kFixRow];
-        long long t = 0;
-        for (unsigned long long j = j0 + lane; j < j1; j += 32) {
-            const uint2 q = __ldg(cw + j);
-            t += (long long)fix_term(__uint_as_float(q.y) * __ldg(pc + q.x), sr);
-        }
-        sum = (double)warp_sum_fixed(t) / sr;
-    } else {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long row0 = ((long long)blockIdx.x * (kIterThreads / 32) + warp) * rows;
+    const long long mine = row0 + lane;  // the row this lane finishes
+    const bool has = lane < rows && mine < n;
+    const unsigned long long ptr = has ? rowptr[mine] : 0ull;
+    const uint32_t len = has ? rowlen[mine] : 0u;
+    float hi = 0.0f, lo = 0.0f;
+    long long exact = 0;
+    const double sr = FIX ? fix[kFixRow] : 1.0;
+    for (int r = 0; r < rows; r++) {
+        if (row0 + r >= n) break;  // whole warps
+        const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, r);
+        const uint32_t m = __shfl_sync(0xffffffffu, len, r);
         float s = 0.0f, comp = 0.0f;
-        for (unsigned long long j = j0 + lane; j < j1; j += 32) {
-            const uint2 q = __ldg(cw + j);
-            kahan_add(s, comp, __uint_as_float(q.y) * __ldg(pc + q.x));
-        }
-        sum = warp_sum_compensated(s, comp);
-    }
-    if (lane == 0) pn[row] = anchor_update(sum, row, bc, vox, p_init, seed, pc);
-}
-
-// Plain method: every weight is 1, so a row is a plain sum of gathered anchor values.
-__global__ void __launch_bounds__(256) k_anchor_spmv_unit(long long n, const unsigned long long *__restrict__ rowptr,
-                                                          const uint32_t *__restrict__ rowlen,
-                                                          const uint32_t *__restrict__ col, const float2 *__restrict__ bc,
-                                                          const uint32_t *__restrict__ vox,
-                                                          const float *__restrict__ p_init, int seed,
-                                                          const float *__restrict__ pc, float *__restrict__ pn,
-                                                          const int *stop, const double *__restrict__ fix)
-{
-    if (stop && *stop) return;
-    long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (row >= n) return;  // whole warps
-    unsigned long long j0 = rowptr[row], j1 = j0 + rowlen[row];
-    double sum;
-    if (fix) {  // bit-reproducible: exact fixed-point sum, whatever the entries' order
-        const double sr = fix[kFixRow];
         long long t = 0;
-        for (unsigned long long j = j0 + lane; j < j1; j += 32) t += (long long)fix_term(__ldg(pc + __ldg(col + j)), sr);
-        sum = (double)warp_sum_fixed(t) / sr;
-    } else {
-        float s = 0.0f, comp = 0.0f;
-        for (unsigned long long j = j0 + lane; j < j1; j += 32) kahan_add(s, comp, __ldg(pc + __ldg(col + j)));
-        sum = warp_sum_compensated(s, comp);
+        auto add = [&](uint32_t c, float w) {
+            const float x = __ldg(pc + c);
+            if (FIX) t += (long long)fix_term(UNIT ? x : w * x, sr);
+            else kahan_add(s, comp, UNIT ? x : w * x);
+        };
+        uint32_t j = lane;
+        for (; j + 96 < m; j += 128) {  // four entries' loads in flight per lane
+            uint32_t c[4];
+            float w[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (UNIT) {
+                    c[u] = __ldg(col + j0 + j + 32 * u);
+                    w[u] = 1.0f;
+                } else {
+                    const uint2 q = __ldg(cw + j0 + j + 32 * u);
+                    c[u] = q.x;
+                    w[u] = __uint_as_float(q.y);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) add(c[u], w[u]);
+        }
+        for (; j < m; j += 32) {
+            if (UNIT) {
+                add(__ldg(col + j0 + j), 1.0f);
+            } else {
+                const uint2 q = __ldg(cw + j0 + j);
+                add(q.x, __uint_as_float(q.y));
+            }
+        }
+        if (FIX) {
+            t = warp_sum_fixed(t);
+            exact = lane == r ? t : exact;
+        } else {
+            float h = s, l = -comp;
+            warp_sum_pair(h, l);
+            hi = lane == r ? h : hi;
+            lo = lane == r ? l : lo;
+        }
     }
-    if (lane == 0) pn[row] = anchor_update(sum, row, bc, vox, p_init, seed, pc);
+    double d = 0.0, p = 0.0;
+    if (has) {
+        const double sum = FIX ? (double)exact / sr : (double)hi + (double)lo;
+        const float2 q = bc[mine];
+        const float old = pc[mine];
+        double numer = (double)q.x + sum;
+        if (seed && p_init) numer += (double)p_init[vox[mine]];
+        const float x = q.y > 0.0f ? (float)(numer / (double)q.y) : old;
+        pn[mine] = x;
+        d = (double)x - (double)old;
+        p = (double)x;
+    }
+    if (!C.red2) return;
+    __shared__ double sh[4][kIterThreads / 32];
+    __shared__ bool last;
+    const double ad = C.about ? C.about[0] : 0.0, ap = C.about ? C.about[1] : 0.0;
+    const double dd = has ? d - ad : 0.0, pp = has ? p - ap : 0.0;
+    const double v[4] = {warp_sum_double(dd), warp_sum_double(dd * dd), warp_sum_double(pp), warp_sum_double(pp * pp)};
+    if (lane == 0)
+        for (int i = 0; i < 4; i++) sh[i][warp] = v[i];
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double t = 0.0;
+        for (int w = 0; w < kIterThreads / 32; w++) t += sh[threadIdx.x][w];
+        C.part[4ull * blockIdx.x + threadIdx.x] = t;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(C.arrived, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;  // the last block adds the blocks' sums in their order
+    __threadfence();
+    const volatile double *part = C.part;
+    const int i = threadIdx.x & 3;
+    double t = 0.0;
+    for (unsigned b = threadIdx.x >> 2; b < gridDim.x; b += kIterThreads / 4) t += part[4ull * b + i];
+    for (int o = 16; o >= 4; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);  // lanes 0..3: this warp's four sums
+    if (lane < 4) sh[lane][warp] = t;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    double S[4];
+    for (int k = 0; k < 4; k++) {
+        S[k] = 0.0;
+        for (int w = 0; w < kIterThreads / 32; w++) S[k] += sh[k][w];
+    }
+    const double N = (double)n;
+    double ed = -ad, ep = -ap;  // the shifts about the old ones (none: 0)
+    if (C.gauge == OMNI3D_GAUGE_POINT && C.ref >= 0) {
+        const volatile float *now = pn;
+        const double at = (double)now[C.ref];
+        ep = at - ap;
+        ed = at - (double)pc[C.ref] - ad;
+    } else if (C.gauge == OMNI3D_GAUGE_MEAN) {
+        ed = S[0] / N;
+        ep = S[2] / N;
+    }
+    const double change = fmax(0.0, S[1] - 2.0 * ed * S[0] + N * ed * ed);
+    const double norm = fmax(0.0, S[3] - 2.0 * ep * S[2] + N * ep * ep);
+    C.red2[0] = change;
+    C.red2[1] = norm;
+    if (C.about) {
+        C.about[0] = ad + ed;
+        C.about[1] = ap + ep;
+    }
+    if (C.stop) {  // the chunk's convergence test: the host loop's formula
+        const double rel = norm > 0 ? sqrt(change / norm) : 0.0;
+        C.rel_out[C.step] = rel;
+        if (rel < C.tol) *C.stop = C.step + 1;
+    }
 }
 
 constexpr int kRedBlocks = 256, kRedThreads = 256;
@@ -576,10 +685,8 @@ __device__ __forceinline__ double block_sum(double x, double *sh)
 }
 
 // Sums of (d, p, 1) over the selected entries (for the mean gauge).
-__global__ void k_sum_dp(long long n, const float *pc, const float *pn, const uint8_t *mask, double *part,
-                         const int *stop)
+__global__ void k_sum_dp(long long n, const float *pc, const float *pn, const uint8_t *mask, double *part)
 {
-    if (stop && *stop) return;
     __shared__ double sh[32];
     double sd = 0.0, sp = 0.0, cn = 0.0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -596,9 +703,8 @@ __global__ void k_sum_dp(long long n, const float *pc, const float *pn, const ui
     }
 }
 
-__global__ void k_finish(const double *part, int nblk, int width, double *out, const int *stop)
+__global__ void k_finish(const double *part, int nblk, int width, double *out)
 {
-    if (stop && *stop) return;
     if ((int)threadIdx.x < width) {
         double s = 0.0;
         for (int i = 0; i < nblk; i++) s += part[width * i + threadIdx.x];
@@ -610,9 +716,8 @@ __global__ void k_finish(const double *part, int nblk, int width, double *out, c
 // sum (p - sp)^2.  The shifts are the reference entry's change and value (point gauge),
 // the means (mean gauge: sums[0..2] = sum d, sum p, count) or 0.
 __global__ void k_change(long long n, const float *pc, const float *pn, const uint8_t *mask, int gauge,
-                         long long ref, const double *sums, double *part, const int *stop)
+                         long long ref, const double *sums, double *part)
 {
-    if (stop && *stop) return;
     __shared__ double sh[32];
     double sd = 0.0, sp = 0.0;
     if (gauge == OMNI3D_GAUGE_POINT && ref >= 0) {
@@ -632,65 +737,6 @@ __global__ void k_change(long long n, const float *pc, const float *pn, const ui
     }
     double ta = block_sum(a, sh), tb = block_sum(bb, sh);
     if (threadIdx.x == 0) { part[2 * blockIdx.x] = ta; part[2 * blockIdx.x + 1] = tb; }
-}
-
-// The gauged squared change and norm of one anchor iteration in one block (operators of up to
-// kChangeBlockMax anchors): the means (mean gauge) in a first pass, then the sums of
-// (d - d_mean)^2 and (p - p_mean)^2 -- one kernel instead of four, and one fixed order of
-// the sums.  red2 = {change, norm}.  One SM's FP64 rate limits it: at 5.8 K anchors it saves
-// 20 us per iteration against the four-kernel form, at 97 K anchors it costs 250 us more.
-constexpr long long kChangeBlockMax = 16384;
-__global__ void __launch_bounds__(1024) k_change_block(long long n, const float *__restrict__ pc,
-                                                       const float *__restrict__ pn, int gauge, long long ref,
-                                                       double *red2, const int *stop)
-{
-    if (stop && *stop) return;
-    __shared__ double sh[32];
-    __shared__ double shift[2];
-    double sd = 0.0, sp = 0.0;
-    if (gauge == OMNI3D_GAUGE_POINT && ref >= 0) {
-        sp = (double)pn[ref];
-        sd = sp - (double)pc[ref];
-    } else if (gauge == OMNI3D_GAUGE_MEAN) {
-        double a = 0.0, b = 0.0;
-        for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-            a += (double)pn[i] - (double)pc[i];
-            b += (double)pn[i];
-        }
-        a = block_sum(a, sh);
-        b = block_sum(b, sh);
-        if (threadIdx.x == 0) {
-            shift[0] = n > 0 ? a / (double)n : 0.0;
-            shift[1] = n > 0 ? b / (double)n : 0.0;
-        }
-        __syncthreads();
-        sd = shift[0];
-        sp = shift[1];
-    }
-    double x = 0.0, y = 0.0;
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        const double d = (double)pn[i] - (double)pc[i] - sd;
-        const double q = (double)pn[i] - sp;
-        x += d * d;
-        y += q * q;
-    }
-    x = block_sum(x, sh);
-    y = block_sum(y, sh);
-    if (threadIdx.x == 0) {
-        red2[0] = x;
-        red2[1] = y;
-    }
-}
-
-// Convergence test of step j of a graph-captured chunk: rel = sqrt(change / norm) (the host
-// loop's formula), recorded in rel_out[j]; *stop = j + 1 when rel < tol, which turns the
-// chunk's remaining kernels into no-ops.
-__global__ void k_converged(const double *red2, double tol, int j, int *stop, double *rel_out)
-{
-    if (*stop) return;
-    const double rel = red2[1] > 0 ? sqrt(red2[0] / red2[1]) : 0.0;
-    rel_out[j] = rel;
-    if (rel < tol) *stop = j + 1;
 }
 
 // The anchor values into the walks' copies of the pressure.
@@ -878,8 +924,7 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     AN_TRY(grow(A->u, cap[3], sizeof(uint32_t) * (size_t)V));
     AN_TRY(grow(A->pos, cap[4], sizeof(uint32_t) * (size_t)(V + 1)));
     AN_TRY(grow(A->tmp, cap[5], sizeof(uint32_t) * scan_tmp_elems(V)));
-    AN_TRY(grow(A->red, cap[6], sizeof(double) * change_scratch_doubles()));
-    Sink S{};
+        Sink S{};
     S.flag = A->flag;
     bool marked = false;
     if (method_accum(method) == kAccSelect) {
@@ -949,6 +994,7 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     if (unit_links) AN_TRY(grow(A->col, cap[11], sizeof(uint32_t) * (size_t)nnz));
     else AN_TRY(grow(A->cw, cap[12], sizeof(uint2) * (size_t)nnz));
     AN_TRY(grow(A->bc, cap[13], sizeof(float2) * (size_t)n));
+    AN_TRY(grow(A->red, cap[6], sizeof(double) * (4 + 4 * (size_t)iter_blocks(std::max<long long>(n, 1)))));
     AN_TRY(grow(A->pa, cap[15], sizeof(float) * (size_t)n));
     AN_TRY(grow(A->pb, cap[16], sizeof(float) * (size_t)n));
     AN_TRY(grow(A->rowlen, cap[17], sizeof(uint32_t) * (size_t)n));
@@ -989,18 +1035,18 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
 size_t change_scratch_doubles() { return 8 + 3 * kRedBlocks; }
 
 cudaError_t change_sums(long long n, const float *pc, const float *pn, int gauge, long long ref, double *scratch,
-                        double *out2, cudaStream_t st, const uint8_t *mask, const int *stop)
+                        double *out2, cudaStream_t st, const uint8_t *mask)
 {
     double *part = scratch + 8;
     if (gauge == OMNI3D_GAUGE_MEAN) {
-        k_sum_dp<<<kRedBlocks, kRedThreads, 0, st>>>(n, pc, pn, mask, part, stop);
+        k_sum_dp<<<kRedBlocks, kRedThreads, 0, st>>>(n, pc, pn, mask, part);
         OM_COUNT_LAUNCH();
-        k_finish<<<1, 32, 0, st>>>(part, kRedBlocks, 3, scratch + 4, stop);
+        k_finish<<<1, 32, 0, st>>>(part, kRedBlocks, 3, scratch + 4);
         OM_COUNT_LAUNCH();
     }
-    k_change<<<kRedBlocks, kRedThreads, 0, st>>>(n, pc, pn, mask, gauge, ref, scratch + 4, part, stop);
+    k_change<<<kRedBlocks, kRedThreads, 0, st>>>(n, pc, pn, mask, gauge, ref, scratch + 4, part);
     OM_COUNT_LAUNCH();
-    k_finish<<<1, 32, 0, st>>>(part, kRedBlocks, 2, out2, stop);
+    k_finish<<<1, 32, 0, st>>>(part, kRedBlocks, 2, out2);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
@@ -1034,41 +1080,44 @@ cudaError_t anchor_mark(const Geometry &geo, const Field &f, int method, long lo
     return e;
 }
 
-cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, int gauge, long long ref_anchor,
-                        const float *p_cur, float *p_next, double *red2, cudaStream_t st, const int *stop,
+cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, bool first, int gauge, long long ref_anchor,
+                        const float *p_cur, float *p_next, double *red2, cudaStream_t st, const ChunkTest *test,
                         const Fixed *fx)
 {
     if (A.n == 0) return cudaSuccess;
-    long long threads = A.n * 32;
+    const int *stop = test ? test->stop : nullptr;
     const double *fix = nullptr;
     if (fx) {  // bit-reproducible: the row sums' scale from this iterate's largest value
         cudaError_t e = fix_row_scale(A.n, p_cur, *fx, st, stop);
         if (e != cudaSuccess) return e;
         fix = fx->scale;
     }
-    if (A.unit_weights)
-        k_anchor_spmv_unit<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(A.n, A.rowptr, A.rowlen, A.col, A.bc, A.vox,
-                                                                               p_init, seed ? 1 : 0, p_cur, p_next, stop,
-                                                                               fix);
-    else
-        k_anchor_spmv<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(A.n, A.rowptr, A.rowlen, A.cw, A.bc,
-                                                                          A.vox, p_init, seed ? 1 : 0, p_cur, p_next,
-                                                                          stop, fix);
-    OM_COUNT_LAUNCH();
-    if (red2 && A.n <= kChangeBlockMax) {
-        k_change_block<<<1, 1024, 0, st>>>(A.n, p_cur, p_next, gauge, ref_anchor, red2, stop);
-        OM_COUNT_LAUNCH();
-    } else if (red2) {
-        return change_sums(A.n, p_cur, p_next, gauge, ref_anchor, A.red, red2, st, nullptr, stop);
+    ChangeOut C{};
+    if (red2) {
+        C.red2 = red2;
+        C.about = A.red;
+        C.arrived = reinterpret_cast<unsigned *>(A.red + 2);
+        C.part = A.red + 4;
+        C.gauge = gauge;
+        C.ref = ref_anchor;
+        if (first) {  // nothing to take the sums about
+            cudaError_t e = cudaMemsetAsync(A.red, 0, sizeof(double) * 4, st);
+            if (e != cudaSuccess) return e;
+        }
+        if (test) {
+            C.tol = test->tol;
+            C.step = test->step;
+            C.stop = test->stop;
+            C.rel_out = test->rel_out;
+        }
     }
-    return cudaGetLastError();
-}
-
-cudaError_t converged_test_launch(const double *red2, double tol, int j, int *stop, double *rel_out,
-                                  cudaStream_t st)
-{
-    k_converged<<<1, 1, 0, st>>>(red2, tol, j, stop, rel_out);
-    OM_COUNT_LAUNCH();
+    auto launch = [&](auto kernel) {
+        kernel<<<iter_blocks(A.n), kIterThreads, 0, st>>>(A.n, iter_rows(A.n), A.rowptr, A.rowlen, A.col, A.cw, A.bc, A.vox,
+                                                          p_init, seed ? 1 : 0, p_cur, p_next, stop, fix, C);
+        OM_COUNT_LAUNCH();
+    };
+    if (A.unit_weights) fix ? launch(k_anchor_iterate<true, true>) : launch(k_anchor_iterate<true, false>);
+    else fix ? launch(k_anchor_iterate<false, true>) : launch(k_anchor_iterate<false, false>);
     return cudaGetLastError();
 }
 
