@@ -458,7 +458,8 @@ cudaError_t enqueue_prepared(omni3d_ctx *ctx, const float *dax, const float *day
     const bool seed = P.seed_first_iteration != 0;
     float *pc = A.pa, *pn = A.pb;
     for (int it = 1; it <= K - 1; it++) {
-        if ((e = anchor_step(A, dpinit, seed && it == 1, it == 1, P.gauge, -1, pc, pn, nullptr, st)) != cudaSuccess) return e;
+        if ((e = anchor_step(A, dpinit, seed && it == 1, it == 1, P.gauge, -1, pc, pn, nullptr, st,
+                             nullptr, nullptr, false)) != cudaSuccess) return e;
         std::swap(pc, pn);
     }
     float2 *acc = ctx->pncnt.as<float2>();
@@ -946,8 +947,8 @@ cudaError_t iterate_chunk(omni3d_ctx *ctx, const Anchor &A, int gauge, long long
     uint64_t tol_bits;
     std::memcpy(&tol_bits, &tol, sizeof(tol_bits));
     const std::vector<const void *> key = {
-        A.rowptr, A.rowlen, A.col, A.cw, A.bc, A.vox, A.red, reinterpret_cast<const void *>((uintptr_t)A.n),
-        reinterpret_cast<const void *>((uintptr_t)A.unit_weights), pc, pn, red2,
+        A.rowptr, A.rowlen, A.links, A.bc, A.vox, A.red, reinterpret_cast<const void *>((uintptr_t)A.n),
+        reinterpret_cast<const void *>((uintptr_t)A.kind), pc, pn, red2,
         reinterpret_cast<const void *>((uintptr_t)gauge), reinterpret_cast<const void *>((intptr_t)ref_anchor),
         reinterpret_cast<const void *>((uintptr_t)tol_bits), stop, fx ? fx->scale : nullptr,
         fx ? fx->bits : nullptr};

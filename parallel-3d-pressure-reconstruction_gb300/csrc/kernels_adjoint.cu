@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <utility>
 
+#include "links.cuh"
 #include "omni3d_internal.h"
 #include "walk.cuh"
 
@@ -220,77 +221,89 @@ __global__ void __launch_bounds__(256) k_adj_grad(Grid g, Layout lay, WalkLines 
     }
 }
 
-// Column and weight of operator entry j: unit-weight operators store the column alone,
-// weighted ones (column, weight bits).
-__device__ __forceinline__ uint32_t entry_col(const uint32_t *col, const uint2 *cw, unsigned long long j)
+// The operator's links, a warp per row: transposed rows' lengths, and the transposed links.
+template <int KIND>
+__global__ void k_adj_tcount(long long n, const unsigned long long *rowptr, const uint32_t *rowlen, const void *links,
+                             uint32_t *tcnt)
 {
-    return col ? col[j] : cw[j].x;
-}
-__device__ __forceinline__ float entry_w(const uint2 *cw, unsigned long long j)
-{
-    return cw ? __uint_as_float(cw[j].y) : 1.0f;
-}
-
-// transposed operator: count entries per column
-__global__ void k_adj_tcount(long long n, const unsigned long long *rowptr, const uint32_t *rowlen,
-                             const uint32_t *col, const uint2 *cw, uint32_t *tcnt)
-{
-    long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
+    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= n) return;
-    unsigned long long j0 = rowptr[row], j1 = j0 + rowlen[row];
-    for (unsigned long long j = j0 + lane; j < j1; j += 32) atomicAdd(tcnt + entry_col(col, cw, j), 1u);
+    if ((threadIdx.x & 31) < lanes_per_row(KIND))
+        row_links<KIND>(links, rowptr[row], rowlen[row], threadIdx.x & 31, [&](uint32_t c, float) { atomicAdd(tcnt + c, 1u); });
 }
 
-__global__ void k_adj_tfill(long long n, const unsigned long long *rowptr, const uint32_t *rowlen, const uint32_t *col,
-                            const uint2 *cw, const unsigned long long *tptr, uint32_t *tcur, uint32_t *trow, float *tw)
+template <int KIND>
+__global__ void k_adj_tfill(long long n, const unsigned long long *rowptr, const uint32_t *rowlen, const void *links,
+                            const unsigned long long *tptr, uint32_t *tcur, void *tlinks)
 {
-    long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
+    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= n) return;
-    unsigned long long j0 = rowptr[row], j1 = j0 + rowlen[row];
-    for (unsigned long long j = j0 + lane; j < j1; j += 32) {
-        const uint32_t c = entry_col(col, cw, j);
-        const unsigned long long pos = tptr[c] + atomicAdd(tcur + c, 1u);
-        trow[pos] = (uint32_t)row;
-        if (tw) tw[pos] = entry_w(cw, j);
-    }
+    if ((threadIdx.x & 31) >= lanes_per_row(KIND)) return;
+    row_links<KIND>(links, rowptr[row], rowlen[row], threadIdx.x & 31, [&](uint32_t c, float w) {
+        store_link<KIND>(tlinks, tptr[c] + atomicAdd(tcur + c, 1u), (uint32_t)row, w);
+    });
 }
 
-__global__ void k_u32_to_u64(long long n, const uint32_t *in, unsigned long long *out)
+// Capacities of the transposed rows: whole 16-byte vectors of `per` links.
+__global__ void k_adj_capacity(long long n, const uint32_t *in, unsigned per, unsigned long long *out)
 {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        out[i] = in[i];
+        out[i] = (in[i] + per - 1) / per * per;
 }
 
-// acc += lambda / c (c > 0)
-__global__ void k_adj_accum(long long n, const float *lam, const float2 *bc, float *acc)
+// u = lambda / c where c > 0, else 0; acc = u: the first term of the backward iterations.
+__global__ void k_adj_first(long long n, const float *lam, const float2 *bc, float *u, float *acc)
 {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float c = bc[i].y;
-        if (c > 0.0f) acc[i] += __fdiv_rn(lam[i], c);
+        const float c = bc[i].y, x = c > 0.0f ? __fdiv_rn(lam[i], c) : 0.0f;
+        u[i] = x;
+        acc[i] = x;
     }
 }
 
-// next = M^T D^-1 lambda (+ lambda where c = 0), a warp per column of M (tw: the entries'
-// weights, null for unit weights)
-__global__ void __launch_bounds__(256) k_adj_spmvT(long long n, const unsigned long long *__restrict__ tptr,
-                                                   const uint32_t *__restrict__ trow, const float *__restrict__ tw,
-                                                   const float *__restrict__ lam, const float2 *__restrict__ bc,
-                                                   float *__restrict__ next)
+// One backward iteration, lambda <- M^T D^-1 lambda (+ lambda where c = 0), from u = D^-1 lambda:
+// a warp per transposed row; then u <- D^-1 lambda and acc += u.  96^3 / 642 directions (34 M
+// links): 133 us with a gather of lambda and of c and a division per link, 46 us with one gather, 30 us with u
+// in shared memory and several rows per warp at a time.
+template <int KIND, bool SMEM>
+__global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 4) k_adj_iterate(
+    long long n, int rows, const unsigned long long *__restrict__ tptr, const uint32_t *__restrict__ tlen,
+    const void *__restrict__ tlinks, const float2 *__restrict__ bc, const float *__restrict__ u, float *__restrict__ unext,
+    float *lam, float *acc)
 {
-    long long a = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (a >= n) return;
-    unsigned long long j0 = tptr[a], j1 = tptr[a + 1];
-    float s = 0.0f;
-    for (unsigned long long j = j0 + lane; j < j1; j += 32) {
-        uint32_t r = __ldg(trow + j);
-        float cr = __ldg(&bc[r].y);
-        if (cr > 0.0f) s += (tw ? __ldg(tw + j) : 1.0f) * __fdiv_rn(__ldg(lam + r), cr);
+    extern __shared__ float4 sh_vector[];
+    const float *x = gather_vector<SMEM>(u, n, reinterpret_cast<float *>(sh_vector));
+    constexpr int kWarps = (SMEM ? 1024 : 256) / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long row0 = ((long long)blockIdx.x * kWarps + warp) * rows;
+    const long long mine = row0 + lane;  // the row this lane finishes
+    const bool has = lane < rows && mine < n;
+    const unsigned long long ptr = has ? tptr[mine] : 0ull;
+    const uint32_t len = has ? tlen[mine] : 0u;
+    float sum = 0.0f;
+    constexpr int kLanes = lanes_per_row(KIND), kRows = 32 / kLanes;
+    for (int r = 0; r < rows; r += kRows) {
+        if (row0 + r >= n) break;  // whole warps
+        const int at = r + lane / kLanes;
+        const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, at & 31);
+        const uint32_t m = __shfl_sync(0xffffffffu, len, at & 31);
+        float s = 0.0f;
+        row_links<KIND>(tlinks, j0, at < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
+            const float y = SMEM ? x[c] : __ldg(x + c);
+            s += KIND == kLinkPair ? w * y : y;
+        });
+        __syncwarp();
+        for (int o = kLanes / 2; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        s = __shfl_sync(0xffffffffu, s, ((lane - r) * kLanes) & 31);  // the row of lane r + i
+        if (lane >= r && lane < r + kRows) sum = s;
     }
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) next[a] = s + (bc[a].y > 0.0f ? 0.0f : lam[a]);
+    if (!has) return;
+    const float c = bc[mine].y;
+    const float l = sum + (c > 0.0f ? 0.0f : lam[mine]);
+    const float t = c > 0.0f ? __fdiv_rn(l, c) : 0.0f;
+    lam[mine] = l;
+    unext[mine] = t;
+    acc[mine] += t;
 }
 
 // dB[vox[a]] += acc[a]
@@ -328,8 +341,15 @@ __global__ void k_sum_g(long long V, const float *g, const float *cnt, double *p
 __global__ void k_gauge_T(long long V, const float *g, const float *cnt, const double *part, int nblk, int gauge,
                           long long ref, float *out)
 {
-    double S = 0.0, N = 0.0;
-    for (int b = 0; b < nblk; b++) { S += part[2 * b]; N += part[2 * b + 1]; }
+    // the blocks' sums, added once per block in their order (a thread each took 0.4 ms at 96^3)
+    __shared__ double sh[2];
+    if (threadIdx.x < 2) {
+        double t = 0.0;
+        for (int b = 0; b < nblk; b++) t += part[2 * b + threadIdx.x];
+        sh[threadIdx.x] = t;
+    }
+    __syncthreads();
+    const double S = sh[0], N = sh[1];
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
         double x = (double)g[v];
         if (gauge == OMNI3D_GAUGE_MEAN && cnt[v] > 0.0f && N > 0) x -= S / N;
@@ -365,12 +385,12 @@ size_t gauge_transpose_scratch_doubles() { return 2 * kRB; }
 void adjoint_free(AdjointBuffers *B)
 {
     cudaFree(B->tptr);
-    cudaFree(B->trow);
-    cudaFree(B->tw);
-    cudaFree(B->tmp);
+    cudaFree(B->tlen);
+    cudaFree(B->tlinks);
     cudaFree(B->mu);
     cudaFree(B->lam);
-    cudaFree(B->nxt);
+    cudaFree(B->u);
+    cudaFree(B->unext);
     cudaFree(B->acc);
     *B = AdjointBuffers();
 }
@@ -412,7 +432,7 @@ void adj_lines(int acc, const Geometry &geo, bool gather, const float4 *f32, con
 cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *B, int K, int method, const float4 *f32,
                           const float *g, const float *cnt, float *gx, float *gy, float *gz, cudaStream_t st)
 {
-    if (!f32 || !A.id || !A.bc || !A.vox || !A.rowptr || !A.rowlen || (A.unit_weights ? !A.col : !A.cw))
+    if (!f32 || !A.id || !A.bc || !A.vox || !A.rowptr || !A.rowlen || !A.links)
         return cudaErrorInvalidValue;
     const int acc = method_accum(method);
     const long long V = geo.grid.V, n = A.n;
@@ -423,38 +443,44 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
     if (!B->mu) ADJ_TRY(cudaMalloc(&B->mu, sizeof(float) * (size_t)V));
     if (!B->lam) {
         ADJ_TRY(cudaMalloc(&B->lam, sizeof(float) * (size_t)std::max(n, 1LL)));
-        ADJ_TRY(cudaMalloc(&B->nxt, sizeof(float) * (size_t)std::max(n, 1LL)));
+        ADJ_TRY(cudaMalloc(&B->u, sizeof(float) * (size_t)std::max(n, 1LL)));
+        ADJ_TRY(cudaMalloc(&B->unext, sizeof(float) * (size_t)std::max(n, 1LL)));
         ADJ_TRY(cudaMalloc(&B->acc, sizeof(float) * (size_t)std::max(n, 1LL)));
     }
     // transposed operator (once per operator)
+    const unsigned row_blocks = (unsigned)((n * 32 + 255) / 256);
     if (!B->tptr) {
-        uint32_t *tcnt = nullptr;
         unsigned long long *t64 = nullptr, *tmp = nullptr;
-        ADJ_TRY(cudaMalloc(&tcnt, sizeof(uint32_t) * (size_t)std::max(n, 1LL)));
+        uint32_t *tcur = nullptr;
+        ADJ_TRY(cudaMalloc(&B->tlen, sizeof(uint32_t) * (size_t)std::max(n, 1LL)));
+        ADJ_TRY(cudaMalloc(&tcur, sizeof(uint32_t) * (size_t)std::max(n, 1LL)));
         ADJ_TRY(cudaMalloc(&t64, sizeof(unsigned long long) * (size_t)std::max(n, 1LL)));
         ADJ_TRY(cudaMalloc(&tmp, sizeof(unsigned long long) * scan_tmp_elems(n)));
         ADJ_TRY(cudaMalloc(&B->tptr, sizeof(unsigned long long) * (size_t)(n + 1)));
-        ADJ_TRY(cudaMemsetAsync(tcnt, 0, sizeof(uint32_t) * (size_t)std::max(n, 1LL), st));
-        long long threads = n * 32;
-        const uint32_t *col = A.unit_weights ? A.col : nullptr;
-        const uint2 *cw = A.unit_weights ? nullptr : A.cw;
-        k_adj_tcount<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(n, A.rowptr, A.rowlen, col, cw, tcnt);
-        OM_COUNT_LAUNCH();
-        k_u32_to_u64<<<grid_for(n), 256, 0, st>>>(n, tcnt, t64);
-        OM_COUNT_LAUNCH();
+        ADJ_TRY(cudaMemsetAsync(B->tlen, 0, sizeof(uint32_t) * (size_t)std::max(n, 1LL), st));
+        auto count = [&](auto kernel) { kernel<<<row_blocks, 256, 0, st>>>(n, A.rowptr, A.rowlen, A.links, B->tlen); };
+        if (n) {
+            A.kind == kLink16 ? count(k_adj_tcount<kLink16>)
+                              : (A.kind == kLink32 ? count(k_adj_tcount<kLink32>) : count(k_adj_tcount<kLinkPair>));
+            OM_COUNT_LAUNCH();
+            k_adj_capacity<<<grid_for(n), 256, 0, st>>>(n, B->tlen, (unsigned)links_per_vector(A.kind), t64);
+            OM_COUNT_LAUNCH();
+        }
         ADJ_TRY(exclusive_scan_u64(t64, B->tptr, n, tmp, st));
         unsigned long long tn = 0;
         ADJ_TRY(cudaMemcpyAsync(&tn, B->tptr + n, sizeof(tn), cudaMemcpyDeviceToHost, st));
         ADJ_TRY(cudaStreamSynchronize(st));
-        ADJ_TRY(cudaMalloc(&B->trow, sizeof(uint32_t) * (size_t)std::max(tn, 1ULL)));
-        if (!A.unit_weights) ADJ_TRY(cudaMalloc(&B->tw, sizeof(float) * (size_t)std::max(tn, 1ULL)));
-        ADJ_TRY(cudaMemsetAsync(tcnt, 0, sizeof(uint32_t) * (size_t)std::max(n, 1LL), st));
-        k_adj_tfill<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(n, A.rowptr, A.rowlen, col, cw, B->tptr, tcnt,
-                                                                       B->trow, B->tw);
-        OM_COUNT_LAUNCH();
+        ADJ_TRY(cudaMalloc(&B->tlinks, link_size(A.kind) * (size_t)std::max(tn, 1ULL)));
+        ADJ_TRY(cudaMemsetAsync(tcur, 0, sizeof(uint32_t) * (size_t)std::max(n, 1LL), st));
+        auto fill = [&](auto kernel) { kernel<<<row_blocks, 256, 0, st>>>(n, A.rowptr, A.rowlen, A.links, B->tptr, tcur, B->tlinks); };
+        if (n) {
+            A.kind == kLink16 ? fill(k_adj_tfill<kLink16>)
+                              : (A.kind == kLink32 ? fill(k_adj_tfill<kLink32>) : fill(k_adj_tfill<kLinkPair>));
+            OM_COUNT_LAUNCH();
+        }
         ADJ_TRY(cudaGetLastError());
         ADJ_TRY(cudaStreamSynchronize(st));
-        cudaFree(tcnt);
+        cudaFree(tcur);
         cudaFree(t64);
         cudaFree(tmp);
     }
@@ -465,20 +491,31 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
     ADJ_TRY(cudaMemsetAsync(B->acc, 0, sizeof(float) * (size_t)std::max(n, 1LL), st));
     adj_lines(acc, geo, true, f32, B->mu, A.id, B->lam, nullptr, nullptr, nullptr, st);
     // anchor iterations, backwards
-    long long threads = n * 32;
-    for (int k = K - 1; k >= 1; k--) {
-        k_adj_accum<<<grid_for(n), 256, 0, st>>>(n, B->lam, A.bc, B->acc);
+    if (K > 1 && n) {
+        k_adj_first<<<grid_for(n), 256, 0, st>>>(n, B->lam, A.bc, B->u, B->acc);
         OM_COUNT_LAUNCH();
-        if (k > 1) {
-            k_adj_spmvT<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(n, B->tptr, B->trow, B->tw, B->lam, A.bc,
-                                                                           B->nxt);
-            OM_COUNT_LAUNCH();
-            std::swap(B->lam, B->nxt);
-        }
+        const IterShape I = iter_shape(n, true);
+        auto launch = [&](auto wide, auto smem) {
+            auto kernel = I.smem ? smem : wide;
+            if (I.bytes > 48 * 1024)
+                ADJ_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIterSmemMax));
+            for (int k = K - 1; k > 1; k--) {
+                kernel<<<I.blocks, I.threads, I.bytes, st>>>(n, I.rows, B->tptr, B->tlen, B->tlinks, A.bc, B->u, B->unext, B->lam,
+                                                             B->acc);
+                OM_COUNT_LAUNCH();
+                std::swap(B->u, B->unext);
+            }
+            return cudaGetLastError();
+        };
+        ADJ_TRY(A.kind == kLink16   ? launch(k_adj_iterate<kLink16, false>, k_adj_iterate<kLink16, true>)
+                : A.kind == kLink32 ? launch(k_adj_iterate<kLink32, false>, k_adj_iterate<kLink32, true>)
+                                    : launch(k_adj_iterate<kLinkPair, false>, k_adj_iterate<kLinkPair, true>));
     }
     // dL/dB = mu + acc on the anchors, then the line scatter
-    k_adj_add_anchor<<<grid_for(n), 256, 0, st>>>(n, A.vox, B->acc, B->mu);
-    OM_COUNT_LAUNCH();
+    if (n) {
+        k_adj_add_anchor<<<grid_for(n), 256, 0, st>>>(n, A.vox, B->acc, B->mu);
+        OM_COUNT_LAUNCH();
+    }
     adj_lines(acc, geo, false, f32, B->mu, nullptr, nullptr, gx, gy, gz, st);
     return cudaGetLastError();
 }

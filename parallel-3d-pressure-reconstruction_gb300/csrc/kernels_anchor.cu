@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include "fixed.cuh"
+#include "links.cuh"
 #include "omni3d_internal.h"
 #include "walk.cuh"
 
@@ -78,8 +79,8 @@ struct Sink {
     const int32_t *id;   // the walks' copies of the anchor ids (-1: no anchor)
     uint8_t *flag;       // row-major (the marking pass walks the row-major layout)
     unsigned long long *next;  // per row: the next free link slot (starts at the row's first slot)
-    uint32_t *col;   // unit-weight operators: the start anchor of each link
-    uint2 *cw;       // weighted operators: (start anchor, weight bits) of each link
+    void *links;     // per link the start anchor, and its weight in weighted operators (links.cuh)
+    int kind;        // LinkKind
     float2 *bc;      // per row: (b, c)
     long long *bc64; // bit-reproducible mode: per row the fixed-point (b, c) instead of bc
     const double *fix;  // its scales (fixed.cuh)
@@ -101,8 +102,9 @@ __device__ __forceinline__ void emit_w(const Sink &S, int row, uint32_t scol, fl
     }
     const unsigned long long slot = atomicAdd(S.next + row, 1ull);
     const float bt = UNIT ? I : wt * I, ct = UNIT ? 1.0f : wt;
-    if (UNIT) S.col[slot] = scol;
-    else S.cw[slot] = make_uint2(scol, __float_as_uint(wt));
+    if (!UNIT) store_link<kLinkPair>(S.links, slot, scol, wt);
+    else if (S.kind == kLink16) store_link<kLink16>(S.links, slot, scol, wt);
+    else store_link<kLink32>(S.links, slot, scol, wt);
     if (S.bc64) {  // bit-reproducible: exact, order-independent fixed-point row sums
         fix_add(S.bc64 + 2 * row, bt, S.fix[kFixB]);
         fix_add(S.bc64 + 2 * row + 1, ct, S.fix[kFixC]);
@@ -465,11 +467,19 @@ __global__ void k_assign_ids(Grid g, Layout lay, const uint8_t *flag, const uint
     }
 }
 
-__global__ void k_row_capacity(long long n, const uint32_t *vox, const uint32_t *lines_through,
-                               unsigned long long *out)
+// Link slots of every row: the lines through its voxel (each contributes at most once), in whole
+// loads of `per` links; *total: the slots before rounding.
+__global__ void k_row_capacity(long long n, const uint32_t *vox, const uint32_t *lines_through, unsigned per,
+                               unsigned long long *out, unsigned long long *total)
 {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        out[i] = lines_through[vox[i]];
+    unsigned long long t = 0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const uint32_t c = lines_through[vox[i]];
+        out[i] = (c + per - 1) / per * per;
+        t += c;
+    }
+    for (int o = 16; o; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0 && t) atomicAdd(total, t);
 }
 
 // Row sums of the anchor iteration: compensated (Kahan) FP32 per lane, the lane sums added as
@@ -477,10 +487,11 @@ __global__ void k_row_capacity(long long n, const uint32_t *vox, const uint32_t 
 // FP64.  A row gathers about as many terms as lines cross its voxel (~1000 at 642 directions);
 // plain FP32 sums of that many terms leave a rounding floor near 1e-6 in the iteration's
 // relative change, above the tolerances the solver is asked for.
+template <int LANES>
 __device__ __forceinline__ void warp_sum_pair(float &hi, float &lo)
 {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
+    for (int o = LANES / 2; o; o >>= 1) {
         const float h2 = __shfl_xor_sync(0xffffffffu, hi, o), l2 = __shfl_xor_sync(0xffffffffu, lo, o);
         const float t = __fadd_rn(hi, h2), b = __fsub_rn(t, hi);
         const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(h2, b));  // hi + h2 = t + e exactly
@@ -489,10 +500,12 @@ __device__ __forceinline__ void warp_sum_pair(float &hi, float &lo)
     }
 }
 
-// The warp's exact sum of fixed-point lane sums (integer additions: order-independent).
+// The exact sum of fixed-point lane sums (integer additions: order-independent).
+template <int LANES>
 __device__ __forceinline__ long long warp_sum_fixed(long long t)
 {
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+#pragma unroll
+    for (int o = LANES / 2; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     return t;
 }
 
@@ -520,109 +533,94 @@ struct ChangeOut {
     double *rel_out;
 };
 
-// Rows per warp: the FP64 work of a row -- its update, one division among it -- is done for a
-// warp's rows together, a lane each, since this GPU's FP64 units take 16 cycles per warp
+// One anchor iteration, p_next = (b + seed p_init + M p_cur) / c; KIND: the links; FIX: the
+// bit-reproducible mode's exact fixed-point sums, whatever the entries' order; SMEM: p_cur in
+// shared memory.  The FP64 work of a row -- its update, one division among it -- is done for a
+// block's rows together, a thread each, since this GPU's FP64 units take 16 cycles per warp
 // instruction and SM: with a row per warp and FP64 lane sums they alone took 0.1 ms of the
-// 0.165 of an iteration at 128^3 / 642 directions (97 K rows).
-constexpr int kIterThreads = 256, kIterRowsMax = 16, kIterWarps = 152 * 48;
-inline int iter_rows(long long n) { return (int)std::max(1LL, std::min<long long>(kIterRowsMax, (n + kIterWarps - 1) / kIterWarps)); }
-inline unsigned iter_blocks(long long n)
-{
-    const long long per = (long long)iter_rows(n) * (kIterThreads / 32);
-    return (unsigned)((n + per - 1) / per);
-}
-
-// One anchor iteration, p_next = (b + seed p_init + M p_cur) / c; UNIT: every weight is 1 (plain
-// method), a row is a sum of gathered anchor values; FIX: the bit-reproducible mode's exact
-// fixed-point sums, whatever the entries' order.
-template <bool UNIT, bool FIX>
-__global__ void __launch_bounds__(kIterThreads) k_anchor_iterate(
+// 0.165 of an iteration at 128^3 / 642 directions (97 K rows).  96^3 / 642 directions (54 K rows,
+// 34 M links): 80 us, 48 with the rows' FP64 work together, 35 with 16-bit links, 28 with
+// p_cur in shared memory; six CTAs of 256 threads per SM at 40 registers (five: 10 to 25 % more).
+template <int KIND, bool FIX, bool SMEM>
+__global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iterate(
     long long n, int rows, const unsigned long long *__restrict__ rowptr, const uint32_t *__restrict__ rowlen,
-    const uint32_t *__restrict__ col, const uint2 *__restrict__ cw, const float2 *__restrict__ bc,
+    const void *__restrict__ links, const float2 *__restrict__ bc,
     const uint32_t *__restrict__ vox, const float *__restrict__ p_init, int seed, const float *__restrict__ pc, float *pn,
     const int *stop, const double *__restrict__ fix, ChangeOut C)
 {
+    extern __shared__ float4 sh_vector[];
     if (stop && *stop) return;  // a graph-captured chunk that has met its tolerance
+    const float *x = gather_vector<SMEM>(pc, n, reinterpret_cast<float *>(sh_vector));
+    constexpr int kWarps = (SMEM ? 1024 : 256) / 32, kLanes = lanes_per_row(KIND), kRows = 32 / kLanes;
+    __shared__ double row_sum[kWarps * kIterRowsMax];  // (hi, lo) pairs, or the exact integers
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long row0 = ((long long)blockIdx.x * (kIterThreads / 32) + warp) * rows;
-    const long long mine = row0 + lane;  // the row this lane finishes
-    const bool has = lane < rows && mine < n;
-    const unsigned long long ptr = has ? rowptr[mine] : 0ull;
-    const uint32_t len = has ? rowlen[mine] : 0u;
-    float hi = 0.0f, lo = 0.0f;
-    long long exact = 0;
+    const long long base = (long long)blockIdx.x * kWarps * rows;  // the block's first row
+    const long long row0 = base + (long long)warp * rows;
+    unsigned long long ptr = 0ull;
+    uint32_t len = 0u;
+    if (lane < rows && row0 + lane < n) {
+        ptr = rowptr[row0 + lane];
+        len = rowlen[row0 + lane];
+    }
     const double sr = FIX ? fix[kFixRow] : 1.0;
-    for (int r = 0; r < rows; r++) {
+    for (int r = 0; r < rows; r += kRows) {
         if (row0 + r >= n) break;  // whole warps
-        const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, r);
-        const uint32_t m = __shfl_sync(0xffffffffu, len, r);
+        const int mine = r + lane / kLanes;  // (lanes past the last row have length 0)
+        const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, mine & 31);
+        const uint32_t m = __shfl_sync(0xffffffffu, len, mine & 31);
         float s = 0.0f, comp = 0.0f;
         long long t = 0;
-        auto add = [&](uint32_t c, float w) {
-            const float x = __ldg(pc + c);
-            if (FIX) t += (long long)fix_term(UNIT ? x : w * x, sr);
-            else kahan_add(s, comp, UNIT ? x : w * x);
-        };
-        uint32_t j = lane;
-        for (; j + 96 < m; j += 128) {  // four entries' loads in flight per lane
-            uint32_t c[4];
-            float w[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (UNIT) {
-                    c[u] = __ldg(col + j0 + j + 32 * u);
-                    w[u] = 1.0f;
-                } else {
-                    const uint2 q = __ldg(cw + j0 + j + 32 * u);
-                    c[u] = q.x;
-                    w[u] = __uint_as_float(q.y);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) add(c[u], w[u]);
-        }
-        for (; j < m; j += 32) {
-            if (UNIT) {
-                add(__ldg(col + j0 + j), 1.0f);
-            } else {
-                const uint2 q = __ldg(cw + j0 + j);
-                add(q.x, __uint_as_float(q.y));
-            }
-        }
+        row_links<KIND>(links, j0, mine < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
+            const float y = SMEM ? x[c] : __ldg(x + c);
+            if (FIX) t += (long long)fix_term(KIND == kLinkPair ? w * y : y, sr);
+            else kahan_add(s, comp, KIND == kLinkPair ? w * y : y);
+        });
+        __syncwarp();
         if (FIX) {
-            t = warp_sum_fixed(t);
-            exact = lane == r ? t : exact;
+            t = warp_sum_fixed<kLanes>(t);
         } else {
             float h = s, l = -comp;
-            warp_sum_pair(h, l);
-            hi = lane == r ? h : hi;
-            lo = lane == r ? l : lo;
+            warp_sum_pair<kLanes>(h, l);
+            t = (long long)(((unsigned long long)__float_as_uint(h) << 32) | __float_as_uint(l));
         }
+        if (lane % kLanes == 0 && mine < rows) row_sum[warp * rows + mine] = __longlong_as_double(t);
     }
-    double d = 0.0, p = 0.0;
-    if (has) {
-        const double sum = FIX ? (double)exact / sr : (double)hi + (double)lo;
+    __syncthreads();
+    // the block's rows, a thread each
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    const double ad = C.about ? C.about[0] : 0.0, ap = C.about ? C.about[1] : 0.0;
+    for (int i = threadIdx.x; i < kWarps * rows; i += 32 * kWarps) {
+        const long long mine = base + i;
+        if (mine >= n) break;
+        const unsigned long long t = (unsigned long long)__double_as_longlong(row_sum[i]);
+        const double sum = FIX ? (double)(long long)t / sr
+                               : (double)__uint_as_float((uint32_t)(t >> 32)) + (double)__uint_as_float((uint32_t)t);
         const float2 q = bc[mine];
-        const float old = pc[mine];
+        const float old = x[mine];
         double numer = (double)q.x + sum;
         if (seed && p_init) numer += (double)p_init[vox[mine]];
-        const float x = q.y > 0.0f ? (float)(numer / (double)q.y) : old;
-        pn[mine] = x;
-        d = (double)x - (double)old;
-        p = (double)x;
+        const float now = q.y > 0.0f ? (float)(numer / (double)q.y) : old;
+        pn[mine] = now;
+        if (C.red2) {
+            const double d = (double)now - (double)old - ad, p = (double)now - ap;
+            v[0] += d;
+            v[1] += d * d;
+            v[2] += p;
+            v[3] += p * p;
+        }
     }
     if (!C.red2) return;
-    __shared__ double sh[4][kIterThreads / 32];
+    __shared__ double sh[4][kWarps];
     __shared__ bool last;
-    const double ad = C.about ? C.about[0] : 0.0, ap = C.about ? C.about[1] : 0.0;
-    const double dd = has ? d - ad : 0.0, pp = has ? p - ap : 0.0;
-    const double v[4] = {warp_sum_double(dd), warp_sum_double(dd * dd), warp_sum_double(pp), warp_sum_double(pp * pp)};
+    if (warp * 32 < kWarps * rows) {  // whole warps: the others have no rows
+        for (int i = 0; i < 4; i++) v[i] = warp_sum_double(v[i]);
+    }
     if (lane == 0)
         for (int i = 0; i < 4; i++) sh[i][warp] = v[i];
     __syncthreads();
     if (threadIdx.x < 4) {
         double t = 0.0;
-        for (int w = 0; w < kIterThreads / 32; w++) t += sh[threadIdx.x][w];
+        for (int w = 0; w < kWarps; w++) t += sh[threadIdx.x][w];
         C.part[4ull * blockIdx.x + threadIdx.x] = t;
         __threadfence();
     }
@@ -634,7 +632,7 @@ __global__ void __launch_bounds__(kIterThreads) k_anchor_iterate(
     const volatile double *part = C.part;
     const int i = threadIdx.x & 3;
     double t = 0.0;
-    for (unsigned b = threadIdx.x >> 2; b < gridDim.x; b += kIterThreads / 4) t += part[4ull * b + i];
+    for (unsigned b = threadIdx.x >> 2; b < gridDim.x; b += 8 * kWarps) t += part[4ull * b + i];
     for (int o = 16; o >= 4; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);  // lanes 0..3: this warp's four sums
     if (lane < 4) sh[lane][warp] = t;
     __syncthreads();
@@ -642,7 +640,7 @@ __global__ void __launch_bounds__(kIterThreads) k_anchor_iterate(
     double S[4];
     for (int k = 0; k < 4; k++) {
         S[k] = 0.0;
-        for (int w = 0; w < kIterThreads / 32; w++) S[k] += sh[k][w];
+        for (int w = 0; w < kWarps; w++) S[k] += sh[k][w];
     }
     const double N = (double)n;
     double ed = -ad, ep = -ap;  // the shifts about the old ones (none: 0)
@@ -859,7 +857,7 @@ cudaError_t run_pass(const Geometry &geo, const Field &f, int method, bool fb, c
     if (PASS == kMark) ok = ok && S.flag;
     else ok = ok && S.id && S.bc;
     const bool unit_links = method_accum(method) == kAccPlain || method_accum(method) == kAccPlainNoEntry;
-    if (PASS == kFill) ok = ok && S.next && (unit_links ? S.col != nullptr : S.cw != nullptr);
+    if (PASS == kFill) ok = ok && S.next && S.links && (unit_links == (S.kind != kLinkPair));
     if (need_field) ok = ok && (f.lay.wrap ? f.edge != nullptr : f.f32 != nullptr);
     const int acc = method_accum(method);
     const bool weighted = acc == kAccWeighted || acc == kAccWeightedRawCurl;
@@ -903,7 +901,7 @@ cudaError_t grow(T *&p, size_t &cap, size_t bytes)
 void anchor_free(Anchor *A)
 {
     cudaFree(A->flag); cudaFree(A->wid); cudaFree(A->id); cudaFree(A->vox); cudaFree(A->rowptr);
-    cudaFree(A->col); cudaFree(A->cw); cudaFree(A->bc); cudaFree(A->pa); cudaFree(A->pb);
+    cudaFree(A->links); cudaFree(A->bc); cudaFree(A->pa); cudaFree(A->pb);
     cudaFree(A->red); cudaFree(A->rowlen); cudaFree(A->u); cudaFree(A->pos); cudaFree(A->tmp); cudaFree(A->cnt64); cudaFree(A->tmp64);
     cudaFree(A->neg); cudaFree(A->next);
     *A = Anchor();
@@ -971,18 +969,23 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     OM_COUNT_LAUNCH();
     AN_TRY(cudaGetLastError());
 
+    const bool unit_links = method_accum(method) == kAccPlain || method_accum(method) == kAccPlainNoEntry;
     // rows: a voxel receives at most one contribution per line through it, so the
     // geometry-only line counts size the rows and no counting pass is needed
     AN_TRY(ensure_lines_through(&geo, f.lay, scratch, st));
-    AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * (size_t)n));
+    AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * (size_t)(n + 1)));
     AN_TRY(grow(A->tmp64, cap[9], sizeof(unsigned long long) * scan_tmp_elems(n)));
     AN_TRY(grow(A->rowptr, cap[10], sizeof(unsigned long long) * (size_t)(n + 1)));
-    k_row_capacity<<<grid_for(n), 256, 0, st>>>(n, A->vox, geo.d_lines_through, A->cnt64);
+    A->kind = !unit_links ? kLinkPair : (n <= 65536 ? kLink16 : kLink32);
+    AN_TRY(cudaMemsetAsync(A->cnt64 + n, 0, sizeof(unsigned long long), st));
+    k_row_capacity<<<grid_for(n), 256, 0, st>>>(n, A->vox, geo.d_lines_through, (unsigned)links_per_vector(A->kind), A->cnt64,
+                                                A->cnt64 + n);
     OM_COUNT_LAUNCH();
     AN_TRY(cudaGetLastError());
     AN_TRY(exclusive_scan_u64(A->cnt64, A->rowptr, n, A->tmp64, st));
-    unsigned long long nnz = 0;
-    AN_TRY(cudaMemcpyAsync(&nnz, A->rowptr + n, sizeof(nnz), cudaMemcpyDeviceToHost, st));
+    unsigned long long slots = 0, nnz = 0;
+    AN_TRY(cudaMemcpyAsync(&slots, A->rowptr + n, sizeof(slots), cudaMemcpyDeviceToHost, st));
+    AN_TRY(cudaMemcpyAsync(&nnz, A->cnt64 + n, sizeof(nnz), cudaMemcpyDeviceToHost, st));
     AN_TRY(cudaStreamSynchronize(st));
     A->nnz = (long long)nnz;
     if (max_nnz >= 0 && (long long)nnz > max_nnz) {
@@ -990,11 +993,11 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
         return cudaErrorNotSupported;
     }
 
-    const bool unit_links = method_accum(method) == kAccPlain || method_accum(method) == kAccPlainNoEntry;
-    if (unit_links) AN_TRY(grow(A->col, cap[11], sizeof(uint32_t) * (size_t)nnz));
-    else AN_TRY(grow(A->cw, cap[12], sizeof(uint2) * (size_t)nnz));
+    const size_t link_bytes = link_size(A->kind);
+    AN_TRY(grow(A->links, cap[11], link_bytes * (size_t)slots));
     AN_TRY(grow(A->bc, cap[13], sizeof(float2) * (size_t)n));
-    AN_TRY(grow(A->red, cap[6], sizeof(double) * (4 + 4 * (size_t)iter_blocks(std::max<long long>(n, 1)))));
+    AN_TRY(grow(A->red, cap[6], sizeof(double) * (4 + 4 * (size_t)std::max(iter_shape(std::max<long long>(n, 1), true).blocks,
+                                                                                iter_shape(std::max<long long>(n, 1), false).blocks))));
     AN_TRY(grow(A->pa, cap[15], sizeof(float) * (size_t)n));
     AN_TRY(grow(A->pb, cap[16], sizeof(float) * (size_t)n));
     AN_TRY(grow(A->rowlen, cap[17], sizeof(uint32_t) * (size_t)n));
@@ -1003,8 +1006,8 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     AN_TRY(cudaMemsetAsync(A->bc, 0, sizeof(float2) * (size_t)std::max<long long>(n, 1), st));
     S.id = lay.wrap ? A->wid : A->id;
     S.next = A->next;
-    S.col = unit_links ? A->col : nullptr;
-    S.cw = unit_links ? nullptr : A->cw;
+    S.links = A->links;
+    S.kind = A->kind;
     S.bc = A->bc;
     if (fx) {  // bit-reproducible: the rows' (b, c) in fixed point (scales set by the caller)
         AN_TRY(grow(fx->bc64, fx->cap_bc64, sizeof(long long) * 2 * (size_t)std::max<long long>(n, 1)));
@@ -1028,7 +1031,6 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
         }
         AN_TRY(cudaGetLastError());
     }
-    A->unit_weights = method_accum(method) == kAccPlain || method_accum(method) == kAccPlainNoEntry;
     return cudaGetLastError();
 }
 
@@ -1082,7 +1084,7 @@ cudaError_t anchor_mark(const Geometry &geo, const Field &f, int method, long lo
 
 cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, bool first, int gauge, long long ref_anchor,
                         const float *p_cur, float *p_next, double *red2, cudaStream_t st, const ChunkTest *test,
-                        const Fixed *fx)
+                        const Fixed *fx, bool alone)
 {
     if (A.n == 0) return cudaSuccess;
     const int *stop = test ? test->stop : nullptr;
@@ -1111,14 +1113,27 @@ cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, bool fi
             C.rel_out = test->rel_out;
         }
     }
-    auto launch = [&](auto kernel) {
-        kernel<<<iter_blocks(A.n), kIterThreads, 0, st>>>(A.n, iter_rows(A.n), A.rowptr, A.rowlen, A.col, A.cw, A.bc, A.vox,
-                                                          p_init, seed ? 1 : 0, p_cur, p_next, stop, fix, C);
+    const IterShape I = iter_shape(A.n, alone);
+    auto launch = [&](auto wide, auto smem) {
+        auto kernel = I.smem ? smem : wide;
+        if (I.bytes > 48 * 1024) {  // (a host-side attribute of the kernel: cheap, and safe while capturing)
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIterSmemMax);
+            if (e != cudaSuccess) return e;
+        }
+        kernel<<<I.blocks, I.threads, I.bytes, st>>>(A.n, I.rows, A.rowptr, A.rowlen, A.links, A.bc, A.vox, p_init, seed ? 1 : 0,
+                                                     p_cur, p_next, stop, fix, C);
         OM_COUNT_LAUNCH();
+        return cudaGetLastError();
     };
-    if (A.unit_weights) fix ? launch(k_anchor_iterate<true, true>) : launch(k_anchor_iterate<true, false>);
-    else fix ? launch(k_anchor_iterate<false, true>) : launch(k_anchor_iterate<false, false>);
-    return cudaGetLastError();
+#define OM_LAUNCH_ITERATE(KIND) \
+    (fix ? launch(k_anchor_iterate<KIND, true, false>, k_anchor_iterate<KIND, true, true>) \
+         : launch(k_anchor_iterate<KIND, false, false>, k_anchor_iterate<KIND, false, true>))
+    switch (A.kind) {
+    case kLink16: return OM_LAUNCH_ITERATE(kLink16);
+    case kLink32: return OM_LAUNCH_ITERATE(kLink32);
+    default: return OM_LAUNCH_ITERATE(kLinkPair);
+    }
+#undef OM_LAUNCH_ITERATE
 }
 
 cudaError_t anchor_refresh_rhs(const Geometry &geo, const Field &f, Anchor *A, cudaStream_t st,

@@ -1,0 +1,127 @@
+// Rows of the anchor operator and of its transpose, as the iterations read them.
+//
+// A row's links are (index, weight) pairs, one load each, or for unit weights (plain method)
+// 16-byte vectors, the row's start aligned, of four 32-bit indices or of eight 16-bit ones where
+// the operator has at most 2^16 anchors.  The gathered vector is kept in shared memory where it
+// fits: the links of a row point all over the volume's faces, so every lane's 4-byte gather is a
+// sector of its own through L2 (293 G gathers/s) but at worst a bank conflict in shared memory.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace omni3d {
+
+enum LinkKind { kLinkPair = 0, kLink32 = 1, kLink16 = 2 };
+
+// Links per load of a row.
+__host__ __device__ constexpr int links_per_vector(int kind) { return kind == kLinkPair ? 1 : (kind == kLink32 ? 4 : 8); }
+
+// Bytes of a link.
+__host__ __device__ constexpr size_t link_size(int kind) { return kind == kLinkPair ? 8 : (kind == kLink32 ? 4 : 2); }
+
+// Lanes that share a row: a row of the 642-direction operators (about 640 links) is then 10 to
+// 20 loads per lane, four of them in flight, and a warp works on several rows at once.
+__host__ __device__ constexpr int lanes_per_row(int kind) { return kind == kLinkPair ? 32 : (kind == kLink32 ? 16 : 8); }
+
+// add(index, weight) for the links of this lane (of lanes_per_row) of a row of m links at
+// `links` (entry j0, aligned).
+template <int KIND, typename F>
+__device__ __forceinline__ void row_links(const void *links, unsigned long long j0, uint32_t m, int lane, F &&add)
+{
+    constexpr uint32_t S = lanes_per_row(KIND);
+    uint32_t v = lane;
+    if constexpr (KIND == kLinkPair) {
+        const uint2 *q = static_cast<const uint2 *>(links) + j0;
+        for (; v < m; v += 4 * S) {
+            uint2 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (v + u * S < m) x[u] = __ldg(q + v + u * S);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (v + u * S < m) add(x[u].x, __uint_as_float(x[u].y));
+        }
+    } else {
+        constexpr uint32_t W = links_per_vector(KIND);
+        const uint4 *q = static_cast<const uint4 *>(links) + j0 / W;
+        auto at = [](const uint4 &x, uint32_t k) {
+            const uint32_t a[4] = {x.x, x.y, x.z, x.w};
+            return KIND == kLink32 ? a[k] : (a[k / 2] >> (16 * (k & 1))) & 0xffffu;
+        };
+        const uint32_t full = m / W;  // whole vectors
+        for (; v + 3 * S < full; v += 4 * S) {
+            uint4 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = __ldg(q + v + u * S);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+#pragma unroll
+                for (uint32_t k = 0; k < W; k++) add(at(x[u], k), 1.0f);
+        }
+        for (; v < full; v += S) {
+            const uint4 x = __ldg(q + v);
+#pragma unroll
+            for (uint32_t k = 0; k < W; k++) add(at(x, k), 1.0f);
+        }
+        if (v == full && W * full < m) {  // the slots past the row's links hold nothing
+            const uint4 x = __ldg(q + full);
+#pragma unroll
+            for (uint32_t k = 0; k < W; k++)
+                if (W * full + k < m) add(at(x, k), 1.0f);
+        }
+    }
+}
+
+// Store link `slot`.
+template <int KIND>
+__device__ __forceinline__ void store_link(void *links, unsigned long long slot, uint32_t index, float weight)
+{
+    if (KIND == kLinkPair) static_cast<uint2 *>(links)[slot] = make_uint2(index, __float_as_uint(weight));
+    else if (KIND == kLink32) static_cast<uint32_t *>(links)[slot] = index;
+    else static_cast<uint16_t *>(links)[slot] = (uint16_t)index;
+}
+
+// The vector an iteration gathers from: copied into shared memory (SMEM) or read through L1.
+constexpr int kIterSmemMax = 220 * 1024;  // bytes of it: beside the rows' sums, what an SM gives one CTA
+template <bool SMEM>
+__device__ __forceinline__ const float *gather_vector(const float *x, long long n, float *sh)
+{
+    if (!SMEM) return x;
+    const long long n4 = n / 4;  // (the iterates' buffers are 256-byte aligned)
+    for (long long i = threadIdx.x; i < n4; i += blockDim.x)
+        reinterpret_cast<float4 *>(sh)[i] = __ldg(reinterpret_cast<const float4 *>(x) + i);
+    for (long long i = 4 * n4 + threadIdx.x; i < n; i += blockDim.x) sh[i] = __ldg(x + i);
+    __syncthreads();
+    return sh;
+}
+
+// Launch shape of an iteration over n rows: CTAs of 256 threads, or with the vector in shared
+// memory CTAs of 1024 (as many as fit per SM), and rows per warp.  alone: the iteration does not
+// share the GPU with others, as it does in a batch's graph, where kernels that fill the SMs'
+// shared memory keep the members apart (16 plain snapshots: 15.6 ms so, 13.8 without).
+constexpr long long kIterSmemMin = 16384;  // smaller vectors stay in L1 anyway
+struct IterShape {
+    bool smem;
+    int threads, rows;
+    unsigned blocks;
+    size_t bytes;
+};
+constexpr int kIterRowsMax = 16;
+inline IterShape iter_shape(long long n, bool alone)
+{
+    IterShape s{};
+    s.bytes = sizeof(float) * (size_t)n;
+    s.smem = alone && n >= kIterSmemMin && s.bytes <= (size_t)kIterSmemMax;
+    s.threads = s.smem ? 1024 : 256;
+    // one CTA per SM above half of its shared memory, else two (2048 threads per SM)
+    const long long warps = s.smem ? 152LL * 32 * (s.bytes > (size_t)kIterSmemMax / 2 ? 1 : 2) : 152LL * 48;
+    const long long rows = (n + warps - 1) / warps;
+    s.rows = (int)(rows < 1 ? 1 : (rows > kIterRowsMax ? kIterRowsMax : rows));
+    const long long per = (long long)s.rows * (s.threads / 32);
+    s.blocks = (unsigned)((n + per - 1) / per);
+    if (!s.smem) s.bytes = 0;
+    return s;
+}
+
+}  // namespace omni3d

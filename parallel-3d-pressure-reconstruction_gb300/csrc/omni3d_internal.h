@@ -341,14 +341,13 @@ struct Anchor {
     int32_t *wid = nullptr;         // the walks' copies of id (skewed layouts)
     int32_t *id = nullptr;          // V: anchor id or -1
     uint32_t *vox = nullptr;        // n: voxel of anchor
-    unsigned long long *rowptr = nullptr;  // n + 1: row capacities (lines through the voxel)
+    unsigned long long *rowptr = nullptr;  // n + 1: row capacities (lines through the voxel, in whole vectors)
     uint32_t *rowlen = nullptr;     // n: entries in each row
-    uint32_t *col = nullptr;        // nnz, unit weights: the start anchor of each link
-    uint2 *cw = nullptr;            // nnz, other methods: (start anchor, weight bits) of each link
+    void *links = nullptr;          // per link the start anchor and, in weighted operators, the weight
+    int kind = 0;                   // LinkKind of the links (links.cuh)
     float2 *bc = nullptr;           // n: (b, c) = (sum of w * I, sum of w)
     float *pa = nullptr, *pb = nullptr;  // iterates
     double *red = nullptr;          // reduction scratch
-    bool unit_weights = false;      // plain method: every w is 1 (the w array is unused)
     // build scratch (kept between builds)
     uint32_t *u = nullptr, *pos = nullptr, *tmp = nullptr;
     unsigned long long *cnt64 = nullptr, *tmp64 = nullptr;
@@ -382,10 +381,11 @@ struct ChunkTest {
 };
 // One iteration p_next = (b + seed * p_init_a + M p_cur) / c.  With red2 also the gauged change
 // and norm sums red2[0..1] of the relative change over all anchors, and the chunk's test;
-// `first`: the solve's first iteration.
+// `first`: the solve's first iteration; alone: see iter_shape.
 cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, bool first, int gauge,
                         long long ref_anchor, const float *p_cur, float *p_next, double *red2,
-                        cudaStream_t st, const ChunkTest *test = nullptr, const Fixed *fx = nullptr);
+                        cudaStream_t st, const ChunkTest *test = nullptr, const Fixed *fx = nullptr,
+                        bool alone = true);
 // Gauged relative-change sums over the n values selected by mask (all when mask is null):
 // out2 = {sum (d - d_ref)^2, sum (p - p_ref)^2} with d = pn - pc; the shift is the value at
 // `ref` (point gauge), the mean (mean gauge) or zero.  Deterministic FP64 reduction;
@@ -406,11 +406,10 @@ cudaError_t anchor_gather(const Anchor &A, const float *vol, float *pa, cudaStre
 
 // Adjoint of the plain-method solve (kernels_adjoint.cu).
 struct AdjointBuffers {
-    unsigned long long *tptr = nullptr;  // transposed operator (built once per operator)
-    uint32_t *trow = nullptr;
-    float *tw = nullptr;                 // weights of the transposed entries (weighted operators)
-    unsigned long long *tmp = nullptr;
-    float *mu = nullptr, *lam = nullptr, *nxt = nullptr, *acc = nullptr;
+    unsigned long long *tptr = nullptr;  // transposed operator (built once per operator): row starts,
+    uint32_t *tlen = nullptr;            // lengths
+    void *tlinks = nullptr;              // and links, of the operator's kind
+    float *mu = nullptr, *lam = nullptr, *u = nullptr, *unext = nullptr, *acc = nullptr;
 };
 void adjoint_free(AdjointBuffers *B);
 // gx, gy, gz = d<g, p_K>/d(ax, ay, az) for `method` after K iterations with the curl held
