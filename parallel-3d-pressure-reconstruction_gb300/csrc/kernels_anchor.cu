@@ -167,7 +167,7 @@ struct FillLine {
     // I += the trapezoid increment of step q of a batch, or 0 on a lane that does not take it
     __device__ __forceinline__ void integrate(uint32_t c, int q, const float4 &gv, bool t)
     {
-        const float x = step_h(L, c, q) * step_sum<GRAD>(c, q, gv, gl);
+        const float x = step_increment<GRAD>(L, c, q, gv, gl);
         I += t ? x : 0.0f;
         if (GRAD != kGradEdge) gl = gv;
     }
@@ -312,9 +312,9 @@ struct SelectFill : FillLine<GRAD> {
         if (!MASK && FB) {
             float lo, hi;
             curl_range<true>(g, lo, hi);
-            return st.run & (lo > 0.0f) & (hi < thr);
+            return st.run() & (lo > 0.0f) & (hi < thr);
         }
-        bool ok = st.run;
+        bool ok = st.run();
 #pragma unroll
         for (int q = 0; q < kWalkBatch; q++) {
             const float cn = curl_of<FB>(g[q]);
@@ -368,7 +368,7 @@ struct SelectFill : FillLine<GRAD> {
         }
         // the ids of the voxels that are anchors or may start a segment, loaded together
         int32_t rows[kWalkBatch];
-        bool open = !st.run;
+        bool open = !st.run();
 #pragma unroll
         for (int q = 0; q < kWalkBatch; q++) {
             rows[q] = -1;
@@ -403,8 +403,8 @@ k_anchor_select(Grid g, Layout lay, WalkLines W, WalkField F, const float *__res
     if (PASS == kFill) S.id += L.copy;
     SelectState st;
     st.enter(PASS == kFill ? curl_of<FB>(gl) : __ldg(curl + L.v), g.thr);
-    if (PASS == kMark && st.run && L.on) S.flag[L.v] = 1;
-    SelectFill<GRAD, PASS, FB> f{{L, S, gl}, curl, g.thr, st, st.run ? start_col<PASS>(S, L.v) : 0u};
+    if (PASS == kMark && st.run() && L.on) S.flag[L.v] = 1;
+    SelectFill<GRAD, PASS, FB> f{{L, S, gl}, curl, g.thr, st, st.run() ? start_col<PASS>(S, L.v) : 0u};
     walk_steps<kWalkBatch, GRAD, PASS == kFill && !FB>(L, field, S.id, f);
 }
 

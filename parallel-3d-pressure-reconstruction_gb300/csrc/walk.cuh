@@ -24,8 +24,8 @@ namespace omni3d {
 constexpr int kIdle = 3;  // step code of a lane that takes no step
 
 // What a walk gathers per step: nothing; the voxel's float4 (ax, ay, az, curl); or its edge
-// record, the sums of the components over the edges by which a line of the octant enters the
-// voxel along x, y and z, and the curl (k_pack).
+// record, the trapezoid increments by which a line of the octant enters the voxel along x, y
+// and z, and the curl (k_pack).
 enum WalkGrad { kNoGrad = 0, kGradVoxel = 1, kGradEdge = 2 };
 
 // The arrays a walk gathers from.
@@ -60,7 +60,7 @@ struct LineWalk {
     uint32_t v;           // index of the current voxel in the copy
     uint32_t wv;          // added when a step leaves the copy's range (see Layout)
     int d0, d1, d2;       // index strides of a step along x, y, z
-    float h0, h1, h2;     // -rho * sign * spacing / 2 per axis (K:1816, 1825, 1834)
+    float h0, h1, h2;     // -rho * sign * spacing / 2 per axis (K:1816, 1825, 1834; in the edge records already)
     uint32_t e;           // entry voxel, row-major
     uint32_t span;        // steps of the group, idle ones included
     size_t copy;          // first entry of the copy
@@ -132,24 +132,36 @@ __device__ __forceinline__ bool taken(uint32_t idle, int q)
     return !MASK || (idle & (1u << (2 * q))) == 0u;
 }
 
-// x, y or z by the axis of step q.  Written as selections: from conditional expressions the
-// compiler makes a three-way branch, which diverges at almost every step.
+// x, y or z by the axis of step q.  Written as selections by the code's two bits: from
+// conditional expressions the compiler makes a three-way branch, which diverges at almost every
+// step.
 __device__ __forceinline__ uint32_t by_axis(uint32_t c, int q, uint32_t x, uint32_t y, uint32_t z)
 {
     uint32_t r;
-    asm("{\n\t.reg .pred px, py;\n\t.reg .b32 t;\n\t"
+    asm("{\n\t.reg .pred py, pz;\n\t.reg .b32 t, u;\n\t"
         "and.b32 t, %4, %5;\n\t"
-        "setp.eq.u32 px, t, 0;\n\t"
-        "setp.eq.u32 py, t, %6;\n\t"
-        "selp.b32 t, %2, %3, py;\n\t"
-        "selp.b32 %0, %1, t, px;\n\t}"
+        "setp.ne.u32 pz, t, 0;\n\t"
+        "and.b32 u, %4, %6;\n\t"
+        "setp.ne.u32 py, u, 0;\n\t"
+        "selp.b32 t, %2, %1, py;\n\t"
+        "selp.b32 %0, %3, t, pz;\n\t}"
         : "=r"(r)
-        : "r"(x), "r"(y), "r"(z), "r"(c), "r"(3u << (2 * q)), "r"(1u << (2 * q)));
+        : "r"(x), "r"(y), "r"(z), "r"(c), "r"(2u << (2 * q)), "r"(1u << (2 * q)));
     return r;
 }
 __device__ __forceinline__ float by_axis(uint32_t c, int q, float x, float y, float z)
 {
     return __uint_as_float(by_axis(c, q, __float_as_uint(x), __float_as_uint(y), __float_as_uint(z)));
+}
+
+// Address of entry v of an array, as one wide multiply-add: the shifted add that the compiler
+// takes is two instructions on the ALU, the busiest unit of a selected sweep.
+template <typename T>
+__device__ __forceinline__ T *entry(T *base, uint32_t v)
+{
+    uint64_t r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(v), "n"(sizeof(T)), "l"((uint64_t)base));
+    return reinterpret_cast<T *>(r);
 }
 
 // Least and greatest of a batch's curls (the magnitudes with ABS), NaN when one of them is NaN.
@@ -178,16 +190,14 @@ __device__ __forceinline__ void curl_range(const float4 (&g)[B], float &lo, floa
     }
 }
 
-// The trapezoid increment of step q without its coefficient: the sum of the component along
-// the step's axis at both its ends, gv the sample of the voxel it enters and gl that of the
-// voxel before (an edge record holds the sum).
+// The trapezoid increment of step q, gv the sample of the voxel it enters and gl that of the
+// voxel before (an edge record holds the increments of the octant's steps).
 template <int GRAD>
-__device__ __forceinline__ float step_sum(uint32_t c, int q, const float4 &gv, const float4 &gl)
+__device__ __forceinline__ float step_increment(const LineWalk &L, uint32_t c, int q, const float4 &gv, const float4 &gl)
 {
     if (GRAD == kGradEdge) return by_axis(c, q, gv.x, gv.y, gv.z);
-    return by_axis(c, q, gv.x + gl.x, gv.y + gl.y, gv.z + gl.z);
+    return by_axis(c, q, L.h0, L.h1, L.h2) * by_axis(c, q, gv.x + gl.x, gv.y + gl.y, gv.z + gl.z);
 }
-__device__ __forceinline__ float step_h(const LineWalk &L, uint32_t c, int q) { return by_axis(c, q, L.h0, L.h1, L.h2); }
 
 // The array a walk gathers from, at the lane's copy.
 template <int GRAD>
@@ -204,15 +214,12 @@ __device__ __forceinline__ float4 sample(const float4 *field, uint32_t v)
 
 // State of the selected method along a line (K:2280-2537): inside a segment (run), or before
 // the first one or between two (a good voxel then starts one).  The decisions of a step depend
-// on the curl of the voxel it enters alone; written with bitwise operators, they stay in
-// predicate registers.
+// on the curl of the voxel it enters alone.  One integer instead of two flags, which the compiler
+// packs into bits and unpacks at every step: 64^3 sweep 1.29 -> 1.25 ms.
 struct SelectState {
-    bool started, run;
-    __device__ __forceinline__ void enter(float curl, float thr)
-    {
-        started = !(curl == 0.0f || curl > thr);
-        run = started;
-    }
+    int phase;  // 0 before the first segment, 1 inside one, 2 between two
+    __device__ __forceinline__ void enter(float curl, float thr) { phase = (curl == 0.0f || curl > thr) ? 0 : 1; }
+    __device__ __forceinline__ bool run() const { return phase == 1; }
     // A step along x, y or z into a voxel of curl cn, taken when `on`: `add`, it adds to the
     // segment; `start`, a segment (re)starts at the voxel; `clear`, that start also clears the
     // running curl sum and count (a restart on a z step keeps them).
@@ -221,11 +228,11 @@ struct SelectState {
         const bool nz = cn != 0.0f;
         const bool good = (cn < thr) & nz;
         const bool pause = (cn >= thr) | (x & !nz);
-        add = on & run & good;
-        start = on & !run & (good | (!started & nz & !x));
-        clear = start & (!started | x | y);
-        run = (run & !(on & pause)) | start;
-        started = started | start;
+        const bool inside = phase == 1, fresh = phase == 0;
+        add = on & inside & good;
+        start = on & !inside & (good | (fresh & nz & !x));
+        clear = start & (fresh | x | y);
+        phase = start ? 1 : (on & inside & pause ? 2 : phase);
     }
     // Whether the step after a voxel of curl cn can start a segment (it cannot after a voxel
     // that is good: that one is in a segment or starts one).
