@@ -1135,7 +1135,7 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
         for (int it = 1; it <= K; it++) {
             CK(ctx, walk_pressure(ctx, lay, pc, &wp, st));
             if (det) {  // exact fixed-point sums, normalised in FP64
-                Fix2 *accf = reinterpret_cast<Fix2 *>(acc64);
+                long long *accf = reinterpret_cast<long long *>(acc64);
                 CK(ctx, fix_sweep_scales(V, pc, *fx, st));
                 CK(ctx, init_accum_fix(g, lay, dpinit, seed && it == 1, *fx, accf, st));
                 cudaEventRecord(ctx->ev[5], st);
@@ -1220,7 +1220,7 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
         }
         if (det) {  // bit-reproducible: exact fixed-point sums, normalised in FP64
             CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)lay.copies * (size_t)V));
-            Fix2 *accf = reinterpret_cast<Fix2 *>(ctx->pncnt64.p);
+            long long *accf = ctx->pncnt64.as<long long>();
             CK(ctx, fix_sweep_scales(V, vol, *fx, st));
             CK(ctx, init_accum_fix(g, lay, dpinit, seed && its == 0, *fx, accf, st));
             cudaEventRecord(ctx->ev[5], st);

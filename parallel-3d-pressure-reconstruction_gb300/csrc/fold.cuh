@@ -60,21 +60,28 @@ __device__ __forceinline__ void fold_add(float2 &a, const float2 &b) { a.x += b.
 __device__ __forceinline__ void fold_add(double2 &a, const double2 &b) { a.x += b.x; a.y += b.y; }
 __device__ __forceinline__ void fold_add(uint32_t &a, const uint32_t &b) { a += b; }
 
+template <typename T>
+__device__ __forceinline__ T fold_load(const T *in, size_t i)
+{
+    return __ldg(in + i);
+}
+
 // f(voxel, sum of the copies' entries of it) for every voxel; the copies are added in the order
 // of their classes.  256^3, float2: 0.45 -> 0.33 ms against one gather per voxel and copy.
-template <typename T, typename F>
-__global__ void __launch_bounds__(kTileThreads) k_fold(Grid g, Layout lay, const T *__restrict__ in, F f)
+template <typename IN, typename F>
+__global__ void __launch_bounds__(kTileThreads) k_fold(Grid g, Layout lay, IN in, F f)
 {
+    using T = decltype(fold_load(in, 0));
     __shared__ T tile[kTile * kTile];
     const TileAt at(g);
     if (!lay.wrap) {
-        at.rows(g, [&](int, long long v, int, int) { f(v, in[v]); });
+        at.rows(g, [&](int, long long v, int, int) { f(v, fold_load(in, (size_t)v)); });
         return;
     }
     for (int c = 0; c < 4; c++) {
-        const T *copy = in + (size_t)c * (size_t)lay.stride;
+        const size_t copy = (size_t)c * (size_t)lay.stride;
         at.diagonals(g, lay, c, [&](int p, uint32_t q) {
-            T x = copy[q];
+            T x = fold_load(in, copy + q);
             if (c) {
                 T s = tile[p];
                 fold_add(s, x);

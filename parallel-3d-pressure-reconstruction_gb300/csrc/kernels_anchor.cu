@@ -96,7 +96,7 @@ __device__ __forceinline__ void emit_w(const Sink &S, int row, uint32_t scol, fl
     if (row < 0) return;  // not an anchor after all: nothing to index
     if (PASS == kFill && (int)scol < 0) return;  // a start that is no anchor: no column to link
     if (PASS == kRhs) {  // plain method, operator cached: only b = sum I is field-dependent
-        if (S.bc64) fix_add(S.bc64 + 2 * row, I, S.fix[kFixB]);
+        if (S.bc64) fix_add(S.bc64 + 2 * row, I, fix_scale(S.fix[kFixB]));
         else atomicAdd(&S.bc[row].x, I);
         return;
     }
@@ -106,8 +106,8 @@ __device__ __forceinline__ void emit_w(const Sink &S, int row, uint32_t scol, fl
     else if (S.kind == kLink16) store_link<kLink16>(S.links, slot, scol, wt);
     else store_link<kLink32>(S.links, slot, scol, wt);
     if (S.bc64) {  // bit-reproducible: exact, order-independent fixed-point row sums
-        fix_add(S.bc64 + 2 * row, bt, S.fix[kFixB]);
-        fix_add(S.bc64 + 2 * row + 1, ct, S.fix[kFixC]);
+        fix_add(S.bc64 + 2 * row, bt, fix_scale(S.fix[kFixB]));
+        fix_add(S.bc64 + 2 * row + 1, ct, fix_scale(S.fix[kFixC]));
     } else {
         atomicAdd(S.bc + row, make_float2(bt, ct));
     }
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iter
         ptr = rowptr[row0 + lane];
         len = rowlen[row0 + lane];
     }
-    const double sr = FIX ? fix[kFixRow] : 1.0;
+    const FixScale sr = FIX ? fix_scale(fix[kFixRow]) : FixScale{};
     for (int r = 0; r < rows; r += kRows) {
         if (row0 + r >= n) break;  // whole warps
         const int mine = r + lane / kLanes;  // (lanes past the last row have length 0)
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iter
         const long long mine = base + i;
         if (mine >= n) break;
         const unsigned long long t = (unsigned long long)__double_as_longlong(row_sum[i]);
-        const double sum = FIX ? (double)(long long)t / sr
+        const double sum = FIX ? (double)(long long)t / fix[kFixRow]
                                : (double)__uint_as_float((uint32_t)(t >> 32)) + (double)__uint_as_float((uint32_t)t);
         const float2 q = bc[mine];
         const float old = x[mine];

@@ -135,9 +135,9 @@ __global__ void k_rows_to_float(long long n, const long long *__restrict__ bc64,
 }
 
 // The seed of a sweep that accumulates on top of p_init: into the first copy.
-__global__ void k_seed_fix(Grid g, Layout lay, const float *__restrict__ p_init, const double *__restrict__ scale, Fix2 *acc)
+__global__ void k_seed_fix(Grid g, Layout lay, const float *__restrict__ p_init, const double *__restrict__ scale, long long *pn)
 {
-    const double sp = scale[kFixPn];
+    const FixScale sp = fix_scale(scale[kFixPn]);
     const long long V = g.V;
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
         size_t at = (size_t)v;
@@ -145,7 +145,7 @@ __global__ void k_seed_fix(Grid g, Layout lay, const float *__restrict__ p_init,
             const VoxelAt q(g, v);
             at = layout_index(lay, g.X, g.Y, 0, q.i, q.j, q.k);
         }
-        acc[at].pn = (long long)fix_term(p_init[v], sp);
+        pn[at] = (long long)fix_term(p_init[v], sp);
     }
 }
 
@@ -207,20 +207,20 @@ cudaError_t fix_rows_to_float(long long n, const Fixed &fx, float2 *bc, bool kee
     return cudaGetLastError();
 }
 
-cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, Fix2 *acc,
+cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, long long *acc,
                            cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(acc, 0, sizeof(Fix2) * (size_t)lay.copies * (size_t)g.V, st);
+    cudaError_t e = cudaMemsetAsync(acc, 0, 2 * sizeof(long long) * (size_t)lay.copies * (size_t)g.V, st);
     if (e != cudaSuccess || !seed || !p_init) return e;
     k_seed_fix<<<grid_for(g.V), 256, 0, st>>>(g, lay, p_init, fx.scale, acc);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
 
-cudaError_t normalize_fix(const Grid &g, const Layout &lay, const Fix2 *acc, const Fixed &fx, const float *p_keep,
+cudaError_t normalize_fix(const Grid &g, const Layout &lay, const long long *acc, const Fixed &fx, const float *p_keep,
                           float *p_out, float *cnt_out, cudaStream_t st)
 {
-    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, acc, NormalizeFix{fx.scale, p_keep, p_out, cnt_out});
+    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, FixSums{acc, acc + (size_t)lay.copies * (size_t)g.V}, NormalizeFix{fx.scale, p_keep, p_out, cnt_out});
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }

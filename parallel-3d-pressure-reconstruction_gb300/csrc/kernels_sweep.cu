@@ -39,33 +39,37 @@ namespace {
 
 // Contributions into the (pn, count) accumulators: one FP32 vector reduction, (the FP64
 // defect-correction sweep) two FP64 reductions, each a native L2 atomic, or (the
-// bit-reproducible mode) two 64-bit fixed-point additions with the scales fs.
-struct FixScale {
-    double pn = 0.0, cnt = 0.0;
+// bit-reproducible mode) two 64-bit fixed-point additions.
+template <typename ACC>
+struct Scales {};
+template <>
+struct Scales<long long> {
+    FixScale pn, cnt;
+    long long *counts;  // the lane's copy
 };
 template <typename ACC>
-__device__ __forceinline__ FixScale load_fix(const double *fix)
+__device__ __forceinline__ Scales<ACC> load_scales(const double *fix, ACC *copy, size_t n)
 {
-    FixScale f;
-    if (std::is_same<ACC, Fix2>::value && fix) {
-        f.pn = fix[kFixPn];
-        f.cnt = fix[kFixCnt];
-    }
-    return f;
+    if constexpr (std::is_same<ACC, long long>::value)
+        return {fix_scale(fix[kFixPn]), fix_scale(fix[kFixCnt]), copy + n};
+    else return {};
 }
-__device__ __forceinline__ void acc_add(const FixScale &, float2 *a, float x, float y)
+__device__ __forceinline__ void acc_add(const Scales<float2> &, float2 *acc, uint32_t v, float x, float y)
 {
+    float2 *a = entry(acc, v);
     asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(__cvta_generic_to_global(a)), "f"(x), "f"(y) : "memory");
 }
-__device__ __forceinline__ void acc_add(const FixScale &, double2 *a, float x, float y)
+__device__ __forceinline__ void acc_add(const Scales<double2> &, double2 *acc, uint32_t v, float x, float y)
 {
-    atomicAdd(&a->x, (double)x);
-    atomicAdd(&a->y, (double)y);
+    double2 *a = entry(acc, v);
+    const size_t g = __cvta_generic_to_global(a);
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(g), "d"((double)x) : "memory");
+    asm volatile("red.global.add.f64 [%0 + 8], %1;" ::"l"(g), "d"((double)y) : "memory");
 }
-__device__ __forceinline__ void acc_add(const FixScale &fs, Fix2 *a, float x, float y)
+__device__ __forceinline__ void acc_add(const Scales<long long> &s, long long *acc, uint32_t v, float x, float y)
 {
-    fix_add(&a->pn, x, fs.pn);
-    fix_add(&a->cnt, y, fs.cnt);
+    fix_add(entry(acc, v), x, s.pn);
+    fix_add(entry(s.counts, v), y, s.cnt);
 }
 
 __device__ __forceinline__ void kahan_add(float &s, float &c, float x)
@@ -93,13 +97,13 @@ template <int GRAD, typename ACC>
 struct LineSum {
     const LineWalk &L;
     ACC *acc;          // the lane's copy
-    const FixScale fs;
+    const Scales<ACC> scales;
     float4 gl;         // sample of the last voxel
     float I = 0.0f, comp = 0.0f;
 
     __device__ __forceinline__ void add(uint32_t v, float x, float y) const
     {
-        acc_add(fs, entry(acc, v), x, y);
+        acc_add(scales, acc, v, x, y);
     }
     // I += the trapezoid increment of step q of a batch, or 0 on a lane that does not take it
     // (`t` false: the lane's line is not in the volume, so that its sums are still zero or not
@@ -149,7 +153,7 @@ k_sweep_plain(Grid g, Layout lay, WalkLines W,
     LineWalk L;
     if (!L.init(g, lay, W)) return;
     const float4 *field = lane_field<GRAD>(F, lay, L);
-    PlainWalk<GRAD, ACC> f{{L, pncnt + L.copy, load_fix<ACC>(fix), sample<GRAD>(field, L.v)}, __ldg(p + L.copy + L.v)};
+    PlainWalk<GRAD, ACC> f{{L, pncnt + L.copy, load_scales(fix, pncnt + L.copy, (size_t)lay.copies * (size_t)g.V), sample<GRAD>(field, L.v)}, __ldg(p + L.copy + L.v)};
     if (SELF && L.on) f.add(L.v, f.pe, 1.0f);
     walk_steps<kWalkBatch, GRAD, false>(L, field, nullptr, f);
 }
@@ -221,7 +225,7 @@ k_sweep_weighted(Grid g, Layout lay, WalkLines W,
     LineWalk L;
     if (!L.init(g, lay, W)) return;
     const float4 *field = lane_field<GRAD>(F, lay, L);
-    WeightedWalk<GRAD, RAW, ACC> f{{L, pncnt + L.copy, load_fix<ACC>(fix), sample<GRAD>(field, L.v)},
+    WeightedWalk<GRAD, RAW, ACC> f{{L, pncnt + L.copy, load_scales(fix, pncnt + L.copy, (size_t)lay.copies * (size_t)g.V), sample<GRAD>(field, L.v)},
                                    __ldg(p + L.copy + L.v), 0.0f, 0.0f};
     if (RAW) {
         f.csum = f.gl.w;
@@ -326,7 +330,7 @@ k_sweep_select(Grid g, Layout lay, WalkLines W,
     const float4 gl = sample<GRAD>(field, L.v);
     SelectState st;
     st.enter(gl.w, g.thr);
-    SelectWalk<GRAD, ACC> f{{L, pncnt + L.copy, load_fix<ACC>(fix), gl}, p, g.thr, st,
+    SelectWalk<GRAD, ACC> f{{L, pncnt + L.copy, load_scales(fix, pncnt + L.copy, (size_t)lay.copies * (size_t)g.V), gl}, p, g.thr, st,
                             st.run() ? __ldg(p + L.v) : 0.0f};
     walk_steps<kWalkBatch, GRAD, false>(L, field, nullptr, f);
 }
@@ -642,7 +646,7 @@ cudaError_t sweep_full64(const Geometry &geo, const Field &f, int method, const 
     return sweep_full_t(geo, f, method, p, pncnt, st);
 }
 
-cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, Fix2 *pncnt,
+cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, long long *pncnt,
                            const double *scale, cudaStream_t st)
 {
     if (!scale) return cudaErrorInvalidValue;

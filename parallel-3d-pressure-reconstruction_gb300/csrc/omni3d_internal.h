@@ -288,8 +288,7 @@ cudaError_t init_accum64(const Grid &g, const Layout &lay, const float *p_init, 
                          cudaStream_t st);
 // The same sweep accumulated in 64-bit fixed point (the bit-reproducible mode), with the
 // voxel scales scale[kFixPn], scale[kFixCnt] (fixed.cuh).
-struct Fix2;
-cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, Fix2 *pncnt,
+cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, long long *pncnt,
                            const double *scale, cudaStream_t st);
 cudaError_t normalize64(const Grid &g, const Layout &lay, const double2 *pncnt, const float *p_keep, float *p_out,
                         float *cnt_out, cudaStream_t st);
@@ -329,9 +328,8 @@ cudaError_t fix_sweep_scales(long long V, const float *vol, const Fixed &fx, cud
 cudaError_t fix_rows_to_float(long long n, const Fixed &fx, float2 *bc, bool keep_c, cudaStream_t st);
 // Fixed-point voxel sums: init (pn = seed ? p_init : 0, count = 0), one full sweep,
 // normalisation (p = pn / count where count > 0, else p_keep) -- in FP64 from the exact sums.
-struct Fix2;
-cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, Fix2 *acc, cudaStream_t st);
-cudaError_t normalize_fix(const Grid &g, const Layout &lay, const Fix2 *acc, const Fixed &fx, const float *p_keep, float *p_out,
+cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, long long *acc, cudaStream_t st);
+cudaError_t normalize_fix(const Grid &g, const Layout &lay, const long long *acc, const Fixed &fx, const float *p_keep, float *p_out,
                           float *cnt_out, cudaStream_t st);
 
 // Anchor operator (kernels_anchor.cu).
