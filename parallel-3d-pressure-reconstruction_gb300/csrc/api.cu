@@ -1357,8 +1357,8 @@ int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *
         gy = gx + V;
         gz = gy + V;
     }
-    CK(ctx, adjoint_solve(ctx->geo, ctx->anc, &ctx->adj, ctx->last_iterations, P.method, ctx->f32.as<float4>(), gg,
-                          ctx->cnt.as<float>(), gx, gy, gz, st));
+    CK(ctx, adjoint_solve(ctx->geo, ctx->anc, &ctx->adj, ctx->last_iterations, P.method, ctx->f32.as<float4>(),
+                          ctx->lay, ctx->pw.as<float>(), gg, ctx->cnt.as<float>(), gx, gy, gz, st));
     if (!dev) {
         CK(ctx, cudaMemcpyAsync(grad_ax, gx, sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, st));
         CK(ctx, cudaMemcpyAsync(grad_ay, gy, sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, st));
