@@ -393,10 +393,19 @@ Layout engine_layout(int engine, const Field &F)
 
 // One full sweep with the chosen engine; p and acc in engine_layout.
 cudaError_t engine_sweep(omni3d_ctx *ctx, int engine, const Field &F, int method, const float *p,
-                         float2 *acc, cudaStream_t st)
+                         const Sums<float> &acc, cudaStream_t st)
 {
-    if (engine == OMNI3D_ENGINE_BRICKS) return brick_sweep(ctx->geo, &ctx->bricks, method, p, acc, st);
+    if (engine == OMNI3D_ENGINE_BRICKS)
+        return brick_sweep(ctx->geo, &ctx->bricks, method, p, reinterpret_cast<float2 *>(acc.mem), st);
     return sweep_full(ctx->geo, F, method, p, acc, st);
+}
+
+// The sums of a sweep in layout lay.
+template <typename T>
+Sums<T> sweep_sums(const omni3d_ctx *ctx, const Layout &lay, const DeviceBuf &mem)
+{
+    const bool counted = lay.wrap && method_accum(ctx->prm.method) == kAccPlain;
+    return Sums<T>{mem.as<T>(), counted ? ctx->geo.d_lines_through : nullptr};
 }
 
 // The pressure copies of a row-major volume p for a sweep in layout lay (p itself when row-major).
@@ -462,7 +471,7 @@ cudaError_t enqueue_prepared(omni3d_ctx *ctx, const float *dax, const float *day
                              nullptr, nullptr, false)) != cudaSuccess) return e;
         std::swap(pc, pn);
     }
-    float2 *acc = ctx->pncnt.as<float2>();
+    const Sums<float> acc = sweep_sums<float>(ctx, F.lay, ctx->pncnt);
     float *vol = ctx->pw.as<float>(), *dout = ctx->pout.as<float>(), *dcnt = ctx->cnt.as<float>();
     if (K == 0) {
         if ((e = cudaMemcpyAsync(dout, dpinit, sizeof(float) * (size_t)V, cudaMemcpyDeviceToDevice, st))) return e;
@@ -575,9 +584,9 @@ cudaError_t tune_line_order(omni3d_ctx *ctx, std::string *err)
         Field F;
         F.f32 = field;
         F.lay = row_major_layout(g);
-        e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, p, acc, ctx->st);  // warm-up
+        e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, p, Sums<float>{(float *)acc}, ctx->st);  // warm-up
         cudaEventRecord(ctx->ev[2], ctx->st);
-        if (e == cudaSuccess) e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, p, acc, ctx->st);
+        if (e == cudaSuccess) e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, p, Sums<float>{(float *)acc}, ctx->st);
         cudaEventRecord(ctx->ev[3], ctx->st);
         if (e == cudaSuccess) e = cudaEventSynchronize(ctx->ev[3]);
         const float ms = ms_between(ctx->ev[2], ctx->ev[3]);
@@ -883,13 +892,13 @@ int sweep_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
     if (ctx->geo.walk_rule == 3) CK(ctx, run_walk(&ctx->geo, 3, F.curl, ctx->st));  // paths follow this field
     const float *dp, *wp;
     if ((rc = stage(ctx, p, dev, ctx->in_pinit, V, &dp))) return rc;
-    float2 *acc = ctx->pncnt.as<float2>();
     const bool bf16 = ctx->prm.grad_storage == OMNI3D_GRAD_BF16;
     int engine = choose_engine(ctx, bf16, &rc);
     if (rc) return rc;
     if ((rc = engine_prepare(ctx, &engine, F, ctx->prm.method))) return rc;
     const Layout lay = engine_layout(engine, F);
     CK(ctx, walk_pressure(ctx, lay, dp, &wp, ctx->st));
+    const Sums<float> acc = sweep_sums<float>(ctx, lay, ctx->pncnt);
     CK(ctx, init_accum(g, lay, nullptr, false, acc, ctx->st));
     CK(ctx, engine_sweep(ctx, engine, F, ctx->prm.method, wp, acc, ctx->st));
     // add (pn, count) to the caller's arrays
@@ -1040,7 +1049,6 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
     CK(ctx, ctx->cnt.ensure(sizeof(float) * (size_t)V));
     CK(ctx, ctx->pvol_a.ensure(sizeof(float) * (size_t)V));
     CK(ctx, ctx->scratch.ensure(sizeof(double) * std::max(change_scratch_doubles(), gauge_scratch_doubles()) + 64));
-    float2 *acc = ctx->pncnt.as<float2>();
     float *dout = ctx->pout.as<float>(), *dcnt = ctx->cnt.as<float>();
     double *scratch = ctx->scratch.as<double>();
     double *red2 = scratch;  // 2 doubles, then the reduction scratch
@@ -1127,28 +1135,26 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
                                 st));
         }
         cudaEventRecord(ctx->ev[1], st);
-        double2 *acc64 = nullptr;
-        if (P.sweep_fp64 || det) {
-            CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)lay.copies * (size_t)V));
-            acc64 = ctx->pncnt64.as<double2>();
-        }
+        if (P.sweep_fp64 || det) CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)lay.copies * (size_t)V));
         for (int it = 1; it <= K; it++) {
             CK(ctx, walk_pressure(ctx, lay, pc, &wp, st));
             if (det) {  // exact fixed-point sums, normalised in FP64
-                long long *accf = reinterpret_cast<long long *>(acc64);
+                const Sums<long long> accf = sweep_sums<long long>(ctx, lay, ctx->pncnt64);
                 CK(ctx, fix_sweep_scales(V, pc, *fx, st));
                 CK(ctx, init_accum_fix(g, lay, dpinit, seed && it == 1, *fx, accf, st));
                 cudaEventRecord(ctx->ev[5], st);
                 CK(ctx, sweep_full_fix(ctx->geo, F, P.method, wp, accf, fx->scale, st));
                 cudaEventRecord(ctx->ev[6], st);
                 CK(ctx, normalize_fix(g, lay, accf, *fx, pc, pn, dcnt, st));
-            } else if (acc64) {
+            } else if (P.sweep_fp64) {
+                const Sums<double> acc64 = sweep_sums<double>(ctx, lay, ctx->pncnt64);
                 CK(ctx, init_accum64(g, lay, dpinit, seed && it == 1, acc64, st));
                 cudaEventRecord(ctx->ev[5], st);
                 CK(ctx, sweep_full64(ctx->geo, F, P.method, wp, acc64, st));
                 cudaEventRecord(ctx->ev[6], st);
                 CK(ctx, normalize64(g, lay, acc64, pc, pn, dcnt, st));
             } else {
+                const Sums<float> acc = sweep_sums<float>(ctx, lay, ctx->pncnt);
                 CK(ctx, init_accum(g, lay, dpinit, seed && it == 1, acc, st));
                 cudaEventRecord(ctx->ev[5], st);
                 CK(ctx, engine_sweep(ctx, engine, F, P.method, wp, acc, st));
@@ -1220,7 +1226,7 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
         }
         if (det) {  // bit-reproducible: exact fixed-point sums, normalised in FP64
             CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)lay.copies * (size_t)V));
-            long long *accf = ctx->pncnt64.as<long long>();
+            const Sums<long long> accf = sweep_sums<long long>(ctx, lay, ctx->pncnt64);
             CK(ctx, fix_sweep_scales(V, vol, *fx, st));
             CK(ctx, init_accum_fix(g, lay, dpinit, seed && its == 0, *fx, accf, st));
             cudaEventRecord(ctx->ev[5], st);
@@ -1229,13 +1235,14 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
             CK(ctx, normalize_fix(g, lay, accf, *fx, dpinit, dout, dcnt, st));
         } else if (P.sweep_fp64) {  // the defect-correction sweep: FP64 sums and normalisation
             CK(ctx, ctx->pncnt64.ensure(sizeof(double2) * (size_t)lay.copies * (size_t)V));
-            double2 *acc64 = ctx->pncnt64.as<double2>();
+            const Sums<double> acc64 = sweep_sums<double>(ctx, lay, ctx->pncnt64);
             CK(ctx, init_accum64(g, lay, dpinit, seed && its == 0, acc64, st));
             cudaEventRecord(ctx->ev[5], st);
             CK(ctx, sweep_full64(ctx->geo, F, P.method, wp, acc64, st));
             cudaEventRecord(ctx->ev[6], st);
             CK(ctx, normalize64(g, lay, acc64, dpinit, dout, dcnt, st));
         } else {
+            const Sums<float> acc = sweep_sums<float>(ctx, lay, ctx->pncnt);
             CK(ctx, init_accum(g, lay, dpinit, seed && its == 0, acc, st));
             cudaEventRecord(ctx->ev[5], st);
             CK(ctx, engine_sweep(ctx, engine, F, P.method, wp, acc, st));

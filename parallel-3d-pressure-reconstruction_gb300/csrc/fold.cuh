@@ -56,6 +56,9 @@ struct TileAt {
     }
 };
 
+__device__ __forceinline__ void fold_add(float &a, const float &b) { a += b; }
+__device__ __forceinline__ void fold_add(double &a, const double &b) { a += b; }
+__device__ __forceinline__ void fold_add(long long &a, const long long &b) { a += b; }
 __device__ __forceinline__ void fold_add(float2 &a, const float2 &b) { a.x += b.x; a.y += b.y; }
 __device__ __forceinline__ void fold_add(double2 &a, const double2 &b) { a.x += b.x; a.y += b.y; }
 __device__ __forceinline__ void fold_add(uint32_t &a, const uint32_t &b) { a += b; }

@@ -153,13 +153,15 @@ struct NormalizeFix {
     const double *scale;
     const float *p_keep;
     float *p_out, *cnt_out;
-    __device__ __forceinline__ void operator()(long long v, const Fix2 &a) const
+    const uint32_t *through;  // the counts where pn alone was summed
+    __device__ __forceinline__ void put(long long v, long long pn, double c) const
     {
-        const double c = (double)a.cnt / scale[kFixCnt];
         const float pk = p_keep ? p_keep[v] : 0.0f;
-        if (p_out) p_out[v] = c > 0.0 ? (float)(((double)a.pn / scale[kFixPn]) / c) : pk;
+        if (p_out) p_out[v] = c > 0.0 ? (float)(((double)pn / scale[kFixPn]) / c) : pk;
         if (cnt_out) cnt_out[v] = (float)c;
     }
+    __device__ __forceinline__ void operator()(long long v, const Fix2 &a) const { put(v, a.pn, (double)a.cnt / scale[kFixCnt]); }
+    __device__ __forceinline__ void operator()(long long v, long long pn) const { put(v, pn, (double)through[v]); }
 };
 
 }  // namespace
@@ -207,20 +209,22 @@ cudaError_t fix_rows_to_float(long long n, const Fixed &fx, float2 *bc, bool kee
     return cudaGetLastError();
 }
 
-cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, long long *acc,
+cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, const Sums<long long> &s,
                            cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(acc, 0, 2 * sizeof(long long) * (size_t)lay.copies * (size_t)g.V, st);
+    cudaError_t e = cudaMemsetAsync(s.mem, 0, (s.through ? 1 : 2) * sizeof(long long) * (size_t)lay.copies * (size_t)g.V, st);
     if (e != cudaSuccess || !seed || !p_init) return e;
-    k_seed_fix<<<grid_for(g.V), 256, 0, st>>>(g, lay, p_init, fx.scale, acc);
+    k_seed_fix<<<grid_for(g.V), 256, 0, st>>>(g, lay, p_init, fx.scale, s.mem);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
 
-cudaError_t normalize_fix(const Grid &g, const Layout &lay, const long long *acc, const Fixed &fx, const float *p_keep,
+cudaError_t normalize_fix(const Grid &g, const Layout &lay, const Sums<long long> &s, const Fixed &fx, const float *p_keep,
                           float *p_out, float *cnt_out, cudaStream_t st)
 {
-    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, FixSums{acc, acc + (size_t)lay.copies * (size_t)g.V}, NormalizeFix{fx.scale, p_keep, p_out, cnt_out});
+    const NormalizeFix f{fx.scale, p_keep, p_out, cnt_out, s.through};
+    if (s.through) k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, (const long long *)s.mem, f);
+    else k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, FixSums{s.mem, s.mem + (size_t)lay.copies * (size_t)g.V}, f);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }

@@ -37,9 +37,12 @@ constexpr int kSweepThreads = 64, kSweepBlocks = 16;  // threads per CTA, CTAs p
 
 namespace {
 
-// Contributions into the (pn, count) accumulators: one FP32 vector reduction, (the FP64
-// defect-correction sweep) two FP64 reductions, each a native L2 atomic, or (the
-// bit-reproducible mode) two 64-bit fixed-point additions.
+// Contributions into the accumulators.  ACC float2: (pn, count), one FP32 vector reduction;
+// double2: the FP64 defect-correction sweep's, two FP64 reductions; long long: the
+// bit-reproducible mode's, two 64-bit fixed-point additions; float, double, unsigned long long:
+// the same with pn alone.  All are stated as reductions: entry() hides from the compiler that the
+// address is global, and of an atomicAdd it would make an atomic with a result (a plain sweep at
+// 128^3: 6.4 ms so with pn alone, 5.0 as a reduction; 5.6 with the counts).
 template <typename ACC>
 struct Scales {};
 template <>
@@ -47,11 +50,16 @@ struct Scales<long long> {
     FixScale pn, cnt;
     long long *counts;  // the lane's copy
 };
+template <>
+struct Scales<unsigned long long> {
+    FixScale pn;
+};
 template <typename ACC>
 __device__ __forceinline__ Scales<ACC> load_scales(const double *fix, ACC *copy, size_t n)
 {
     if constexpr (std::is_same<ACC, long long>::value)
         return {fix_scale(fix[kFixPn]), fix_scale(fix[kFixCnt]), copy + n};
+    else if constexpr (std::is_same<ACC, unsigned long long>::value) return {fix_scale(fix[kFixPn])};
     else return {};
 }
 __device__ __forceinline__ void acc_add(const Scales<float2> &, float2 *acc, uint32_t v, float x, float y)
@@ -70,6 +78,19 @@ __device__ __forceinline__ void acc_add(const Scales<long long> &s, long long *a
 {
     fix_add(entry(acc, v), x, s.pn);
     fix_add(entry(s.counts, v), y, s.cnt);
+}
+
+__device__ __forceinline__ void acc_add(const Scales<float> &, float *acc, uint32_t v, float x, float)
+{
+    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(entry(acc, v))), "f"(x) : "memory");
+}
+__device__ __forceinline__ void acc_add(const Scales<double> &, double *acc, uint32_t v, float x, float)
+{
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(entry(acc, v))), "d"((double)x) : "memory");
+}
+__device__ __forceinline__ void acc_add(const Scales<unsigned long long> &s, unsigned long long *acc, uint32_t v, float x, float)
+{
+    fix_add(reinterpret_cast<long long *>(entry(acc, v)), x, s.pn);
 }
 
 __device__ __forceinline__ void kahan_add(float &s, float &c, float x)
@@ -350,6 +371,21 @@ struct Normalize {
     static __device__ __forceinline__ float quotient(const double2 &a) { return (float)(a.x / a.y); }
 };
 
+// f(v, (pn, count)) of sums of pn alone, the counts known.
+template <typename ACC, typename F>
+struct Counted {
+    F f;
+    const uint32_t *through;
+    template <typename T>
+    __device__ __forceinline__ void operator()(long long v, T pn) const
+    {
+        ACC a;
+        a.x = pn;
+        a.y = (T)through[v];
+        f(v, a);
+    }
+};
+
 struct AddTo {
     float *pn, *cnt;
     __device__ __forceinline__ void operator()(long long v, const float2 &a) const
@@ -358,6 +394,11 @@ struct AddTo {
         cnt[v] += a.y;
     }
 };
+
+__device__ __forceinline__ float &pn_of(float &a) { return a; }
+__device__ __forceinline__ float &pn_of(float2 &a) { return a.x; }
+__device__ __forceinline__ double &pn_of(double &a) { return a; }
+__device__ __forceinline__ double &pn_of(double2 &a) { return a.x; }
 
 // The seed of a sweep that accumulates on top of p_init: into the first copy.
 template <typename ACC>
@@ -371,7 +412,7 @@ __global__ void k_seed_accum(Grid g, Layout lay, const float *__restrict__ p_ini
             const VoxelAt q(g, v);
             at = layout_index(lay, g.X, g.Y, 0, q.i, q.j, q.k);
         }
-        pncnt[at].x = p_init[v];
+        pn_of(pncnt[at]) = p_init[v];
     }
 }
 
@@ -622,35 +663,43 @@ cudaError_t sweep_full_t(const Geometry &geo, const Field &f, int method, const 
         kernel<<<blocks, kSweepThreads, 0, st>>>(geo.grid, f.lay, W, F, p, pncnt, fix);
         OM_COUNT_LAUNCH();
     };
-    switch (method_accum(method)) {
-    case kAccWeighted: launch(k_sweep_weighted<kGradEdge, false, ACC>, k_sweep_weighted<kGradVoxel, false, ACC>); break;
-    case kAccWeightedRawCurl: launch(k_sweep_weighted<kGradEdge, true, ACC>, k_sweep_weighted<kGradVoxel, true, ACC>); break;
-    case kAccSelect: launch(k_sweep_select<kGradEdge, ACC>, k_sweep_select<kGradVoxel, ACC>); break;
-    case kAccPlainNoEntry: launch(k_sweep_plain<kGradEdge, false, ACC>, k_sweep_plain<kGradVoxel, false, ACC>); break;
-    default: launch(k_sweep_plain<kGradEdge, true, ACC>, k_sweep_plain<kGradVoxel, true, ACC>); break;
+    if constexpr (std::is_same<ACC, float>::value || std::is_same<ACC, double>::value || std::is_same<ACC, unsigned long long>::value) {
+        if (method_accum(method) != kAccPlain) return cudaErrorInvalidValue;  // the other methods' counts are sums of weights
+        launch(k_sweep_plain<kGradEdge, true, ACC>, k_sweep_plain<kGradVoxel, true, ACC>);
+    } else {
+        switch (method_accum(method)) {
+        case kAccWeighted: launch(k_sweep_weighted<kGradEdge, false, ACC>, k_sweep_weighted<kGradVoxel, false, ACC>); break;
+        case kAccWeightedRawCurl: launch(k_sweep_weighted<kGradEdge, true, ACC>, k_sweep_weighted<kGradVoxel, true, ACC>); break;
+        case kAccSelect: launch(k_sweep_select<kGradEdge, ACC>, k_sweep_select<kGradVoxel, ACC>); break;
+        case kAccPlainNoEntry: launch(k_sweep_plain<kGradEdge, false, ACC>, k_sweep_plain<kGradVoxel, false, ACC>); break;
+        default: launch(k_sweep_plain<kGradEdge, true, ACC>, k_sweep_plain<kGradVoxel, true, ACC>); break;
+        }
     }
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t sweep_full(const Geometry &geo, const Field &f, int method, const float *p, float2 *pncnt,
+cudaError_t sweep_full(const Geometry &geo, const Field &f, int method, const float *p, const Sums<float> &s,
                        cudaStream_t st)
 {
-    return sweep_full_t(geo, f, method, p, pncnt, st);
+    if (s.through) return sweep_full_t(geo, f, method, p, s.mem, st);
+    return sweep_full_t(geo, f, method, p, reinterpret_cast<float2 *>(s.mem), st);
 }
 
-cudaError_t sweep_full64(const Geometry &geo, const Field &f, int method, const float *p, double2 *pncnt,
+cudaError_t sweep_full64(const Geometry &geo, const Field &f, int method, const float *p, const Sums<double> &s,
                          cudaStream_t st)
 {
-    return sweep_full_t(geo, f, method, p, pncnt, st);
+    if (s.through) return sweep_full_t(geo, f, method, p, s.mem, st);
+    return sweep_full_t(geo, f, method, p, reinterpret_cast<double2 *>(s.mem), st);
 }
 
-cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, long long *pncnt,
+cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, const Sums<long long> &s,
                            const double *scale, cudaStream_t st)
 {
     if (!scale) return cudaErrorInvalidValue;
-    return sweep_full_t(geo, f, method, p, pncnt, st, scale);
+    if (s.through) return sweep_full_t(geo, f, method, p, reinterpret_cast<unsigned long long *>(s.mem), st, scale);
+    return sweep_full_t(geo, f, method, p, s.mem, st, scale);
 }
 
 namespace {
@@ -665,39 +714,45 @@ cudaError_t init_accum_t(const Grid &g, const Layout &lay, const float *p_init, 
     return cudaGetLastError();
 }
 
+// f of every voxel's (pn, count), a pair ACC of T
+template <typename ACC, typename T, typename F>
+cudaError_t fold_sums(const Grid &g, const Layout &lay, const Sums<T> &s, const F &f, cudaStream_t st)
+{
+    if (s.through) k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, (const T *)s.mem, Counted<ACC, F>{f, s.through});
+    else k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, reinterpret_cast<const ACC *>(s.mem), f);
+    OM_COUNT_LAUNCH();
+    return cudaGetLastError();
+}
+
 }  // namespace
 
-cudaError_t init_accum64(const Grid &g, const Layout &lay, const float *p_init, bool seed, double2 *pncnt, cudaStream_t st)
+cudaError_t init_accum64(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Sums<double> &s, cudaStream_t st)
 {
-    return init_accum_t(g, lay, p_init, seed, pncnt, st);
+    if (s.through) return init_accum_t(g, lay, p_init, seed, s.mem, st);
+    return init_accum_t(g, lay, p_init, seed, reinterpret_cast<double2 *>(s.mem), st);
 }
 
-cudaError_t normalize64(const Grid &g, const Layout &lay, const double2 *pncnt, const float *p_keep, float *p_out,
+cudaError_t normalize64(const Grid &g, const Layout &lay, const Sums<double> &s, const float *p_keep, float *p_out,
                         float *cnt_out, cudaStream_t st)
 {
-    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, pncnt, Normalize<double2>{p_keep, p_out, cnt_out});
-    OM_COUNT_LAUNCH();
-    return cudaGetLastError();
+    return fold_sums<double2>(g, lay, s, Normalize<double2>{p_keep, p_out, cnt_out}, st);
 }
 
-cudaError_t normalize(const Grid &g, const Layout &lay, const float2 *pncnt, const float *p_keep, float *p_out,
+cudaError_t normalize(const Grid &g, const Layout &lay, const Sums<float> &s, const float *p_keep, float *p_out,
                       float *cnt_out, cudaStream_t st)
 {
-    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, pncnt, Normalize<float2>{p_keep, p_out, cnt_out});
-    OM_COUNT_LAUNCH();
-    return cudaGetLastError();
+    return fold_sums<float2>(g, lay, s, Normalize<float2>{p_keep, p_out, cnt_out}, st);
 }
 
-cudaError_t accum_split(const Grid &g, const Layout &lay, const float2 *acc, float *pn, float *cnt, cudaStream_t st)
+cudaError_t accum_split(const Grid &g, const Layout &lay, const Sums<float> &s, float *pn, float *cnt, cudaStream_t st)
 {
-    k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, acc, AddTo{pn, cnt});
-    OM_COUNT_LAUNCH();
-    return cudaGetLastError();
+    return fold_sums<float2>(g, lay, s, AddTo{pn, cnt}, st);
 }
 
-cudaError_t init_accum(const Grid &g, const Layout &lay, const float *p_init, bool seed, float2 *pncnt, cudaStream_t st)
+cudaError_t init_accum(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Sums<float> &s, cudaStream_t st)
 {
-    return init_accum_t(g, lay, p_init, seed, pncnt, st);
+    if (s.through) return init_accum_t(g, lay, p_init, seed, s.mem, st);
+    return init_accum_t(g, lay, p_init, seed, reinterpret_cast<float2 *>(s.mem), st);
 }
 
 cudaError_t spread_volume(const Grid &g, const Layout &lay, const float *in, float *out, cudaStream_t st)

@@ -117,9 +117,9 @@ extern "C" int omni3d_sweep_noalloc(omni3d_ctx *ctx, const float *ax, const floa
     F.lay = row_major_layout(geo->grid);  // one copy: what the static scratch holds
     F.curl = const_cast<float *>(curl);
     if ((e = pack_field(geo->grid, ax, ay, az, curl, &F, false, st)) != cudaSuccess ||
-        (e = init_accum(geo->grid, F.lay, nullptr, false, accum, st)) != cudaSuccess ||  // the last call's sums are cleared
-        (e = sweep_full(*geo, F, P->method, p, accum, st)) != cudaSuccess ||
-        (e = accum_split(geo->grid, F.lay, accum, pn, count, st)) != cudaSuccess)
+        (e = init_accum(geo->grid, F.lay, nullptr, false, Sums<float>{(float *)accum}, st)) != cudaSuccess ||  // the last call's sums are cleared
+        (e = sweep_full(*geo, F, P->method, p, Sums<float>{(float *)accum}, st)) != cudaSuccess ||
+        (e = accum_split(geo->grid, F.lay, Sums<float>{(float *)accum}, pn, count, st)) != cudaSuccess)
         return fail(OMNI3D_ERR_CUDA, std::string("omni3d_sweep_noalloc: ") + cudaGetErrorString(e));
     return OMNI3D_OK;
 }

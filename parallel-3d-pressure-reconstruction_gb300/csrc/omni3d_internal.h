@@ -217,6 +217,15 @@ struct Field {
     float *curl = nullptr;          // curl (methods that read it), also in f32[v].w
 };
 
+// Sums of a full sweep, in the walks' copies: (pn, count) of every voxel, or pn alone where the
+// count is known beforehand (`through`: the plain method's is the number of lines through the
+// voxel, which the geometry has once an operator has been built).
+template <typename T>
+struct Sums {
+    T *mem = nullptr;
+    const uint32_t *through = nullptr;  // row-major counts: pn alone is summed
+};
+
 // Brick passes B1 + L for the field f (FP32) and the method: per-segment carry-in states.
 cudaError_t brick_prepare(const Geometry &geo, Bricks *B, const Field &f, int method, cudaStream_t st,
                           std::string *err);
@@ -279,28 +288,28 @@ inline int method_accum(int method)
 
 // method: OMNI3D_METHOD_*; p is read at line entries / segment starts.
 cudaError_t sweep_full(const Geometry &geo, const Field &f, int method,
-                       const float *p, float2 *pncnt, cudaStream_t st);
+                       const float *p, const Sums<float> &pncnt, cudaStream_t st);
 // The same sweep accumulated in FP64 (two FP64 L2 reductions per contribution): the
 // defect-correction sweep of params.sweep_fp64.
 cudaError_t sweep_full64(const Geometry &geo, const Field &f, int method, const float *p,
-                         double2 *pncnt, cudaStream_t st);
-cudaError_t init_accum64(const Grid &g, const Layout &lay, const float *p_init, bool seed, double2 *pncnt,
+                         const Sums<double> &pncnt, cudaStream_t st);
+cudaError_t init_accum64(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Sums<double> &pncnt,
                          cudaStream_t st);
 // The same sweep accumulated in 64-bit fixed point (the bit-reproducible mode), with the
 // voxel scales scale[kFixPn], scale[kFixCnt] (fixed.cuh).
-cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, long long *pncnt,
+cudaError_t sweep_full_fix(const Geometry &geo, const Field &f, int method, const float *p, const Sums<long long> &pncnt,
                            const double *scale, cudaStream_t st);
-cudaError_t normalize64(const Grid &g, const Layout &lay, const double2 *pncnt, const float *p_keep, float *p_out,
+cudaError_t normalize64(const Grid &g, const Layout &lay, const Sums<double> &pncnt, const float *p_keep, float *p_out,
                         float *cnt_out, cudaStream_t st);
 
 // p_out[v] = cnt > 0 ? pn / cnt : p_keep[v]; cnt_out[v] = cnt (either may be null), with
 // (pn, cnt) the sum of the copies' accumulators.
-cudaError_t normalize(const Grid &g, const Layout &lay, const float2 *pncnt, const float *p_keep, float *p_out,
+cudaError_t normalize(const Grid &g, const Layout &lay, const Sums<float> &pncnt, const float *p_keep, float *p_out,
                       float *cnt_out, cudaStream_t st);
 // pn[v] += acc[v].x, cnt[v] += acc[v].y (summed over the copies)
-cudaError_t accum_split(const Grid &g, const Layout &lay, const float2 *acc, float *pn, float *cnt, cudaStream_t st);
+cudaError_t accum_split(const Grid &g, const Layout &lay, const Sums<float> &acc, float *pn, float *cnt, cudaStream_t st);
 // pncnt = (seed ? p_init : 0, 0): the seed in the first copy, zero in the others
-cudaError_t init_accum(const Grid &g, const Layout &lay, const float *p_init, bool seed, float2 *pncnt, cudaStream_t st);
+cudaError_t init_accum(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Sums<float> &pncnt, cudaStream_t st);
 // The walks' copies of a row-major volume (a row-major layout has one, the volume itself).
 cudaError_t spread_volume(const Grid &g, const Layout &lay, const float *in, float *out, cudaStream_t st);
 
@@ -328,8 +337,8 @@ cudaError_t fix_sweep_scales(long long V, const float *vol, const Fixed &fx, cud
 cudaError_t fix_rows_to_float(long long n, const Fixed &fx, float2 *bc, bool keep_c, cudaStream_t st);
 // Fixed-point voxel sums: init (pn = seed ? p_init : 0, count = 0), one full sweep,
 // normalisation (p = pn / count where count > 0, else p_keep) -- in FP64 from the exact sums.
-cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, long long *acc, cudaStream_t st);
-cudaError_t normalize_fix(const Grid &g, const Layout &lay, const long long *acc, const Fixed &fx, const float *p_keep, float *p_out,
+cudaError_t init_accum_fix(const Grid &g, const Layout &lay, const float *p_init, bool seed, const Fixed &fx, const Sums<long long> &acc, cudaStream_t st);
+cudaError_t normalize_fix(const Grid &g, const Layout &lay, const Sums<long long> &acc, const Fixed &fx, const float *p_keep, float *p_out,
                           float *cnt_out, cudaStream_t st);
 
 // Anchor operator (kernels_anchor.cu).
