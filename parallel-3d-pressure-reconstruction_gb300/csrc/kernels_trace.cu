@@ -44,6 +44,7 @@ struct CandOrder {
     int s_log2;       // log2 of the super-tile side in tiles (0..kSuperLog2Max)
     int gsize;        // directions per group
     int nv;
+    bool narrow;      // fewer than 2^32 candidates
 };
 
 // Super-tile side (log2) for a lattice of tu x tv tiles: the smallest power of two that
@@ -72,15 +73,24 @@ __device__ __forceinline__ bool trace_candidate(const Grid &g, const DirEntry *d
 {
     const long long per_block = (long long)co.gsize * 32;
     const long long per_group = co.nblk * per_block;
-    long long grp = c / per_group;
-    long long r = c - grp * per_group;
-    long long blk = r / per_block;
-    r -= blk * per_block;
-    int d = (int)(grp * co.gsize + r / 32);
-    const long long sup = blk >> (2 * co.s_log2);
+    long long grp, r, blk;
+    if (co.narrow) {  // 32-bit divisions
+        const uint32_t n = (uint32_t)c, q = n / (uint32_t)per_group, rest = n - q * (uint32_t)per_group;
+        const uint32_t b = rest / (uint32_t)per_block;
+        grp = q;
+        blk = b;
+        r = rest - b * (uint32_t)per_block;
+    } else {
+        grp = c / per_group;
+        r = c - grp * per_group;
+        blk = r / per_block;
+        r -= blk * per_block;
+    }
+    int d = (int)grp * co.gsize + ((int)r >> 5);
+    const uint32_t sup = (uint32_t)(blk >> (2 * co.s_log2)), srow = sup / (uint32_t)co.su;  // (a direction's tiles fit 32 bits)
     const uint32_t z = (uint32_t)(blk & ((1LL << (2 * co.s_log2)) - 1));
-    const long long tx = (sup % co.su) * (1LL << co.s_log2) + z_compact(z);
-    const long long ty = (sup / co.su) * (1LL << co.s_log2) + z_compact(z >> 1);
+    const long long tx = (long long)(sup - srow * (uint32_t)co.su) * (1LL << co.s_log2) + z_compact(z);
+    const long long ty = (long long)srow * (1LL << co.s_log2) + z_compact(z >> 1);
     const long long u = tx * (1LL << co.tw_log2) + (r & ((1LL << co.tw_log2) - 1));
     const long long v = ty * (32LL >> co.tw_log2) + ((r & 31) >> co.tw_log2);
     *dir = d;
@@ -88,6 +98,7 @@ __device__ __forceinline__ bool trace_candidate(const Grid &g, const DirEntry *d
     const long long pt = u + v * g.ng;  // lattice point: column u, row v
     DirEntry D = dirs[d];
     om_line_offset(pt, g.ng, g.ls, D, o[0], o[1], o[2]);
+    if (om_certain_miss(g, o[0], o[1], o[2], D.k1, D.k2, D.k3, D.cas)) return false;
     om_cross2point(g, o[0], o[1], o[2], D.k1, D.k2, D.k3, D.cas, in, out);
     return om_line_valid(g, in, out);
 }
@@ -204,7 +215,7 @@ __global__ void k_group_offsets(long long n_groups, const uint32_t *off, GroupRe
 // exit), so a re-walk with another field fits the words reserved for the line.  counters[0]
 // counts walks that stopped early under rule 0 (the reference's "Wrong Point" error; under the
 // other rules stopping early is their design), counters[1] the voxel visits.
-template <int RULE, bool FAST>
+template <int RULE, typename WALKER>
 __global__ void __launch_bounds__(kWalkThreads) k_walk(Grid g, const DirEntry *dirs, LineRec *lines,
                                                        const float4 *off, const GroupRec *groups,
                                                        uint32_t *desc, long long n_groups,
@@ -221,7 +232,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk(Grid g, const DirEntry *d
     const float4 o = off[li];
     const DirEntry D = dirs[r.dir];
     const LaneLine L = lane_line(g, r, (int)(G.info >> kGroupSigns));
-    std::conditional_t<FAST, OmFastWalker, OmWalker> w;
+    WALKER w;
     w.init(g, o.x, o.y, o.z, D.k1, D.k2, D.k3, L.ie, L.je, L.ke, L.ix, L.jx, L.kx);
     uint32_t *dp = desc + 32ull * G.word0 + lane;
     int s = 0;
@@ -232,8 +243,8 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk(Grid g, const DirEntry *d
         const int n1 = min(16, end - t0);
         for (int t = max(0, first - t0); t < n1; t++) {
             int a;
-            if constexpr (FAST) a = w.template step<RULE>();
-            else a = w.template step<RULE>(curl, g.X, g.XY, g.V);
+            if constexpr (std::is_same<WALKER, OmWalker>::value) a = w.template step<RULE>(curl, g.X, g.XY, g.V);
+            else a = w.template step<RULE>();
             if (a < 0) {  // the reference's loop ends here and keeps the steps taken
                 end = 0;
                 break;
@@ -515,6 +526,7 @@ cudaError_t build_geometry(Geometry *g, cudaStream_t st, std::string *err)
     co.nv = g->nv;
     long long ngroups = (g->nv + co.gsize - 1) / co.gsize;
     long long ncand = ngroups * co.nblk * co.gsize * 32;
+    co.narrow = ncand < (1LL << 32);
     long long nblk = (ncand + kTraceBlock - 1) / kTraceBlock;
     if (nblk > 0x7fffffffLL) {
         if (err) *err = "too many lattice candidates";
@@ -580,16 +592,20 @@ cudaError_t run_walk(Geometry *g, int rule, const float *curl, cudaStream_t st)
     cudaError_t e = cudaMemsetAsync(g->d_counters, 0, 2 * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     const Grid &G = g->grid;
-    const bool fast = std::max(std::max(G.X, G.Y), G.Z) < kFastWalkMax;
+    const int side = std::max(std::max(G.X, G.Y), G.Z);
+    const bool fast = side < kFastWalkMax, filtered = side <= kFilterMax;
     auto launch = [&](auto kernel) {
         kernel<<<group_blocks(*g, kWalkThreads), kWalkThreads, 0, st>>>(G, g->d_dirs, g->d_lines, g->d_off, g->d_groups, g->d_desc,
                                                                         g->n_groups, g->d_counters, curl);
     };
     switch (rule) {
-    case 1: fast ? launch(k_walk<1, true>) : launch(k_walk<1, false>); break;
-    case 2: fast ? launch(k_walk<2, true>) : launch(k_walk<2, false>); break;
-    case 3: launch(k_walk<3, false>); break;
-    default: fast ? launch(k_walk<0, true>) : launch(k_walk<0, false>); break;
+    case 1: fast ? launch(k_walk<1, OmFastWalker>) : launch(k_walk<1, OmWalker>); break;
+    case 2: fast ? launch(k_walk<2, OmFastWalker>) : launch(k_walk<2, OmWalker>); break;
+    case 3: launch(k_walk<3, OmWalker>); break;
+    default:
+        if (filtered) launch(k_walk<0, OmFilteredWalker>);
+        else fast ? launch(k_walk<0, OmFastWalker>) : launch(k_walk<0, OmWalker>);
+        break;
     }
     OM_COUNT_LAUNCH();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
