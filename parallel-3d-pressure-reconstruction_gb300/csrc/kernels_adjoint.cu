@@ -355,26 +355,33 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_edges(Grid g, Layout lay, 
 }
 
 // The operator's links, a warp per row: transposed rows' lengths, and the transposed links.
+// With two panels (split columns each) of both: row 2 i + p holds row i's links into panel p.
 template <int KIND>
-__global__ void k_adj_tcount(long long n, const unsigned long long *rowptr, const uint32_t *rowlen, const void *links,
-                             uint32_t *tcnt)
+__global__ void k_adj_tcount(long long n, uint32_t split, const unsigned long long *rowptr, const uint32_t *rowlen,
+                             const void *links, uint32_t *tcnt)
 {
     const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= n) return;
-    if ((threadIdx.x & 31) < lanes_per_row(KIND))
-        row_links<KIND>(links, rowptr[row], rowlen[row], threadIdx.x & 31, [&](uint32_t c, float) { atomicAdd(tcnt + c, 1u); });
+    if ((threadIdx.x & 31) >= lanes_per_row(KIND)) return;
+    const uint32_t panels = split ? 2 : 1, mine = split && row >= split ? 1 : 0;
+    for (uint32_t p = 0; p < panels; p++)
+        row_links<KIND>(links, rowptr[row * panels + p], rowlen[row * panels + p], threadIdx.x & 31,
+                        [&](uint32_t c, float) { atomicAdd(tcnt + (size_t)(c + p * split) * panels + mine, 1u); });
 }
 
 template <int KIND>
-__global__ void k_adj_tfill(long long n, const unsigned long long *rowptr, const uint32_t *rowlen, const void *links,
+__global__ void k_adj_tfill(long long n, uint32_t split, const unsigned long long *rowptr, const uint32_t *rowlen, const void *links,
                             const unsigned long long *tptr, uint32_t *tcur, void *tlinks)
 {
     const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= n) return;
     if ((threadIdx.x & 31) >= lanes_per_row(KIND)) return;
-    row_links<KIND>(links, rowptr[row], rowlen[row], threadIdx.x & 31, [&](uint32_t c, float w) {
-        store_link<KIND>(tlinks, tptr[c] + atomicAdd(tcur + c, 1u), (uint32_t)row, w);
-    });
+    const uint32_t panels = split ? 2 : 1, mine = split && row >= split ? 1 : 0;
+    for (uint32_t p = 0; p < panels; p++)
+        row_links<KIND>(links, rowptr[row * panels + p], rowlen[row * panels + p], threadIdx.x & 31, [&](uint32_t c, float w) {
+            const size_t t = (size_t)(c + p * split) * panels + mine;
+            store_link<KIND>(tlinks, tptr[t] + atomicAdd(tcur + t, 1u), (uint32_t)row - mine * split, w);
+        });
 }
 
 // Capacities of the transposed rows: whole 16-byte vectors of `per` links.
@@ -400,35 +407,40 @@ __global__ void k_adj_first(long long n, const float *lam, const float2 *bc, flo
 // in shared memory and several rows per warp at a time.
 template <int KIND, bool SMEM>
 __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 4) k_adj_iterate(
-    long long n, int rows, const unsigned long long *__restrict__ tptr, const uint32_t *__restrict__ tlen,
+    long long n, int rows, uint32_t split, const unsigned long long *__restrict__ tptr, const uint32_t *__restrict__ tlen,
     const void *__restrict__ tlinks, const float2 *__restrict__ bc, const float *__restrict__ u, float *__restrict__ unext,
     float *lam, float *acc)
 {
     extern __shared__ float4 sh_vector[];
-    const float *x = gather_vector<SMEM>(u, n, reinterpret_cast<float *>(sh_vector));
     constexpr int kWarps = (SMEM ? 1024 : 256) / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long row0 = ((long long)blockIdx.x * kWarps + warp) * rows;
     const long long mine = row0 + lane;  // the row this lane finishes
     const bool has = lane < rows && mine < n;
-    const unsigned long long ptr = has ? tptr[mine] : 0ull;
-    const uint32_t len = has ? tlen[mine] : 0u;
     float sum = 0.0f;
     constexpr int kLanes = lanes_per_row(KIND), kRows = 32 / kLanes;
-    for (int r = 0; r < rows; r += kRows) {
-        if (row0 + r >= n) break;  // whole warps
-        const int at = r + lane / kLanes;
-        const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, at & 31);
-        const uint32_t m = __shfl_sync(0xffffffffu, len, at & 31);
-        float s = 0.0f;
-        row_links<KIND>(tlinks, j0, at < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
-            const float y = SMEM ? x[c] : __ldg(x + c);
-            s += KIND == kLinkPair ? w * y : y;
-        });
-        __syncwarp();
-        for (int o = kLanes / 2; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        s = __shfl_sync(0xffffffffu, s, ((lane - r) * kLanes) & 31);  // the row of lane r + i
-        if (lane >= r && lane < r + kRows) sum = s;
+    const int panels = KIND == kLink16 && split ? 2 : 1;
+    for (int p = 0; p < panels; p++) {
+        if (SMEM && p) __syncthreads();  // the first panel has been read
+        const long long c0 = p ? (long long)split : 0;
+        const float *x = gather_vector<SMEM>(u + c0, panels == 1 ? n : min((long long)split, n - c0), reinterpret_cast<float *>(sh_vector));
+        const unsigned long long ptr = has ? tptr[mine * panels + p] : 0ull;
+        const uint32_t len = has ? tlen[mine * panels + p] : 0u;
+        for (int r = 0; r < rows; r += kRows) {
+            if (row0 + r >= n) break;  // whole warps
+            const int at = r + lane / kLanes;
+            const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, at & 31);
+            const uint32_t m = __shfl_sync(0xffffffffu, len, at & 31);
+            float s = 0.0f;
+            row_links<KIND>(tlinks, j0, at < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
+                const float y = SMEM ? x[c] : __ldg(x + c);
+                s += KIND == kLinkPair ? w * y : y;
+            });
+            __syncwarp();
+            for (int o = kLanes / 2; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            s = __shfl_sync(0xffffffffu, s, ((lane - r) * kLanes) & 31);  // the row of lane r + i
+            if (lane >= r && lane < r + kRows) sum += s;
+        }
     }
     if (!has) return;
     const float c = bc[mine].y;
@@ -597,29 +609,30 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
     // transposed operator (once per operator)
     const unsigned row_blocks = (unsigned)((n * 32 + 255) / 256);
     if (!B->tptr) {
+        const long long trows = n * A.panels();
         unsigned long long *t64 = nullptr, *tmp = nullptr;
         uint32_t *tcur = nullptr;
-        ADJ_TRY(cudaMalloc(&B->tlen, sizeof(uint32_t) * (size_t)std::max(n, 1LL)));
-        ADJ_TRY(cudaMalloc(&tcur, sizeof(uint32_t) * (size_t)std::max(n, 1LL)));
-        ADJ_TRY(cudaMalloc(&t64, sizeof(unsigned long long) * (size_t)std::max(n, 1LL)));
-        ADJ_TRY(cudaMalloc(&tmp, sizeof(unsigned long long) * scan_tmp_elems(n)));
-        ADJ_TRY(cudaMalloc(&B->tptr, sizeof(unsigned long long) * (size_t)(n + 1)));
-        ADJ_TRY(cudaMemsetAsync(B->tlen, 0, sizeof(uint32_t) * (size_t)std::max(n, 1LL), st));
-        auto count = [&](auto kernel) { kernel<<<row_blocks, 256, 0, st>>>(n, A.rowptr, A.rowlen, A.links, B->tlen); };
+        ADJ_TRY(cudaMalloc(&B->tlen, sizeof(uint32_t) * (size_t)std::max(trows, 1LL)));
+        ADJ_TRY(cudaMalloc(&tcur, sizeof(uint32_t) * (size_t)std::max(trows, 1LL)));
+        ADJ_TRY(cudaMalloc(&t64, sizeof(unsigned long long) * (size_t)std::max(trows, 1LL)));
+        ADJ_TRY(cudaMalloc(&tmp, sizeof(unsigned long long) * scan_tmp_elems(trows)));
+        ADJ_TRY(cudaMalloc(&B->tptr, sizeof(unsigned long long) * (size_t)(trows + 1)));
+        ADJ_TRY(cudaMemsetAsync(B->tlen, 0, sizeof(uint32_t) * (size_t)std::max(trows, 1LL), st));
+        auto count = [&](auto kernel) { kernel<<<row_blocks, 256, 0, st>>>(n, A.split, A.rowptr, A.rowlen, A.links, B->tlen); };
         if (n) {
             A.kind == kLink16 ? count(k_adj_tcount<kLink16>)
                               : (A.kind == kLink32 ? count(k_adj_tcount<kLink32>) : count(k_adj_tcount<kLinkPair>));
             OM_COUNT_LAUNCH();
-            k_adj_capacity<<<grid_for(n), 256, 0, st>>>(n, B->tlen, (unsigned)links_per_vector(A.kind), t64);
+            k_adj_capacity<<<grid_for(trows), 256, 0, st>>>(trows, B->tlen, (unsigned)links_per_vector(A.kind), t64);
             OM_COUNT_LAUNCH();
         }
-        ADJ_TRY(exclusive_scan_u64(t64, B->tptr, n, tmp, st));
+        ADJ_TRY(exclusive_scan_u64(t64, B->tptr, trows, tmp, st));
         unsigned long long tn = 0;
-        ADJ_TRY(cudaMemcpyAsync(&tn, B->tptr + n, sizeof(tn), cudaMemcpyDeviceToHost, st));
+        ADJ_TRY(cudaMemcpyAsync(&tn, B->tptr + trows, sizeof(tn), cudaMemcpyDeviceToHost, st));
         ADJ_TRY(cudaStreamSynchronize(st));
         ADJ_TRY(cudaMalloc(&B->tlinks, link_size(A.kind) * (size_t)std::max(tn, 1ULL)));
-        ADJ_TRY(cudaMemsetAsync(tcur, 0, sizeof(uint32_t) * (size_t)std::max(n, 1LL), st));
-        auto fill = [&](auto kernel) { kernel<<<row_blocks, 256, 0, st>>>(n, A.rowptr, A.rowlen, A.links, B->tptr, tcur, B->tlinks); };
+        ADJ_TRY(cudaMemsetAsync(tcur, 0, sizeof(uint32_t) * (size_t)std::max(trows, 1LL), st));
+        auto fill = [&](auto kernel) { kernel<<<row_blocks, 256, 0, st>>>(n, A.split, A.rowptr, A.rowlen, A.links, B->tptr, tcur, B->tlinks); };
         if (n) {
             A.kind == kLink16 ? fill(k_adj_tfill<kLink16>)
                               : (A.kind == kLink32 ? fill(k_adj_tfill<kLink32>) : fill(k_adj_tfill<kLinkPair>));
@@ -651,13 +664,13 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
     if (K > 1 && n) {
         k_adj_first<<<grid_for(n), 256, 0, st>>>(n, B->lam, A.bc, B->u, B->acc);
         OM_COUNT_LAUNCH();
-        const IterShape I = iter_shape(n, true);
+        const IterShape I = iter_shape(n, true, A.kind, A.split);
         auto launch = [&](auto wide, auto smem) {
             auto kernel = I.smem ? smem : wide;
             if (I.bytes > 48 * 1024)
                 ADJ_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIterSmemMax));
             for (int k = K - 1; k > 1; k--) {
-                kernel<<<I.blocks, I.threads, I.bytes, st>>>(n, I.rows, B->tptr, B->tlen, B->tlinks, A.bc, B->u, B->unext, B->lam,
+                kernel<<<I.blocks, I.threads, I.bytes, st>>>(n, I.rows, A.split, B->tptr, B->tlen, B->tlinks, A.bc, B->u, B->unext, B->lam,
                                                              B->acc);
                 OM_COUNT_LAUNCH();
                 std::swap(B->u, B->unext);

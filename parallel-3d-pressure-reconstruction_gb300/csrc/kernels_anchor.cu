@@ -81,6 +81,7 @@ struct Sink {
     unsigned long long *next;  // per row: the next free link slot (starts at the row's first slot)
     void *links;     // per link the start anchor, and its weight in weighted operators (links.cuh)
     int kind;        // LinkKind
+    uint32_t split;  // columns of a panel (links.cuh), 0: one panel
     float2 *bc;      // per row: (b, c)
     long long *bc64; // bit-reproducible mode: per row the fixed-point (b, c) instead of bc
     const double *fix;  // its scales (fixed.cuh)
@@ -100,7 +101,9 @@ __device__ __forceinline__ void emit_w(const Sink &S, int row, uint32_t scol, fl
         else atomicAdd(&S.bc[row].x, I);
         return;
     }
-    const unsigned long long slot = atomicAdd(S.next + row, 1ull);
+    const bool upper = UNIT && S.split && scol >= S.split;  // the second panel's
+    const unsigned long long slot = atomicAdd(S.next + (UNIT && S.split ? 2u * (uint32_t)row + (upper ? 1u : 0u) : (uint32_t)row), 1ull);
+    if (upper) scol -= S.split;
     const float bt = UNIT ? I : wt * I, ct = UNIT ? 1.0f : wt;
     if (!UNIT) store_link<kLinkPair>(S.links, slot, scol, wt);
     else if (S.kind == kLink16) store_link<kLink16>(S.links, slot, scol, wt);
@@ -469,13 +472,13 @@ __global__ void k_assign_ids(Grid g, Layout lay, const uint8_t *flag, const uint
 
 // Link slots of every row: the lines through its voxel (each contributes at most once), in whole
 // loads of `per` links; *total: the slots before rounding.
-__global__ void k_row_capacity(long long n, const uint32_t *vox, const uint32_t *lines_through, unsigned per,
+__global__ void k_row_capacity(long long n, const uint32_t *vox, const uint32_t *lines_through, unsigned per, int panels,
                                unsigned long long *out, unsigned long long *total)
 {
     unsigned long long t = 0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const uint32_t c = lines_through[vox[i]];
-        out[i] = (c + per - 1) / per * per;
+        for (int p = 0; p < panels; p++) out[i * panels + p] = (c + per - 1) / per * per;
         t += c;
     }
     for (int o = 16; o; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
@@ -487,17 +490,19 @@ __global__ void k_row_capacity(long long n, const uint32_t *vox, const uint32_t 
 // FP64.  A row gathers about as many terms as lines cross its voxel (~1000 at 642 directions);
 // plain FP32 sums of that many terms leave a rounding floor near 1e-6 in the iteration's
 // relative change, above the tolerances the solver is asked for.
+__device__ __forceinline__ void add_pair(float &hi, float &lo, float h2, float l2)
+{
+    const float t = __fadd_rn(hi, h2), b = __fsub_rn(t, hi);
+    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(h2, b));  // hi + h2 = t + e exactly
+    lo = __fadd_rn(__fadd_rn(lo, l2), e);
+    hi = t;
+}
 template <int LANES>
 __device__ __forceinline__ void warp_sum_pair(float &hi, float &lo)
 {
 #pragma unroll
-    for (int o = LANES / 2; o; o >>= 1) {
-        const float h2 = __shfl_xor_sync(0xffffffffu, hi, o), l2 = __shfl_xor_sync(0xffffffffu, lo, o);
-        const float t = __fadd_rn(hi, h2), b = __fsub_rn(t, hi);
-        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(h2, b));  // hi + h2 = t + e exactly
-        lo = __fadd_rn(__fadd_rn(lo, l2), e);
-        hi = t;
-    }
+    for (int o = LANES / 2; o; o >>= 1)
+        add_pair(hi, lo, __shfl_xor_sync(0xffffffffu, hi, o), __shfl_xor_sync(0xffffffffu, lo, o));
 }
 
 // The exact sum of fixed-point lane sums (integer additions: order-independent).
@@ -543,47 +548,57 @@ struct ChangeOut {
 // p_cur in shared memory; six CTAs of 256 threads per SM at 40 registers (five: 10 to 25 % more).
 template <int KIND, bool FIX, bool SMEM>
 __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iterate(
-    long long n, int rows, const unsigned long long *__restrict__ rowptr, const uint32_t *__restrict__ rowlen,
-    const void *__restrict__ links, const float2 *__restrict__ bc,
+    long long n, int rows, uint32_t split, const unsigned long long *__restrict__ rowptr,
+    const uint32_t *__restrict__ rowlen, const void *__restrict__ links, const float2 *__restrict__ bc,
     const uint32_t *__restrict__ vox, const float *__restrict__ p_init, int seed, const float *__restrict__ pc, float *pn,
     const int *stop, const double *__restrict__ fix, ChangeOut C)
 {
     extern __shared__ float4 sh_vector[];
     if (stop && *stop) return;  // a graph-captured chunk that has met its tolerance
-    const float *x = gather_vector<SMEM>(pc, n, reinterpret_cast<float *>(sh_vector));
     constexpr int kWarps = (SMEM ? 1024 : 256) / 32, kLanes = lanes_per_row(KIND), kRows = 32 / kLanes;
-    __shared__ double row_sum[kWarps * kIterRowsMax];  // (hi, lo) pairs, or the exact integers
+    __shared__ double row_sum[kWarps * iter_rows_max(SMEM)];  // (hi, lo) pairs, or the exact integers
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long base = (long long)blockIdx.x * kWarps * rows;  // the block's first row
     const long long row0 = base + (long long)warp * rows;
-    unsigned long long ptr = 0ull;
-    uint32_t len = 0u;
-    if (lane < rows && row0 + lane < n) {
-        ptr = rowptr[row0 + lane];
-        len = rowlen[row0 + lane];
-    }
     const FixScale sr = FIX ? fix_scale(fix[kFixRow]) : FixScale{};
-    for (int r = 0; r < rows; r += kRows) {
-        if (row0 + r >= n) break;  // whole warps
-        const int mine = r + lane / kLanes;  // (lanes past the last row have length 0)
-        const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, mine & 31);
-        const uint32_t m = __shfl_sync(0xffffffffu, len, mine & 31);
-        float s = 0.0f, comp = 0.0f;
-        long long t = 0;
-        row_links<KIND>(links, j0, mine < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
-            const float y = SMEM ? x[c] : __ldg(x + c);
-            if (FIX) t += (long long)fix_term(KIND == kLinkPair ? w * y : y, sr);
-            else kahan_add(s, comp, KIND == kLinkPair ? w * y : y);
-        });
-        __syncwarp();
-        if (FIX) {
-            t = warp_sum_fixed<kLanes>(t);
-        } else {
-            float h = s, l = -comp;
-            warp_sum_pair<kLanes>(h, l);
-            t = (long long)(((unsigned long long)__float_as_uint(h) << 32) | __float_as_uint(l));
+    const int panels = KIND == kLink16 && split ? 2 : 1;
+    for (int p = 0; p < panels; p++) {
+        if (SMEM && p) __syncthreads();  // the first panel has been read
+        const long long c0 = p ? (long long)split : 0;
+        const float *x = gather_vector<SMEM>(pc + c0, panels == 1 ? n : min((long long)split, n - c0), reinterpret_cast<float *>(sh_vector));
+        unsigned long long ptr = 0ull;
+        uint32_t len = 0u;
+        if (lane < rows && row0 + lane < n) {
+            ptr = rowptr[(row0 + lane) * panels + p];
+            len = rowlen[(row0 + lane) * panels + p];
         }
-        if (lane % kLanes == 0 && mine < rows) row_sum[warp * rows + mine] = __longlong_as_double(t);
+        for (int r = 0; r < rows; r += kRows) {
+            if (row0 + r >= n) break;  // whole warps
+            const int mine = r + lane / kLanes;  // (lanes past the last row have length 0)
+            const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, mine & 31);
+            const uint32_t m = __shfl_sync(0xffffffffu, len, mine & 31);
+            float s = 0.0f, comp = 0.0f;
+            long long t = 0;
+            row_links<KIND>(links, j0, mine < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
+                const float y = SMEM ? x[c] : __ldg(x + c);
+                if (FIX) t += (long long)fix_term(KIND == kLinkPair ? w * y : y, sr);
+                else kahan_add(s, comp, KIND == kLinkPair ? w * y : y);
+            });
+            __syncwarp();
+            if (FIX) {
+                t = warp_sum_fixed<kLanes>(t);
+                if (p && mine < rows) t += __double_as_longlong(row_sum[warp * rows + mine]);
+            } else {
+                float h = s, l = -comp;
+                warp_sum_pair<kLanes>(h, l);
+                if (p && mine < rows) {  // the first panel's pair
+                    const unsigned long long f = (unsigned long long)__double_as_longlong(row_sum[warp * rows + mine]);
+                    add_pair(h, l, __uint_as_float((uint32_t)(f >> 32)), __uint_as_float((uint32_t)f));
+                }
+                t = (long long)(((unsigned long long)__float_as_uint(h) << 32) | __float_as_uint(l));
+            }
+            if (lane % kLanes == 0 && mine < rows) row_sum[warp * rows + mine] = __longlong_as_double(t);
+        }
     }
     __syncthreads();
     // the block's rows, a thread each
@@ -596,7 +611,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iter
         const double sum = FIX ? (double)(long long)t / fix[kFixRow]
                                : (double)__uint_as_float((uint32_t)(t >> 32)) + (double)__uint_as_float((uint32_t)t);
         const float2 q = bc[mine];
-        const float old = x[mine];
+        const float old = pc[mine];
         double numer = (double)q.x + sum;
         if (seed && p_init) numer += (double)p_init[vox[mine]];
         const float now = q.y > 0.0f ? (float)(numer / (double)q.y) : old;
@@ -629,19 +644,19 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iter
     __syncthreads();
     if (!last) return;  // the last block adds the blocks' sums in their order
     __threadfence();
-    const volatile double *part = C.part;
     const int i = threadIdx.x & 3;
     double t = 0.0;
-    for (unsigned b = threadIdx.x >> 2; b < gridDim.x; b += 8 * kWarps) t += part[4ull * b + i];
+#pragma unroll 4
+    for (unsigned b = threadIdx.x >> 2; b < gridDim.x; b += 8 * kWarps) t += __ldcg(C.part + 4ull * b + i);
     for (int o = 16; o >= 4; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);  // lanes 0..3: this warp's four sums
     if (lane < 4) sh[lane][warp] = t;
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    if (warp != 0) return;
+    t = 0.0;  // lanes 0..3 (and those that repeat them): the block's four
+    for (int w = 0; w < kWarps; w++) t += sh[i][w];
     double S[4];
-    for (int k = 0; k < 4; k++) {
-        S[k] = 0.0;
-        for (int w = 0; w < kWarps; w++) S[k] += sh[k][w];
-    }
+    for (int k = 0; k < 4; k++) S[k] = __shfl_sync(0xffffffffu, t, k);
+    if (lane != 0) return;
     const double N = (double)n;
     double ed = -ad, ep = -ap;  // the shifts about the old ones (none: 0)
     if (C.gauge == OMNI3D_GAUGE_POINT && C.ref >= 0) {
@@ -973,19 +988,21 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     // rows: a voxel receives at most one contribution per line through it, so the
     // geometry-only line counts size the rows and no counting pass is needed
     AN_TRY(ensure_lines_through(&geo, f.lay, scratch, st));
-    AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * (size_t)(n + 1)));
-    AN_TRY(grow(A->tmp64, cap[9], sizeof(unsigned long long) * scan_tmp_elems(n)));
-    AN_TRY(grow(A->rowptr, cap[10], sizeof(unsigned long long) * (size_t)(n + 1)));
-    A->kind = !unit_links ? kLinkPair : (n <= 65536 ? kLink16 : kLink32);
-    AN_TRY(cudaMemsetAsync(A->cnt64 + n, 0, sizeof(unsigned long long), st));
-    k_row_capacity<<<grid_for(n), 256, 0, st>>>(n, A->vox, geo.d_lines_through, (unsigned)links_per_vector(A->kind), A->cnt64,
-                                                A->cnt64 + n);
+    A->kind = link_kind(n, unit_links);
+    A->split = link_split(n, unit_links);
+    const long long subrows = (long long)n * A->panels();
+    AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * (size_t)(subrows + 1)));
+    AN_TRY(grow(A->tmp64, cap[9], sizeof(unsigned long long) * scan_tmp_elems(subrows)));
+    AN_TRY(grow(A->rowptr, cap[10], sizeof(unsigned long long) * (size_t)(subrows + 1)));
+    AN_TRY(cudaMemsetAsync(A->cnt64 + subrows, 0, sizeof(unsigned long long), st));
+    k_row_capacity<<<grid_for(n), 256, 0, st>>>(n, A->vox, geo.d_lines_through, (unsigned)links_per_vector(A->kind), A->panels(),
+                                                A->cnt64, A->cnt64 + subrows);
     OM_COUNT_LAUNCH();
     AN_TRY(cudaGetLastError());
-    AN_TRY(exclusive_scan_u64(A->cnt64, A->rowptr, n, A->tmp64, st));
+    AN_TRY(exclusive_scan_u64(A->cnt64, A->rowptr, subrows, A->tmp64, st));
     unsigned long long slots = 0, nnz = 0;
-    AN_TRY(cudaMemcpyAsync(&slots, A->rowptr + n, sizeof(slots), cudaMemcpyDeviceToHost, st));
-    AN_TRY(cudaMemcpyAsync(&nnz, A->cnt64 + n, sizeof(nnz), cudaMemcpyDeviceToHost, st));
+    AN_TRY(cudaMemcpyAsync(&slots, A->rowptr + subrows, sizeof(slots), cudaMemcpyDeviceToHost, st));
+    AN_TRY(cudaMemcpyAsync(&nnz, A->cnt64 + subrows, sizeof(nnz), cudaMemcpyDeviceToHost, st));
     AN_TRY(cudaStreamSynchronize(st));
     A->nnz = (long long)nnz;
     if (max_nnz >= 0 && (long long)nnz > max_nnz) {
@@ -996,18 +1013,19 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     const size_t link_bytes = link_size(A->kind);
     AN_TRY(grow(A->links, cap[11], link_bytes * (size_t)slots));
     AN_TRY(grow(A->bc, cap[13], sizeof(float2) * (size_t)n));
-    AN_TRY(grow(A->red, cap[6], sizeof(double) * (4 + 4 * (size_t)std::max(iter_shape(std::max<long long>(n, 1), true).blocks,
-                                                                                iter_shape(std::max<long long>(n, 1), false).blocks))));
+    AN_TRY(grow(A->red, cap[6], sizeof(double) * (4 + 4 * (size_t)std::max(iter_shape(std::max<long long>(n, 1), true, A->kind, A->split).blocks,
+                                                                                iter_shape(std::max<long long>(n, 1), false, A->kind, A->split).blocks))));
     AN_TRY(grow(A->pa, cap[15], sizeof(float) * (size_t)n));
     AN_TRY(grow(A->pb, cap[16], sizeof(float) * (size_t)n));
-    AN_TRY(grow(A->rowlen, cap[17], sizeof(uint32_t) * (size_t)n));
-    AN_TRY(grow(A->next, cap[19], sizeof(unsigned long long) * (size_t)std::max<long long>(n, 1)));
-    if (n) AN_TRY(cudaMemcpyAsync(A->next, A->rowptr, sizeof(unsigned long long) * (size_t)n, cudaMemcpyDeviceToDevice, st));
+    AN_TRY(grow(A->rowlen, cap[17], sizeof(uint32_t) * (size_t)subrows));
+    AN_TRY(grow(A->next, cap[19], sizeof(unsigned long long) * (size_t)std::max<long long>(subrows, 1)));
+    if (n) AN_TRY(cudaMemcpyAsync(A->next, A->rowptr, sizeof(unsigned long long) * (size_t)subrows, cudaMemcpyDeviceToDevice, st));
     AN_TRY(cudaMemsetAsync(A->bc, 0, sizeof(float2) * (size_t)std::max<long long>(n, 1), st));
     S.id = lay.wrap ? A->wid : A->id;
     S.next = A->next;
     S.links = A->links;
     S.kind = A->kind;
+    S.split = A->split;
     S.bc = A->bc;
     if (fx) {  // bit-reproducible: the rows' (b, c) in fixed point (scales set by the caller)
         AN_TRY(grow(fx->bc64, fx->cap_bc64, sizeof(long long) * 2 * (size_t)std::max<long long>(n, 1)));
@@ -1023,7 +1041,7 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     AN_TRY(run_pass<kFill>(geo, f, method, fb, S, st));
     if (fx) AN_TRY(fix_rows_to_float(n, *fx, A->bc, false, st));
     if (n) {
-        k_row_lengths<<<grid_for(n), 256, 0, st>>>(n, A->rowptr, A->next, A->rowlen);
+        k_row_lengths<<<grid_for(subrows), 256, 0, st>>>(subrows, A->rowptr, A->next, A->rowlen);
         OM_COUNT_LAUNCH();
         if (fb) {  // the sweeps read the field unflagged
             k_field_flags<<<grid_for(n * 8), 256, 0, st>>>(geo.grid, f.lay, n, A->vox, f.lay.wrap ? f.edge : f.f32, 0);
@@ -1113,14 +1131,14 @@ cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, bool fi
             C.rel_out = test->rel_out;
         }
     }
-    const IterShape I = iter_shape(A.n, alone);
+    const IterShape I = iter_shape(A.n, alone, A.kind, A.split);
     auto launch = [&](auto wide, auto smem) {
         auto kernel = I.smem ? smem : wide;
         if (I.bytes > 48 * 1024) {  // (a host-side attribute of the kernel: cheap, and safe while capturing)
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIterSmemMax);
             if (e != cudaSuccess) return e;
         }
-        kernel<<<I.blocks, I.threads, I.bytes, st>>>(A.n, I.rows, A.rowptr, A.rowlen, A.links, A.bc, A.vox, p_init, seed ? 1 : 0,
+        kernel<<<I.blocks, I.threads, I.bytes, st>>>(A.n, I.rows, A.split, A.rowptr, A.rowlen, A.links, A.bc, A.vox, p_init, seed ? 1 : 0,
                                                      p_cur, p_next, stop, fix, C);
         OM_COUNT_LAUNCH();
         return cudaGetLastError();

@@ -1,10 +1,14 @@
 // Rows of the anchor operator and of its transpose, as the iterations read them.
 //
 // A row's links are (index, weight) pairs, one load each, or for unit weights (plain method)
-// 16-byte vectors, the row's start aligned, of four 32-bit indices or of eight 16-bit ones where
-// the operator has at most 2^16 anchors.  The gathered vector is kept in shared memory where it
-// fits: the links of a row point all over the volume's faces, so every lane's 4-byte gather is a
-// sector of its own through L2 (293 G gathers/s) but at worst a bank conflict in shared memory.
+// 16-byte vectors, the row's start aligned, of four 32-bit indices or of eight 16-bit ones.  The
+// gathered vector is kept in shared memory where it fits: the links of a row point all over the
+// volume's faces, so every lane's 4-byte gather is a sector of its own through L2 (293 G gathers/s)
+// but at worst a bank conflict in shared memory.  Up to kIterSplitMax anchors the columns are
+// split into two panels that fit one after the other, a row being two rows of 16-bit links, one
+// per panel, each with room for all of the row's links (as many bytes as 32-bit links take).
+// 128^3 / 642 directions (97 K anchors, 61 M links): 96 us an iteration with 32-bit links through
+// L1, 76 us with two panels.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -83,7 +87,8 @@ __device__ __forceinline__ void store_link(void *links, unsigned long long slot,
 }
 
 // The vector an iteration gathers from: copied into shared memory (SMEM) or read through L1.
-constexpr int kIterSmemMax = 220 * 1024;  // bytes of it: beside the rows' sums, what an SM gives one CTA
+constexpr int kIterSmemMax = 216 * 1024;  // bytes of it: beside the rows' sums, what an SM gives one CTA
+constexpr long long kIterPanelMax = kIterSmemMax / 4, kIterSplitMax = 2 * kIterPanelMax;
 template <bool SMEM>
 __device__ __forceinline__ const float *gather_vector(const float *x, long long n, float *sh)
 {
@@ -107,17 +112,32 @@ struct IterShape {
     unsigned blocks;
     size_t bytes;
 };
-constexpr int kIterRowsMax = 16;
-inline IterShape iter_shape(long long n, bool alone)
+// Rows per warp at most.  In shared memory enough for a single wave over kIterSplitMax rows; else
+// more blocks end more evenly (paired links, 112^3 selected: 0.77 ms of iterations at 16, 0.81 at 24).
+__host__ __device__ constexpr int iter_rows_max(bool smem) { return smem ? 24 : 16; }
+
+// Columns of a panel of an operator of n anchors (whole 16-byte vectors), 0: not split.
+inline uint32_t link_split(long long n, bool unit)
+{
+    return unit && n > kIterPanelMax && n <= kIterSplitMax ? (uint32_t)((n + 7) / 8 * 4) : 0u;
+}
+inline int link_kind(long long n, bool unit)
+{
+    return !unit ? kLinkPair : (n <= kIterSplitMax ? kLink16 : kLink32);
+}
+
+inline IterShape iter_shape(long long n, bool alone, int kind, uint32_t split)
 {
     IterShape s{};
-    s.bytes = sizeof(float) * (size_t)n;
+    s.bytes = sizeof(float) * (split ? (size_t)split : (size_t)n);
     s.smem = alone && n >= kIterSmemMin && s.bytes <= (size_t)kIterSmemMax;
     s.threads = s.smem ? 1024 : 256;
     // one CTA per SM above half of its shared memory, else two (2048 threads per SM)
+    // at least as many rows as a warp takes at once: fewer blocks then hand in fewer change sums (32^3
+    // / 162 directions: 15.2 -> 12.3 us an iteration with its test)
     const long long warps = s.smem ? 152LL * 32 * (s.bytes > (size_t)kIterSmemMax / 2 ? 1 : 2) : 152LL * 48;
-    const long long rows = (n + warps - 1) / warps;
-    s.rows = (int)(rows < 1 ? 1 : (rows > kIterRowsMax ? kIterRowsMax : rows));
+    const long long rows = (n + warps - 1) / warps, least = 32 / lanes_per_row(kind);
+    s.rows = (int)(rows < least ? least : (rows > iter_rows_max(s.smem) ? iter_rows_max(s.smem) : rows));
     const long long per = (long long)s.rows * (s.threads / 32);
     s.blocks = (unsigned)((n + per - 1) / per);
     if (!s.smem) s.bytes = 0;

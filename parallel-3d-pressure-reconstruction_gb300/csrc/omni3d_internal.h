@@ -348,10 +348,12 @@ struct Anchor {
     int32_t *wid = nullptr;         // the walks' copies of id (skewed layouts)
     int32_t *id = nullptr;          // V: anchor id or -1
     uint32_t *vox = nullptr;        // n: voxel of anchor
-    unsigned long long *rowptr = nullptr;  // n + 1: row capacities (lines through the voxel, in whole vectors)
-    uint32_t *rowlen = nullptr;     // n: entries in each row
+    unsigned long long *rowptr = nullptr;  // n x panels + 1: row capacities (lines through the voxel, in whole vectors)
+    uint32_t *rowlen = nullptr;     // n x panels: entries in each row
     void *links = nullptr;          // per link the start anchor and, in weighted operators, the weight
     int kind = 0;                   // LinkKind of the links (links.cuh)
+    uint32_t split = 0;             // columns of a panel (links.cuh); 0: one panel.  Two: rows 2 i, 2 i + 1 are row i's
+    int panels() const { return split ? 2 : 1; }
     float2 *bc = nullptr;           // n: (b, c) = (sum of w * I, sum of w)
     float *pa = nullptr, *pb = nullptr;  // iterates
     double *red = nullptr;          // reduction scratch
@@ -359,7 +361,7 @@ struct Anchor {
     uint32_t *u = nullptr, *pos = nullptr, *tmp = nullptr;
     unsigned long long *cnt64 = nullptr, *tmp64 = nullptr;
     uint32_t *neg = nullptr;        // 1 word: some curl value has its sign bit set
-    unsigned long long *next = nullptr;  // n: next free link slot of each row while filling
+    unsigned long long *next = nullptr;  // n x panels: next free link slot of each row while filling
     // capacities in bytes, one per buffer above, so that rebuilding for a new field of the
     // same geometry allocates nothing
     size_t cap[20] = {};
