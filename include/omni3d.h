@@ -69,7 +69,7 @@ extern "C" {
 
 /* Sweep engine.  Both give the same contributions; they differ in how the volume is read. */
 #define OMNI3D_ENGINE_AUTO 0    /* the faster engine for the solve: lines (measured on GB300
-                                   at 256^3 / 642 directions: lines 97 ms per sweep, bricks
+                                   at 256^3 / 642 directions: lines 44 ms per sweep, bricks
                                    145 ms + 95 ms of per-field passes) */
 #define OMNI3D_ENGINE_LINES 1   /* one thread per line, gathers and reductions through L2 */
 #define OMNI3D_ENGINE_BRICKS 2  /* lines cut into 16^3-brick segments; each brick's field is

@@ -258,10 +258,9 @@ int ensure_layout(omni3d_ctx *ctx)
         ctx->lay = skewed_layout(g);
         const omni3d_params &P = ctx->prm;
         const size_t entry = 2 * sizeof(float4) + sizeof(float) + sizeof(int32_t) + sizeof(float2) + (P.sweep_fp64 || P.deterministic ? sizeof(double2) : 0);
-        size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess ||
-            entry * (size_t)ctx->lay.copies * (size_t)g.V > fr / 2)
-            ctx->lay = row_major_layout(g);
+        const size_t need = entry * (size_t)ctx->lay.copies * (size_t)g.V;
+        size_t fr = 0, tot = 0;  // (a small context does not ask: the query takes longer than its first pass)
+        if (need > (64u << 20) && (cudaMemGetInfo(&fr, &tot) != cudaSuccess || need > fr / 2)) ctx->lay = row_major_layout(g);
         ctx->lay_set = true;
     }
     const size_t n = (size_t)ctx->lay.copies * (size_t)g.V;
@@ -1093,13 +1092,8 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
             aerr = cudaGetErrorString(e);
         } else {
             ctx->anc_cached = false;
-            long long max_links = P.anchor_max_links;
-            if (max_links <= 0) {  // what 80 % of the free memory holds (column + weight)
-                size_t fr = 0, tot = 0;
-                cudaMemGetInfo(&fr, &tot);
-                max_links = (long long)(0.8 * (double)fr / 8.0);
-            }
-            e = anchor_build(ctx->geo, F, P.method, P.gauge == OMNI3D_GAUGE_POINT ? ref : -1, max_links,
+            e = anchor_build(ctx->geo, F, P.method, P.gauge == OMNI3D_GAUGE_POINT ? ref : -1,
+                             std::max(P.anchor_max_links, 0LL),
                              &ctx->anc, st, &aerr, fx, ctx->pw.as<uint32_t>());
             ctx->anc_cached = e == cudaSuccess && P.method == OMNI3D_METHOD_PLAIN;
             adjoint_free(&ctx->adj);

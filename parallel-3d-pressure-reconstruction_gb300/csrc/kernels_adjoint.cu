@@ -665,8 +665,7 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
         k_adj_first<<<grid_for(n), 256, 0, st>>>(n, B->lam, A.bc, B->u, B->acc);
         OM_COUNT_LAUNCH();
         const IterShape I = iter_shape(n, true, A.kind, A.split);
-        auto launch = [&](auto wide, auto smem) {
-            auto kernel = I.smem ? smem : wide;
+        auto launch = [&](auto kernel) {
             if (I.bytes > 48 * 1024)
                 ADJ_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIterSmemMax));
             for (int k = K - 1; k > 1; k--) {
@@ -677,9 +676,9 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
             }
             return cudaGetLastError();
         };
-        ADJ_TRY(A.kind == kLink16   ? launch(k_adj_iterate<kLink16, false>, k_adj_iterate<kLink16, true>)
-                : A.kind == kLink32 ? launch(k_adj_iterate<kLink32, false>, k_adj_iterate<kLink32, true>)
-                                    : launch(k_adj_iterate<kLinkPair, false>, k_adj_iterate<kLinkPair, true>));
+        ADJ_TRY(A.kind == kLink16   ? (I.smem ? launch(k_adj_iterate<kLink16, true>) : launch(k_adj_iterate<kLink16, false>))
+                : A.kind == kLink32 ? launch(k_adj_iterate<kLink32, false>)
+                                    : launch(k_adj_iterate<kLinkPair, false>));
     }
     // dL/dB = mu + acc on the anchors, then the line scatter
     if (n) {

@@ -91,19 +91,22 @@ struct Sink {
 // the segment whose start anchor is scol (its id, loaded once per segment).  A link costs one
 // row lookup, one 64-bit slot atomic, one store and one vector reduction of (b, c); UNIT
 // operators (every weight 1) store no weight.
-template <int PASS, bool UNIT>
-__device__ __forceinline__ void emit_w(const Sink &S, int row, uint32_t scol, float wt, float I)
+//
+// take_slot reserves the link's slot (the row's next), put_link fills it.
+template <bool UNIT>
+__device__ __forceinline__ bool upper_panel(const Sink &S, uint32_t scol)
 {
-    if (row < 0) return;  // not an anchor after all: nothing to index
-    if (PASS == kFill && (int)scol < 0) return;  // a start that is no anchor: no column to link
-    if (PASS == kRhs) {  // plain method, operator cached: only b = sum I is field-dependent
-        if (S.bc64) fix_add(S.bc64 + 2 * row, I, fix_scale(S.fix[kFixB]));
-        else atomicAdd(&S.bc[row].x, I);
-        return;
-    }
-    const bool upper = UNIT && S.split && scol >= S.split;  // the second panel's
-    const unsigned long long slot = atomicAdd(S.next + (UNIT && S.split ? 2u * (uint32_t)row + (upper ? 1u : 0u) : (uint32_t)row), 1ull);
-    if (upper) scol -= S.split;
+    return UNIT && S.split && scol >= S.split;
+}
+template <bool UNIT>
+__device__ __forceinline__ unsigned long long take_slot(const Sink &S, int row, uint32_t scol)
+{
+    return atomicAdd(S.next + (UNIT && S.split ? 2u * (uint32_t)row + (upper_panel<UNIT>(S, scol) ? 1u : 0u) : (uint32_t)row), 1ull);
+}
+template <bool UNIT>
+__device__ __forceinline__ void put_link(const Sink &S, int row, unsigned long long slot, uint32_t scol, float wt, float I)
+{
+    if (upper_panel<UNIT>(S, scol)) scol -= S.split;
     const float bt = UNIT ? I : wt * I, ct = UNIT ? 1.0f : wt;
     if (!UNIT) store_link<kLinkPair>(S.links, slot, scol, wt);
     else if (S.kind == kLink16) store_link<kLink16>(S.links, slot, scol, wt);
@@ -113,6 +116,51 @@ __device__ __forceinline__ void emit_w(const Sink &S, int row, uint32_t scol, fl
         fix_add(S.bc64 + 2 * row + 1, ct, fix_scale(S.fix[kFixC]));
     } else {
         atomicAdd(S.bc + row, make_float2(bt, ct));
+    }
+}
+// Plain method, operator cached: only b = sum I is field-dependent.
+__device__ __forceinline__ void put_rhs(const Sink &S, int row, float I)
+{
+    if (S.bc64) fix_add(S.bc64 + 2 * row, I, fix_scale(S.fix[kFixB]));
+    else atomicAdd(&S.bc[row].x, I);
+}
+template <int PASS, bool UNIT>
+__device__ __forceinline__ void emit_w(const Sink &S, int row, uint32_t scol, float wt, float I)
+{
+    if (row < 0) return;  // not an anchor after all: nothing to index
+    if (PASS == kRhs) {
+        put_rhs(S, row, I);
+        return;
+    }
+    if (PASS == kFill && (int)scol < 0) return;  // a start that is no anchor: no column to link
+    put_link<UNIT>(S, row, take_slot<UNIT>(S, row, scol), scol, wt, I);
+}
+
+// The contributions of a batch's steps `todo` (bits 2q) into the anchors they enter, unit weights:
+// the row lookups of all steps wait together, then their slots (128^3: 3.02 -> 2.98 ms against a
+// step at a time; the weighted forms have no registers for it and spill: 29.0 -> 32.4 ms at 256^3).
+template <int PASS>
+__device__ __forceinline__ void emit_units(const Sink &S, uint32_t todo, const uint32_t (&v)[kWalkBatch], uint32_t scol,
+                                           const float (&I)[kWalkBatch])
+{
+    int rows[kWalkBatch];
+    unsigned long long slot[kWalkBatch];
+#pragma unroll
+    for (int q = 0; q < kWalkBatch; q++) {
+        rows[q] = -1;
+        if (todo & (1u << (2 * q))) rows[q] = __ldg(S.id + v[q]);
+        if (PASS == kFill && (int)scol < 0) rows[q] = -1;
+    }
+    if (PASS == kFill) {
+#pragma unroll
+        for (int q = 0; q < kWalkBatch; q++)
+            if (rows[q] >= 0) slot[q] = take_slot<true>(S, rows[q], scol);
+    }
+#pragma unroll
+    for (int q = 0; q < kWalkBatch; q++) {
+        if (rows[q] < 0) continue;
+        if (PASS == kFill) put_link<true>(S, rows[q], slot[q], scol, 1.0f, I[q]);
+        else put_rhs(S, rows[q], I[q]);
     }
 }
 
@@ -157,9 +205,9 @@ __device__ __forceinline__ bool any_anchor(const float4 (&g)[kWalkBatch], const 
 
 // What every operator pass keeps along a line.  A batch without an anchor only sums; in one
 // with anchors the sums at its steps stay in registers and the lanes then record their
-// contributions together, each lane its next one per round, instead of step by step with the
-// few lanes that enter an anchor at that step (three of 32 on average): a record waits for a
-// row lookup and an atomic, and a round of them waits once.
+// contributions together, each lane its next one per round (unit weights: all at once), instead
+// of step by step with the few lanes that enter an anchor at that step (three of 32 on average):
+// a record waits for a row lookup and an atomic, and a round of them waits once.
 template <int GRAD>
 struct FillLine {
     const LineWalk &L;
@@ -200,10 +248,7 @@ struct PlainFill : FillLine<GRAD> {
             this->integrate(c, q, g[q], taken<MASK>(idle, q));
             Is[q] = this->I;
         }
-        for (uint32_t todo = anchor_steps<FB>(idle, g, id); todo; todo &= todo - 1u) {
-            const int q = (__ffs(todo) - 1) >> 1;
-            emit_w<PASS, true>(this->S, __ldg(this->S.id + pick(v, q)), ecol, 1.0f, pick(Is, q));
-        }
+        emit_units<PASS>(this->S, anchor_steps<FB>(idle, g, id), v, ecol, Is);
     }
     template <bool MASK>
     __device__ __forceinline__ void general(uint32_t, uint32_t, const uint32_t (&)[kWalkBatch],
@@ -927,37 +972,10 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
 {
     const long long V = geo.grid.V;
     size_t *cap = A->cap;
-    AN_TRY(grow(A->flag, cap[0], (size_t)V));
     const Layout &lay = f.lay;
-    if (lay.wrap) {
-        AN_TRY(grow(A->wid, cap[1], sizeof(int32_t) * (size_t)lay.copies * (size_t)V));
-        AN_TRY(cudaMemsetAsync(A->wid, 0xff, sizeof(int32_t) * (size_t)lay.copies * (size_t)V, st));
-    }
-    AN_TRY(grow(A->id, cap[2], sizeof(int32_t) * (size_t)V));
-    AN_TRY(grow(A->u, cap[3], sizeof(uint32_t) * (size_t)V));
-    AN_TRY(grow(A->pos, cap[4], sizeof(uint32_t) * (size_t)(V + 1)));
-    AN_TRY(grow(A->tmp, cap[5], sizeof(uint32_t) * scan_tmp_elems(V)));
-        Sink S{};
-    S.flag = A->flag;
-    bool marked = false;
-    if (method_accum(method) == kAccSelect) {
-        // cheap superset of the segment starts; used when it stays small
-        AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * 1));
-        unsigned long long *dcount = A->cnt64;
-        AN_TRY(cudaMemsetAsync(dcount, 0, sizeof(unsigned long long), st));
-        k_select_candidates<<<grid_for(V), 256, 0, st>>>(geo.grid, f.curl, A->flag, dcount);
-        OM_COUNT_LAUNCH();
-        AN_TRY(cudaGetLastError());
-        unsigned long long nc = 0;
-        AN_TRY(cudaMemcpyAsync(&nc, dcount, sizeof(nc), cudaMemcpyDeviceToHost, st));
-        AN_TRY(cudaStreamSynchronize(st));
-        marked = (long long)nc <= V / 16;
-    }
-    if (!marked) {
-        AN_TRY(cudaMemsetAsync(A->flag, 0, (size_t)V, st));
-        AN_TRY(run_pass<kMark>(geo, f, method, false, S, st));
-    }
-    if (ref_voxel >= 0 && ref_voxel < V) AN_TRY(cudaMemsetAsync(A->flag + ref_voxel, 1, 1, st));
+    const int acc = method_accum(method);
+    const bool unit_links = acc == kAccPlain || acc == kAccPlainNoEntry;
+    Sink S{};
     // the field carries curl in .w: its sign bit can flag the anchors unless a curl value
     // already has it set
     const bool check_sign = f.curl != nullptr;
@@ -968,50 +986,94 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
         OM_COUNT_LAUNCH();
         AN_TRY(cudaGetLastError());
     }
+    uint32_t n = (uint32_t)A->n, neg = 0;
+    // The anchors and their rows' capacities.  Those of the methods whose anchors are the lines'
+    // entries follow from the geometry's walks alone: a later field finds them in place (40^3 /
+    // 642 directions, weighted: 0.95 -> 0.84 ms a solve).
+    if (A->placed == geo.walk_generation + 1 && acc != kAccSelect) {
+        AN_TRY(cudaMemcpyAsync(&neg, A->neg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        AN_TRY(cudaStreamSynchronize(st));
+    } else {
+        A->placed = 0;
+        AN_TRY(grow(A->flag, cap[0], (size_t)V));
+        if (lay.wrap) {
+            AN_TRY(grow(A->wid, cap[1], sizeof(int32_t) * (size_t)lay.copies * (size_t)V));
+            AN_TRY(cudaMemsetAsync(A->wid, 0xff, sizeof(int32_t) * (size_t)lay.copies * (size_t)V, st));
+        }
+        AN_TRY(grow(A->id, cap[2], sizeof(int32_t) * (size_t)V));
+        AN_TRY(grow(A->u, cap[3], sizeof(uint32_t) * (size_t)V));
+        AN_TRY(grow(A->pos, cap[4], sizeof(uint32_t) * (size_t)(V + 1)));
+        AN_TRY(grow(A->tmp, cap[5], sizeof(uint32_t) * scan_tmp_elems(V)));
+        S.flag = A->flag;
+        bool marked = false;
+        if (acc == kAccSelect) {
+            // cheap superset of the segment starts; used when it stays small
+            AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * 1));
+            unsigned long long *dcount = A->cnt64;
+            AN_TRY(cudaMemsetAsync(dcount, 0, sizeof(unsigned long long), st));
+            k_select_candidates<<<grid_for(V), 256, 0, st>>>(geo.grid, f.curl, A->flag, dcount);
+            OM_COUNT_LAUNCH();
+            AN_TRY(cudaGetLastError());
+            unsigned long long nc = 0;
+            AN_TRY(cudaMemcpyAsync(&nc, dcount, sizeof(nc), cudaMemcpyDeviceToHost, st));
+            AN_TRY(cudaStreamSynchronize(st));
+            marked = (long long)nc <= V / 16;
+        }
+        if (!marked) {
+            AN_TRY(cudaMemsetAsync(A->flag, 0, (size_t)V, st));
+            AN_TRY(run_pass<kMark>(geo, f, method, false, S, st));
+        }
+        if (ref_voxel >= 0 && ref_voxel < V) AN_TRY(cudaMemsetAsync(A->flag + ref_voxel, 1, 1, st));
+        k_flag_to_u32<<<grid_for(V), 256, 0, st>>>(V, A->flag, A->u);
+        OM_COUNT_LAUNCH();
+        AN_TRY(cudaGetLastError());
+        AN_TRY(exclusive_scan_u32(A->u, A->pos, V, A->tmp, st));
+        AN_TRY(cudaMemcpyAsync(&n, A->pos + V, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        AN_TRY(cudaMemcpyAsync(&neg, A->neg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        AN_TRY(cudaStreamSynchronize(st));
+        A->n = n;
+        AN_TRY(grow(A->vox, cap[7], sizeof(uint32_t) * (size_t)n));
+        k_assign_ids<<<grid_for(V), 256, 0, st>>>(geo.grid, lay, A->flag, A->pos, A->id, A->vox, A->wid);
+        OM_COUNT_LAUNCH();
+        AN_TRY(cudaGetLastError());
 
-    k_flag_to_u32<<<grid_for(V), 256, 0, st>>>(V, A->flag, A->u);
-    OM_COUNT_LAUNCH();
-    AN_TRY(cudaGetLastError());
-    AN_TRY(exclusive_scan_u32(A->u, A->pos, V, A->tmp, st));
-    uint32_t n = 0, neg = 0;
-    AN_TRY(cudaMemcpyAsync(&n, A->pos + V, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    AN_TRY(cudaMemcpyAsync(&neg, A->neg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    AN_TRY(cudaStreamSynchronize(st));
-    A->n = n;
+        // rows: a voxel receives at most one contribution per line through it, so the
+        // geometry-only line counts size the rows and no counting pass is needed
+        AN_TRY(ensure_lines_through(&geo, f.lay, scratch, st));
+        A->kind = link_kind(n, unit_links);
+        A->split = link_split(n, unit_links);
+        const long long rows = (long long)n * A->panels();
+        AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * (size_t)(rows + 1)));
+        AN_TRY(grow(A->tmp64, cap[9], sizeof(unsigned long long) * scan_tmp_elems(rows)));
+        AN_TRY(grow(A->rowptr, cap[10], sizeof(unsigned long long) * (size_t)(rows + 1)));
+        AN_TRY(cudaMemsetAsync(A->cnt64 + rows, 0, sizeof(unsigned long long), st));
+        k_row_capacity<<<grid_for(n), 256, 0, st>>>(n, A->vox, geo.d_lines_through, (unsigned)links_per_vector(A->kind),
+                                                    A->panels(), A->cnt64, A->cnt64 + rows);
+        OM_COUNT_LAUNCH();
+        AN_TRY(cudaGetLastError());
+        AN_TRY(exclusive_scan_u64(A->cnt64, A->rowptr, rows, A->tmp64, st));
+        unsigned long long nnz = 0;
+        AN_TRY(cudaMemcpyAsync(&A->slots, A->rowptr + rows, sizeof(A->slots), cudaMemcpyDeviceToHost, st));
+        AN_TRY(cudaMemcpyAsync(&nnz, A->cnt64 + rows, sizeof(nnz), cudaMemcpyDeviceToHost, st));
+        AN_TRY(cudaStreamSynchronize(st));
+        A->nnz = (long long)nnz;
+        if (acc != kAccSelect) A->placed = geo.walk_generation + 1;
+    }
     const bool fb = neg == 0u;
-    AN_TRY(grow(A->vox, cap[7], sizeof(uint32_t) * (size_t)n));
-    k_assign_ids<<<grid_for(V), 256, 0, st>>>(geo.grid, lay, A->flag, A->pos, A->id, A->vox, A->wid);
-    OM_COUNT_LAUNCH();
-    AN_TRY(cudaGetLastError());
-
-    const bool unit_links = method_accum(method) == kAccPlain || method_accum(method) == kAccPlainNoEntry;
-    // rows: a voxel receives at most one contribution per line through it, so the
-    // geometry-only line counts size the rows and no counting pass is needed
-    AN_TRY(ensure_lines_through(&geo, f.lay, scratch, st));
-    A->kind = link_kind(n, unit_links);
-    A->split = link_split(n, unit_links);
     const long long subrows = (long long)n * A->panels();
-    AN_TRY(grow(A->cnt64, cap[8], sizeof(unsigned long long) * (size_t)(subrows + 1)));
-    AN_TRY(grow(A->tmp64, cap[9], sizeof(unsigned long long) * scan_tmp_elems(subrows)));
-    AN_TRY(grow(A->rowptr, cap[10], sizeof(unsigned long long) * (size_t)(subrows + 1)));
-    AN_TRY(cudaMemsetAsync(A->cnt64 + subrows, 0, sizeof(unsigned long long), st));
-    k_row_capacity<<<grid_for(n), 256, 0, st>>>(n, A->vox, geo.d_lines_through, (unsigned)links_per_vector(A->kind), A->panels(),
-                                                A->cnt64, A->cnt64 + subrows);
-    OM_COUNT_LAUNCH();
-    AN_TRY(cudaGetLastError());
-    AN_TRY(exclusive_scan_u64(A->cnt64, A->rowptr, subrows, A->tmp64, st));
-    unsigned long long slots = 0, nnz = 0;
-    AN_TRY(cudaMemcpyAsync(&slots, A->rowptr + subrows, sizeof(slots), cudaMemcpyDeviceToHost, st));
-    AN_TRY(cudaMemcpyAsync(&nnz, A->cnt64 + subrows, sizeof(nnz), cudaMemcpyDeviceToHost, st));
-    AN_TRY(cudaStreamSynchronize(st));
-    A->nnz = (long long)nnz;
-    if (max_nnz >= 0 && (long long)nnz > max_nnz) {
+    const size_t link_bytes = link_size(A->kind);
+    long long limit = max_nnz;
+    if (max_nnz == 0) {  // what 80 % of the free memory holds (column + weight); links that fit in place always do (asking takes 23 us)
+        size_t fr = 0, tot = 0;
+        if (link_bytes * (size_t)A->slots <= cap[11]) limit = -1;
+        else if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) limit = (long long)(0.8 * (double)fr / 8.0);
+    }
+    if (limit >= 0 && A->nnz > limit) {
         if (err) *err = "anchor operator larger than its limit";
         return cudaErrorNotSupported;
     }
 
-    const size_t link_bytes = link_size(A->kind);
-    AN_TRY(grow(A->links, cap[11], link_bytes * (size_t)slots));
+    AN_TRY(grow(A->links, cap[11], link_bytes * (size_t)A->slots));
     AN_TRY(grow(A->bc, cap[13], sizeof(float2) * (size_t)n));
     AN_TRY(grow(A->red, cap[6], sizeof(double) * (4 + 4 * (size_t)std::max(iter_shape(std::max<long long>(n, 1), true, A->kind, A->split).blocks,
                                                                                 iter_shape(std::max<long long>(n, 1), false, A->kind, A->split).blocks))));
@@ -1132,8 +1194,7 @@ cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, bool fi
         }
     }
     const IterShape I = iter_shape(A.n, alone, A.kind, A.split);
-    auto launch = [&](auto wide, auto smem) {
-        auto kernel = I.smem ? smem : wide;
+    auto launch = [&](auto kernel) {
         if (I.bytes > 48 * 1024) {  // (a host-side attribute of the kernel: cheap, and safe while capturing)
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIterSmemMax);
             if (e != cudaSuccess) return e;
@@ -1143,13 +1204,11 @@ cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, bool fi
         OM_COUNT_LAUNCH();
         return cudaGetLastError();
     };
-#define OM_LAUNCH_ITERATE(KIND) \
-    (fix ? launch(k_anchor_iterate<KIND, true, false>, k_anchor_iterate<KIND, true, true>) \
-         : launch(k_anchor_iterate<KIND, false, false>, k_anchor_iterate<KIND, false, true>))
+#define OM_LAUNCH_ITERATE(KIND, SMEM) (fix ? launch(k_anchor_iterate<KIND, true, SMEM>) : launch(k_anchor_iterate<KIND, false, SMEM>))
     switch (A.kind) {
-    case kLink16: return OM_LAUNCH_ITERATE(kLink16);
-    case kLink32: return OM_LAUNCH_ITERATE(kLink32);
-    default: return OM_LAUNCH_ITERATE(kLinkPair);
+    case kLink16: return I.smem ? OM_LAUNCH_ITERATE(kLink16, true) : OM_LAUNCH_ITERATE(kLink16, false);
+    case kLink32: return OM_LAUNCH_ITERATE(kLink32, false);
+    default: return OM_LAUNCH_ITERATE(kLinkPair, false);
     }
 #undef OM_LAUNCH_ITERATE
 }

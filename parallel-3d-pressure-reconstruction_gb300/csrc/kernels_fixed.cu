@@ -223,10 +223,8 @@ cudaError_t normalize_fix(const Grid &g, const Layout &lay, const Sums<long long
                           float *p_out, float *cnt_out, cudaStream_t st)
 {
     const NormalizeFix f{fx.scale, p_keep, p_out, cnt_out, s.through};
-    if (s.through) k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, (const long long *)s.mem, f);
-    else k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, FixSums{s.mem, s.mem + (size_t)lay.copies * (size_t)g.V}, f);
-    OM_COUNT_LAUNCH();
-    return cudaGetLastError();
+    if (s.through) return fold_copies(g, lay, (const long long *)s.mem, f, st);
+    return fold_copies(g, lay, FixSums{s.mem, s.mem + (size_t)lay.copies * (size_t)g.V}, f, st);
 }
 
 }  // namespace omni3d

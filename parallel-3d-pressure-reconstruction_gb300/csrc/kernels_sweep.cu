@@ -427,6 +427,16 @@ __global__ void __launch_bounds__(kTileThreads) k_spread(Grid g, Layout lay, con
         at.diagonals(g, lay, c, [&](int p, uint32_t q) { out[(size_t)c * (size_t)lay.stride + q] = tile[p]; });
 }
 
+__global__ void __launch_bounds__(kTileThreads) k_spread_voxels(Grid g, Layout lay, const float *__restrict__ in, float *out)
+{
+    const long long v = (long long)blockIdx.x * kTileThreads + threadIdx.x;
+    if (v >= g.V) return;
+    const VoxelAt at(g, v);
+    const float x = in[v];
+#pragma unroll
+    for (int c = 0; c < 4; c++) out[(size_t)c * (size_t)lay.stride + layout_index(lay, g.X, g.Y, c, at.i, at.j, at.k)] = x;
+}
+
 __device__ __forceinline__ uint32_t to_bf16(float x)
 {
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x));
@@ -468,48 +478,77 @@ __device__ __forceinline__ uint32_t curl_bf16(float c, const Grid &g)
 // same field.
 // The records of a tile are put together in shared memory and written diagonal by diagonal
 // (fold.cuh): 256^3, 2.46 -> 0.50 ms against eight scattered records per voxel.
-__global__ void __launch_bounds__(kTileThreads) k_pack(Grid g, const float *__restrict__ ax, const float *__restrict__ ay,
-                       const float *__restrict__ az, const float *curl, float4 *f32, Layout lay, float4 *edge,
-                       float *curl_out, int round16)
-{
-    __shared__ float sxl[kTile * kTile], sxu[kTile * kTile], syl[kTile * kTile], syu[kTile * kTile], szl[kTile * kTile],
-        szu[kTile * kTile], sc[kTile * kTile];
+struct PackIn {
+    const float *ax, *ay, *az, *curl;
+    int round16;
     // a component as stored
-    auto stored = [&](float x) { return round16 ? __uint_as_float(to_bf16(x) << 16) : x; };
+    __device__ __forceinline__ float at(const float *a, long long v) const
+    {
+        const float x = a[v];
+        return round16 ? __uint_as_float(to_bf16(x) << 16) : x;
+    }
+};
+// The sums of the components over a voxel's two edges along each axis (lower, upper), and its curl.
+struct VoxelEdges {
+    float xl, xu, yl, yu, zl, zu, c;
+};
+// Packs voxel v into f32 and curl_out; its edges' sums where a layout needs them.
+__device__ __forceinline__ VoxelEdges pack_voxel(const Grid &g, const PackIn &in, long long v, int i, int j, int k, bool edges,
+                                                 float4 *f32, float *curl_out)
+{
+    VoxelEdges E{};
+    const float x = in.at(in.ax, v), y = in.at(in.ay, v), z = in.at(in.az, v);
+    E.c = in.curl ? in.curl[v] : 0.0f;
+    if (in.round16) {
+        E.c = __uint_as_float(curl_bf16(E.c, g) << 16);
+        if (curl_out) curl_out[v] = E.c;
+    }
+    f32[v] = make_float4(x, y, z, E.c);
+    if (!edges) return E;
+    if (i > 0) E.xl = x + in.at(in.ax, v - 1);
+    if (i < g.X - 1) E.xu = x + in.at(in.ax, v + 1);
+    if (j > 0) E.yl = y + in.at(in.ay, v - g.X);
+    if (j < g.Y - 1) E.yu = y + in.at(in.ay, v + g.X);
+    if (k > 0) E.zl = z + in.at(in.az, v - g.XY);
+    if (k < g.Z - 1) E.zu = z + in.at(in.az, v + g.XY);
+    return E;
+}
+// The edge records of a voxel in class c: entry q of its two octants' copies.
+__device__ __forceinline__ void store_edges(const Grid &g, const Layout &lay, int c, uint32_t q, const VoxelEdges &E, float4 *edge)
+{
+    // the coefficients of the octant that steps upward along x
+    const float hx = __fmul_rn(-g.rho, g.dx) * 0.5f, h1 = __fmul_rn(-g.rho, g.dy) * 0.5f, h2 = __fmul_rn(-g.rho, g.dz) * 0.5f;
+    const float hy = (c & 1) ? -h1 : h1, hz = (c & 2) ? -h2 : h2;
+    // a step upward along an axis crosses the voxel's lower edge
+    const float yd = (c & 1) ? E.yl : E.yu, yu = (c & 1) ? E.yu : E.yl, zd = (c & 2) ? E.zl : E.zu, zu = (c & 2) ? E.zu : E.zl;
+    edge[(size_t)(2 * c) * (size_t)lay.stride + q] = make_float4(-hx * E.xu, -hy * yd, -hz * zd, E.c);
+    edge[(size_t)(2 * c + 1) * (size_t)lay.stride + q] = make_float4(hx * E.xl, hy * yu, hz * zu, E.c);
+}
+
+__global__ void __launch_bounds__(kTileThreads) k_pack(Grid g, PackIn in, float4 *f32, Layout lay, float4 *edge, float *curl_out)
+{
+    __shared__ float sums[7][kTile * kTile];
     const TileAt at(g);
     at.rows(g, [&](int p, long long v, int i, int j) {
-        const float x = stored(ax[v]), y = stored(ay[v]), z = stored(az[v]);
-        float c = curl ? curl[v] : 0.0f;
-        if (round16) {
-            c = __uint_as_float(curl_bf16(c, g) << 16);
-            if (curl_out) curl_out[v] = c;
-        }
-        f32[v] = make_float4(x, y, z, c);
-        if (!lay.wrap) return;
-        // the sums over each axis' two edges
-        sxl[p] = i > 0 ? x + stored(ax[v - 1]) : 0.0f;
-        sxu[p] = i < g.X - 1 ? x + stored(ax[v + 1]) : 0.0f;
-        syl[p] = j > 0 ? y + stored(ay[v - g.X]) : 0.0f;
-        syu[p] = j < g.Y - 1 ? y + stored(ay[v + g.X]) : 0.0f;
-        szl[p] = at.k > 0 ? z + stored(az[v - g.XY]) : 0.0f;
-        szu[p] = at.k < g.Z - 1 ? z + stored(az[v + g.XY]) : 0.0f;
-        sc[p] = c;
+        const VoxelEdges E = pack_voxel(g, in, v, i, j, at.k, true, f32, curl_out);
+        sums[0][p] = E.xl; sums[1][p] = E.xu; sums[2][p] = E.yl; sums[3][p] = E.yu;
+        sums[4][p] = E.zl; sums[5][p] = E.zu; sums[6][p] = E.c;
     });
-    if (!lay.wrap) return;
     __syncthreads();
-    const float hx = __fmul_rn(-g.rho, g.dx) * 0.5f, h1 = __fmul_rn(-g.rho, g.dy) * 0.5f, h2 = __fmul_rn(-g.rho, g.dz) * 0.5f;
-    for (int c = 0; c < 4; c++) {
-        // the steps' signs along y and z where the one along x is upward
-        const float hy = (c & 1) ? -h1 : h1, hz = (c & 2) ? -h2 : h2;
-        // a step upward along an axis crosses the voxel's lower edge
-        const float *yd = (c & 1) ? syl : syu, *yu = (c & 1) ? syu : syl;
-        const float *zd = (c & 2) ? szl : szu, *zu = (c & 2) ? szu : szl;
+    for (int c = 0; c < 4; c++)
         at.diagonals(g, lay, c, [&](int p, uint32_t q) {
-            const float w = sc[p];
-            edge[(size_t)(2 * c) * (size_t)lay.stride + q] = make_float4(-hx * sxu[p], -hy * yd[p], -hz * zd[p], w);
-            edge[(size_t)(2 * c + 1) * (size_t)lay.stride + q] = make_float4(hx * sxl[p], hy * yu[p], hz * zu[p], w);
+            store_edges(g, lay, c, q, VoxelEdges{sums[0][p], sums[1][p], sums[2][p], sums[3][p], sums[4][p], sums[5][p], sums[6][p]}, edge);
         });
-    }
+}
+__global__ void __launch_bounds__(kTileThreads) k_pack_voxels(Grid g, PackIn in, float4 *f32, Layout lay, float4 *edge, float *curl_out)
+{
+    const long long v = (long long)blockIdx.x * kTileThreads + threadIdx.x;
+    if (v >= g.V) return;
+    const VoxelAt at(g, v);
+    const VoxelEdges E = pack_voxel(g, in, v, at.i, at.j, at.k, lay.wrap != 0, f32, curl_out);
+    if (!lay.wrap) return;
+#pragma unroll
+    for (int c = 0; c < 4; c++) store_edges(g, lay, c, layout_index(lay, g.X, g.Y, c, at.i, at.j, at.k), E, edge);
 }
 
 // |curl a| x mask with the reference's stencil and evaluation order (K:8352-8378).
@@ -718,10 +757,8 @@ cudaError_t init_accum_t(const Grid &g, const Layout &lay, const float *p_init, 
 template <typename ACC, typename T, typename F>
 cudaError_t fold_sums(const Grid &g, const Layout &lay, const Sums<T> &s, const F &f, cudaStream_t st)
 {
-    if (s.through) k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, (const T *)s.mem, Counted<ACC, F>{f, s.through});
-    else k_fold<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, reinterpret_cast<const ACC *>(s.mem), f);
-    OM_COUNT_LAUNCH();
-    return cudaGetLastError();
+    if (s.through) return fold_copies(g, lay, (const T *)s.mem, Counted<ACC, F>{f, s.through}, st);
+    return fold_copies(g, lay, reinterpret_cast<const ACC *>(s.mem), f, st);
 }
 
 }  // namespace
@@ -758,7 +795,8 @@ cudaError_t init_accum(const Grid &g, const Layout &lay, const float *p_init, bo
 cudaError_t spread_volume(const Grid &g, const Layout &lay, const float *in, float *out, cudaStream_t st)
 {
     if (!lay.wrap) return in == out ? cudaSuccess : cudaErrorInvalidValue;
-    k_spread<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, in, out);
+    if (by_tiles(g, lay)) k_spread<<<tile_blocks(g), kTileThreads, 0, st>>>(g, lay, in, out);
+    else k_spread_voxels<<<voxel_blocks(g), kTileThreads, 0, st>>>(g, lay, in, out);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }
@@ -767,7 +805,9 @@ cudaError_t pack_field(const Grid &g, const float *ax, const float *ay, const fl
                        Field *f, bool round_bf16, cudaStream_t st, float *curl_rounded)
 {
     if (!f->f32 || (f->lay.wrap && !f->edge)) return cudaErrorInvalidValue;
-    k_pack<<<tile_blocks(g), kTileThreads, 0, st>>>(g, ax, ay, az, curl, f->f32, f->lay, f->edge, curl_rounded, round_bf16 ? 1 : 0);
+    const PackIn in{ax, ay, az, curl, round_bf16 ? 1 : 0};
+    if (by_tiles(g, f->lay)) k_pack<<<tile_blocks(g), kTileThreads, 0, st>>>(g, in, f->f32, f->lay, f->edge, curl_rounded);
+    else k_pack_voxels<<<voxel_blocks(g), kTileThreads, 0, st>>>(g, in, f->f32, f->lay, f->edge, curl_rounded);
     OM_COUNT_LAUNCH();
     return cudaGetLastError();
 }

@@ -449,9 +449,7 @@ cudaError_t ensure_lines_through(Geometry *g, const Layout &lay, uint32_t *scrat
         OM_COUNT_LAUNCH();
         if ((e = cudaGetLastError()) != cudaSuccess || !fold) return e;
     }
-    k_fold<<<tile_blocks(g->grid), kTileThreads, 0, st>>>(g->grid, lay, (const uint32_t *)cnt, StoreCount{g->d_lines_through});
-    OM_COUNT_LAUNCH();
-    return cudaGetLastError();
+    return fold_copies(g->grid, lay, (const uint32_t *)cnt, StoreCount{g->d_lines_through}, st);
 }
 
 namespace {

@@ -106,6 +106,8 @@ __device__ __forceinline__ const float *gather_vector(const float *x, long long 
 // share the GPU with others, as it does in a batch's graph, where kernels that fill the SMs'
 // shared memory keep the members apart (16 plain snapshots: 15.6 ms so, 13.8 without).
 constexpr long long kIterSmemMin = 16384;  // smaller vectors stay in L1 anyway
+// (paired links always gather through L1: their stream takes longer than the gathers; 25 K anchors, 40^3
+// selected: 44 us an iteration from shared memory, 32 through L1)
 struct IterShape {
     bool smem;
     int threads, rows;
@@ -130,7 +132,7 @@ inline IterShape iter_shape(long long n, bool alone, int kind, uint32_t split)
 {
     IterShape s{};
     s.bytes = sizeof(float) * (split ? (size_t)split : (size_t)n);
-    s.smem = alone && n >= kIterSmemMin && s.bytes <= (size_t)kIterSmemMax;
+    s.smem = alone && kind == kLink16 && n >= kIterSmemMin;
     s.threads = s.smem ? 1024 : 256;
     // one CTA per SM above half of its shared memory, else two (2048 threads per SM)
     // at least as many rows as a warp takes at once: fewer blocks then hand in fewer change sums (32^3

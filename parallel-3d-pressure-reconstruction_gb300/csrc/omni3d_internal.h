@@ -344,6 +344,8 @@ cudaError_t normalize_fix(const Grid &g, const Layout &lay, const Sums<long long
 // Anchor operator (kernels_anchor.cu).
 struct Anchor {
     long long n = 0, nnz = 0;
+    unsigned long long slots = 0;   // link slots of all rows
+    long long placed = 0;           // walk generation + 1 whose lines' entries the anchors and row capacities are (0: none)
     uint8_t *flag = nullptr;        // V bytes: voxel is an anchor
     int32_t *wid = nullptr;         // the walks' copies of id (skewed layouts)
     int32_t *id = nullptr;          // V: anchor id or -1
@@ -368,7 +370,7 @@ struct Anchor {
 };
 // Builds the operator from the float4 entries of f (with BF16 storage they hold the stored
 // values); returns cudaErrorNotSupported (nothing filled) when it would hold more than
-// max_nnz entries (max_nnz < 0: no limit).
+// max_nnz entries (max_nnz < 0: no limit; 0: what 80 % of the free memory holds).
 // fx (bit-reproducible mode): the rows' (b, c) are summed in fixed point with the scales of
 // fix_fill_scales, which the caller sets before.
 // scratch: the layout's copies of a 4-byte volume, overwritten.

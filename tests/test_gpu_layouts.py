@@ -23,7 +23,7 @@ def _random_field(dims, seed, scale=1.0):
 @pytest.mark.parametrize("dims", [(2, 3, 5), (5, 2, 3), (31, 33, 32), (65, 5, 7), (4, 64, 33), (33, 3, 66)])
 def test_sweep_over_skewed_copies(omni, orc, dims, method):
     """One sweep of every method against the FP64 oracle, at the bar of the sweep parity test."""
-    h = 1e-3
+    h = (1e-3, 1e-3, 1e-3)
     dirs = omni.icosphere(3)
     a = _random_field(dims, 100)
     p = np.random.default_rng(101).normal(size=int(np.prod(dims))).astype(np.float32)
@@ -82,8 +82,9 @@ def test_plain_adjoint_is_the_transpose(omni, dims):
     assert abs(lhs - rhs) <= 1e-4 * abs(lhs)
 
 
-@pytest.mark.parametrize("scale", [1e-25, 1.0, 1e15])
-@pytest.mark.parametrize("method", ["plain", "select"])
+# (below about 1e-19 the curl's squares underflow, and a selected solve has no anchor to start from)
+@pytest.mark.parametrize("method,scale", [("plain", 1e-25), ("plain", 1.0), ("plain", 1e15), ("select", 1e-15),
+                                          ("select", 1.0), ("select", 1e15)])
 def test_fixed_point_scales(omni, method, scale):
     """The bit-reproducible mode's terms are scaled in FP32 by two factors: over magnitudes that
     need either, it agrees with the default mode to that mode's FP32 rounding."""
