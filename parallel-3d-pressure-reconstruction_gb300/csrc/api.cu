@@ -31,21 +31,30 @@ thread_local std::string g_error;
 struct DeviceBuf {
     void *p = nullptr;
     size_t n = 0;
+    bool part = false;  // a part of another buffer
     cudaError_t ensure(size_t bytes)
     {
         if (bytes <= n) return cudaSuccess;
-        cudaFree(p);
-        p = nullptr;
-        n = 0;
+        release();
         cudaError_t e = cudaMalloc(&p, bytes);
         if (e == cudaSuccess) n = bytes;
         return e;
     }
     void release()
     {
-        cudaFree(p);
+        if (!part) cudaFree(p);
         p = nullptr;
         n = 0;
+        part = false;
+    }
+    // Makes this buffer `bytes` of `whole` from `at` on; returns where they end.
+    size_t place(const DeviceBuf &whole, size_t at, size_t bytes)
+    {
+        release();
+        p = static_cast<char *>(whole.p) + at;
+        n = bytes;
+        part = true;
+        return at + (bytes + 255) / 256 * 256;
     }
     template <typename T>
     T *as() const { return reinterpret_cast<T *>(p); }
@@ -72,7 +81,8 @@ struct omni3d_ctx {
     DeviceBuf f32, curl;
     Layout lay;               // layout of the walks' copies of the field, pressure and sums
     bool lay_set = false;
-    DeviceBuf edge, pw;       // the walks' edge records (skewed layouts) and copies of the pressure
+    DeviceBuf copies;         // what the walks read and add to, one allocation:
+    DeviceBuf edge, pw;       // its edge records (skewed layouts), copies of the pressure (and pncnt)
     DeviceBuf pvol_a, pvol_b, pout, cnt, pncnt, scratch, flags;
     Anchor anc;
     bool anc_cached = false;  // plain method: operator structure built for this geometry
@@ -264,9 +274,13 @@ int ensure_layout(omni3d_ctx *ctx)
         ctx->lay_set = true;
     }
     const size_t n = (size_t)ctx->lay.copies * (size_t)g.V;
-    if (ctx->lay.wrap) CK(ctx, ctx->edge.ensure(2 * sizeof(float4) * n));
-    CK(ctx, ctx->pw.ensure(sizeof(float) * n));
-    CK(ctx, ctx->pncnt.ensure(sizeof(float2) * n));
+    if (!ctx->copies.p) {  // (a context's grid and layout never grow)
+        const size_t edge = ctx->lay.wrap ? 2 * sizeof(float4) * n : 0;
+        CK(ctx, ctx->copies.ensure(edge + (sizeof(float) + sizeof(float2)) * n + 3 * 256));
+        size_t at = ctx->edge.place(ctx->copies, 0, edge);
+        at = ctx->pw.place(ctx->copies, at, sizeof(float) * n);
+        ctx->pncnt.place(ctx->copies, at, sizeof(float2) * n);
+    }
     return OMNI3D_OK;
 }
 
@@ -278,7 +292,7 @@ bool drop_skewed(omni3d_ctx *ctx, int rc)
     cudaGetLastError();
     if (ctx->st) cudaStreamSynchronize(ctx->st);
     ctx->lay = row_major_layout(ctx->geo.grid);
-    for (DeviceBuf *b : {&ctx->edge, &ctx->pw, &ctx->pncnt, &ctx->pncnt64}) b->release();
+    for (DeviceBuf *b : {&ctx->edge, &ctx->pw, &ctx->pncnt, &ctx->pncnt64, &ctx->copies}) b->release();
     anchor_free(&ctx->anc);
     ctx->anc_cached = ctx->anc_last = false;
     return true;
@@ -294,7 +308,7 @@ cudaError_t start_volume(const Grid &g, const Layout &lay, const float *dpinit, 
 
 // Build the device field (float4 ax, ay, az, curl; optional bf16 copy; curl array).
 int prepare_field(omni3d_ctx *ctx, const float *ax, const float *ay, const float *az, const float *curl,
-                  const float *mask, bool dev, Field *F)
+                  const float *mask, bool dev, Field *F, const float *p = nullptr)
 {
     const Grid &g = ctx->geo.grid;
     const long long V = g.V;
@@ -327,7 +341,7 @@ int prepare_field(omni3d_ctx *ctx, const float *ax, const float *ay, const float
         rounded = ctx->curl.as<float>();
     }
     F->curl = rounded ? rounded : const_cast<float *>(dcurl);
-    CK(ctx, pack_field(g, dax, day, daz, dcurl, F, bf16, ctx->st, rounded));
+    CK(ctx, pack_field(g, dax, day, daz, dcurl, F, bf16, ctx->st, rounded, p, ctx->pw.as<float>()));
     return OMNI3D_OK;
 }
 
@@ -721,7 +735,7 @@ int omni3d_destroy(omni3d_ctx *ctx)
     adjoint_free(&ctx->adj);
     ctx->adj_g.release();
     ctx->adj_out.release();
-    for (DeviceBuf *b : {&ctx->in_ax, &ctx->in_ay, &ctx->in_az, &ctx->in_aux, &ctx->in_pinit, &ctx->f32, &ctx->edge, &ctx->pw,
+    for (DeviceBuf *b : {&ctx->in_ax, &ctx->in_ay, &ctx->in_az, &ctx->in_aux, &ctx->in_pinit, &ctx->f32, &ctx->copies, &ctx->edge, &ctx->pw,
                          &ctx->curl, &ctx->pvol_a, &ctx->pvol_b, &ctx->pout, &ctx->cnt, &ctx->pncnt, &ctx->scratch,
                          &ctx->flags, &ctx->centre, &ctx->pncnt64})
         b->release();
@@ -886,17 +900,17 @@ int sweep_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
     const Grid &g = ctx->geo.grid;
     const long long V = g.V;
     Field F;
-    int rc = prepare_field(ctx, ax, ay, az, curl, nullptr, dev, &F);
+    const float *dp;
+    int rc = stage(ctx, p, dev, ctx->in_pinit, V, &dp);
     if (rc) return rc;
+    if ((rc = prepare_field(ctx, ax, ay, az, curl, nullptr, dev, &F, dp))) return rc;  // and the copies of dp
     if (ctx->geo.walk_rule == 3) CK(ctx, run_walk(&ctx->geo, 3, F.curl, ctx->st));  // paths follow this field
-    const float *dp, *wp;
-    if ((rc = stage(ctx, p, dev, ctx->in_pinit, V, &dp))) return rc;
     const bool bf16 = ctx->prm.grad_storage == OMNI3D_GRAD_BF16;
     int engine = choose_engine(ctx, bf16, &rc);
     if (rc) return rc;
     if ((rc = engine_prepare(ctx, &engine, F, ctx->prm.method))) return rc;
     const Layout lay = engine_layout(engine, F);
-    CK(ctx, walk_pressure(ctx, lay, dp, &wp, ctx->st));
+    const float *wp = lay.wrap ? ctx->pw.as<float>() : dp;
     const Sums<float> acc = sweep_sums<float>(ctx, lay, ctx->pncnt);
     CK(ctx, init_accum(g, lay, nullptr, false, acc, ctx->st));
     CK(ctx, engine_sweep(ctx, engine, F, ctx->prm.method, wp, acc, ctx->st));

@@ -540,15 +540,22 @@ __global__ void __launch_bounds__(kTileThreads) k_pack(Grid g, PackIn in, float4
             store_edges(g, lay, c, q, VoxelEdges{sums[0][p], sums[1][p], sums[2][p], sums[3][p], sums[4][p], sums[5][p], sums[6][p]}, edge);
         });
 }
-__global__ void __launch_bounds__(kTileThreads) k_pack_voxels(Grid g, PackIn in, float4 *f32, Layout lay, float4 *edge, float *curl_out)
+// p, pw: as k_spread_voxels (null: not given); a launch less for a small sweep.
+__global__ void __launch_bounds__(kTileThreads) k_pack_voxels(Grid g, PackIn in, float4 *f32, Layout lay, float4 *edge, float *curl_out,
+                                                              const float *__restrict__ p, float *pw)
 {
     const long long v = (long long)blockIdx.x * kTileThreads + threadIdx.x;
     if (v >= g.V) return;
     const VoxelAt at(g, v);
     const VoxelEdges E = pack_voxel(g, in, v, at.i, at.j, at.k, lay.wrap != 0, f32, curl_out);
     if (!lay.wrap) return;
+    const float pv = p ? p[v] : 0.0f;
 #pragma unroll
-    for (int c = 0; c < 4; c++) store_edges(g, lay, c, layout_index(lay, g.X, g.Y, c, at.i, at.j, at.k), E, edge);
+    for (int c = 0; c < 4; c++) {
+        const uint32_t q = layout_index(lay, g.X, g.Y, c, at.i, at.j, at.k);
+        store_edges(g, lay, c, q, E, edge);
+        if (p) pw[(size_t)c * (size_t)lay.stride + q] = pv;
+    }
 }
 
 // |curl a| x mask with the reference's stencil and evaluation order (K:8352-8378).
@@ -802,14 +809,16 @@ cudaError_t spread_volume(const Grid &g, const Layout &lay, const float *in, flo
 }
 
 cudaError_t pack_field(const Grid &g, const float *ax, const float *ay, const float *az, const float *curl,
-                       Field *f, bool round_bf16, cudaStream_t st, float *curl_rounded)
+                       Field *f, bool round_bf16, cudaStream_t st, float *curl_rounded,
+                       const float *p, float *pw)
 {
     if (!f->f32 || (f->lay.wrap && !f->edge)) return cudaErrorInvalidValue;
     const PackIn in{ax, ay, az, curl, round_bf16 ? 1 : 0};
     if (by_tiles(g, f->lay)) k_pack<<<tile_blocks(g), kTileThreads, 0, st>>>(g, in, f->f32, f->lay, f->edge, curl_rounded);
-    else k_pack_voxels<<<voxel_blocks(g), kTileThreads, 0, st>>>(g, in, f->f32, f->lay, f->edge, curl_rounded);
+    else k_pack_voxels<<<voxel_blocks(g), kTileThreads, 0, st>>>(g, in, f->f32, f->lay, f->edge, curl_rounded, p, pw);
     OM_COUNT_LAUNCH();
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess && p && by_tiles(g, f->lay) ? spread_volume(g, f->lay, p, pw, st) : e;
 }
 
 namespace {

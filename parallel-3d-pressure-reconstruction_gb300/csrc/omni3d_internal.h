@@ -243,10 +243,10 @@ cudaError_t centre_integration(const Grid &g, const float *ax, const float *ay, 
 
 // Pack three component arrays (+ optional curl) into the field and its edge records.  With
 // round_bf16 the values are rounded to BF16 first, and the rounded curl is also written to
-// curl_rounded (when given; it may be curl).
+// curl_rounded (when given; it may be curl).  With p its copies for a sweep go to pw (skewed layouts).
 cudaError_t pack_field(const Grid &g, const float *ax, const float *ay, const float *az,
                        const float *curl, Field *f, bool round_bf16, cudaStream_t st,
-                       float *curl_rounded = nullptr);
+                       float *curl_rounded = nullptr, const float *p = nullptr, float *pw = nullptr);
 // The curl a solve used (.w of its packed FP32 field) into out.
 cudaError_t field_curl(long long V, const float4 *f32, float *out, cudaStream_t st);
 // |curl a| x mask into out (and into field .w when f is given).
