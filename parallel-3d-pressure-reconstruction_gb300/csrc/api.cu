@@ -1571,7 +1571,11 @@ int omni3d_batch_solve(omni3d_batch *b, const float *const *ax, const float *con
     }
     std::vector<const void *> key;
     for (int i = 0; i < n; i++) {
+        const omni3d_ctx *c = b->ctx[i];
         key.insert(key.end(), {dax[i], day[i], daz[i], dp0[i], dout[i], dcnt[i]});
+        // a member's own solve may have given up its copies, and its operator with them, since the capture
+        key.insert(key.end(), {c->f32.p, c->copies.p, reinterpret_cast<const void *>((uintptr_t)c->lay.wrap), c->anc.rowptr,
+                               c->anc.links, c->anc.wid, c->geo.d_lines_through});
     }
     cudaError_t e;
     if (!dev) {
