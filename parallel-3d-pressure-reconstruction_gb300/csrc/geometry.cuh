@@ -408,10 +408,15 @@ struct OmFastWalker {
 //
 // An axis at its exit coordinate has its candidate 60000 cells away, across the line by
 // 60000 sqrt(1 - k_a^2), far beyond the others unless the direction is within two degrees of the
-// axis: such directions take the exact form throughout.
+// axis: such directions take the exact form throughout.  So do those whose e = |k|^2 - 1 is above
+// kUnitMax: the "distances" then hold (e r)^2 with r up to 1.7 M, whose rounding is of first order
+// in r's.  Up to kUnitMax (directions in FP32, or written with five decimals) that adds
+// 2 e x 1.7 M x 12 u M, 5 u M at kFilterMax, and a candidate is at most e x 1.7 M = 0.2 further away,
+// which adds 2 u M.
 // 256^3 / 642 directions: 60 -> 31 ms (23.6 G steps over 67 grids and sets of directions: no step
 // other than the exact form's).
 constexpr int kFilterMax = 2048;
+constexpr float kUnitMax = 6.103515625e-5f;  // 2^-14
 struct OmFilteredWalker {
     float x, y, z, k1, k2, k3;
     float oi, oj, ok;     // exit voxel
@@ -432,14 +437,14 @@ struct OmFilteredWalker {
         ni = fabsf(oi - (float)ie); nj = fabsf(oj - (float)je); nk = fabsf(ok - (float)ke);
         const float a = (float)ie - x, b = (float)je - y, c = (float)ke - z;
         const float e = fmaf(k3, k3, fmaf(k2, k2, fmaf(k1, k1, -1.0f)));  // |k|^2 - 1
-        const float r = fmaf(k1, a, fmaf(k2, b, k3 * c)), t = fmaf(-e, r, r);
-        const float root = fmaf(-0.5f, e, 1.0f);
+        const float r = fmaf(k1, a, fmaf(k2, b, k3 * c)), t = fmaf(-e, r, r), f = 1.0f - e;  // g (k.w), g
+        const float root = sqrtf(f);
         ci = si * k1 * root; cj = sj * k2 * root; ck = sk * k3 * root;
-        Di = fmaf(2.0f * si, fmaf(-k1, t, a), -k1 * k1);
-        Dj = fmaf(2.0f * sj, fmaf(-k2, t, b), -k2 * k2);
-        Dk = fmaf(2.0f * sk, fmaf(-k3, t, c), -k3 * k3);
+        Di = fmaf(2.0f * si, fmaf(-k1, t, a), -f * k1 * k1);
+        Dj = fmaf(2.0f * sj, fmaf(-k2, t, b), -f * k2 * k2);
+        Dk = fmaf(2.0f * sk, fmaf(-k3, t, c), -f * k3 * k3);
         const float km = fmaxf(fmaxf(fabsf(k1), fabsf(k2)), fabsf(k3));
-        margin = km * km <= 0.999f ? 208.0f * 5.9604644775390625e-8f * (float)(max(max(g.X, g.Y), g.Z) + 8) : INFINITY;
+        margin = km * km <= 0.999f && fabsf(e) <= kUnitMax ? 208.0f * 5.9604644775390625e-8f * (float)(max(max(g.X, g.Y), g.Z) + 8) : INFINITY;
     }
 
     // OmFastWalker's step from the current voxel.
