@@ -207,13 +207,14 @@ __device__ __forceinline__ void om_cross2point(const Grid &g, float x, float y, 
 // A line of a general direction (case 7 alone) that certainly misses the volume: some pair of
 // axes has its projection outside the rectangle's by more than a thousand times what the roundings
 // of om_cross2point amount to (its accepted face points are off by 10 u M at most, M the longest
-// side).  Half of the lattice points of a cube miss, almost all of a long volume's; the full
+// side, times the largest component of k: of the rotation's k2 and k3 none is above 1, but k1 may be
+// anything).  Half of the lattice points of a cube miss, almost all of a long volume's; the full
 // evaluation takes 12 divisions.
 __device__ __forceinline__ bool om_certain_miss(const Grid &g, float x, float y, float z, float k1, float k2, float k3, int cases)
 {
     if (cases != 64) return false;
-    const float slack = 1.0e-3f * (float)max(max(g.X, g.Y), g.Z);
     const float a1 = fabsf(k1), a2 = fabsf(k2), a3 = fabsf(k3);
+    const float slack = 1.0e-3f * (float)max(max(g.X, g.Y), g.Z) * fmaxf(a1, 1.0f);
     return (fabsf(x * k2 - y * k1) > g.cx * a2 + g.cy * a1 + slack) | (fabsf(x * k3 - z * k1) > g.cx * a3 + g.cz * a1 + slack) |
            (fabsf(y * k3 - z * k2) > g.cy * a3 + g.cz * a2 + slack);
 }

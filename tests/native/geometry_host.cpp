@@ -61,13 +61,18 @@ long long filtered_walk_differences(int X, int Y, int Z, const float *k, long lo
     return differ;
 }
 
-// Of the n offsets, those om_certain_miss leaves out although `valid` says that the line crosses.
-long long wrong_misses(int X, int Y, int Z, const float *k, long long n, const int *valid, const float *xyz)
+// Of the n offsets, those that om_certain_miss leaves out although the line of direction k (case 7)
+// through them crosses the grid.
+long long wrong_misses(int X, int Y, int Z, const float *k, long long n, const float *xyz)
 {
     const Grid g = grid_of(X, Y, Z);
     long long wrong = 0;
-    for (long long l = 0; l < n; l++)
-        wrong += valid[l] && om_certain_miss(g, xyz[3 * l], xyz[3 * l + 1], xyz[3 * l + 2], k[0], k[1], k[2], 64);
+    for (long long l = 0; l < n; l++) {
+        const float *o = xyz + 3 * l;
+        int in[3], out[3];
+        om_cross2point(g, o[0], o[1], o[2], k[0], k[1], k[2], 64, in, out);
+        wrong += om_line_valid(g, in, out) && om_certain_miss(g, o[0], o[1], o[2], k[0], k[1], k[2], 64);
+    }
     return wrong;
 }
 

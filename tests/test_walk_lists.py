@@ -23,9 +23,9 @@ def native(tmp_path_factory):
                            "-I" + os.path.join(PKG, "csrc"), "-I" + os.path.join(REPO, "include"), "-I" + cuda,
                            os.path.join(HERE, "native", "geometry_host.cpp"), "-o", so])
     L = C.CDLL(so)
-    for f in (L.filtered_walk_differences, L.wrong_misses):
-        f.restype = C.c_longlong
-        f.argtypes = [C.c_int] * 3 + [C.c_void_p, C.c_longlong, C.c_void_p, C.c_void_p]
+    L.filtered_walk_differences.argtypes = [C.c_int] * 3 + [C.c_void_p, C.c_longlong, C.c_void_p, C.c_void_p]
+    L.wrong_misses.argtypes = [C.c_int] * 3 + [C.c_void_p, C.c_longlong, C.c_void_p]
+    L.filtered_walk_differences.restype = L.wrong_misses.restype = C.c_longlong
     return L
 
 
@@ -58,6 +58,26 @@ def test_filtered_walk_takes_the_reference_steps(orc, native, kind, dims):
         at = np.nonzero(valid)[0]
         io, o = np.ascontiguousarray(inout[at], np.int32), np.ascontiguousarray(xyz[at], np.float32)
         assert native.filtered_walk_differences(*dims, k.ctypes.data, len(at), io.ctypes.data, o.ctypes.data) == 0
+
+
+@pytest.mark.parametrize("k1", [0.8660254, -30.0, 3e3, -2e5, 1e8])
+def test_certain_misses_miss(native, k1):
+    """Lines through points within a few roundings of the grid's silhouette.  The rotation takes its
+    angles from k2 and k3, so a first component of any size is accepted, and the roundings grow with it."""
+    dims = (40, 37, 41)
+    c = (np.array(dims) - 1) / 2
+    rng = np.random.default_rng(111)
+    n = 200000
+    for k2, k3 in ((0.3, 0.4), (0.5, -0.2), (-0.01, 0.7)):
+        k = np.array([k1, k2, k3], np.float32)
+        # a point on an edge of the grid, moved along the direction and off it by a few ulp
+        at = rng.uniform(-1, 1, (n, 3)) * c
+        for a, side in zip(rng.permuted(np.tile(np.arange(3), (n, 1)), axis=1)[:, :2].T, rng.choice([-1, 1], (2, n))):
+            at[np.arange(n), a] = side * c[a]
+        at += rng.uniform(-60, 60, (n, 1)) * (k / np.linalg.norm(k))
+        at *= 1 + rng.integers(-8, 9, (n, 3)) * 2.0**-24
+        o = np.ascontiguousarray(at, np.float32)
+        assert native.wrong_misses(*dims, k.ctypes.data, n, o.ctypes.data) == 0
 
 
 @pytest.mark.gpu
