@@ -81,6 +81,7 @@ struct omni3d_ctx {
     DeviceBuf f32, curl;
     Layout lay;               // layout of the walks' copies of the field, pressure and sums
     bool lay_set = false;
+    bool no_copies = false;   // tests: the next use of the skewed copies finds no memory for them
     DeviceBuf copies;         // what the walks read and add to, one allocation:
     DeviceBuf edge, pw;       // its edge records (skewed layouts), copies of the pressure (and pncnt)
     DeviceBuf pvol_a, pvol_b, pout, cnt, pncnt, scratch, flags;
@@ -272,6 +273,10 @@ int ensure_layout(omni3d_ctx *ctx)
         size_t fr = 0, tot = 0;  // (a small context does not ask: the query takes longer than its first pass)
         if (need > (64u << 20) && (cudaMemGetInfo(&fr, &tot) != cudaSuccess || need > fr / 2)) ctx->lay = row_major_layout(g);
         ctx->lay_set = true;
+    }
+    if (ctx->no_copies && ctx->lay.wrap) {
+        ctx->no_copies = false;
+        return cuda_fail(ctx, cudaErrorMemoryAllocation, "skewed copies");
     }
     const size_t n = (size_t)ctx->lay.copies * (size_t)g.V;
     if (!ctx->copies.p) {  // (a context's grid and layout never grow)
@@ -1394,6 +1399,14 @@ void context_set_error(omni3d_ctx *ctx, const std::string &msg) { ctx->err = msg
 }  // namespace omni3d
 
 extern "C" {
+
+// For the tests, not part of omni3d.h: whether ctx walks skewed copies; with `lose` its next call
+// that uses them finds no memory for them.
+int omni3d_test_copies(omni3d_ctx *ctx, int lose)
+{
+    if (lose) ctx->no_copies = true;
+    return ctx->lay_set && ctx->lay.wrap ? 1 : 0;
+}
 
 // ------------------------------------------------------------------------- batches
 
