@@ -65,14 +65,6 @@ __device__ __forceinline__ float curl_of(const float4 &gv)
     return FB ? fabsf(gv.w) : gv.w;
 }
 
-__device__ __forceinline__ void kahan_add(float &s, float &c, float x)
-{
-    float y = x - c;
-    float t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
 enum Pass { kMark = 0, kFill = 2, kRhs = 3 };
 
 struct Sink {
@@ -219,7 +211,7 @@ struct FillLine {
     __device__ __forceinline__ void integrate(uint32_t c, int q, const float4 &gv, bool t)
     {
         const float x = step_increment<GRAD>(L, c, q, gv, gl);
-        I += t ? x : 0.0f;
+        I = __fadd_rn(I, t ? x : 0.0f);
         if (GRAD != kGradEdge) gl = gv;
     }
 };
@@ -373,7 +365,7 @@ struct SelectFill : FillLine<GRAD> {
     template <bool FLAGS>  // FLAGS: the curl may carry an anchor flag
     __device__ __forceinline__ void step(uint32_t c, int q, const float4 &gv, bool t)
     {
-        csum += (t ? curl_of<FLAGS>(gv) : 0.0f) * 1.0e-4f;  // the weights as in k_sweep_select
+        csum = add_curl(csum, t ? curl_of<FLAGS>(gv) : 0.0f);  // the weights as in k_sweep_select
         this->integrate(c, q, gv, t);
         nseg += t ? 1.0f : 0.0f;
     }
@@ -627,7 +619,8 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iter
             row_links<KIND>(links, j0, mine < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
                 const float y = SMEM ? x[c] : __ldg(x + c);
                 if (FIX) t += (long long)fix_term(KIND == kLinkPair ? w * y : y, sr);
-                else kahan_add(s, comp, KIND == kLinkPair ? w * y : y);
+                else if (KIND == kLinkPair) kahan_add_product(s, comp, w, y);
+                else kahan_add(s, comp, y);
             });
             __syncwarp();
             if (FIX) {

@@ -93,14 +93,6 @@ __device__ __forceinline__ void acc_add(const Scales<unsigned long long> &s, uns
     fix_add(reinterpret_cast<long long *>(entry(acc, v)), x, s.pn);
 }
 
-__device__ __forceinline__ void kahan_add(float &s, float &c, float x)
-{
-    float y = x - c;
-    float t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
 // n / csum for a batch of the walk (f.quick has seen csum far from the subnormal range): the
 // reciprocal's and the product's rounding, as __fdividef's within 2 ulp, without its scaling.
 __device__ __forceinline__ float quick_div(float n, float csum)
@@ -294,7 +286,7 @@ struct SelectWalk : LineSum<GRAD, ACC> {
         for (int q = 0; q < kWalkBatch; q++)
         {
             const bool t = taken<MASK>(idle, q);
-            csum += (t ? g[q].w : 0.0f) * 1.0e-4f;
+            csum = add_curl(csum, t ? g[q].w : 0.0f);
             this->integrate(c, q, g[q], t);
             nseg += t ? 1.0f : 0.0f;
             const float w = quick_div(nseg, csum);
@@ -323,7 +315,7 @@ struct SelectWalk : LineSum<GRAD, ACC> {
                 // weight n / sum(curl / 1e4) of the reference (K:2390-2392), as one fast
                 // division (within 2 ulp) instead of its two correctly rounded ones: the
                 // weights only scale averages, and the FP64-oracle bars hold
-                csum += g[q].w * 1.0e-4f;
+                csum = add_curl(csum, g[q].w);
                 nseg += 1.0f;
                 this->integrate(c, q, g[q], true);
                 const float w = __fdividef(nseg, csum);

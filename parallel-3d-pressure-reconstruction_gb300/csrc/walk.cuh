@@ -191,13 +191,32 @@ __device__ __forceinline__ void curl_range(const float4 (&g)[B], float &lo, floa
 }
 
 // The trapezoid increment of step q, gv the sample of the voxel it enters and gl that of the
-// voxel before (an edge record holds the increments of the octant's steps).
+// voxel before (an edge record holds the increments of the octant's steps).  Its roundings are
+// named, as are those of the sums it enters: an expression that the compiler may fuse with the next
+// addition would give other bits than the stored product of an edge record.
 template <int GRAD>
 __device__ __forceinline__ float step_increment(const LineWalk &L, uint32_t c, int q, const float4 &gv, const float4 &gl)
 {
     if (GRAD == kGradEdge) return by_axis(c, q, gv.x, gv.y, gv.z);
-    return by_axis(c, q, L.h0, L.h1, L.h2) * by_axis(c, q, gv.x + gl.x, gv.y + gl.y, gv.z + gl.z);
+    return __fmul_rn(by_axis(c, q, L.h0, L.h1, L.h2),
+                     by_axis(c, q, __fadd_rn(gv.x, gl.x), __fadd_rn(gv.y, gl.y), __fadd_rn(gv.z, gl.z)));
 }
+
+__device__ __forceinline__ void kahan_add(float &s, float &c, float x)
+{
+    const float y = __fsub_rn(x, c), t = __fadd_rn(s, y);
+    c = __fsub_rn(__fsub_rn(t, s), y);
+    s = t;
+}
+// s += w y, the product not rounded.
+__device__ __forceinline__ void kahan_add_product(float &s, float &c, float w, float y)
+{
+    const float p = __fmaf_rn(w, y, -c), t = __fadd_rn(s, p);
+    c = __fsub_rn(__fsub_rn(t, s), p);
+    s = t;
+}
+// The curl sum of the selected method after a voxel of curl cn.
+__device__ __forceinline__ float add_curl(float csum, float cn) { return __fmaf_rn(cn, 1.0e-4f, csum); }
 
 // The array a walk gathers from, at the lane's copy.
 template <int GRAD>

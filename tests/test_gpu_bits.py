@@ -1,0 +1,39 @@
+"""The bit-reproducible mode (params.deterministic) gives the bits of the inputs: not those of the
+layout a context's free memory allowed, of the line order, or of a field solved before."""
+import numpy as np
+import pytest
+from test_gpu_row_major import METHODS, _copies
+
+from omni3d import synthetic
+
+pytestmark = pytest.mark.gpu
+
+DIMS = (29, 33, 26)
+
+
+def _bits(a):
+    return np.ascontiguousarray(np.asarray(a, np.float32)).view(np.uint32)
+
+
+def _equal(a, b):
+    np.testing.assert_array_equal(_bits(a.p), _bits(b.p))
+    np.testing.assert_array_equal(_bits(a.count), _bits(b.count))
+
+
+def _field(orc):
+    f = synthetic.blobs(dims=DIMS, count=4, sigma_range=(2.0, 6.0), noise=0.10, seed=130, sphere_radius=4.0)
+    curl = orc.curl(DIMS, f["spacing"], f["ax"], f["ay"], f["az"], f["mask"])
+    return f, [f[k] for k in ("ax", "ay", "az")], curl, float(np.percentile(curl[curl > 0], 85))
+
+
+@pytest.mark.parametrize("solver", ["anchor", "sweep"])
+@pytest.mark.parametrize("method", METHODS)
+def test_bits_do_not_depend_on_the_layout(omni, orc, method, solver):
+    f, a, curl, thr = _field(orc)
+    with omni.Omni3D(DIMS, f["spacing"], omni.icosphere(3), max_iter=5, method=method, threshold=thr, gauge="mean",
+                     solver=solver, deterministic=True) as s:
+        skewed = s.solve(*a, curl=curl)
+        _copies(s, lose=True)
+        row_major = s.solve(*a, curl=curl)
+        assert _copies(s) == 0
+    _equal(row_major, skewed)
