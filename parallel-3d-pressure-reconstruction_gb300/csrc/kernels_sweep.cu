@@ -101,6 +101,15 @@ __device__ __forceinline__ float quick_div(float n, float csum)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(csum));
     return n * r;
 }
+// n / csum of a batch's contribution.  The fixed-point sums take the division of the general form:
+// which form a batch takes depends on all of a warp's lines, and the bits of the bit-reproducible mode
+// must not depend on the line order.
+template <typename ACC>
+__device__ __forceinline__ float batch_weight(float n, float csum)
+{
+    constexpr bool kFixed = std::is_same<ACC, long long>::value || std::is_same<ACC, unsigned long long>::value;
+    return kFixed ? __fdividef(n, csum) : quick_div(n, csum);
+}
 constexpr float kQuickMin = 1e-30f;  // least csum of a batch that uses quick_div
 constexpr float kQuickCurl = 1e-25f; // least curl of one that starts a sum
 constexpr uint32_t kAllIdle = 0x55555555u & ((1u << (2 * kWalkBatch)) - 1u);  // no step of the batch is the lane's
@@ -208,7 +217,7 @@ struct WeightedWalk : LineSum<GRAD, ACC> {
             csum += RAW ? cn : __fdiv_rn(cn, 1.0e4f);
             this->integrate(c, q, g[q], t);
             nseg += t ? 1.0f : 0.0f;
-            const float w = quick_div(nseg, csum);
+            const float w = batch_weight<ACC>(nseg, csum);
             if (t) this->add(v[q], (pe + this->I) * w, w);
         }
     }
@@ -289,7 +298,7 @@ struct SelectWalk : LineSum<GRAD, ACC> {
             csum = add_curl(csum, t ? g[q].w : 0.0f);
             this->integrate(c, q, g[q], t);
             nseg += t ? 1.0f : 0.0f;
-            const float w = quick_div(nseg, csum);
+            const float w = batch_weight<ACC>(nseg, csum);
             if (t) this->add(v[q], (p0 + this->I) * w, w);
         }
     }

@@ -37,3 +37,16 @@ def test_bits_do_not_depend_on_the_layout(omni, orc, method, solver):
         row_major = s.solve(*a, curl=curl)
         assert _copies(s) == 0
     _equal(row_major, skewed)
+
+
+@pytest.mark.parametrize("solver", ["anchor", "sweep"])
+@pytest.mark.parametrize("method", METHODS)
+def test_bits_do_not_depend_on_the_line_order(omni, orc, method, solver):
+    f, a, curl, thr = _field(orc)
+    runs = []
+    for tile_width, dir_group in ((8, 32), (4, 1), (16, 5)):
+        with omni.Omni3D(DIMS, f["spacing"], omni.icosphere(3), max_iter=5, method=method, threshold=thr, gauge="mean",
+                         solver=solver, deterministic=True, tile_width=tile_width, dir_group=dir_group) as s:
+            runs.append(s.solve(*a, curl=curl))
+    for r in runs[1:]:
+        _equal(r, runs[0])
