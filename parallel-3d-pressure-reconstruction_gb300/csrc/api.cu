@@ -971,14 +971,15 @@ cudaError_t iterate_chunk(omni3d_ctx *ctx, const Anchor &A, int gauge, long long
     if (e != cudaSuccess) return e;
     int *stop = ctx->iter_buf.as<int>();
     double *rels = ctx->iter_buf.as<double>() + 1;
-    uint64_t tol_bits;
+    uint64_t tol_bits, lmax_bits = 0;
     std::memcpy(&tol_bits, &tol, sizeof(tol_bits));
+    if (fx) std::memcpy(&lmax_bits, &fx->lmax, sizeof(lmax_bits));  // (its other bounds are the context's)
     const std::vector<const void *> key = {
         A.rowptr, A.rowlen, A.links, A.bc, A.vox, A.red, reinterpret_cast<const void *>((uintptr_t)A.n),
         reinterpret_cast<const void *>((uintptr_t)A.kind), pc, pn, red2,
         reinterpret_cast<const void *>((uintptr_t)gauge), reinterpret_cast<const void *>((intptr_t)ref_anchor),
         reinterpret_cast<const void *>((uintptr_t)tol_bits), stop, fx ? fx->scale : nullptr,
-        fx ? fx->bits : nullptr};
+        fx ? fx->bits : nullptr, reinterpret_cast<const void *>((uintptr_t)lmax_bits)};
     if (!ctx->iter_exec || ctx->iter_key != key) {
         if (ctx->iter_exec) cudaGraphExecDestroy(ctx->iter_exec);
         ctx->iter_exec = nullptr;
