@@ -706,8 +706,13 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iter
         ed = S[0] / N;
         ep = S[2] / N;
     }
-    const double change = fmax(0.0, S[1] - 2.0 * ed * S[0] + N * ed * ed);
-    const double norm = fmax(0.0, S[3] - 2.0 * ep * S[2] + N * ep * ep);
+    // sum (x - shift)^2 from sum x^2 and sum x: infinite and NaN sums stay so
+    auto moved = [&](double square, double linear, double shift) {
+        if (shift == 0.0 || (isfinite(shift) && !isfinite(square))) return square;
+        const double r = square - 2.0 * shift * linear + N * shift * shift;
+        return r < 0.0 ? 0.0 : r;
+    };
+    const double change = moved(S[1], S[0], ed), norm = moved(S[3], S[2], ep);
     C.red2[0] = change;
     C.red2[1] = norm;
     if (C.about) {
