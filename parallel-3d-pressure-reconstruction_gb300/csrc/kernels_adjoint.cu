@@ -107,23 +107,20 @@ struct LineProg {
     }
 };
 
-// Step decoder over a line's staircase (2-bit steps between its group's idle codes).
+// Step decoder over a line's staircase (2-bit steps), from its own entry.
 struct StepCursor {
     uint32_t word;
     uint32_t s;
     uint32_t v;
     __device__ __forceinline__ bool next(const LineWalk &L, int &a, uint32_t &prev)
     {
-        do {
-            if (s >= L.span) return false;
-            if ((s & 15) == 0) word = __ldg(L.dp + 32 * (s >> 4));
-            a = (int)(word & 3u);
-            word >>= 2;
-            s++;
-        } while (a == kIdle);
+        if (s >= L.m) return false;
+        if ((s & 15) == 0) word = L.own(s >> 4);
+        a = (int)(word & 3u);
+        word >>= 2;
+        s++;
         prev = v;
         v += (uint32_t)(a == 0 ? L.d0 : (a == 1 ? L.d1 : L.d2));
-        v = min(v, v + L.wv);
         return true;
     }
 };
@@ -144,7 +141,7 @@ __global__ void __launch_bounds__(256) k_adj_gather(Grid g, Layout lay, WalkLine
                                                     const int32_t *__restrict__ id, float *lam)
 {
     LineWalk L;
-    if (!L.init(g, lay, W) || !L.on) return;
+    if (!L.init<true>(g, lay, W) || !L.on) return;
     LineProg<ACC> P;
     float w;
     bool seg;
@@ -199,7 +196,7 @@ __global__ void __launch_bounds__(256) k_adj_grad(Grid g, Layout lay, WalkLines 
                                                   float *gx, float *gy, float *gz)
 {
     LineWalk L;
-    if (!L.init(g, lay, W) || !L.on) return;
+    if (!L.init<true>(g, lay, W) || !L.on) return;
     LineProg<ACC> P;
     float w;
     bool seg;
@@ -255,7 +252,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks) k_adj_gather_plain(Gr
     if (!L.init(g, lay, W)) return;
     mu += L.copy;
     SumAlong f{SELF ? __ldg(mu + L.v) : 0.0f};
-    walk_steps<kAdjBatch, kNoGrad, true>(L, nullptr, reinterpret_cast<const int32_t *>(mu), f);
+    walk_steps<kAdjBatch, kNoGrad, true, false>(L, nullptr, reinterpret_cast<const int32_t *>(mu), f);
     if (!L.on || f.t == 0.0f) return;
     const int row = __ldg(id + L.e);
     if (row >= 0) atomicAdd(lam + row, f.t);

@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kFillThreads, kFillBlocks)
 k_anchor_plain(Grid g, Layout lay, WalkLines W, WalkField F, Sink S)
 {
     LineWalk L;
-    if (!L.init(g, lay, W)) return;
+    if (!L.init<GRAD != kGradEdge>(g, lay, W)) return;
     if (PASS == kMark) {
         if (L.on) S.flag[L.e] = 1;
         return;
@@ -264,7 +264,7 @@ k_anchor_plain(Grid g, Layout lay, WalkLines W, WalkField F, Sink S)
     S.id += L.copy;
     PlainFill<GRAD, PASS, FB> f{{L, S, sample<GRAD>(field, L.v)}, start_col<PASS>(S, L.v)};
     if (SELF && L.on) emit_w<PASS, true>(S, __ldg(S.id + L.v), f.ecol, 1.0f, 0.0f);
-    walk_steps<kWalkBatch, GRAD, !FB>(L, field, S.id, f);
+    walk_steps<kWalkBatch, GRAD, !FB, GRAD != kGradEdge>(L, field, S.id, f);
 }
 
 // Weighted methods: the walks of k_sweep_weighted (K:1993-2135, RAW: K:2937-3085); anchors are
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kFillThreads, kFillBlocks)
 k_anchor_weighted(Grid g, Layout lay, WalkLines W, WalkField F, Sink S)
 {
     LineWalk L;
-    if (!L.init(g, lay, W)) return;
+    if (!L.init<GRAD != kGradEdge>(g, lay, W)) return;
     const float4 *field = lane_field<GRAD>(F, lay, L);
     S.id += L.copy;
     WeightedFill<GRAD, RAW, FB> f{{L, S, sample<GRAD>(field, L.v)}, start_col<kFill>(S, L.v), 0.0f, 0.0f};
@@ -331,7 +331,7 @@ k_anchor_weighted(Grid g, Layout lay, WalkLines W, WalkField F, Sink S)
         f.nseg = 1.0f;
         if (L.on) emit_w<kFill, false>(S, __ldg(S.id + L.v), f.ecol, __frcp_rn(f.csum), 0.0f);
     }
-    walk_steps<kWalkBatch, GRAD, !FB>(L, field, S.id, f);
+    walk_steps<kWalkBatch, GRAD, !FB, GRAD != kGradEdge>(L, field, S.id, f);
 }
 
 // Selected method: the state machine of k_sweep_select (K:2280-2537); anchors are the
@@ -412,7 +412,7 @@ struct SelectFill : FillLine<GRAD> {
 #pragma unroll
         for (int q = 0; q < kWalkBatch; q++) {
             rows[q] = -1;
-            if (open | anchor_of<FB>(g[q], id[q])) rows[q] = __ldg(this->S.id + v[q]);
+            if ((open | anchor_of<FB>(g[q], id[q])) & taken<MASK>(idle, q)) rows[q] = __ldg(this->S.id + v[q]);
             open = st.may_start_after(curl_of<FB>(g[q]), thr) | !taken<MASK>(idle, q);
         }
 #pragma unroll
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kFillThreads, kFillBlocks)
 k_anchor_select(Grid g, Layout lay, WalkLines W, WalkField F, const float *__restrict__ curl, Sink S)
 {
     LineWalk L;
-    if (!L.init(g, lay, W)) return;
+    if (!L.init<GRAD != kGradEdge>(g, lay, W)) return;
     const float4 *field = lane_field<GRAD>(F, lay, L);
     const float4 gl = sample<GRAD>(field, L.v);
     if (PASS == kFill) S.id += L.copy;
@@ -445,7 +445,7 @@ k_anchor_select(Grid g, Layout lay, WalkLines W, WalkField F, const float *__res
     st.enter(PASS == kFill ? curl_of<FB>(gl) : __ldg(curl + L.v), g.thr);
     if (PASS == kMark && st.run() && L.on) S.flag[L.v] = 1;
     SelectFill<GRAD, PASS, FB> f{{L, S, gl}, curl, g.thr, st, st.run() ? start_col<PASS>(S, L.v) : 0u};
-    walk_steps<kWalkBatch, GRAD, PASS == kFill && !FB>(L, field, S.id, f);
+    walk_steps<kWalkBatch, GRAD, PASS == kFill && !FB, GRAD != kGradEdge>(L, field, S.id, f);
 }
 
 // Selected method: a voxel can start a segment only if it is on the boundary (a line entry)

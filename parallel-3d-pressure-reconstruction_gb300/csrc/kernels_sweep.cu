@@ -173,11 +173,11 @@ k_sweep_plain(Grid g, Layout lay, WalkLines W,
               WalkField F, const float *__restrict__ p, ACC *pncnt, const double *__restrict__ fix)
 {
     LineWalk L;
-    if (!L.init(g, lay, W)) return;
+    if (!L.init<GRAD == kGradVoxel>(g, lay, W)) return;
     const float4 *field = lane_field<GRAD>(F, lay, L);
     PlainWalk<GRAD, ACC> f{{L, pncnt + L.copy, load_scales(fix, pncnt + L.copy, (size_t)lay.copies * (size_t)g.V), sample<GRAD>(field, L.v)}, __ldg(p + L.copy + L.v)};
     if (SELF && L.on) f.add(L.v, f.pe, 1.0f);
-    walk_steps<kWalkBatch, GRAD, false>(L, field, nullptr, f);
+    walk_steps<kWalkBatch, GRAD, false, GRAD == kGradVoxel>(L, field, nullptr, f);
 }
 
 // Weighted methods.  RAW = false (K:1993-2135): the entry receives nothing; step s of the line
@@ -245,7 +245,7 @@ k_sweep_weighted(Grid g, Layout lay, WalkLines W,
                  WalkField F, const float *__restrict__ p, ACC *pncnt, const double *__restrict__ fix)
 {
     LineWalk L;
-    if (!L.init(g, lay, W)) return;
+    if (!L.init<GRAD == kGradVoxel>(g, lay, W)) return;
     const float4 *field = lane_field<GRAD>(F, lay, L);
     WeightedWalk<GRAD, RAW, ACC> f{{L, pncnt + L.copy, load_scales(fix, pncnt + L.copy, (size_t)lay.copies * (size_t)g.V), sample<GRAD>(field, L.v)},
                                    __ldg(p + L.copy + L.v), 0.0f, 0.0f};
@@ -255,7 +255,7 @@ k_sweep_weighted(Grid g, Layout lay, WalkLines W,
         const float w0 = __frcp_rn(f.csum);
         if (L.on) f.add(L.v, f.pe * w0, w0);
     }
-    walk_steps<kWalkBatch, GRAD, false>(L, field, nullptr, f);
+    walk_steps<kWalkBatch, GRAD, false, GRAD == kGradVoxel>(L, field, nullptr, f);
 }
 
 // Selected method (K:2280-2537), state machine and asymmetries included: the entry is a
@@ -313,7 +313,7 @@ struct SelectWalk : LineSum<GRAD, ACC> {
 #pragma unroll
         for (int q = 0; q < kWalkBatch; q++) {
             ps[q] = 0.0f;
-            if (open) ps[q] = __ldg(p + v[q]);
+            if (open & taken<MASK>(idle, q)) ps[q] = __ldg(p + v[q]);
             open = st.may_start_after(g[q].w, thr) | !taken<MASK>(idle, q);
         }
 #pragma unroll
@@ -346,7 +346,7 @@ k_sweep_select(Grid g, Layout lay, WalkLines W,
                WalkField F, const float *__restrict__ p, ACC *pncnt, const double *__restrict__ fix)
 {
     LineWalk L;
-    if (!L.init(g, lay, W)) return;
+    if (!L.init<GRAD == kGradVoxel>(g, lay, W)) return;
     const float4 *field = lane_field<GRAD>(F, lay, L);
     p += L.copy;
     const float4 gl = sample<GRAD>(field, L.v);
@@ -354,7 +354,7 @@ k_sweep_select(Grid g, Layout lay, WalkLines W,
     st.enter(gl.w, g.thr);
     SelectWalk<GRAD, ACC> f{{L, pncnt + L.copy, load_scales(fix, pncnt + L.copy, (size_t)lay.copies * (size_t)g.V), gl}, p, g.thr, st,
                             st.run() ? __ldg(p + L.v) : 0.0f};
-    walk_steps<kWalkBatch, GRAD, false>(L, field, nullptr, f);
+    walk_steps<kWalkBatch, GRAD, false, GRAD == kGradVoxel>(L, field, nullptr, f);
 }
 
 // p = pn / count where count > 0, else the kept value; a pair of sums in FP32 or FP64.

@@ -167,10 +167,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_emit(Grid g, const DirEnt
 }
 
 // A lane's line of a group: its end voxels, its staircase length and the idle steps before it
-// enters, which bring the group's lines to one level.  A line that moves against its
-// direction's signs (directions with k3 = 0 have some, see om_cross2point) starts at once.
-// Every lane of the warp calls it; the lanes beyond the group's lines repeat the last one, so
-// that the walks need no test for them but where they write.
+// enters (line_lag).  Every lane of the warp calls it; the lanes beyond the group's lines repeat the
+// last one, so that the walks need no test for them but where they write.
 struct LaneLine {
     int ie, je, ke, ix, jx, kx, m, lag;
 };
@@ -180,10 +178,7 @@ __device__ __forceinline__ LaneLine lane_line(const Grid &g, const LineRec &r, i
     L.ie = (int)(r.e % (uint32_t)g.X); L.je = (int)((r.e / (uint32_t)g.X) % (uint32_t)g.Y); L.ke = (int)(r.e / (uint32_t)g.XY);
     L.ix = (int)(r.x % (uint32_t)g.X); L.jx = (int)((r.x / (uint32_t)g.X) % (uint32_t)g.Y); L.kx = (int)(r.x / (uint32_t)g.XY);
     L.m = abs(L.ix - L.ie) + abs(L.jx - L.je) + abs(L.kx - L.ke);
-    const bool regular = line_signs(L.ie, L.je, L.ke, L.ix, L.jx, L.kx, dir_signs) == (dir_signs & 7);
-    const int level = ((dir_signs & 1) ? L.ie : -L.ie) + ((dir_signs & 2) ? L.je : -L.je) + ((dir_signs & 4) ? L.ke : -L.ke);
-    const int low = __reduce_min_sync(0xffffffffu, regular ? level : 0x7fffffff);
-    L.lag = regular ? level - low : 0;
+    L.lag = line_lag(L.ie, L.je, L.ke, line_signs(L.ie, L.je, L.ke, L.ix, L.jx, L.kx, dir_signs), dir_signs);
     return L;
 }
 
@@ -278,13 +273,14 @@ struct CountVisits {
     __device__ __forceinline__ void general(uint32_t, uint32_t, const uint32_t (&)[4], const float4 (&)[4], const int32_t (&)[4]) const {}
 };
 
+template <bool OWN>
 __global__ void __launch_bounds__(kWalkThreads) k_lines_through(Grid g, Layout lay, WalkLines W, uint32_t *cnt)
 {
     LineWalk L;
-    if (!L.init(g, lay, W)) return;
+    if (!L.init<OWN>(g, lay, W)) return;
     CountVisits f{cnt + L.copy};
     if (L.on) atomicAdd(f.cnt + L.v, 1u);
-    walk_steps<4, kNoGrad, false>(L, nullptr, nullptr, f);
+    walk_steps<4, kNoGrad, false, OWN>(L, nullptr, nullptr, f);
 }
 
 // ---------------------------------------------------------------- scan
@@ -444,7 +440,8 @@ cudaError_t ensure_lines_through(Geometry *g, const Layout &lay, uint32_t *scrat
     e = cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (size_t)(fold ? lay.copies : 1) * (size_t)V, st);
     if (e != cudaSuccess || (g->n_lines == 0 && !fold)) return e;
     if (g->n_lines) {
-        k_lines_through<<<group_blocks(*g, kWalkThreads), kWalkThreads, 0, st>>>(
+        auto kernel = fold ? k_lines_through<false> : k_lines_through<true>;
+        kernel<<<group_blocks(*g, kWalkThreads), kWalkThreads, 0, st>>>(
             g->grid, fold ? lay : row_major_layout(g->grid), WalkLines{g->d_groups, g->n_groups, g->d_lines, g->d_desc}, cnt);
         OM_COUNT_LAUNCH();
         if ((e = cudaGetLastError()) != cudaSuccess || !fold) return e;

@@ -7,6 +7,12 @@
 // together.  The group's step words begin with idle codes on the lanes whose lines enter at a
 // higher level, and end with them on the lanes whose lines leave earlier.
 //
+// Over a row-major volume a level brings nothing: no two of its voxels share a row.  There every lane
+// starts at its own entry (OWN), its step words shifted past the idle codes: neighbouring lines
+// that enter by one face then read and write its rows together, and the warp is done after its
+// longest line.  64^3 / 642 directions, a row-major sweep: 1.41 -> 1.18 ms (1.12 before groups were
+// aligned by level, with warps of any 32 lines).
+//
 // A line's voxel addresses follow from its 2-bit steps alone, not from the values loaded
 // along it.  The walk therefore decodes a batch of B steps, issues the B gathers (and, with
 // AUX, B loads of an int32 per voxel from `aux`) before using any of them.  Without the batch
@@ -54,6 +60,17 @@ struct VoxelAt {
     }
 };
 
+// Idle steps before a lane's line enters, which bring the group's lines to one level: sg its step
+// signs, ds its direction's.  A line that moves against its direction's signs (directions with k3 = 0
+// have some, see om_cross2point) starts at once.  Every lane of the warp calls it.
+__device__ __forceinline__ int line_lag(int ie, int je, int ke, int sg, int ds)
+{
+    const bool regular = sg == (ds & 7);
+    const int level = ((ds & 1) ? ie : -ie) + ((ds & 2) ? je : -je) + ((ds & 4) ? ke : -ke);
+    const int low = __reduce_min_sync(0xffffffffu, regular ? level : 0x7fffffff);
+    return regular ? level - low : 0;
+}
+
 // One lane of a group: its line (none on the lanes beyond the group's lines) and where and
 // how it steps in the layout's copy for its step signs.
 struct LineWalk {
@@ -68,8 +85,12 @@ struct LineWalk {
     bool on;              // the lane has a line of its own (the lanes beyond the group's repeat the last one)
     uint32_t line;        // that line
     const uint32_t *dp;   // this lane's first step word
+    uint32_t m;           // steps of the line
+    uint32_t words;       // OWN: words at dp,
+    uint32_t shift;       // bits of the first one before the line's first step
 
-    // False when the warp has no group (whole warps).
+    // False when the warp has no group (whole warps).  OWN: the lane starts at its own entry.
+    template <bool OWN = false>
     __device__ __forceinline__ bool init(const Grid &g, const Layout &lay, const WalkLines &W)
     {
         const long long gi = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -86,7 +107,15 @@ struct LineWalk {
         const uint32_t X = (uint32_t)g.X, Y = (uint32_t)g.Y;
         const int ie = (int)(r.x % X), je = (int)((r.x / X) % Y), ke = (int)(r.x / (uint32_t)g.XY);
         const int ix = (int)(r.y % X), jx = (int)((r.y / X) % Y), kx = (int)(r.y / (uint32_t)g.XY);
-        const int sg = line_signs(ie, je, ke, ix, jx, kx, (int)(q.w >> kGroupSigns));
+        const int ds = (int)(q.w >> kGroupSigns), sg = line_signs(ie, je, ke, ix, jx, kx, ds);
+        m = r.w;
+        if (OWN) {
+            const uint32_t lag = (uint32_t)line_lag(ie, je, ke, sg, ds);
+            words = ((span + 15u) >> 4) - (lag >> 4);
+            dp += 32u * (lag >> 4);
+            shift = 2u * (lag & 15u);
+            span = __reduce_max_sync(0xffffffffu, m);
+        }
         const int si = (sg & 1) ? 1 : -1, sj = (sg & 2) ? 1 : -1, sk = (sg & 4) ? 1 : -1;
         // the reference forms -rho*s*dl in float and halves it in double (exact)
         h0 = __fmul_rn(-g.rho * (float)si, g.dx) * 0.5f;
@@ -113,6 +142,10 @@ struct LineWalk {
         }
         return true;
     }
+
+    // Word i of the lane's stored steps, OWN (idle past them), and the codes of its own steps 16 i on.
+    __device__ __forceinline__ uint32_t stored(uint32_t i) const { return i < words ? __ldg(dp + 32u * i) : 0xffffffffu; }
+    __device__ __forceinline__ uint32_t own(uint32_t i) const { return __funnelshift_r(stored(i), stored(i + 1), shift); }
 
     // The next voxel along axis code a (0, 1, 2).
     __device__ __forceinline__ void step(int a)
@@ -267,17 +300,24 @@ struct SelectState {
 //     f.quick<true>(idle, ...) holds on every lane (the ends of the groups: a third of the
 //     batches at 96^3, an eighth at 256^3);
 //   f.general<false or true>(...) otherwise.
-// The lanes beyond the group's lines take no steps.
-template <int B, int GRAD, bool AUX, typename F>
+// The lanes beyond the group's lines take no steps.  OWN: as L was initialised; a lane then gathers
+// nothing for a step that it does not take (1.18 -> 1.11 ms; over skewed copies it gathers its last
+// voxel again: the selected method's walks, bound by the ALU, were 2 % slower with the tests).
+template <int B, int GRAD, bool AUX, bool OWN, typename F>
 __device__ __forceinline__ void walk_steps(LineWalk &L, const float4 *field, const int32_t *aux, F &f)
 {
     static_assert(16 % B == 0, "a batch may not straddle step words");
     constexpr uint32_t kOnes = 0x55555555u & ((1u << (2 * B)) - 1u);
     const uint32_t off = L.on ? 0u : 0xffffffffu;
-    uint32_t next = L.span ? __ldg(L.dp) : 0u;
+    uint32_t next = L.span ? __ldg(L.dp) : 0u, after = OWN ? L.stored(1) : 0u;
     for (uint32_t s0 = 0; s0 < L.span; s0 += 16) {
-        uint32_t w = next | off;
-        if (s0 + 16 < L.span) next = __ldg(L.dp + 2 * s0 + 32);
+        uint32_t w = (OWN ? __funnelshift_r(next, after, L.shift) : next) | off;
+        if (OWN) {
+            next = after;
+            after = L.stored((s0 >> 4) + 2);
+        } else if (s0 + 16 < L.span) {
+            next = __ldg(L.dp + 2 * s0 + 32);
+        }
         const uint32_t n = min(16u, L.span - s0);  // codes past the span are idle
         for (uint32_t t0 = 0; t0 < n; t0 += B) {
             const uint32_t c = w;
@@ -303,10 +343,22 @@ __device__ __forceinline__ void walk_steps(LineWalk &L, const float4 *field, con
                     vv[q] = L.v;
                 }
             }
+            if (all | !OWN) {
 #pragma unroll
-            for (int q = 0; q < B; q++) {
-                g[q] = sample<GRAD>(field, vv[q]);
-                xw[q] = AUX ? __ldg(aux + vv[q]) : 0;
+                for (int q = 0; q < B; q++) {
+                    g[q] = sample<GRAD>(field, vv[q]);
+                    xw[q] = AUX ? __ldg(aux + vv[q]) : 0;
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < B; q++) {
+                    g[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    xw[q] = -1;
+                    if (taken<true>(idle, q)) {
+                        g[q] = sample<GRAD>(field, vv[q]);
+                        if (AUX) xw[q] = __ldg(aux + vv[q]);
+                    }
+                }
             }
             if (all) {
                 if (__all_sync(0xffffffffu, f.template quick<false>(0u, g, xw))) f.template batch<false>(c, 0u, vv, g, xw);

@@ -91,7 +91,7 @@ def test_row_major_operator_with_signed_curls(omni, orc):
 
 
 @pytest.mark.parametrize("method,mode", [("plain", 0), ("select", 1), ("weighted", 2)])
-@pytest.mark.parametrize("dims", [(2, 3, 5), (31, 33, 32), (65, 5, 7)])
+@pytest.mark.parametrize("dims", [(2, 3, 5), (31, 33, 32), (65, 5, 7), (4, 64, 33), (33, 3, 66), (48, 50, 47)])
 def test_row_major_sweep(omni, orc, dims, method, mode):
     rng = np.random.default_rng(121)
     a = [rng.normal(size=int(np.prod(dims))).astype(np.float32) for _ in range(3)]
