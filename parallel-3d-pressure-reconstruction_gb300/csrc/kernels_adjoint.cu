@@ -661,7 +661,7 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
     if (K > 1 && n) {
         k_adj_first<<<grid_for(n), 256, 0, st>>>(n, B->lam, A.bc, B->u, B->acc);
         OM_COUNT_LAUNCH();
-        const IterShape I = iter_shape(n, true, A.kind, A.split);
+        const IterShape I = iter_shape(n, true, A.kind, A.split, A.uneven);
         auto launch = [&](auto kernel) {
             if (I.bytes > 48 * 1024)
                 ADJ_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIterSmemMax));

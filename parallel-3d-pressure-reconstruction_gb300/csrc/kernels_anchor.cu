@@ -1073,8 +1073,10 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
 
     AN_TRY(grow(A->links, cap[11], link_bytes * (size_t)A->slots));
     AN_TRY(grow(A->bc, cap[13], sizeof(float2) * (size_t)n));
-    AN_TRY(grow(A->red, cap[6], sizeof(double) * (4 + 4 * (size_t)std::max(iter_shape(std::max<long long>(n, 1), true, A->kind, A->split).blocks,
-                                                                                iter_shape(std::max<long long>(n, 1), false, A->kind, A->split).blocks))));
+    A->uneven = geo.walk_rule == 3;
+    const long long n1 = std::max<long long>(n, 1);
+    AN_TRY(grow(A->red, cap[6], sizeof(double) * (4 + 4 * (size_t)std::max(iter_shape(n1, true, A->kind, A->split, A->uneven).blocks,
+                                                                           iter_shape(n1, false, A->kind, A->split, A->uneven).blocks))));
     AN_TRY(grow(A->pa, cap[15], sizeof(float) * (size_t)n));
     AN_TRY(grow(A->pb, cap[16], sizeof(float) * (size_t)n));
     AN_TRY(grow(A->rowlen, cap[17], sizeof(uint32_t) * (size_t)subrows));
@@ -1191,7 +1193,7 @@ cudaError_t anchor_step(const Anchor &A, const float *p_init, bool seed, bool fi
             C.rel_out = test->rel_out;
         }
     }
-    const IterShape I = iter_shape(A.n, alone, A.kind, A.split);
+    const IterShape I = iter_shape(A.n, alone, A.kind, A.split, A.uneven);
     auto launch = [&](auto kernel) {
         if (I.bytes > 48 * 1024) {  // (a host-side attribute of the kernel: cheap, and safe while capturing)
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIterSmemMax);

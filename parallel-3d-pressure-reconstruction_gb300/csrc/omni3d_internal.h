@@ -355,6 +355,7 @@ struct Anchor {
     void *links = nullptr;          // per link the start anchor and, in weighted operators, the weight
     int kind = 0;                   // LinkKind of the links (links.cuh)
     uint32_t split = 0;             // columns of a panel (links.cuh); 0: one panel.  Two: rows 2 i, 2 i + 1 are row i's
+    bool uneven = false;            // rows of very unequal lengths (minimum-curl walks; see iter_shape)
     int panels() const { return split ? 2 : 1; }
     float2 *bc = nullptr;           // n: (b, c) = (sum of w * I, sum of w)
     float *pa = nullptr, *pb = nullptr;  // iterates
