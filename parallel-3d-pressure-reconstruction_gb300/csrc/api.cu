@@ -1378,8 +1378,13 @@ int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *
         gy = gx + V;
         gz = gy + V;
     }
-    CK(ctx, adjoint_solve(ctx->geo, ctx->anc, &ctx->adj, ctx->last_iterations, P.method, ctx->f32.as<float4>(),
-                          ctx->lay, ctx->pw.as<float>(), gg, ctx->cnt.as<float>(), gx, gy, gz, st));
+    const cudaError_t ae = adjoint_solve(ctx->geo, ctx->anc, &ctx->adj, ctx->last_iterations, P.method, ctx->f32.as<float4>(),
+                                         ctx->lay, ctx->pw.as<float>(), gg, ctx->cnt.as<float>(), gx, gy, gz, st);
+    if (ae != cudaSuccess) {
+        cudaGetLastError();
+        adjoint_free(&ctx->adj);  // the next call must not find half of a transposed operator
+        return cuda_fail(ctx, ae, "adjoint");
+    }
     if (!dev) {
         CK(ctx, cudaMemcpyAsync(grad_ax, gx, sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, st));
         CK(ctx, cudaMemcpyAsync(grad_ay, gy, sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, st));
@@ -1408,6 +1413,8 @@ int omni3d_test_copies(omni3d_ctx *ctx, int lose)
     if (lose) ctx->no_copies = true;
     return ctx->lay_set && ctx->lay.wrap ? 1 : 0;
 }
+// The transposed operator's links of ctx's next adjoint find no memory.
+void omni3d_test_no_adjoint_links(omni3d_ctx *ctx) { ctx->adj.no_links = true; }
 
 // ------------------------------------------------------------------------- batches
 

@@ -544,6 +544,19 @@ void adjoint_free(AdjointBuffers *B)
         if (e_ != cudaSuccess) return e_;        \
     } while (0)
 
+// A temporary of the transposed operator's build, freed on every way out.
+struct AdjTemp {
+    void *p = nullptr;
+    template <typename T>
+    cudaError_t alloc(T **out, size_t elems)
+    {
+        const cudaError_t e = cudaMalloc(&p, sizeof(T) * std::max<size_t>(elems, 1));
+        *out = e == cudaSuccess ? static_cast<T *>(p) : nullptr;
+        return e;
+    }
+    ~AdjTemp() { cudaFree(p); }
+};
+
 template <int ACC>
 void launch_adj_lines(const Geometry &geo, bool gather, const float4 *f32, const float *in, const int32_t *id,
                       float *lam, float *gx, float *gy, float *gz, cudaStream_t st)
@@ -607,12 +620,13 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
     const unsigned row_blocks = (unsigned)((n * 32 + 255) / 256);
     if (!B->tptr) {
         const long long trows = n * A.panels();
+        AdjTemp t64_mem, tmp_mem, tcur_mem;
         unsigned long long *t64 = nullptr, *tmp = nullptr;
         uint32_t *tcur = nullptr;
         ADJ_TRY(cudaMalloc(&B->tlen, sizeof(uint32_t) * (size_t)std::max(trows, 1LL)));
-        ADJ_TRY(cudaMalloc(&tcur, sizeof(uint32_t) * (size_t)std::max(trows, 1LL)));
-        ADJ_TRY(cudaMalloc(&t64, sizeof(unsigned long long) * (size_t)std::max(trows, 1LL)));
-        ADJ_TRY(cudaMalloc(&tmp, sizeof(unsigned long long) * scan_tmp_elems(trows)));
+        ADJ_TRY(tcur_mem.alloc(&tcur, (size_t)trows));
+        ADJ_TRY(t64_mem.alloc(&t64, (size_t)trows));
+        ADJ_TRY(tmp_mem.alloc(&tmp, scan_tmp_elems(trows)));
         ADJ_TRY(cudaMalloc(&B->tptr, sizeof(unsigned long long) * (size_t)(trows + 1)));
         ADJ_TRY(cudaMemsetAsync(B->tlen, 0, sizeof(uint32_t) * (size_t)std::max(trows, 1LL), st));
         auto count = [&](auto kernel) { kernel<<<row_blocks, 256, 0, st>>>(n, A.split, A.rowptr, A.rowlen, A.links, B->tlen); };
@@ -627,6 +641,7 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
         unsigned long long tn = 0;
         ADJ_TRY(cudaMemcpyAsync(&tn, B->tptr + trows, sizeof(tn), cudaMemcpyDeviceToHost, st));
         ADJ_TRY(cudaStreamSynchronize(st));
+        if (B->no_links) return cudaErrorMemoryAllocation;
         ADJ_TRY(cudaMalloc(&B->tlinks, link_size(A.kind) * (size_t)std::max(tn, 1ULL)));
         ADJ_TRY(cudaMemsetAsync(tcur, 0, sizeof(uint32_t) * (size_t)std::max(trows, 1LL), st));
         auto fill = [&](auto kernel) { kernel<<<row_blocks, 256, 0, st>>>(n, A.split, A.rowptr, A.rowlen, A.links, B->tptr, tcur, B->tlinks); };
@@ -637,9 +652,6 @@ cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *
         }
         ADJ_TRY(cudaGetLastError());
         ADJ_TRY(cudaStreamSynchronize(st));
-        cudaFree(tcur);
-        cudaFree(t64);
-        cudaFree(tmp);
     }
     // mu = g / c; lambda_{K-1} = S^T mu
     k_adj_mu<<<grid_for(V), 256, 0, st>>>(V, g, cnt, B->mu);

@@ -423,11 +423,13 @@ struct AdjointBuffers {
     void *tlinks = nullptr;              // and links, of the operator's kind
     float *mu = nullptr, *lam = nullptr, *u = nullptr, *unext = nullptr, *acc = nullptr;
     float *edges = nullptr;  // the plain methods' dL/de, 3 axes of every copy of the layout
+    bool no_links = false;   // tests: the transposed links find no memory
 };
 void adjoint_free(AdjointBuffers *B);
 // gx, gy, gz = d<g, p_K>/d(ax, ay, az) for `method` after K iterations with the curl held
 // fixed, given the operator A of that solve, its per-voxel count cnt and its packed FP32
-// field f32 (whose .w holds the curl the solve used); copies: a volume in every copy of lay.
+// field f32 (whose .w holds the curl the solve used); copies: a volume in every copy of lay.  After an
+// error B may hold a part of the transposed operator: adjoint_free it.
 cudaError_t adjoint_solve(const Geometry &geo, const Anchor &A, AdjointBuffers *B, int K, int method,
                           const float4 *f32, const Layout &lay, float *copies, const float *g, const float *cnt,
                           float *gx, float *gy, float *gz, cudaStream_t st);

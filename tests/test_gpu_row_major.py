@@ -152,3 +152,25 @@ def test_batch_member_that_loses_its_copies(omni, method):
     finally:
         for s in members:
             s.close()
+
+
+@pytest.mark.parametrize("method", ["plain", "select"])
+def test_adjoint_after_one_that_found_no_memory(omni, orc, method):
+    """An adjoint that could not allocate its transposed links leaves nothing of them behind."""
+    dims = (13, 11, 10)
+    f, curl, thr = _field(orc, dims, 124)
+    g = np.random.default_rng(8).normal(size=int(np.prod(dims))).astype(np.float32)
+    with omni.Omni3D(dims, f["spacing"], omni.icosphere(2), max_iter=4, method=method, threshold=thr) as s:
+        _copies(s, lose=True)
+        s.solve(f["ax"], f["ay"], f["az"], curl=curl)
+        fail = lib().omni3d_test_no_adjoint_links
+        fail.restype, fail.argtypes = None, [C.c_void_p]
+        fail(s.handle)
+        with pytest.raises(omni.Omni3DError) as e:
+            s.adjoint(g)
+        assert e.value.code == -4
+        after = s.adjoint(g)
+    with omni.Omni3D(dims, f["spacing"], omni.icosphere(2), max_iter=4, method=method, threshold=thr) as s:
+        s.solve(f["ax"], f["ay"], f["az"], curl=curl)
+        for a, b in zip(after, s.adjoint(g)):
+            assert synthetic.relative_l2(a, b, gauge="none") < 1e-5
