@@ -1327,19 +1327,18 @@ int omni3d_solve(omni3d_ctx *ctx, const float *ax, const float *ay, const float 
     return rc;
 }
 
-int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *grad_ay, float *grad_az,
-                   int device_ptrs)
+namespace {
+
+// The adjoint of the gauged g (ctx->adj_g) into gx, gy, gz.  *nomem: an allocation failed.
+int adjoint_impl(omni3d_ctx *ctx, float *gx, float *gy, float *gz, bool *nomem)
 {
-    if (!ctx || !grad_p || !grad_ax || !grad_ay || !grad_az) return fail(ctx, OMNI3D_ERR_ARG, "NULL argument");
-    if (ctx->last_iterations < 0) return fail(ctx, OMNI3D_ERR_STATE, "no solve to differentiate on this context");
-    cudaSetDevice(ctx->prm.device);
     const omni3d_params &P = ctx->prm;
     const Grid &g = ctx->geo.grid;
     const long long V = g.V;
-    const bool dev = device_ptrs != 0;
     cudaStream_t st = ctx->st;
     const long long ref = (long long)P.ref_i + (long long)P.ref_j * g.X + (long long)P.ref_k * g.XY;
     const bool plain = P.method == OMNI3D_METHOD_PLAIN;
+    *nomem = false;
     // the plain operator's structure and anchor counts depend on the geometry alone; the other
     // methods' weights depend on the curl, so their operator must be the last solve's
     if (plain ? !ctx->anc_cached : !ctx->anc_last) {  // the last solve ran the sweep form: build it now
@@ -1355,11 +1354,37 @@ int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *
         std::string aerr;
         cudaError_t e = anchor_build(ctx->geo, F, P.method, P.gauge == OMNI3D_GAUGE_POINT ? ref : -1,
                                      -1, &ctx->anc, st, &aerr, nullptr, ctx->pw.as<uint32_t>());
-        if (e != cudaSuccess) return fail(ctx, OMNI3D_ERR_CUDA, "anchor operator: " + aerr);
+        if (e != cudaSuccess) {
+            *nomem = e == cudaErrorMemoryAllocation;
+            return fail(ctx, OMNI3D_ERR_CUDA, "anchor operator: " + aerr);
+        }
         ctx->anc_cached = plain;
         ctx->anc_last = true;
         adjoint_free(&ctx->adj);
     }
+    const cudaError_t e = adjoint_solve(ctx->geo, ctx->anc, &ctx->adj, ctx->last_iterations, P.method, ctx->f32.as<float4>(),
+                                        ctx->lay, ctx->pw.as<float>(), ctx->adj_g.as<float>(), ctx->cnt.as<float>(), gx, gy, gz, st);
+    if (e == cudaSuccess) return OMNI3D_OK;
+    *nomem = e == cudaErrorMemoryAllocation;
+    cudaGetLastError();
+    adjoint_free(&ctx->adj);  // the next call must not find half of a transposed operator
+    return cuda_fail(ctx, e, "adjoint");
+}
+
+}  // namespace
+
+int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *grad_ay, float *grad_az,
+                   int device_ptrs)
+{
+    if (!ctx || !grad_p || !grad_ax || !grad_ay || !grad_az) return fail(ctx, OMNI3D_ERR_ARG, "NULL argument");
+    if (ctx->last_iterations < 0) return fail(ctx, OMNI3D_ERR_STATE, "no solve to differentiate on this context");
+    cudaSetDevice(ctx->prm.device);
+    const omni3d_params &P = ctx->prm;
+    const Grid &g = ctx->geo.grid;
+    const long long V = g.V;
+    const bool dev = device_ptrs != 0;
+    cudaStream_t st = ctx->st;
+    const long long ref = (long long)P.ref_i + (long long)P.ref_j * g.X + (long long)P.ref_k * g.XY;
     const float *dg = grad_p;
     CK(ctx, ctx->adj_g.ensure(sizeof(float) * (size_t)V));
     if (!dev) {
@@ -1370,21 +1395,22 @@ int omni3d_adjoint(omni3d_ctx *ctx, const float *grad_p, float *grad_ax, float *
     CK(ctx, ctx->scratch.ensure(sizeof(double) * std::max(change_scratch_doubles(),
                                                           std::max(gauge_scratch_doubles(),
                                                                    gauge_transpose_scratch_doubles())) + 64));
-    float *gg = ctx->adj_g.as<float>();
-    CK(ctx, gauge_transpose(V, P.gauge, ref, dg, ctx->cnt.as<float>(), gg, ctx->scratch.as<double>() + 4, st));
+    CK(ctx, gauge_transpose(V, P.gauge, ref, dg, ctx->cnt.as<float>(), ctx->adj_g.as<float>(), ctx->scratch.as<double>() + 4,
+                            st));
     float *gx = grad_ax, *gy = grad_ay, *gz = grad_az;
     if (!dev) {
         gx = ctx->adj_out.as<float>();
         gy = gx + V;
         gz = gy + V;
     }
-    const cudaError_t ae = adjoint_solve(ctx->geo, ctx->anc, &ctx->adj, ctx->last_iterations, P.method, ctx->f32.as<float4>(),
-                                         ctx->lay, ctx->pw.as<float>(), gg, ctx->cnt.as<float>(), gx, gy, gz, st);
-    if (ae != cudaSuccess) {
-        cudaGetLastError();
-        adjoint_free(&ctx->adj);  // the next call must not find half of a transposed operator
-        return cuda_fail(ctx, ae, "adjoint");
+    bool nomem;
+    int rc = adjoint_impl(ctx, gx, gy, gz, &nomem);
+    if (nomem && drop_skewed(ctx, OMNI3D_ERR_NOMEM)) {  // the memory may be in the skewed copies: once more without
+        adjoint_free(&ctx->adj);
+        if ((rc = ensure_layout(ctx))) return rc;
+        rc = adjoint_impl(ctx, gx, gy, gz, &nomem);
     }
+    if (rc) return rc;
     if (!dev) {
         CK(ctx, cudaMemcpyAsync(grad_ax, gx, sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, st));
         CK(ctx, cudaMemcpyAsync(grad_ay, gy, sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, st));

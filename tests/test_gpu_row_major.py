@@ -174,3 +174,37 @@ def test_adjoint_after_one_that_found_no_memory(omni, orc, method):
         s.solve(f["ax"], f["ay"], f["az"], curl=curl)
         for a, b in zip(after, s.adjoint(g)):
             assert synthetic.relative_l2(a, b, gauge="none") < 1e-5
+
+
+@pytest.mark.parametrize("gauge", ["none", "mean"])
+@pytest.mark.parametrize("method", METHODS)
+def test_adjoint_gives_up_the_copies_for_memory(omni, orc, method, gauge):
+    """Links that find no memory beside the skewed copies find it without them: the adjoint starts over
+    row-major, and the solves after it are."""
+    torch = pytest.importorskip("torch")
+    dims = (13, 11, 10)
+    f, curl, thr = _field(orc, dims, 125)
+    g = np.random.default_rng(9).normal(size=int(np.prod(dims))).astype(np.float32)
+    a = [f[k] for k in ("ax", "ay", "az")]
+    fail = lib().omni3d_test_no_adjoint_links
+    fail.restype, fail.argtypes = None, [C.c_void_p]
+    with omni.Omni3D(dims, f["spacing"], omni.icosphere(2), max_iter=4, method=method, threshold=thr, gauge=gauge) as s:
+        first = s.solve(*a, curl=curl)
+        want = s.adjoint(g)
+        for device in (False, True):
+            with omni.Omni3D(dims, f["spacing"], omni.icosphere(2), max_iter=4, method=method, threshold=thr,
+                             gauge=gauge) as t:
+                t.solve(*a, curl=curl)
+                fail(t.handle)
+                if device:  # the gradient's own memory takes the result
+                    x = torch.tensor(g, device="cuda")
+                    rest = [torch.empty_like(x) for _ in range(2)]
+                    torch.cuda.synchronize()
+                    assert lib().omni3d_adjoint(t.handle, x.data_ptr(), x.data_ptr(), *[r.data_ptr() for r in rest], 1) == 0
+                    got = [r.cpu().numpy().reshape(dims[::-1]) for r in (x, *rest)]
+                else:
+                    got = t.adjoint(g)
+                assert _copies(t) == 0
+                for p, q in zip(got, want):
+                    assert synthetic.relative_l2(p, q, gauge="none") < 1e-5
+                _same(t.solve(*a, curl=curl), first, method)
