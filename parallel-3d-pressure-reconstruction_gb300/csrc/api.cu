@@ -82,6 +82,7 @@ struct omni3d_ctx {
     Layout lay;               // layout of the walks' copies of the field, pressure and sums
     bool lay_set = false;
     bool no_copies = false;   // tests: the next use of the skewed copies finds no memory for them
+    size_t test_memory = 0;   // tests: device memory there would be without the copies (0: ask the driver)
     DeviceBuf copies;         // what the walks read and add to, one allocation:
     DeviceBuf edge, pw;       // its edge records (skewed layouts), copies of the pressure (and pncnt)
     DeviceBuf pvol_a, pvol_b, pout, cnt, pncnt, scratch, flags;
@@ -260,6 +261,15 @@ int stage(omni3d_ctx *ctx, const float *src, bool dev, DeviceBuf &buf, long long
     return OMNI3D_OK;
 }
 
+// Free device memory; false when the driver does not say.
+bool free_memory(const omni3d_ctx *ctx, size_t *fr)
+{
+    size_t tot = 0;
+    if (!ctx->test_memory) return cudaMemGetInfo(fr, &tot) == cudaSuccess;
+    *fr = ctx->test_memory - std::min(ctx->test_memory, ctx->copies.n);
+    return true;
+}
+
 // The layout of a context's walks, chosen at its first field: skewed copies, unless they and
 // what goes with them would take more than half of the free device memory.
 int ensure_layout(omni3d_ctx *ctx)
@@ -270,8 +280,8 @@ int ensure_layout(omni3d_ctx *ctx)
         const omni3d_params &P = ctx->prm;
         const size_t entry = 2 * sizeof(float4) + sizeof(float) + sizeof(int32_t) + sizeof(float2) + (P.sweep_fp64 || P.deterministic ? sizeof(double2) : 0);
         const size_t need = entry * (size_t)ctx->lay.copies * (size_t)g.V;
-        size_t fr = 0, tot = 0;  // (a small context does not ask: the query takes longer than its first pass)
-        if (need > (64u << 20) && (cudaMemGetInfo(&fr, &tot) != cudaSuccess || need > fr / 2)) ctx->lay = row_major_layout(g);
+        size_t fr = 0;  // (a small context does not ask: the query takes longer than its first pass)
+        if ((need > (64u << 20) || ctx->test_memory) && (!free_memory(ctx, &fr) || need > fr / 2)) ctx->lay = row_major_layout(g);
         ctx->lay_set = true;
     }
     if (ctx->no_copies && ctx->lay.wrap) {
@@ -1112,8 +1122,10 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
             aerr = cudaGetErrorString(e);
         } else {
             ctx->anc_cached = false;
-            e = anchor_build(ctx->geo, F, P.method, P.gauge == OMNI3D_GAUGE_POINT ? ref : -1,
-                             std::max(P.anchor_max_links, 0LL),
+            long long limit = std::max(P.anchor_max_links, 0LL);
+            size_t fr = 0;
+            if (limit == 0 && ctx->test_memory && free_memory(ctx, &fr)) limit = anchor_link_limit(fr);
+            e = anchor_build(ctx->geo, F, P.method, P.gauge == OMNI3D_GAUGE_POINT ? ref : -1, limit,
                              &ctx->anc, st, &aerr, fx, ctx->pw.as<uint32_t>());
             ctx->anc_cached = e == cudaSuccess && P.method == OMNI3D_METHOD_PLAIN;
             adjoint_free(&ctx->adj);
@@ -1121,6 +1133,11 @@ int solve_impl(omni3d_ctx *ctx, const float *ax, const float *ay, const float *a
         ctx->anc_last = e == cudaSuccess;
         if (e == cudaErrorNotSupported) {
             cudaGetLastError();
+            // the copies' memory would let it pass: iterations without copies cost less than sweeps with them
+            size_t fr = 0;
+            const size_t held = ctx->copies.n + ctx->pncnt64.n + ctx->anc.cap[1] - (sizeof(float) + sizeof(float2)) * (size_t)V;
+            if (P.anchor_max_links == 0 && ctx->lay.wrap && free_memory(ctx, &fr) && ctx->anc.nnz <= anchor_link_limit(fr + held))
+                return fail(ctx, OMNI3D_ERR_NOMEM, "anchor operator: no room beside the skewed copies");
             solver = OMNI3D_SOLVER_SWEEP;  // operator not profitable: one sweep per iteration
         } else if (e != cudaSuccess) {
             return fail(ctx, e == cudaErrorMemoryAllocation ? OMNI3D_ERR_NOMEM : OMNI3D_ERR_CUDA,
@@ -1439,6 +1456,8 @@ int omni3d_test_copies(omni3d_ctx *ctx, int lose)
     if (lose) ctx->no_copies = true;
     return ctx->lay_set && ctx->lay.wrap ? 1 : 0;
 }
+// ctx takes this for the device memory that is free when it holds no copies.
+void omni3d_test_memory(omni3d_ctx *ctx, long long bytes) { ctx->test_memory = (size_t)bytes; }
 // The transposed operator's links of ctx's next adjoint find no memory.
 void omni3d_test_no_adjoint_links(omni3d_ctx *ctx) { ctx->adj.no_links = true; }
 

@@ -1061,10 +1061,10 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
     const long long subrows = (long long)n * A->panels();
     const size_t link_bytes = link_size(A->kind);
     long long limit = max_nnz;
-    if (max_nnz == 0) {  // what 80 % of the free memory holds (column + weight); links that fit in place always do (asking takes 23 us)
+    if (max_nnz == 0) {  // links that fit in place always pass (asking takes 23 us)
         size_t fr = 0, tot = 0;
         if (link_bytes * (size_t)A->slots <= cap[11]) limit = -1;
-        else if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) limit = (long long)(0.8 * (double)fr / 8.0);
+        else if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) limit = anchor_link_limit(fr);
     }
     if (limit >= 0 && A->nnz > limit) {
         if (err) *err = "anchor operator larger than its limit";

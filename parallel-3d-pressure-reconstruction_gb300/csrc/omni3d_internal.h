@@ -379,6 +379,8 @@ cudaError_t anchor_build(Geometry &geo, const Field &f, int method, long long re
                          long long max_nnz, Anchor *A, cudaStream_t st, std::string *err,
                          Fixed *fx, uint32_t *scratch);
 void anchor_free(Anchor *A);
+// Entries that an operator may hold in `fr` bytes of free memory: 80 % of it (column + weight).
+inline long long anchor_link_limit(size_t fr) { return (long long)(0.8 * (double)fr / 8.0); }
 // Plain method: recompute only b (the field-dependent part) of an operator built by
 // anchor_build for the same geometry; rows, columns and c depend on the geometry alone.
 cudaError_t anchor_refresh_rhs(const Geometry &geo, const Field &f, Anchor *A, cudaStream_t st,

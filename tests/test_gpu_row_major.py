@@ -208,3 +208,32 @@ def test_adjoint_gives_up_the_copies_for_memory(omni, orc, method, gauge):
                 for p, q in zip(got, want):
                     assert synthetic.relative_l2(p, q, gauge="none") < 1e-5
                 _same(t.solve(*a, curl=curl), first, method)
+
+
+def test_operator_that_fits_without_the_copies(omni):
+    """Whether the anchor operator passes its automatic limit does not depend on the skewed copies: they
+    go when it fits only without them.  40^3 voxels: copies of 176 bytes a voxel, at most half of the free memory."""
+    dims = (40, 40, 40)
+    f = synthetic.blobs(dims=dims, count=4, sigma_range=(3.0, 8.0), noise=0.05, seed=126)
+    a = [f[k] for k in ("ax", "ay", "az")]
+    memory = lib().omni3d_test_memory
+    memory.restype, memory.argtypes = None, [C.c_void_p, C.c_longlong]
+
+    def solve(nbytes):
+        with omni.Omni3D(dims, f["spacing"], omni.icosphere(4), max_iter=5, gauge="mean") as s:
+            if nbytes:
+                memory(s.handle, nbytes)
+            r = s.solve(*a)
+            return r, _copies(s)
+
+    want, copies = solve(0)
+    assert copies == 1
+    need = 10 * want.stats["n_links"]  # 80 % hold 8 bytes a link
+    copied = 176 * 40**3
+    assert 2 * 192 * 40**3 < need - need // 100  # skewed copies are taken in all three
+    for nbytes, solver, skewed in ((need + copied // 2, 0, 0),  # the operator fits without the copies,
+                                   (need + copied + 4096, 0, 1),  # beside them,
+                                   (need - need // 100, 1, 1)):  # not at all
+        r, copies = solve(nbytes)
+        assert (r.stats["solver_used"], copies) == (solver, skewed)
+        _same(r, want, "plain")
