@@ -82,6 +82,7 @@ struct omni3d_ctx {
     Layout lay;               // layout of the walks' copies of the field, pressure and sums
     bool lay_set = false;
     bool no_copies = false;   // tests: the next use of the skewed copies finds no memory for them
+    int tuned = -1;           // the line order was timed over skewed copies (1), row-major (0)
     size_t test_memory = 0;   // tests: device memory there would be without the copies (0: ask the driver)
     DeviceBuf copies;         // what the walks read and add to, one allocation:
     DeviceBuf edge, pw;       // its edge records (skewed layouts), copies of the pressure (and pncnt)
@@ -270,18 +271,26 @@ bool free_memory(const omni3d_ctx *ctx, size_t *fr)
     return true;
 }
 
-// The layout of a context's walks, chosen at its first field: skewed copies, unless they and
-// what goes with them would take more than half of the free device memory.
+// The layout of a context's walks: skewed copies, unless they and what goes with them would take more
+// than half of the free device memory.
+Layout choose_layout(const omni3d_ctx *ctx)
+{
+    const Grid &g = ctx->geo.grid;
+    const omni3d_params &P = ctx->prm;
+    const Layout lay = skewed_layout(g);
+    const size_t entry = 2 * sizeof(float4) + sizeof(float) + sizeof(int32_t) + sizeof(float2) + (P.sweep_fp64 || P.deterministic ? sizeof(double2) : 0);
+    const size_t need = entry * (size_t)lay.copies * (size_t)g.V;
+    size_t fr = 0;  // (a small context does not ask: the query takes longer than its first pass)
+    if ((need > (64u << 20) || ctx->test_memory) && (!free_memory(ctx, &fr) || need > fr / 2)) return row_major_layout(g);
+    return lay;
+}
+
+// Chooses the layout at a context's first field and allocates the copies.
 int ensure_layout(omni3d_ctx *ctx)
 {
     const Grid &g = ctx->geo.grid;
     if (!ctx->lay_set) {
-        ctx->lay = skewed_layout(g);
-        const omni3d_params &P = ctx->prm;
-        const size_t entry = 2 * sizeof(float4) + sizeof(float) + sizeof(int32_t) + sizeof(float2) + (P.sweep_fp64 || P.deterministic ? sizeof(double2) : 0);
-        const size_t need = entry * (size_t)ctx->lay.copies * (size_t)g.V;
-        size_t fr = 0;  // (a small context does not ask: the query takes longer than its first pass)
-        if ((need > (64u << 20) || ctx->test_memory) && (!free_memory(ctx, &fr) || need > fr / 2)) ctx->lay = row_major_layout(g);
+        ctx->lay = choose_layout(ctx);
         ctx->lay_set = true;
     }
     if (ctx->no_copies && ctx->lay.wrap) {
@@ -560,17 +569,17 @@ namespace {
 
 // Line-order tuning (params.autotune).  The line order decides which voxels the lanes of a
 // warp, and the warps of a block, touch at the same time, so the best tile width and
-// direction group depend on the grid and the direction set.  Each candidate pair is built
-// and timed with one plain sweep of a zero field (the sweep's cost depends on where its
-// gathers and reductions land, not on the values); the fastest pair is kept for the process,
-// per device and size class.
+// direction group depend on the grid and the direction set.  Each candidate pair is built and timed
+// with one plain sweep of a zero field over the layout that the context's walks will have (the
+// sweep's cost depends on where its gathers and reductions land, not on the values); the
+// fastest pair is kept for the process, per device, layout and size class.
 struct TuneKey {
-    int device, size_class, nv, rule;
+    int device, size_class, nv, rule, skewed;
     uint32_t ls_bits;
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(device, size_class, nv, rule, ls_bits) <
-               std::tie(o.device, o.size_class, o.nv, o.rule, o.ls_bits);
+        return std::tie(device, size_class, nv, rule, skewed, ls_bits) <
+               std::tie(o.device, o.size_class, o.nv, o.rule, o.skewed, o.ls_bits);
     }
 };
 std::mutex g_tune_mutex;
@@ -583,55 +592,57 @@ cudaError_t tune_line_order(omni3d_ctx *ctx, std::string *err)
     uint32_t ls_bits;
     std::memcpy(&ls_bits, &g.ls, sizeof(ls_bits));
     const int mx = std::max(std::max(g.X, g.Y), g.Z);
-    const TuneKey key{ctx->prm.device, (mx + 31) / 32, geo.nv, geo.walk_rule, ls_bits};
     std::lock_guard<std::mutex> lock(g_tune_mutex);
+    TuneKey key{ctx->prm.device, (mx + 31) / 32, geo.nv, geo.walk_rule, choose_layout(ctx).wrap ? 1 : 0, ls_bits};
     auto it = g_tune_cache.find(key);
-    if (it != g_tune_cache.end()) {
-        geo.tile_width = it->second.first;
-        geo.dir_group = it->second.second;
-        return cudaSuccess;
-    }
-    static const int kCand[][2] = {{8, 4}, {4, 4}, {16, 4}, {8, 2}, {8, 8}};
-    float4 *field = nullptr;
-    float *p = nullptr;
-    float2 *acc = nullptr;
-    const size_t V = (size_t)g.V;
-    cudaError_t e = cudaMalloc(&field, sizeof(float4) * V);
-    if (e == cudaSuccess) e = cudaMalloc(&p, sizeof(float) * V);
-    if (e == cudaSuccess) e = cudaMalloc(&acc, sizeof(float2) * V);
-    if (e == cudaSuccess) e = cudaMemsetAsync(field, 0, sizeof(float4) * V, ctx->st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, sizeof(float) * V, ctx->st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, sizeof(float2) * V, ctx->st);
-    float best = 0.0f;
     int bt = 8, bg = 4;
-    for (const auto &c : kCand) {
-        if (e != cudaSuccess) break;
-        geo.tile_width = c[0];
-        geo.dir_group = c[1];
-        if ((e = build_geometry(&geo, ctx->st, err)) != cudaSuccess) break;
+    cudaError_t e = cudaSuccess;
+    if (it != g_tune_cache.end()) {
+        bt = it->second.first;
+        bg = it->second.second;
+    } else {  // over the copies that the context's first field would get, given back below
+        DeviceBuf field;
+        int rc = ensure_layout(ctx);
+        if (drop_skewed(ctx, rc)) rc = ensure_layout(ctx);
+        if (rc != OMNI3D_OK) e = rc == OMNI3D_ERR_NOMEM ? cudaErrorMemoryAllocation : cudaErrorUnknown;
         Field F;
-        F.f32 = field;
-        F.lay = row_major_layout(g);
-        e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, p, Sums<float>{(float *)acc}, ctx->st);  // warm-up
-        cudaEventRecord(ctx->ev[2], ctx->st);
-        if (e == cudaSuccess) e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, p, Sums<float>{(float *)acc}, ctx->st);
-        cudaEventRecord(ctx->ev[3], ctx->st);
-        if (e == cudaSuccess) e = cudaEventSynchronize(ctx->ev[3]);
-        const float ms = ms_between(ctx->ev[2], ctx->ev[3]);
-        free_geometry(&geo);
-        if (e == cudaSuccess && (best == 0.0f || ms < best)) {
-            best = ms;
-            bt = c[0];
-            bg = c[1];
+        F.lay = ctx->lay;
+        key.skewed = F.lay.wrap ? 1 : 0;
+        if (e == cudaSuccess && !F.lay.wrap) e = field.ensure(sizeof(float4) * (size_t)g.V);
+        if (e == cudaSuccess && !F.lay.wrap) e = cudaMemsetAsync(field.p, 0, field.n, ctx->st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(ctx->copies.p, 0, ctx->copies.n, ctx->st);
+        F.f32 = field.as<float4>();
+        F.edge = F.lay.wrap ? ctx->edge.as<float4>() : nullptr;
+        const Sums<float> acc{ctx->pncnt.as<float>(), nullptr};
+        float best = 0.0f;
+        static const int kCand[][2] = {{8, 4}, {4, 4}, {16, 4}, {8, 2}, {8, 8}};
+        for (const auto &c : kCand) {
+            if (e != cudaSuccess) break;
+            geo.tile_width = c[0];
+            geo.dir_group = c[1];
+            if ((e = build_geometry(&geo, ctx->st, err)) != cudaSuccess) break;
+            e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, ctx->pw.as<float>(), acc, ctx->st);  // warm-up
+            cudaEventRecord(ctx->ev[2], ctx->st);
+            if (e == cudaSuccess) e = sweep_full(geo, F, OMNI3D_METHOD_PLAIN, ctx->pw.as<float>(), acc, ctx->st);
+            cudaEventRecord(ctx->ev[3], ctx->st);
+            if (e == cudaSuccess) e = cudaEventSynchronize(ctx->ev[3]);
+            const float ms = ms_between(ctx->ev[2], ctx->ev[3]);
+            free_geometry(&geo);
+            if (e == cudaSuccess && (best == 0.0f || ms < best)) {
+                best = ms;
+                bt = c[0];
+                bg = c[1];
+            }
         }
+        if (e == cudaSuccess) g_tune_cache[key] = {bt, bg};
+        field.release();
+        for (DeviceBuf *b : {&ctx->edge, &ctx->pw, &ctx->pncnt, &ctx->copies}) b->release();
+        ctx->lay_set = false;
     }
-    cudaFree(field);
-    cudaFree(p);
-    cudaFree(acc);
     if (e != cudaSuccess) return e;
     geo.tile_width = bt;
     geo.dir_group = bg;
-    g_tune_cache[key] = {bt, bg};
+    ctx->tuned = key.skewed;
     return cudaSuccess;
 }
 
@@ -707,10 +718,11 @@ int omni3d_create(const omni3d_params *params, omni3d_ctx **out)
         return bail(e, "upload dirs");
     ctx->geo.tile_width = params->tile_width ? params->tile_width : 8;
     // Direction groups: up to 2^24 voxels, 32 directions walked through each lattice patch
-    // together share the filling pass's gathers in L1 and L2 (256^3 / 642 directions: 124.8
-    // against 127.2 ms per solve with groups of 4; 192^3: 53.5 against 55.1 ms); on larger
-    // grids the final sweep's footprint outgrows the L2 and groups of 4 win (320^3: 256.7
-    // against 260.9 ms with 16; 512^3: 1385 against 1551 ms with 32).
+    // together share the passes' gathers in L1 and L2 (642 directions, a solve over skewed copies:
+    // 256^3 77.4 against 84.5 ms with groups of 4; 192^3 34.1 against 36.1 ms; 128^3 11.3 ms with
+    // either).  The line lies where the row-major walks' footprint outgrew the L2 (320^3: 256.7 ms
+    // with 4, 260.9 with 16; 512^3: 1385 with 4, 1551 with 32).  Skewed copies take larger groups well
+    // above it too: 320^3 193.8 ms with 4, 164.1 with 16, 162.8 with 32; 384^3 379.6, 326.0, 332.2.
     ctx->geo.dir_group = params->dir_group ? params->dir_group : (ctx->geo.grid.V <= (1LL << 24) ? 32 : 4);
     std::string gerr;
     if (params->autotune && (e = tune_line_order(ctx, &gerr)) != cudaSuccess) {
@@ -1456,6 +1468,8 @@ int omni3d_test_copies(omni3d_ctx *ctx, int lose)
     if (lose) ctx->no_copies = true;
     return ctx->lay_set && ctx->lay.wrap ? 1 : 0;
 }
+// What ctx's line order was tuned on: 1 skewed copies, 0 the row-major volume, -1 nothing.
+int omni3d_test_tuned(const omni3d_ctx *ctx) { return ctx->tuned; }
 // ctx takes this for the device memory that is free when it holds no copies.
 void omni3d_test_memory(omni3d_ctx *ctx, long long bytes) { ctx->test_memory = (size_t)bytes; }
 // The transposed operator's links of ctx's next adjoint find no memory.
