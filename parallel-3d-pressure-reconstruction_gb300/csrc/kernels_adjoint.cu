@@ -27,6 +27,7 @@
 #include "fold.cuh"
 #include "links.cuh"
 #include "omni3d_internal.h"
+#include "sums.cuh"
 #include "walk.cuh"
 
 namespace omni3d {
@@ -363,7 +364,7 @@ __global__ void k_adj_tcount(long long n, uint32_t split, const unsigned long lo
     const uint32_t panels = split ? 2 : 1, mine = split && row >= split ? 1 : 0;
     for (uint32_t p = 0; p < panels; p++)
         row_links<KIND>(links, rowptr[row * panels + p], rowlen[row * panels + p], threadIdx.x & 31,
-                        [&](uint32_t c, float) { atomicAdd(tcnt + (size_t)(c + p * split) * panels + mine, 1u); });
+                        [&](uint32_t c, float, int) { atomicAdd(tcnt + (size_t)(c + p * split) * panels + mine, 1u); });
 }
 
 template <int KIND>
@@ -375,7 +376,7 @@ __global__ void k_adj_tfill(long long n, uint32_t split, const unsigned long lon
     if ((threadIdx.x & 31) >= lanes_per_row(KIND)) return;
     const uint32_t panels = split ? 2 : 1, mine = split && row >= split ? 1 : 0;
     for (uint32_t p = 0; p < panels; p++)
-        row_links<KIND>(links, rowptr[row * panels + p], rowlen[row * panels + p], threadIdx.x & 31, [&](uint32_t c, float w) {
+        row_links<KIND>(links, rowptr[row * panels + p], rowlen[row * panels + p], threadIdx.x & 31, [&](uint32_t c, float w, int) {
             const size_t t = (size_t)(c + p * split) * panels + mine;
             store_link<KIND>(tlinks, tptr[t] + atomicAdd(tcur + t, 1u), (uint32_t)row - mine * split, w);
         });
@@ -428,11 +429,12 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 4) k_adj_iterate
             const int at = r + lane / kLanes;
             const unsigned long long j0 = __shfl_sync(0xffffffffu, ptr, at & 31);
             const uint32_t m = __shfl_sync(0xffffffffu, len, at & 31);
-            float s = 0.0f;
-            row_links<KIND>(tlinks, j0, at < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
+            LaneSum q;
+            row_links<KIND>(tlinks, j0, at < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w, int i) {
                 const float y = SMEM ? x[c] : __ldg(x + c);
-                s += KIND == kLinkPair ? w * y : y;
+                q.add(i, KIND == kLinkPair ? w * y : y);
             });
+            float s = q.total();
             __syncwarp();
             for (int o = kLanes / 2; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             s = __shfl_sync(0xffffffffu, s, ((lane - r) * kLanes) & 31);  // the row of lane r + i

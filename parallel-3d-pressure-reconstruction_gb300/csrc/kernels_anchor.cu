@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iter
             const uint32_t m = __shfl_sync(0xffffffffu, len, mine & 31);
             float s = 0.0f, comp = 0.0f;
             long long t = 0;
-            row_links<KIND>(links, j0, mine < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w) {
+            row_links<KIND>(links, j0, mine < rows ? m : 0u, lane % kLanes, [&](uint32_t c, float w, int) {
                 const float y = SMEM ? x[c] : __ldg(x + c);
                 if (FIX) t += (long long)fix_term(KIND == kLinkPair ? w * y : y, sr);
                 else if (KIND == kLinkPair) kahan_add_product(s, comp, w, y);

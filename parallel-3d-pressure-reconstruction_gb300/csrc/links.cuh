@@ -28,8 +28,8 @@ __host__ __device__ constexpr size_t link_size(int kind) { return kind == kLinkP
 // 20 loads per lane, four of them in flight, and a warp works on several rows at once.
 __host__ __device__ constexpr int lanes_per_row(int kind) { return kind == kLinkPair ? 32 : (kind == kLink32 ? 16 : 8); }
 
-// add(index, weight) for the links of this lane (of lanes_per_row) of a row of m links at
-// `links` (entry j0, aligned).
+// add(index, weight, i) for the links of this lane (of lanes_per_row) of a row of m links at
+// `links` (entry j0, aligned); i: the link's place in its unrolled load, known at compile time.
 template <int KIND, typename F>
 __device__ __forceinline__ void row_links(const void *links, unsigned long long j0, uint32_t m, int lane, F &&add)
 {
@@ -44,7 +44,7 @@ __device__ __forceinline__ void row_links(const void *links, unsigned long long 
                 if (v + u * S < m) x[u] = __ldg(q + v + u * S);
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                if (v + u * S < m) add(x[u].x, __uint_as_float(x[u].y));
+                if (v + u * S < m) add(x[u].x, __uint_as_float(x[u].y), u);
         }
     } else {
         constexpr uint32_t W = links_per_vector(KIND);
@@ -61,18 +61,18 @@ __device__ __forceinline__ void row_links(const void *links, unsigned long long 
 #pragma unroll
             for (int u = 0; u < 4; u++)
 #pragma unroll
-                for (uint32_t k = 0; k < W; k++) add(at(x[u], k), 1.0f);
+                for (uint32_t k = 0; k < W; k++) add(at(x[u], k), 1.0f, (int)k);
         }
         for (; v < full; v += S) {
             const uint4 x = __ldg(q + v);
 #pragma unroll
-            for (uint32_t k = 0; k < W; k++) add(at(x, k), 1.0f);
+            for (uint32_t k = 0; k < W; k++) add(at(x, k), 1.0f, (int)k);
         }
         if (v == full && W * full < m) {  // the slots past the row's links hold nothing
             const uint4 x = __ldg(q + full);
 #pragma unroll
             for (uint32_t k = 0; k < W; k++)
-                if (W * full + k < m) add(at(x, k), 1.0f);
+                if (W * full + k < m) add(at(x, k), 1.0f, (int)k);
         }
     }
 }
