@@ -522,18 +522,11 @@ __global__ void k_row_capacity(long long n, const uint32_t *vox, const uint32_t 
     if ((threadIdx.x & 31) == 0 && t) atomicAdd(total, t);
 }
 
-// Row sums of the anchor iteration: compensated (Kahan) FP32 per lane, the lane sums added as
-// unevaluated pairs (hi, lo) with error-free additions, about 46 bits, and the row's update in
-// FP64.  A row gathers about as many terms as lines cross its voxel (~1000 at 642 directions);
-// plain FP32 sums of that many terms leave a rounding floor near 1e-6 in the iteration's
-// relative change, above the tolerances the solver is asked for.
-__device__ __forceinline__ void add_pair(float &hi, float &lo, float h2, float l2)
-{
-    const float t = __fadd_rn(hi, h2), b = __fsub_rn(t, hi);
-    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(h2, b));  // hi + h2 = t + e exactly
-    lo = __fadd_rn(__fadd_rn(lo, l2), e);
-    hi = t;
-}
+// Row sums of the anchor iteration.  A row gathers about as many terms as lines cross its voxel
+// (~1000 at 642 directions); plain FP32 sums of that many terms leave a rounding floor near 1e-6 in
+// the iteration's relative change, above the tolerances the solver is asked for.  A lane's links are
+// summed with their errors (sums.cuh), the lane sums added as unevaluated pairs (hi, lo), and the
+// row's update is in FP64.
 template <int LANES>
 __device__ __forceinline__ void warp_sum_pair(float &hi, float &lo)
 {
@@ -620,14 +613,14 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, SMEM ? 1 : 6) k_anchor_iter
                 const float y = SMEM ? x[c] : __ldg(x + c);
                 if (FIX) t += (long long)fix_term(KIND == kLinkPair ? w * y : y, sr);
                 else if (KIND == kLinkPair) kahan_add_product(s, comp, w, y);
-                else kahan_add(s, comp, y);
+                else two_sum_add(s, comp, y);
             });
             __syncwarp();
             if (FIX) {
                 t = warp_sum_fixed<kLanes>(t);
                 if (p && mine < rows) t += __double_as_longlong(row_sum[warp * rows + mine]);
             } else {
-                float h = s, l = -comp;
+                float h = s, l = KIND == kLinkPair ? -comp : comp;
                 warp_sum_pair<kLanes>(h, l);
                 if (p && mine < rows) {  // the first panel's pair
                     const unsigned long long f = (unsigned long long)__double_as_longlong(row_sum[warp * rows + mine]);

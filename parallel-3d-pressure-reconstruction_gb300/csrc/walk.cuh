@@ -24,6 +24,7 @@
 #include <stdint.h>
 
 #include "omni3d_internal.h"
+#include "sums.cuh"
 
 namespace omni3d {
 
@@ -235,19 +236,6 @@ __device__ __forceinline__ float step_increment(const LineWalk &L, uint32_t c, i
                      by_axis(c, q, __fadd_rn(gv.x, gl.x), __fadd_rn(gv.y, gl.y), __fadd_rn(gv.z, gl.z)));
 }
 
-__device__ __forceinline__ void kahan_add(float &s, float &c, float x)
-{
-    const float y = __fsub_rn(x, c), t = __fadd_rn(s, y);
-    c = __fsub_rn(__fsub_rn(t, s), y);
-    s = t;
-}
-// s += w y, the product not rounded.
-__device__ __forceinline__ void kahan_add_product(float &s, float &c, float w, float y)
-{
-    const float p = __fmaf_rn(w, y, -c), t = __fadd_rn(s, p);
-    c = __fsub_rn(__fsub_rn(t, s), p);
-    s = t;
-}
 // The curl sum of the selected method after a voxel of curl cn.
 __device__ __forceinline__ float add_curl(float csum, float cn) { return __fmaf_rn(cn, 1.0e-4f, csum); }
 

@@ -49,3 +49,26 @@ def test_adjoint_row_sums_are_as_exact_as_with_32_lanes(native, lanes, per, n):
         want.append((_lanes32(x) - exact) / exact)
     rms = lambda e: float(np.sqrt(np.mean(np.square(e))))
     assert rms(mine) <= 1.1 * rms(want)
+
+
+@pytest.mark.parametrize("lanes,per", [(8, 8), (16, 4)])  # 16-bit and 32-bit links
+@pytest.mark.parametrize("n", [1, 7, 60, 640, 7305])
+def test_unit_row_sums_hold_twice_the_precision(native, lanes, per, n):
+    """Within the bound of a sum in twice FP32's precision, gamma_n^2 of the sum of magnitudes (n u squared,
+    and u of a lane's correction where its terms nearly cancel stays below it)."""
+    row_sum = native.unit_row_sum
+    row_sum.restype, row_sum.argtypes = C.c_double, [C.c_void_p, C.c_longlong, C.c_int, C.c_int]
+    rng = np.random.default_rng(150)
+    for trial in range(40):
+        x = rng.normal(size=n)
+        if trial % 4 == 1:
+            x = x * 10.0 ** rng.uniform(-4, 0, n)
+        elif trial % 4 == 2:
+            x = 5.0 + 0.3 * x
+        elif trial % 4 == 3:
+            x = x - x.mean()
+        x = np.ascontiguousarray(x, np.float32)
+        exact = math.fsum(x.astype(np.float64))
+        size = math.fsum(np.abs(x.astype(np.float64)))
+        gamma = (n + 8) * 2.0**-24
+        assert abs(row_sum(x.ctypes.data, n, lanes, per) - exact) <= max(gamma * gamma, 2.0**-46) * size
