@@ -102,10 +102,13 @@ __device__ __forceinline__ const float *gather_vector(const float *x, long long 
 }
 
 // Launch shape of an iteration over n rows: CTAs of 256 threads, or with the vector in shared
-// memory CTAs of 1024 (as many as fit per SM), and rows per warp.  alone: the iteration does not
+// memory one CTA of 1024 per SM, and rows per warp.  alone: the iteration does not
 // share the GPU with others, as it does in a batch's graph, where kernels that fill the SMs'
 // shared memory keep the members apart (16 plain snapshots: 15.6 ms so, 13.8 without).
-constexpr long long kIterSmemMin = 16384;  // smaller vectors stay in L1 anyway
+// Vectors below kIterSmemMin stay in L1 anyway: 642 directions, 54^3 (17 K rows) 16.4 us through L1,
+// 12.3 from shared memory, 72^3 26.7 and 18.5; 162 directions 9.7 and 8.4, 12.3 with either (60^3 to
+// 68^3 10.3 and 12.3: a second row for some warps).
+constexpr long long kIterSmemMin = 16384;
 // (paired links always gather through L1: their stream takes longer than the gathers; 25 K anchors, 40^3
 // selected: 44 us an iteration from shared memory, 32 through L1)
 struct IterShape {
@@ -137,10 +140,11 @@ inline IterShape iter_shape(long long n, bool alone, int kind, uint32_t split, b
     s.bytes = sizeof(float) * (split ? (size_t)split : (size_t)n);
     s.smem = alone && kind == kLink16 && n >= kIterSmemMin;
     s.threads = s.smem ? 1024 : 256;
-    // one CTA per SM above half of its shared memory, else two (2048 threads per SM)
+    // with the vector in shared memory one CTA per SM (1024 threads at 48 to 64 registers): a shape for two
+    // took 60^3 to 68^3 / 642 directions, 21 to 27 K rows, 22.6 instead of 18.5 us in two rounds
     // at least as many rows as a warp takes at once: fewer blocks then hand in fewer change sums (32^3
     // / 162 directions: 15.2 -> 12.3 us an iteration with its test)
-    const long long warps = s.smem ? 152LL * 32 * (s.bytes > (size_t)kIterSmemMax / 2 ? 1 : 2) : 152LL * 48;
+    const long long warps = 152LL * (s.smem ? 32 : 48);
     const long long rows = (n + warps - 1) / warps, least = 32 / lanes_per_row(kind);
     s.rows = (int)(rows < least || (uneven && kind == kLinkPair) ? least : (rows > iter_rows_max(s.smem) ? iter_rows_max(s.smem) : rows));
     const long long per = (long long)s.rows * (s.threads / 32);
