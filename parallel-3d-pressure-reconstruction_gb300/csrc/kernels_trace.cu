@@ -104,10 +104,11 @@ __device__ __forceinline__ bool trace_candidate(const Grid &g, const DirEntry *d
 }
 
 // The 32 candidates of a warp are one tile of one direction: its valid lines form one group.
-// Pass 1: lines (low word) and groups (high word) per block of candidates.
+// Pass 1: lines (low word) and groups (high word) per block of candidates; where the low words' sum may
+// overflow, also all lines in *lines.
 __global__ void __launch_bounds__(kTraceBlock) k_trace_count(Grid g, const DirEntry *dirs,
                                                              long long ncand, CandOrder co,
-                                                             unsigned long long *blk_cnt)
+                                                             unsigned long long *blk_cnt, unsigned long long *lines)
 {
     __shared__ uint32_t warp_cnt[kTraceBlock / 32];
     long long c = (long long)blockIdx.x * kTraceBlock + threadIdx.x;
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_count(Grid g, const DirEn
         unsigned long long s = 0;
         for (int w = 0; w < kTraceBlock / 32; w++) s += warp_cnt[w] ? (1ull << 32) + warp_cnt[w] : 0ull;
         blk_cnt[blockIdx.x] = s;
+        if (lines && s) atomicAdd(lines, s & 0xffffffffull);
     }
 }
 
@@ -196,6 +198,15 @@ __global__ void k_group_words(Grid g, const LineRec *lines, long long n_groups, 
         groups[gi].span = (uint32_t)span;
         gw[gi] = (uint32_t)((span + 15) >> 4);
     }
+}
+
+// *total += the words of all groups.
+__global__ void k_words_total(long long n_groups, const uint32_t *gw, unsigned long long *total)
+{
+    unsigned long long s = 0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_groups; i += (long long)gridDim.x * blockDim.x) s += gw[i];
+    for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0 && s) atomicAdd(total, s);
 }
 
 __global__ void k_group_offsets(long long n_groups, const uint32_t *off, GroupRec *groups)
@@ -533,9 +544,25 @@ cudaError_t build_geometry(Geometry *g, cudaStream_t st, std::string *err)
     OM_TRY(tb_blk.alloc(&blk, (size_t)(2 * nblk + 1)));
     OM_TRY(tb_tmp.alloc(&tmp, scan_tmp_elems(nblk)));
     unsigned long long *blk_off = blk + nblk;
-    k_trace_count<<<(unsigned)nblk, kTraceBlock, 0, st>>>(G, g->d_dirs, ncand, co, blk);
+    // lines and groups are numbered in 32 bits: more lines than that (their records alone would take 137 GB)
+    // or more words (550 GB) find no memory
+    TmpBuf tb_wide;
+    unsigned long long *wide = nullptr, wide_total = 0;
+    if (!co.narrow) {
+        OM_TRY(tb_wide.alloc(&wide, 1));
+        OM_TRY(cudaMemsetAsync(wide, 0, sizeof(*wide), st));
+    }
+    k_trace_count<<<(unsigned)nblk, kTraceBlock, 0, st>>>(G, g->d_dirs, ncand, co, blk, wide);
     OM_COUNT_LAUNCH();
     OM_TRY(cudaGetLastError());
+    if (wide) {
+        OM_TRY(cudaMemcpyAsync(&wide_total, wide, sizeof(wide_total), cudaMemcpyDeviceToHost, st));
+        OM_TRY(cudaStreamSynchronize(st));
+        if (wide_total >> 32) {
+            if (err) *err = "more than 2^32 lines";
+            return cudaErrorMemoryAllocation;
+        }
+    }
     OM_TRY(exclusive_scan_u64(blk, blk_off, nblk, tmp, st));
     unsigned long long total = 0;
     OM_TRY(cudaMemcpyAsync(&total, blk_off + nblk, sizeof(total), cudaMemcpyDeviceToHost, st));
@@ -563,6 +590,20 @@ cudaError_t build_geometry(Geometry *g, cudaStream_t st, std::string *err)
     k_group_words<<<group_blocks(*g, 256), 256, 0, st>>>(G, g->d_lines, g->n_groups, g->d_groups, gw);
     OM_COUNT_LAUNCH();
     OM_TRY(cudaGetLastError());
+    if (g->n_groups * (((long long)G.X + G.Y + G.Z + 15) / 16) >> 32) {  // the scan may overflow
+        TmpBuf tb_words;
+        unsigned long long *words = nullptr, words_total = 0;
+        OM_TRY(tb_words.alloc(&words, 1));
+        OM_TRY(cudaMemsetAsync(words, 0, sizeof(*words), st));
+        k_words_total<<<152 * 8, 256, 0, st>>>(g->n_groups, gw, words);
+        OM_COUNT_LAUNCH();
+        OM_TRY(cudaMemcpyAsync(&words_total, words, sizeof(words_total), cudaMemcpyDeviceToHost, st));
+        OM_TRY(cudaStreamSynchronize(st));
+        if (words_total >> 32) {
+            if (err) *err = "more than 2^32 step words";
+            return cudaErrorMemoryAllocation;
+        }
+    }
     OM_TRY(exclusive_scan_u32(gw, goff, g->n_groups, gtmp, st));
     k_group_offsets<<<(unsigned)std::min<long long>((g->n_groups + 255) / 256, 152LL * 64), 256, 0, st>>>(g->n_groups, goff,
                                                                                                          g->d_groups);
