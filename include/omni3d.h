@@ -125,7 +125,8 @@ typedef struct {
                                   sweep of each of a few candidate pairs on this grid and
                                   direction set, and keeps the choice for the process, per
                                   device and size class (largest grid dimension rounded up to
-                                  a multiple of 32, direction count, line spacing, walk rule);
+                                  a multiple of 32, direction count, line spacing, walk rule,
+                                  volume layout);
                                   tile_width and dir_group are then ignored */
     int deterministic;         /* 1: bit-reproducible solves.  The sums whose order the GPU does
                                   not fix -- the voxels' (pn, count) of every full sweep, the
