@@ -670,6 +670,9 @@ int omni3d_create(const omni3d_params *params, omni3d_ctx **out)
     for (int d : sphere_order(ctx->dirs)) {
         ctx->table.push_back(make_dir(ctx->dirs[3 * d], ctx->dirs[3 * d + 1], ctx->dirs[3 * d + 2]));
         ctx->table.back().orig = d;
+        const float *k = &ctx->dirs[3 * d];
+        const double e = (double)k[0] * k[0] + (double)k[1] * k[1] + (double)k[2] * k[2] - 1.0;
+        ctx->geo.unit_dirs += std::fabs(e) <= (double)kUnitMax ? 1 : 0;
     }
 
     Grid &g = ctx->geo.grid;

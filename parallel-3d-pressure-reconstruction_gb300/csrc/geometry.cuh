@@ -417,7 +417,6 @@ struct OmFastWalker {
 // 256^3 / 642 directions: 60 -> 31 ms (23.6 G steps over 67 grids and sets of directions: no step
 // other than the exact form's).
 constexpr int kFilterMax = 2048;
-constexpr float kUnitMax = 6.103515625e-5f;  // 2^-14
 struct OmFilteredWalker {
     float x, y, z, k1, k2, k3;
     float oi, oj, ok;     // exit voxel

@@ -59,6 +59,9 @@ struct GroupRec {
 constexpr uint32_t kGroupCount = 0xffu;
 constexpr int kGroupSigns = 8;
 
+// The filtered walk (geometry.cuh) takes directions with | |k|^2 - 1 | up to this.
+constexpr float kUnitMax = 6.103515625e-5f;  // 2^-14
+
 // Device-resident geometry of one (grid, direction set, line spacing) triple.  Lines are
 // grouped by (direction, lattice tile), a warp each; a group's step words are interleaved
 // lane by lane, 16 steps of 2 bits per word: the axis of the step or kIdle (walk.cuh).
@@ -75,6 +78,7 @@ struct Geometry {
     uint32_t *d_lines_through = nullptr;  // per voxel: lines through it (built on first use)
     unsigned max_through = 0;       // the most lines through one voxel (0: not computed)
     unsigned long long *d_counters = nullptr;  // walk counters (early stops, voxel visits)
+    int unit_dirs = 0;              // directions of unit length to within kUnitMax (the filtered walk's)
     int walk_rule = 0;              // OmWalker rule of the staircases (3: per field, minimum curl)
     long long walk_generation = 0;  // incremented by every walk
     long long n_lines = 0, n_groups = 0, n_words = 0;
